@@ -12,11 +12,14 @@
 // kernel (all projections at once) and one update kernel, applied twice
 // (classical Gram-Schmidt with reorthogonalisation): the same projector up to
 // rounding, with better orthogonality, in 4 launches per step instead of
-// 2 * idx.  The small exponential runs on the host (dense.h).
+// 2 * idx.  The small exponential runs on the host (dense.h).  This form serves
+// the requests of the serving loop and sectors too large for the persistent
+// recurrence (arnres.cu), which takes all other calls.
 #include <algorithm>
 #include <cstring>
 #include <vector>
 
+#include "arnres.cuh"
 #include "dense.h"
 #include "tridiag.cuh"
 #include "evolve.cuh"
@@ -190,6 +193,12 @@ __global__ void __launch_bounds__(kEvThreads) ev_combine_kernel(int64_t n, const
   }
 }
 
+void launch_ev_combine(Ctx* ctx, int64_t n, const cplx* V, int64_t ld, int a, const cplx* e, cplx* out) {
+  ev_combine_kernel<<<ev_stream_grid(ctx, n), kEvThreads, 0, ctx->stream>>>(n, V, ld, a, e, out);
+  QD_CHECK_LAUNCH();
+  QD_LAUNCHED(ctx);
+}
+
 void ArnoldiBuffers::drop_graph() {
   if (steps_exec) cudaGraphExecDestroy(steps_exec);
   steps_exec = nullptr;
@@ -254,6 +263,10 @@ void arnoldi_evolve(qd_ham* H, const cplx* psi_in, cplx* psi_out, double h, int 
   Ctx* ctx = H->ctx;
   QD_REQUIRE(m >= 2 && m <= 33, QD_ERR_UNSUPPORTED, "Krylov dimension m must be in 2..33");
   const int64_t n = H->dim;
+  if (arn_res_fits(H, m - 1)) {
+    if (!H->arn_ev) H->arn_ev.reset(new ArnRes());
+    if (arn_res_evolve(H, *H->arn_ev, psi_in, psi_out, h, m - 1, act_out)) return;
+  }
   if (!H->arnoldi) H->arnoldi.reset(new ArnoldiBuffers());
   ArnoldiBuffers& B = *H->arnoldi;
   const int g = ev_grid(ctx, n);
@@ -334,9 +347,7 @@ void arnoldi_evolve(qd_ham* H, const cplx* psi_in, cplx* psi_out, double h, int 
   std::vector<cplx> e(act);
   for (int j = 0; j < act; ++j) e[j] = mkc(E[j].real(), E[j].imag());
   QD_CUDA(cudaMemcpyAsync(B.e.p, e.data(), act * sizeof(cplx), cudaMemcpyHostToDevice, ctx->stream));
-  ev_combine_kernel<<<ev_stream_grid(ctx, n), kEvThreads, 0, ctx->stream>>>(n, B.V.p, B.ld, act, B.e.p, psi_out);
-  QD_CHECK_LAUNCH();
-  QD_LAUNCHED(ctx);
+  launch_ev_combine(ctx, n, B.V.p, B.ld, act, B.e.p, psi_out);
   QD_CUDA(cudaStreamSynchronize(ctx->stream));
   if (act_out) *act_out = act;
 }
@@ -467,12 +478,67 @@ static void arnoldi_ground_steps(qd_ham* H, const MV* vals, ArnoldiGround& B, in
   }
 }
 
+// The persistent form of arnoldi_ground (arnres.cu).  False, with nothing run, when it does not take
+// the solve; a solve that it began it also continues.
+static bool arnoldi_ground_res(qd_ham* H, cplx* psi, int kdim, int add_dim, bool extend, double* evals_out,
+                               qd_lanczos_result* res) {
+  Ctx* ctx = H->ctx;
+  if (!extend) {
+    if (H->arn_gs) H->arn_gs->open = false;
+    if (!arn_res_fits(H, kdim)) return false;
+    if (!H->arn_gs) H->arn_gs.reset(new ArnRes());
+    bool has_imag = false;
+    const double n0 = state_norm2_imag(H, psi, &has_imag);
+    QD_REQUIRE(n0 > 0.0, QD_ERR_INVALID, "start vector is zero");
+    H->arn_gs->act = 0;
+    H->arn_gs->broke = false;
+    // a real operator keeps a real start vector's Krylov space real
+    H->arn_gs->real_start = !has_imag && (H->flags & QD_HAM_REAL);
+  } else if (!H->arn_gs || !H->arn_gs->open || H->arn_gs->kdim != kdim) {
+    return false;
+  }
+  ArnRes& B = *H->arn_gs;
+  int steps = (add_dim <= 0 || B.act + add_dim > kdim) ? kdim - B.act : add_dim;
+  if (B.broke) steps = 0;
+  const int act_prev = B.act;
+  if (steps > 0) {
+    B.open = false;
+    if (!arn_res_steps(H, B, psi, kdim, B.real_start, B.act + 1, B.act + steps)) return false;
+    B.open = true;
+    if (H->arnoldi_gs) H->arnoldi_gs->open = false;
+    B.act = B.host.stop ? B.host.stop : B.act + steps;  // expandBasis<0>: the breaking step counts
+    B.broke = B.host.stop != 0;
+  }
+  const int act = B.act;
+  QD_REQUIRE(act >= 1, QD_ERR_INVALID, "no Krylov step was run");
+  std::vector<double> d(act), e(act), ev(act), y(act);
+  for (int i = 0; i < act; ++i) {
+    d[i] = B.host.alpha[i + 1];
+    e[i] = (i + 1 < act) ? B.host.nrm[i + 1] : 0.0;
+  }
+  QD_REQUIRE(tridiag_lowest<double>(act, d.data(), e.data(), ev.data(), y.data()) == 0, QD_ERR_INVALID,
+             "tridiagonal eigensolver did not converge");
+  for (int j = 0; j < act; ++j) y[j] *= B.host.scl[j];
+  double* yd = reinterpret_cast<double*>(B.hcol.p);
+  QD_CUDA(cudaMemcpyAsync(yd, y.data(), act * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  launch_ritz(ctx, H->dim, B.V.p, B.real_v, B.ld, yd, act, psi);
+  QD_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (evals_out) std::memcpy(evals_out, ev.data(), act * sizeof(double));
+  res->act_dim = act;
+  res->breakdown = B.broke ? 1 : 0;
+  res->matvecs = act - act_prev;
+  res->ritz_value = ev[0];
+  res->err = std::fabs(ev[0]);
+  return true;
+}
+
 void arnoldi_ground(qd_ham* H, cplx* psi, int kdim, int add_dim, bool extend, double* evals_out,
                     qd_lanczos_result* res) {
   Ctx* ctx = H->ctx;
   const int64_t n = H->dim;
   QD_REQUIRE(kdim >= 1 && kdim <= 4096, QD_ERR_INVALID, "krylov_dim must be in 1..4096");
   QD_REQUIRE(n >= 1, QD_ERR_INVALID, "empty sector");
+  if (arnoldi_ground_res(H, psi, kdim, add_dim, extend, evals_out, res)) return;
   const int g = ev_grid(ctx, n);
   if (extend) {
     QD_REQUIRE(H->arnoldi_gs && H->arnoldi_gs->open && H->arnoldi_gs->kdim == kdim, QD_ERR_INVALID,
@@ -547,6 +613,8 @@ void arnoldi_ground(qd_ham* H, cplx* psi, int kdim, int add_dim, bool extend, do
 }
 
 void ArnoldiGroundDeleter::operator()(ArnoldiGround* b) const { delete b; }
+
+void ArnResDeleter::operator()(ArnRes* b) const { delete b; }
 
 void ArnoldiDeleter::operator()(ArnoldiBuffers* b) const { delete b; }
 

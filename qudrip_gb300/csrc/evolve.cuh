@@ -33,6 +33,9 @@ struct ArnoldiBuffers {
   ~ArnoldiBuffers() { drop_graph(); }
 };
 
+// out = sum_{j<a} e_j V_j
+void launch_ev_combine(Ctx* ctx, int64_t n, const cplx* V, int64_t ld, int a, const cplx* e, cplx* out);
+
 void arnoldi_evolve(qd_ham* H, const cplx* psi_in, cplx* psi_out, double h, int m, int* act_out);
 
 // Solve state of the Arnoldi ground state (ArnoldiSolver<T, herm=0>::getGroundState), kept per

@@ -30,6 +30,11 @@ struct ArnoldiGroundDeleter {
   void operator()(ArnoldiGround* b) const;
 };
 
+struct ArnRes;
+struct ArnResDeleter {
+  void operator()(ArnRes* b) const;
+};
+
 struct GateDev {
   int kind, site, site_b, string;
   cplx u[4];  // u[b*2 + o] = amplitude from input bit b to output bit o = U(b, o)
@@ -118,6 +123,7 @@ struct qd_ham {
   std::unique_ptr<qd::Workspace, qd::WorkspaceDeleter> ws;  // solver buffers, reused across calls
   std::unique_ptr<qd::ArnoldiBuffers, qd::ArnoldiDeleter> arnoldi;
   std::unique_ptr<qd::ArnoldiGround, qd::ArnoldiGroundDeleter> arnoldi_gs;  // Arnoldi ground-state solve
+  std::unique_ptr<qd::ArnRes, qd::ArnResDeleter> arn_ev, arn_gs;  // the persistent recurrence: evolve, ground state
   double arnoldi_gs_ritz = 0.0;  // its last lowest eigenvalue (the error of a grown solve)
 };
 

@@ -301,6 +301,16 @@ __global__ void __launch_bounds__(kVecThreads) ritz_kernel(int64_t n, const VV* 
   }
 }
 
+void launch_ritz(Ctx* ctx, int64_t n, const void* V, bool real_v, int64_t ld, const double* y, int act, cplx* psi) {
+  const int vg = vec_grid(ctx, n);
+  if (real_v)
+    ritz_kernel<double><<<vg, kVecThreads, 0, ctx->stream>>>(n, static_cast<const double*>(V), ld, y, act, psi);
+  else
+    ritz_kernel<cplx><<<vg, kVecThreads, 0, ctx->stream>>>(n, static_cast<const cplx*>(V), ld, y, act, psi);
+  QD_CHECK_LAUNCH();
+  QD_LAUNCHED(ctx);
+}
+
 // <a, b> over complex columns (a^dagger b).
 __global__ void __launch_bounds__(kVecThreads) cdot_kernel(int64_t n, const cplx* a, const cplx* b, cplx* out,
                                                            GridRed<cplx> red) {
@@ -396,6 +406,25 @@ void obs_eval_many(qd_ham* const* obs, int nobs, const cplx* psi, cplx* out_host
   QD_CUDA(cudaStreamSynchronize(ctx->stream));
 }
 
+double state_norm2_imag(qd_ham* H, const cplx* psi, bool* has_imag) {
+  Ctx* ctx = H->ctx;
+  Workspace& W = ham_workspace(H);
+  if (!W.start_nrm2.p) W.start_nrm2.alloc(1);
+  if (!W.start_has_im.p) W.start_has_im.alloc(1);
+  QD_CUDA(cudaMemsetAsync(W.start_has_im.p, 0, sizeof(int), ctx->stream));
+  colnorm_kernel<<<vec_grid(ctx, H->dim), kVecThreads, 0, ctx->stream>>>(H->dim, psi, W.start_nrm2.p, W.red_d(0),
+                                                                         W.start_has_im.p);
+  QD_CHECK_LAUNCH();
+  QD_LAUNCHED(ctx);
+  double n2 = 0.0;
+  int im = 0;
+  QD_CUDA(cudaMemcpyAsync(&n2, W.start_nrm2.p, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  QD_CUDA(cudaMemcpyAsync(&im, W.start_has_im.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  QD_CUDA(cudaStreamSynchronize(ctx->stream));
+  *has_imag = im != 0;
+  return n2;
+}
+
 // ||psi||^2 on the Hamiltonian's stream.
 double state_norm2(qd_ham* H, const cplx* psi) {
   Ctx* ctx = H->ctx;
@@ -450,7 +479,7 @@ static bool fx_one_launch_step() {
 // publishing alpha and beta and lets every block give up after <polls> polls, so each step's
 // wait runs out and the solve returns QD_ERR_TIMEOUT with the kernel finished.
 // Read per solve; 0 when unset.
-static unsigned step_wait_out_polls() {
+unsigned step_wait_out_polls() {
   const char* e = std::getenv("QD_STEP_WAIT_OUT");
   if (!e) return 0;
   const long v = std::strtol(e, nullptr, 10);

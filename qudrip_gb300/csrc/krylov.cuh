@@ -137,6 +137,13 @@ struct Workspace {
 };
 
 Workspace& ham_workspace(qd_ham* H);
+// Test control of the bounded device waits (polls before a block gives up, the publishing block
+// held back); 0 when QD_STEP_WAIT_OUT is unset.
+unsigned step_wait_out_polls();
+// ||psi||^2 and whether psi has an imaginary part, on the host.
+double state_norm2_imag(qd_ham* H, const cplx* psi, bool* has_imag);
+// psi = sum_{k < act} y_k V[k] for a basis of reals or complex numbers.
+void launch_ritz(Ctx* ctx, int64_t n, const void* V, bool real_v, int64_t ld, const double* y, int act, cplx* psi);
 void ham_apply_c(qd_ham* H, const cplx* x, cplx* y);
 cplx state_eval(qd_ham* H, const cplx* psi);
 double state_norm2(qd_ham* H, const cplx* psi);
