@@ -386,23 +386,99 @@ cplx state_eval(qd_ham* H, const cplx* psi) {
 }
 
 // <psi|O_i|psi> for a list of operators (McManager::incrAllObs,
-// mc_manager.hpp:88-106): every product is fused with its inner product and
-// the launches go back to back on one stream, with one copy of all results.
+// mc_manager.hpp:88-106) in one launch per kObsBatch operators: row y of the grid
+// is operator y, its blocks share the rows, and the last of them to finish adds
+// their partials in block order.  One launch per operator left each at the
+// launch's own 4-5 us (a diagonal operator's work at dim 4,900 is a tenth of
+// that), and the product's result was written for nobody: 15 operators at dim
+// 4,900 took 180 us a call with their allocations, now 35.
+constexpr int kObsBatch = 32;
+
+struct ObsOp {
+  const int64_t* rowptr;
+  const int32_t* colidx;
+  const void* vals;  // double or cplx
+  int real;
+};
+struct ObsArgs {
+  int64_t n;
+  const cplx* psi;
+  cplx* partials;     // gridDim.x per operator
+  unsigned* tickets;  // one per operator, 0 at rest
+  cplx* out;
+  ObsOp op[kObsBatch];
+};
+
+template <typename MV>
+__device__ __forceinline__ cplx obs_rows(const ObsArgs& A, const ObsOp& O) {
+  const MV* vals = static_cast<const MV*>(O.vals);
+  cplx acc = mkc(0.0, 0.0);
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < A.n; r += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t b = O.rowptr[r], e = O.rowptr[r + 1];
+    if (b == e) continue;
+    cplx y = mkc(0.0, 0.0);
+    int64_t k = b;
+    for (; k + 4 <= e; k += 4) {
+      int32_t c[4];
+      MV v[4];
+      cplx x[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        c[u] = ld_plain(O.colidx + k + u);
+        v[u] = ld_plain(vals + k + u);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) x[u] = ld_ro(A.psi + c[u]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) y = vfma(v[u], x[u], y);
+    }
+    for (; k < e; ++k) y = vfma(ld_plain(vals + k), ld_ro(A.psi + ld_plain(O.colidx + k)), y);
+    acc = vdotfma(ld_ro(A.psi + r), y, acc);
+  }
+  return acc;
+}
+
+__global__ void __launch_bounds__(kVecThreads) obs_kernel(const __grid_constant__ ObsArgs A) {
+  const ObsOp& O = A.op[blockIdx.y];
+  const cplx acc = O.real ? obs_rows<double>(A, O) : obs_rows<cplx>(A, O);
+  GridRed<cplx> red{A.partials + (size_t)blockIdx.y * gridDim.x, A.tickets + blockIdx.y};
+  grid_sum_flat(acc, red, A.out + blockIdx.y);
+}
+
 void obs_eval_many(qd_ham* const* obs, int nobs, const cplx* psi, cplx* out_host) {
   Ctx* ctx = obs[0]->ctx;
   const int64_t n = obs[0]->dim;
-  DBuf<cplx> tmp(n + 1);
-  DBuf<cplx> out(nobs);
-  for (int i = 0; i < nobs; ++i) {
-    qd_ham* H = obs[i];
-    QD_REQUIRE(H->ctx == ctx && H->dim == n, QD_ERR_INVALID, "observable %d: other context or dimension", i);
-    Workspace& W = ham_workspace(H);
-    if (H->flags & QD_HAM_REAL)
-      launch_spmv<double, cplx>(ctx, H, H->vals_r.p, psi, tmp.p, 1.0, psi, W.red_c(0), out.p + i, nullptr, 0, -1);
-    else
-      launch_spmv<cplx, cplx>(ctx, H, H->vals_c.p, psi, tmp.p, 1.0, psi, W.red_c(0), out.p + i, nullptr, 0, -1);
+  for (int i = 0; i < nobs; ++i)
+    QD_REQUIRE(obs[i]->ctx == ctx && obs[i]->dim == n, QD_ERR_INVALID, "observable %d: other context or dimension", i);
+  // the first operator's workspace, kept between calls
+  Workspace& W = ham_workspace(obs[0]);
+  if (!W.obs_tickets.p) {
+    W.obs_tickets.alloc(kObsBatch);
+    QD_CUDA(cudaMemsetAsync(W.obs_tickets.p, 0, W.obs_tickets.bytes(), ctx->stream));
   }
-  QD_CUDA(cudaMemcpyAsync(out_host, out.p, nobs * sizeof(cplx), cudaMemcpyDeviceToHost, ctx->stream));
+  if (W.obs_out.n < (size_t)nobs) W.obs_out.alloc(nobs);
+  ObsArgs A;
+  std::memset(&A, 0, sizeof(A));
+  A.n = n;
+  A.psi = psi;
+  A.partials = W.partials_c.p;
+  A.tickets = W.obs_tickets.p;
+  for (int i0 = 0; i0 < nobs; i0 += kObsBatch) {
+    const int cnt = std::min(kObsBatch, nobs - i0);
+    for (int i = 0; i < cnt; ++i) {
+      const qd_ham* H = obs[i0 + i];
+      const bool real = (H->flags & QD_HAM_REAL) != 0;
+      A.op[i] = ObsOp{H->rowptr.p, H->colidx.p, real ? (const void*)H->vals_r.p : (const void*)H->vals_c.p, real};
+    }
+    A.out = W.obs_out.p + i0;
+    // enough blocks for eight per SM over all operators, one row per thread at least
+    const int64_t gx = std::max<int64_t>(
+        1, std::min<int64_t>(ceil_div(n, kVecThreads), std::max<int64_t>(1, (int64_t)ctx->num_sms * 8 / cnt)));
+    obs_kernel<<<dim3((unsigned)gx, (unsigned)cnt), kVecThreads, 0, ctx->stream>>>(A);
+    QD_CHECK_LAUNCH();
+    QD_LAUNCHED(ctx);
+  }
+  QD_CUDA(cudaMemcpyAsync(out_host, W.obs_out.p, nobs * sizeof(cplx), cudaMemcpyDeviceToHost, ctx->stream));
   QD_CUDA(cudaStreamSynchronize(ctx->stream));
 }
 

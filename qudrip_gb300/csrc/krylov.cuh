@@ -114,6 +114,8 @@ struct Workspace {
   // H psi and the result of state_eval, kept between calls (a device allocation
   // and free per call would wait for the whole device)
   DBuf<cplx> eval_y, eval_out;
+  DBuf<cplx> obs_out;  // obs_eval_many's results and its operators' tickets
+  DBuf<unsigned> obs_tickets;
   DBuf<double> eval_real;  // the uniform-coupling form's value and its imaginary-part flag
   DBuf<int> eval_flag;
   DBuf<double> start_nrm2;  // ||v0||^2 of the last ground-state solve (read by its first kernels)
