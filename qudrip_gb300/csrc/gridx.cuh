@@ -88,6 +88,24 @@ __device__ __forceinline__ cplx x_peek(const cplx* p) {
 }
 __device__ __forceinline__ bool x_filled(double v) { return !x_is_empty(v); }
 __device__ __forceinline__ bool x_filled(cplx v) { return !x_is_empty(v.re) && !x_is_empty(v.im); }
+// 128-bit integers of magnitude below 2^125 as two words that are never kXEmpty: hi 2^63 + lo, 0 <= lo < 2^63.
+struct __align__(16) XInt {
+  unsigned long long lo;
+  long long hi;
+};
+__device__ __forceinline__ void x_put(XInt* p, __int128 v) {
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p),
+               "l"((unsigned long long)v & 0x7fffffffffffffffull), "l"((long long)(v >> 63))
+               : "memory");
+}
+__device__ __forceinline__ XInt x_peek(const XInt* p) {
+  XInt v;
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.lo), "=l"(v.hi) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ bool x_filled(XInt v) { return v.lo != kXEmpty && (unsigned long long)v.hi != kXEmpty; }
+__device__ __forceinline__ __int128 x_value(XInt v) { return ((__int128)v.hi << 63) + v.lo; }
+
 template <typename VV>
 __device__ __forceinline__ bool x_await(const GridX& X, const VV* p, VV& v) {
   unsigned polls = 0;
@@ -115,29 +133,30 @@ __device__ __forceinline__ void x_sum(const GridX& X, double* slots, double* v, 
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank(), ncl = (int)gridDim.x / C, me = (int)blockIdx.x / C;
-    const int per = (nv + C - 1) / C;  // values per block: C lanes each
+    const int per = (nv + C - 1) / C;  // values per block
     cl.sync();
-    const int g = tid / C, l = tid & (C - 1);
-    if ((tid & ~31) / C < per) {  // whole warps
+    // a value takes C lanes, or a warp where there are many clusters to collect from
+    const int L = ncl > 2 * C ? 32 : C;
+    const int l = tid & (L - 1);
+    for (int g = tid / L; (g & ~(32 / L - 1)) < per; g += blockDim.x / L) {  // whole warps
       const int q = rank * per + g;
       const bool on = g < per && q < nv;
-      double a = on ? *cl.map_shared_rank(v + q, l) : 0.0;
+      double a = (on && l < C) ? *cl.map_shared_rank(v + q, l) : 0.0;
 #pragma unroll
       for (int o = C / 2; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
       if (ncl > 1) {
         if (on && l == 0 && !(X.hold && me == 0)) x_st(slots + (size_t)me * nv + q, x_clean(a));
         double t = 0.0;
-        bool ok = true;
-        for (int c = l; c < ncl && on && ok; c += C) {
-          double b = x_ld(slots + (size_t)c * nv + q);
-          ok = x_wait(X, slots + (size_t)c * nv + q, b);
-          t += b;
-        }
-#pragma unroll
-        for (int o = C / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (on)
+          for (int c = l; c < ncl; c += L) {
+            double b = x_ld(slots + (size_t)c * nv + q);
+            x_wait(X, slots + (size_t)c * nv + q, b);
+            t += b;
+          }
+        for (int o = L / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
         a = t;
       }
-      if (on) *cl.map_shared_rank(out + q, l) = a;
+      if (on && l < C) *cl.map_shared_rank(out + q, l) = a;
     }
     cl.sync();
   }

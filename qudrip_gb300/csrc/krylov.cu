@@ -25,12 +25,23 @@
 
 #include "fxstep.cuh"
 #include "krylov.cuh"
+#include "lanres.cuh"
 #include "spmv.cuh"
 #include "tridiag.cuh"
 
 namespace qd {
 
 constexpr int kVecThreads = 256;
+// Most rows of the persistent recurrence (lan_res_takes).  Whole solves of 3 L steps, launched step by step
+// -> persistent: real couplings per bond L = 17 1,338 -> 693 us, L = 21 (352,716 rows) 2,953 -> 2,444, L = 22
+// (705,432) 4,806 -> 5,474; complex L = 21 6,523 -> 5,213, L = 22 the same: the line lies between them.
+constexpr int64_t kLanResMax = 1 << 19;
+// With the uniform-coupling form, whose one-launch step is faster: L = 12 686 -> 433 us, L = 16 906 -> 647,
+// L = 18 (48,620 rows) 1,152 -> 822, L = 19 (92,378) 1,356 -> 1,227 on the stored columns but 1,436 -> 1,682
+// matrix-free, and both keep one route so that their bits stay the same.
+constexpr int64_t kLanResMaxUniform = 1 << 16;
+// Hermitian::LanczosSolver keeps its basis up to this size instead of forming it twice
+constexpr int64_t kHermBasisBytes = 256ll << 20;
 
 static int vec_grid(Ctx* ctx, int64_t n) {
   const int64_t want = ceil_div(n, kVecThreads);
@@ -743,6 +754,54 @@ void time_spmv(qd_ham* H, int spmv, int iters, double* avg_ms, double* bytes_per
 }
 
 // ---------------------------------------------------------------- Lanczos
+// Whether a solve takes the persistent recurrence (lanres.cu): sectors up to kLanResMax rows, where the
+// launches and reductions of a step outweigh its memory traffic.  Served requests keep the
+// separate launches (a co-resident grid waits for room beside the other lanes' kernels), and so do
+// QD_KRYLOV_STEP=split and QD_LANCZOS_STEP=split.
+static bool lan_res_takes(const qd_ham* H, bool uniform) {
+  const char* e = std::getenv("QD_KRYLOV_STEP");
+  if (H->one_shot || !fx_one_launch_step() || (e && std::strcmp(e, "split") == 0)) return false;
+  static const bool coop = [&] {  // once per process (thread-safe initialisation)
+    int v = 0;
+    return cudaDeviceGetAttribute(&v, cudaDevAttrCooperativeLaunch, H->ctx->device) == cudaSuccess && v != 0;
+  }();
+  return coop && H->dim >= 1 && H->dim <= (uniform ? kLanResMaxUniform : kLanResMax);
+}
+
+// The flags of a persistent run, cleared on the stream.
+static int* lan_flags(Workspace& W) {
+  if (!W.lan_flags.p) W.lan_flags.alloc(2);
+  QD_CUDA(cudaMemsetAsync(W.lan_flags.p, 0, 2 * sizeof(int), W.ctx->stream));
+  return W.lan_flags.p;
+}
+
+// Steps k_first .. k_last in one persistent launch; false: not launched.
+template <typename MV, typename VV>
+static bool lanczos_run_res(qd_ham* H, const MV* vals, LanczosBuffers<VV>& B, int k_first, int k_last, Workspace& W,
+                            const FxForm* form) {
+  LanRun<MV, VV> r{};
+  r.vals = vals;
+  r.rule = kLanLocal;
+  r.form = form;
+  r.V = B.V.p;
+  r.ld = B.ld;
+  r.kdim = B.kdim;
+  r.first = k_first;
+  r.last = k_last;
+  r.stop_below = 1e-10;  // sparse_algorithm.hpp:421
+  r.alpha = B.alpha.p;
+  r.beta = B.beta.p;
+  r.nrm = B.nrm.p;
+  r.scl = B.scl.p;
+  r.stop = B.stop.p;
+  r.flags = lan_flags(W);
+  r.slots = &W.lan_slots;
+  r.xv = &W.lan_x;
+  if (!lan_res_run(H, r)) return false;
+  if (form) form->step_fused = 1;
+  return true;
+}
+
 template <typename MV, typename VV>
 // fxk: 0 the product alone (CSR or matrix-free), then K2; 1 the uniform-
 // coupling form with fixed-point sums fused with the step's inner products.
@@ -833,7 +892,7 @@ LanczosBuffers<cplx>& buffers_for<cplx>(Workspace& W, int64_t n, int kdim) {
 template <typename MV, typename VV>
 static void lanczos_finish(qd_ham* H, cplx* psi, const double* psi_nrm2, const qd_lanczos_opts& o,
                            LanczosBuffers<VV>& B, Workspace& W, const MV* vals, bool mf, int fxk,
-                           const FxForm* form, double* evals_out, qd_lanczos_result* res);
+                           const FxForm* form, bool res_run, double* evals_out, qd_lanczos_result* res);
 
 template <typename MV, typename VV>
 static void lanczos_ground_impl(qd_ham* H, cplx* psi, const double* psi_nrm2, const qd_lanczos_opts& o,
@@ -868,6 +927,8 @@ static void lanczos_ground_impl(qd_ham* H, cplx* psi, const double* psi_nrm2, co
   }
   fxk = form ? 1 : 0;
   const bool fx = fxk == 1;
+  const int steps = (o.add_dim > 0 && o.add_dim < kdim) ? o.add_dim : kdim;  // add_dim of an incremental start
+  const bool res_run = lan_res_takes(H, fx) && lanczos_run_res<MV, VV>(H, vals, B, 1, steps, W, form);
   const int fxF = fx ? form->F : 0;
   const bool one_launch = fx && fx_one_launch_step() && !H->one_shot;
   // the column source of the fixed-point form is part of what a captured recurrence launches
@@ -878,13 +939,13 @@ static void lanczos_ground_impl(qd_ham* H, cplx* psi, const double* psi_nrm2, co
     B.drop_graph();
     B.kind = kind;
   }
-  if (fx) {
+  if (fx && !res_run) {
     B.ensure_fx(ctx->stream);
     QD_CUDA(cudaMemsetAsync(B.ovf.p, 0, 2 * sizeof(int), ctx->stream));
     if constexpr (std::is_same<VV, double>::value) launch_fx_shadow(ctx, n, B.V.p, B.X.p, fxF, B.ovf.p);
   }
-  const int steps = (o.add_dim > 0 && o.add_dim < kdim) ? o.add_dim : kdim;  // add_dim of an incremental start
-  if (steps == kdim && !H->one_shot)
+  if (res_run) {
+  } else if (steps == kdim && !H->one_shot)
     B.run_graph(ctx, [&]() { lanczos_run<MV, VV>(H, vals, B, 1, kdim, W, mf, fxk, form); });
   else
     lanczos_run<MV, VV>(H, vals, B, 1, steps, W, mf, fxk, form);
@@ -893,8 +954,9 @@ static void lanczos_ground_impl(qd_ham* H, cplx* psi, const double* psi_nrm2, co
   W.lz_mv = std::is_same<MV, double>::value ? 1 : 2;
   W.lz_mf = mf;
   W.lz_fxk = fxk;
-  if (fx) {
-    const int ov = fx_flags(ctx, B.ovf.p);
+  W.lz_res = res_run;
+  if (fx || res_run) {
+    const int ov = fx_flags(ctx, res_run ? W.lan_flags.p : B.ovf.p);
     if (ov) {  // a vector left the fixed-point range: redo the solve on the FP64 CSR product
       H->fx_allowed = false;
       lanczos_ground_impl<MV, VV>(H, psi, psi_nrm2, o, evals_out, res);
@@ -903,7 +965,7 @@ static void lanczos_ground_impl(qd_ham* H, cplx* psi, const double* psi_nrm2, co
     }
   }
   if (timing) QD_CUDA(cudaEventRecord(ctx->events[13], ctx->stream));
-  lanczos_finish<MV, VV>(H, psi, psi_nrm2, o, B, W, vals, mf, fxk, form, evals_out, res);
+  lanczos_finish<MV, VV>(H, psi, psi_nrm2, o, B, W, vals, mf, fxk, form, res_run, evals_out, res);
   if (timing) {
     float g = 0.f;
     QD_CUDA(cudaEventElapsedTime(&g, ctx->events[12], ctx->events[13]));
@@ -919,7 +981,7 @@ static void lanczos_ground_impl(qd_ham* H, cplx* psi, const double* psi_nrm2, co
 template <typename MV, typename VV>
 static void lanczos_finish(qd_ham* H, cplx* psi, const double* psi_nrm2, const qd_lanczos_opts& o,
                            LanczosBuffers<VV>& B, Workspace& W, const MV* vals, bool mf, int fxk,
-                           const FxForm* form, double* evals_out, qd_lanczos_result* res) {
+                           const FxForm* form, bool res_run, double* evals_out, qd_lanczos_result* res) {
   Ctx* ctx = H->ctx;
   const int64_t n = H->dim;
   const int kdim = B.done;
@@ -954,12 +1016,18 @@ static void lanczos_finish(qd_ham* H, cplx* psi, const double* psi_nrm2, const q
     QD_CHECK_LAUNCH();
     QD_LAUNCHED(ctx);
     QD_CUDA(cudaMemsetAsync(B.stop.p, 0, sizeof(int), ctx->stream));
-    if (fx) {
-      QD_CUDA(cudaMemsetAsync(B.ovf.p, 0, 2 * sizeof(int), ctx->stream));
-      if constexpr (std::is_same<VV, double>::value) launch_fx_shadow(ctx, n, B.V.p, B.X.p, fxF, B.ovf.p);
+    if (res_run) {
+      QD_REQUIRE((lanczos_run_res<MV, VV>(H, vals, B, 1, act, W, form)), QD_ERR_UNSUPPORTED,
+                 "the persistent recurrence's grid does not fit any more");
+      fx_flags(ctx, W.lan_flags.p);
+    } else {
+      if (fx) {
+        QD_CUDA(cudaMemsetAsync(B.ovf.p, 0, 2 * sizeof(int), ctx->stream));
+        if constexpr (std::is_same<VV, double>::value) launch_fx_shadow(ctx, n, B.V.p, B.X.p, fxF, B.ovf.p);
+      }
+      lanczos_run<MV, VV>(H, vals, B, 1, act, W, mf, fxk, form);
+      if (fx) fx_flags(ctx, B.ovf.p);
     }
-    lanczos_run<MV, VV>(H, vals, B, 1, act, W, mf, fxk, form);
-    if (fx) fx_flags(ctx, B.ovf.p);
     matvecs += act;
   }
   // psi = sum_k y_k v_k = sum_k (y_k s_k) V[k]
@@ -999,16 +1067,20 @@ static void lanczos_extend_impl(qd_ham* H, cplx* psi, const qd_lanczos_opts& o, 
   const int add = (o.add_dim > 0) ? std::min(o.add_dim, B.kdim - B.done) : B.kdim - B.done;
   const FxForm* form = W.lz_fxk == 1 ? (W.lz_mf ? H->mfx.get() : H->fx.get()) : nullptr;
   if (!stop && add > 0) {
-    lanczos_run<MV, VV>(H, vals, B, B.done + 1, B.done + add, W, W.lz_mf, W.lz_fxk, form);
+    if (W.lz_res)
+      QD_REQUIRE((lanczos_run_res<MV, VV>(H, vals, B, B.done + 1, B.done + add, W, form)), QD_ERR_UNSUPPORTED,
+                 "the persistent recurrence's grid does not fit any more");
+    else
+      lanczos_run<MV, VV>(H, vals, B, B.done + 1, B.done + add, W, W.lz_mf, W.lz_fxk, form);
     B.done += add;
   }
-  if (W.lz_fxk == 1) {
-    const int ov = fx_flags(ctx, B.ovf.p);
+  if (W.lz_fxk == 1 || W.lz_res) {
+    const int ov = fx_flags(ctx, W.lz_res ? W.lan_flags.p : B.ovf.p);
     QD_REQUIRE(!ov, QD_ERR_OVERFLOW, "a Lanczos vector left the fixed-point range; restart the solve");
   }
   qd_lanczos_opts o2 = o;
   o2.ritz = QD_RITZ_STORED_BASIS;
-  lanczos_finish<MV, VV>(H, psi, nullptr, o2, B, W, vals, W.lz_mf, W.lz_fxk, form, evals_out, res);
+  lanczos_finish<MV, VV>(H, psi, nullptr, o2, B, W, vals, W.lz_mf, W.lz_fxk, form, W.lz_res, evals_out, res);
 }
 
 void lanczos_extend(qd_ham* H, cplx* psi, const qd_lanczos_opts& o, double* evals_out, qd_lanczos_result* res) {
@@ -1036,20 +1108,10 @@ void lanczos_ground(qd_ham* H, cplx* psi, const qd_lanczos_opts& o, double* eval
   QD_REQUIRE(o.krylov_dim >= 1 && o.krylov_dim <= 4096, QD_ERR_INVALID, "krylov_dim must be in 1..4096");
   QD_REQUIRE(n >= 1, QD_ERR_INVALID, "empty sector");
   Workspace& W = ham_workspace(H);
-  // ||psi||^2 and whether the start vector is real (buffers kept in the workspace)
-  if (!W.start_nrm2.p) W.start_nrm2.alloc(1);
-  if (!W.start_has_im.p) W.start_has_im.alloc(1);
+  // ||psi||^2 and whether the start vector is real
+  bool him = false;
+  const double hn = state_norm2_imag(H, psi, &him);
   DBuf<double>& nrm2 = W.start_nrm2;
-  DBuf<int>& has_im = W.start_has_im;
-  QD_CUDA(cudaMemsetAsync(has_im.p, 0, sizeof(int), ctx->stream));
-  colnorm_kernel<<<vec_grid(ctx, n), kVecThreads, 0, ctx->stream>>>(n, psi, nrm2.p, W.red_d(0), has_im.p);
-  QD_CHECK_LAUNCH();
-  QD_LAUNCHED(ctx);
-  int him = 0;
-  double hn = 0.0;
-  QD_CUDA(cudaMemcpyAsync(&him, has_im.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  QD_CUDA(cudaMemcpyAsync(&hn, nrm2.p, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  QD_CUDA(cudaStreamSynchronize(ctx->stream));
   QD_REQUIRE(hn > 0.0 && std::isfinite(hn), QD_ERR_INVALID, "start vector has zero or non-finite norm");
   if (o.spmv == QD_SPMV_MATRIX_FREE) ham_build_matrix_free(H);
   const bool real_h = (o.spmv == QD_SPMV_MATRIX_FREE) ? H->mf_real : (H->flags & QD_HAM_REAL) != 0;
@@ -1119,6 +1181,12 @@ __global__ void __launch_bounds__(kVecThreads) herm_accum_kernel(int64_t n, doub
   }
 }
 
+template <typename VV>
+static LanczosBuffers<VV>& herm_buffers(Workspace& W) {
+  if constexpr (std::is_same<VV, double>::value) return W.hl_d;
+  else return W.hl_c;
+}
+
 template <typename MV, typename VV>
 static void herm_lanczos_impl(qd_ham* H, cplx* psi, const double* psi_nrm2, int kdim, double* evals_out,
                               qd_lanczos_result* res) {
@@ -1129,6 +1197,62 @@ static void herm_lanczos_impl(qd_ham* H, cplx* psi, const double* psi_nrm2, int 
   if constexpr (std::is_same<MV, double>::value) vals = H->vals_r.p;
   else vals = H->vals_c.p;
   const int vg = vec_grid(ctx, n);
+  // the basis kept, in one persistent launch (lanres.cu): the second pass would form the same vectors again
+  const int64_t ldv = (n + 31) / 32 * 32;
+  if (lan_res_takes(H, false) && (int64_t)(kdim + 2) * ldv * (int64_t)sizeof(VV) <= kHermBasisBytes) {
+    LanczosBuffers<VV>& B = herm_buffers<VV>(W);
+    B.ensure(n, kdim + 1);
+    QD_CUDA(cudaMemsetAsync(B.stop.p, 0, sizeof(int), ctx->stream));
+    const double one = 1.0;
+    QD_CUDA(cudaMemcpyAsync(B.scl.p, &one, sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+    init_v0_kernel<VV><<<vg, kVecThreads, 0, ctx->stream>>>(n, psi, psi_nrm2, B.V.p);
+    QD_CHECK_LAUNCH();
+    QD_LAUNCHED(ctx);
+    LanRun<MV, VV> r{};
+    r.vals = vals;
+    r.rule = kLanPaige;
+    r.V = B.V.p;
+    r.ld = B.ld;
+    r.kdim = B.kdim;
+    r.first = 1;
+    r.last = kdim + 1;       // a_0 and kdim more (the reference's idx runs 1..kdim)
+    r.stop_below = 1e-5;     // nn <= 1e-10 (qudrip.hpp:18)
+    r.alpha = B.alpha.p;
+    r.nrm = B.nrm.p;
+    r.scl = B.scl.p;
+    r.stop = B.stop.p;
+    r.flags = lan_flags(W);
+    r.slots = &W.lan_slots;
+    if (lan_res_run(H, r)) {
+      std::vector<VV> ha(kdim + 2);
+      std::vector<double> hn(kdim + 2), hs(kdim + 2);
+      int st = 0;
+      QD_CUDA(cudaMemcpyAsync(ha.data(), B.alpha.p, (kdim + 2) * sizeof(VV), cudaMemcpyDeviceToHost, ctx->stream));
+      QD_CUDA(cudaMemcpyAsync(hn.data(), B.nrm.p, (kdim + 2) * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+      QD_CUDA(cudaMemcpyAsync(hs.data(), B.scl.p, (kdim + 2) * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+      QD_CUDA(cudaMemcpyAsync(&st, B.stop.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+      fx_flags(ctx, W.lan_flags.p);
+      const int K = st ? st : kdim + 1;
+      std::vector<double> d(K), e(K), ev(K), z(K);
+      for (int i = 0; i < K; ++i) {
+        d[i] = real_part(ha[i + 1]);
+        e[i] = (i + 1 < K) ? hn[i + 1] : 0.0;
+      }
+      QD_REQUIRE(tridiag_lowest<double>(K, d.data(), e.data(), ev.data(), z.data()) == 0, QD_ERR_INVALID,
+                 "tridiagonal eigensolver did not converge");
+      for (int i = 0; i < K; ++i) z[i] *= hs[i];
+      QD_CUDA(cudaMemcpyAsync(B.y.p, z.data(), K * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+      launch_ritz(ctx, n, B.V.p, std::is_same<VV, double>::value, B.ld, B.y.p, K, psi);
+      QD_CUDA(cudaStreamSynchronize(ctx->stream));
+      if (evals_out) std::memcpy(evals_out, ev.data(), K * sizeof(double));
+      res->act_dim = K;
+      res->breakdown = st ? 1 : 0;
+      res->matvecs = 2 * K - 1;  // as the two passes count them
+      res->ritz_value = ev[0];
+      res->err = hn[K];
+      return;
+    }
+  }
   DBuf<VV> v(n), w(n), h(n), a(kdim + 2);
   DBuf<double> nn(kdim + 2);
   DBuf<int> stop(1);
@@ -1195,17 +1319,9 @@ void hermitian_lanczos_ground(qd_ham* H, cplx* psi, int kdim, double* evals_out,
   QD_REQUIRE(kdim >= 1 && kdim <= 4096, QD_ERR_INVALID, "krylov_dim must be in 1..4096");
   QD_REQUIRE(H->flags & QD_HAM_HERMITIAN, QD_ERR_NOT_HERMITIAN, "Hermitian::LanczosSolver needs a Hermitian operator");
   Workspace& W = ham_workspace(H);
-  DBuf<double> nrm2(1);
-  DBuf<int> has_im(1);
-  QD_CUDA(cudaMemsetAsync(has_im.p, 0, sizeof(int), ctx->stream));
-  colnorm_kernel<<<vec_grid(ctx, n), kVecThreads, 0, ctx->stream>>>(n, psi, nrm2.p, W.red_d(0), has_im.p);
-  QD_CHECK_LAUNCH();
-  QD_LAUNCHED(ctx);
-  int him = 0;
-  double hn = 0.0;
-  QD_CUDA(cudaMemcpyAsync(&him, has_im.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  QD_CUDA(cudaMemcpyAsync(&hn, nrm2.p, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  QD_CUDA(cudaStreamSynchronize(ctx->stream));
+  bool him = false;
+  const double hn = state_norm2_imag(H, psi, &him);
+  const DBuf<double>& nrm2 = W.start_nrm2;
   QD_REQUIRE(hn > 0.0 && std::isfinite(hn), QD_ERR_INVALID, "start vector has zero or non-finite norm");
   const bool real_h = (H->flags & QD_HAM_REAL) != 0;
   if (real_h && !him)
@@ -1330,8 +1446,27 @@ static void lanczos_evolve_steps(qd_ham* H, cplx* psi, double h, int m, int nste
     G.matvecs.alloc(1);
   }
   const double one = 1.0;
-  QD_CUDA(cudaMemcpyAsync(B.scl.p, &one, sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
   QD_CUDA(cudaMemsetAsync(G.matvecs.p, 0, sizeof(long long), ctx->stream));
+  // one launch per Krylov step (lanres.cu) where the recurrence fits the grid
+  bool res_run = lan_res_takes(H, false);
+  if (res_run) {
+    int* flags = lan_flags(W);
+    for (int s = 0; s < nsteps && res_run; ++s) {
+      res_run = lan_res_evolve<MV>(H, vals, psi, B.V.p, B.ld, kdim, h, G.act.p, G.matvecs.p, flags, &W.lan_slots);
+      QD_REQUIRE(res_run || s == 0, QD_ERR_UNSUPPORTED, "the persistent recurrence's grid does not fit any more");
+    }
+  }
+  if (res_run) {
+    int act = 0;
+    long long mv = 0;
+    QD_CUDA(cudaMemcpyAsync(&act, G.act.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    QD_CUDA(cudaMemcpyAsync(&mv, G.matvecs.p, sizeof(long long), cudaMemcpyDeviceToHost, ctx->stream));
+    fx_flags(ctx, W.lan_flags.p);
+    if (act_out) *act_out = act;
+    if (matvecs_out) *matvecs_out = mv;
+    return;
+  }
+  QD_CUDA(cudaMemcpyAsync(B.scl.p, &one, sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
   if (B.kind != 0) {
     B.drop_graph();
     B.kind = 0;
@@ -1404,19 +1539,9 @@ void lanczos_evolve(qd_ham* H, const cplx* psi_in, cplx* psi_out, double h, int 
   QD_REQUIRE(nsteps >= 1, QD_ERR_INVALID, "nsteps must be positive");
   QD_REQUIRE(H->flags & QD_HAM_HERMITIAN, QD_ERR_NOT_HERMITIAN,
              "the short-recurrence Krylov exponential needs a Hermitian operator");
-  Workspace& W = ham_workspace(H);
-  {
-    DBuf<double> nrm2(1);
-    DBuf<int> has_im(1);
-    QD_CUDA(cudaMemsetAsync(has_im.p, 0, sizeof(int), ctx->stream));
-    colnorm_kernel<<<vec_grid(ctx, n), kVecThreads, 0, ctx->stream>>>(n, psi_in, nrm2.p, W.red_d(0), has_im.p);
-    QD_CHECK_LAUNCH();
-    QD_LAUNCHED(ctx);
-    double hn = 0.0;
-    QD_CUDA(cudaMemcpyAsync(&hn, nrm2.p, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    QD_CUDA(cudaStreamSynchronize(ctx->stream));
-    QD_REQUIRE(hn > 0.0 && std::isfinite(hn), QD_ERR_INVALID, "input state has zero or non-finite norm");
-  }
+  bool has_imag = false;
+  const double hn = state_norm2_imag(H, psi_in, &has_imag);
+  QD_REQUIRE(hn > 0.0 && std::isfinite(hn), QD_ERR_INVALID, "input state has zero or non-finite norm");
   if (psi_out != psi_in)
     QD_CUDA(cudaMemcpyAsync(psi_out, psi_in, n * sizeof(cplx), cudaMemcpyDeviceToDevice, ctx->stream));
   if (H->flags & QD_HAM_REAL)

@@ -98,12 +98,21 @@ struct EvolveGraphDeleter {
   void operator()(EvolveGraph* g) const;
 };
 
+// The grid of a persistent Lanczos recurrence (lanres.cu), chosen on its first run on an operator.
+struct LanPlan {
+  bool ok = false;
+  int csize = 1, ncl = 1;  // blocks per cluster, clusters
+  int rows = 0;            // most rows of a block
+  DBuf<int> first;         // first row of each block, and the number of rows
+};
+
 struct Workspace {
   Ctx* ctx;
   std::unique_ptr<EvolveGraph, EvolveGraphDeleter> evolve;  // cached Krylov-step graph
   // the last Lanczos ground-state run: vector type (1 real, 2 complex), value
   // type (1 real, 2 complex), product kind -- what a continuation must reuse
   int lz_vv = 0, lz_mv = 0, lz_mf = 0, lz_fxk = 0;
+  bool lz_res = false;  // ... and whether the persistent form ran it
   DBuf<double> partials_d, gpart_d;
   DBuf<cplx> partials_c, gpart_c;
   DBuf<Tri<double>> partials_td, gpart_td;
@@ -111,6 +120,12 @@ struct Workspace {
   DBuf<unsigned> tickets;
   LanczosBuffers<double> lz_d;
   LanczosBuffers<cplx> lz_c;
+  LanczosBuffers<double> hl_d;  // Hermitian::LanczosSolver's, apart from an open incremental solve
+  LanczosBuffers<cplx> hl_c;
+  LanPlan lan_plan[5];          // real and complex, local and Paige's rule, the exponential
+  DBuf<double> lan_slots;
+  DBuf<char> lan_x;             // fixed-point copies of the basis (uniform couplings)
+  DBuf<int> lan_flags;
   // H psi and the result of state_eval, kept between calls (a device allocation
   // and free per call would wait for the whole device)
   DBuf<cplx> eval_y, eval_out;

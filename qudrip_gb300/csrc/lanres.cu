@@ -1,0 +1,702 @@
+// lanres.cu -- the Lanczos recurrence as one persistent launch.
+//
+// A step (krylov.cu) is a product, three inner products, an update and a norm.
+// Launched step by step it cannot take less than its launches and their
+// reductions: at dim 12,870 the one-launch step of the uniform-coupling form
+// took 18 us, at dim 184,756 the three kernels of a complex step 66 us, where
+// the arithmetic is 0.3 and 15.  Here the grid (clusters of eight blocks, one
+// block per SM) stays for all steps, a block keeps its rows of the last two
+// vectors and of w in shared memory, and the blocks exchange one small sum a
+// step (gridx.cuh): the inner products of the product with the two last
+// vectors, and, from the update before, the norm of the newest vector and its
+// overlap with the one before, which scale everything.  The product gathers
+// the newest vector as its rows arrive from the other blocks.
+//
+// The block's sums of its threads' partial sums are integer adds: a warp-wide
+// FP64 add takes 76 cycles on GB300 and a butterfly of seven values over
+// sixteen warps 10,600; as 53-bit integers on the scale of the largest partial
+// sum it is 2,200, and each partial sum keeps what an FP64 sum would round.
+//
+// Hermitian::LanczosSolver runs here with its basis kept, where the reference
+// forms every vector a second time for the Ritz vector.
+//
+// Measured (GB300): a step at dim 12,870 (uniform couplings) 18 -> 9 us, complex
+// at dim 184,756 61 -> 28 us (the FP64 product is 14 of them, rows of unequal
+// length in a warp and the exchange most of the rest), real couplings per bond
+// there 41 -> 22 us; Hermitian solver at dim 4,900 2.3 -> 0.42 ms a solve.
+// Mean error against 64-bit references over ten random cases each: ground-state
+// eigenvalues 5.4e-16 (launched step by step: 5.6e-16), evolved states 1.95e-15
+// (1.99e-15).
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <vector>
+
+#include "gridx.cuh"
+#include "lanres.cuh"
+#include "qvec.cuh"
+
+namespace qd {
+
+constexpr int kLanThreads = 512;
+constexpr int kLanMinRows = 96;  // rows of a block before the grid covers every SM
+// Clusters of eight keep the exchange short; of four cover more SMs (148 of 152 against 120, which is
+// what one block per SM and whole clusters per GPC leave), which pays once a block's rows outweigh it.
+constexpr int64_t kLanWideRows = 1 << 16;
+constexpr int kLanMaxExp = 32;
+
+template <typename MV, typename VV>
+struct LanArgs {
+  int64_t n, ld;
+  int rows;               // most rows of a block
+  const int* row_first;   // first row of each block, then n
+  const int64_t* rowptr;
+  const int32_t* colidx;
+  const MV* vals;
+  const double* fxdiag;  // uniform couplings: the diagonal (null: zero), c 2^-F and F
+  double cF;
+  int F;
+  const int32_t *fxptr, *fxcol;  // its off-diagonal columns (null: from the CSR rows)
+  XInt* XV;              // fixed-point copy of V[k] at XV + (k - first + 1) ld
+  VV* V;
+  int first, last;
+  double stop_below;
+  VV *alpha, *beta;
+  double *nrm, *scl;
+  int* stop;
+  int* ovf;
+  // the Krylov exponential
+  cplx* psi;
+  double h;
+  int* act;
+  long long* matvecs;
+  double* slots;
+  int xstride;
+  GridX X;
+};
+
+__device__ __forceinline__ __int128 lan_shfl(__int128 v, int o) {
+  const unsigned long long lo = __shfl_xor_sync(0xffffffffu, (unsigned long long)v, o);
+  const long long hi = __shfl_xor_sync(0xffffffffu, (long long)(v >> 64), o);
+  return ((__int128)hi << 64) | lo;
+}
+
+// One row of H x (FP64), shared by `lanes` threads, four loads in flight.  wait: x is being written in
+// this launch, an element is taken once it is there.
+template <typename MV, typename VV>
+__device__ __forceinline__ VV lan_row(const LanArgs<MV, VV>& A, const VV* x, int64_t r, bool live, int sub, int lanes,
+                                      bool wait) {
+  VV acc = vzero(VV{});
+  if (live) {
+    const int64_t e = __ldg(A.rowptr + r + 1);
+    for (int64_t k = __ldg(A.rowptr + r) + sub; k < e; k += 4 * lanes) {
+      int32_t c[4];
+      MV v[4];
+      VV xv[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (k + u * lanes < e) {
+          c[u] = __ldg(A.colidx + k + u * lanes);
+          v[u] = ld_ro(A.vals + k + u * lanes);
+        }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (k + u * lanes < e) xv[u] = x_peek(x + c[u]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (k + u * lanes < e) {
+          if (wait) x_await(A.X, x + c[u], xv[u]);
+          acc = vfma(v[u], xv[u], acc);
+        }
+    }
+  }
+  for (int o = lanes >> 1; o > 0; o >>= 1) acc = vadd(acc, shfl_xor(acc, o));
+  return acc;
+}
+
+// The same for uniform couplings: the 128-bit fixed-point copies (fxsum.cuh) that the blocks keep beside
+// their rows, summed exactly and rounded once; the diagonal apart.  Every off-diagonal value is one c,
+// explicit zeros skipped.  (Converting each gathered double instead took twice the FP64 product's time.)
+__device__ __forceinline__ double lan_row_uniform(const LanArgs<double, double>& A, const XInt* x, int64_t r,
+                                                  bool live, int sub, int lanes, double own) {
+  __int128 acc = 0;
+  if (live) {
+    const bool listed = A.fxptr != nullptr;  // the form's own list of off-diagonal columns
+    const int32_t* col = listed ? A.fxcol : A.colidx;
+    const int64_t e = listed ? (int64_t)__ldg(A.fxptr + r + 1) : __ldg(A.rowptr + r + 1);
+    for (int64_t k = (listed ? (int64_t)__ldg(A.fxptr + r) : __ldg(A.rowptr + r)) + sub; k < e; k += 4 * lanes) {
+      int32_t c[4];
+      XInt xv[4];
+      bool on[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        on[u] = k + u * lanes < e;
+        if (on[u]) c[u] = __ldg(col + k + u * lanes);
+        if (!listed && on[u]) on[u] = c[u] != (int32_t)r && __ldg(A.vals + k + u * lanes) != 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (on[u]) xv[u] = x_peek(x + c[u]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (on[u]) {
+          x_await(A.X, x + c[u], xv[u]);
+          acc += x_value(xv[u]);
+        }
+    }
+  }
+  for (int o = lanes >> 1; o > 0; o >>= 1) acc += lan_shfl(acc, o);
+  const double dx = (live && A.fxdiag) ? __ldg(A.fxdiag + r) * own : 0.0;
+  return fma(A.cF, (double)acc, dx);
+}
+
+// v on the scale 2^E (|v| < 2^E) in units of 2^(E - 53)
+__device__ __forceinline__ long long lan_fix(double v, int E) {
+  const long long b = __double_as_longlong(v);
+  const int e = (int)((b >> 52) & 0x7ff);
+  const unsigned long long m = ((unsigned long long)b & 0xfffffffffffffull) | 0x10000000000000ull;
+  const int sh = E + 1022 - e;  // >= 0
+  long long q = (e == 0 || sh > 53) ? 0ll : (long long)(sh > 0 ? (m + (1ull << (sh - 1))) >> sh : m);
+  return b < 0 ? -q : q;
+}
+
+template <int T>
+struct LanShared {
+  unsigned mx[8][T / 32];
+  long long q[8][T / 32];
+  double v[8], red[8];
+  double sw, c1[2], c2[2];  // the update's scale and coefficients (re, im)
+  double s1, s2;            // scales of V[k-1] and V[k-2]
+  int stop;
+};
+
+// The block's sums of NV values per thread into S.v (complete after the next block barrier).
+// Only the first nact warps hold any (the others' slots are zero from the start).
+template <int NV, int T>
+__device__ __forceinline__ void lan_block_sums(LanShared<T>& S, const double (&v)[NV], int nact) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int nw = T / 32;
+  if (warp < nact) {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const unsigned m = __reduce_max_sync(0xffffffffu, q_mag(v[i]));
+      if (lane == 0) S.mx[i][warp] = m;
+    }
+  }
+  __syncthreads();
+  unsigned mag[NV];
+  if (warp < nact) {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      mag[i] = __reduce_max_sync(0xffffffffu, lane < nw ? S.mx[i][lane] : 0u);
+      long long q = lan_fix(v[i], (int)(mag[i] >> 20) - 1022);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+      if (lane == 0) S.q[i][warp] = q;
+    }
+  }
+  __syncthreads();
+  if (warp == 0) {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      long long q = lane < nw ? S.q[i][lane] : 0ll;
+#pragma unroll
+      for (int o = nw / 2; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+      if (lane == i) {
+        const int e = (int)(mag[i] >> 20), ue = e - 1022 - 53 + 1023;
+        S.v[i] = (e == 0x7ff) ? __longlong_as_double(0x7ff8000000000000ll)
+                              : (ue > 0 ? (double)q * __hiloint2double(ue << 20, 0) : 0.0);
+      }
+    }
+  }
+}
+
+__device__ __forceinline__ double lan_re(double v) { return v; }
+__device__ __forceinline__ double lan_re(cplx v) { return v.re; }
+__device__ __forceinline__ double lan_im(double) { return 0.0; }
+__device__ __forceinline__ double lan_im(cplx v) { return v.im; }
+__device__ __forceinline__ void lan_make(double& d, double re, double) { d = re; }
+__device__ __forceinline__ void lan_make(cplx& d, double re, double im) { d = mkc(re, im); }
+__device__ __forceinline__ double lan_redot(double a, double b, double acc) { return fma(a, b, acc); }
+__device__ __forceinline__ double lan_redot(cplx a, cplx b, double acc) {
+  return fma(a.im, b.im, fma(a.re, b.re, acc));
+}
+
+// y = exp(-i h T) e_0, T = tridiag(al[0 .. act), be[1 .. act)), by one warp: Taylor terms on sub-steps of
+// infinity-norm at most 1 (as texp_kernel, krylov.cu, with its terms counted from the remainder bound).
+__device__ __forceinline__ void lan_texp(int act, double h, double d, double e, double& yr, double& yi) {
+  const int lane = threadIdx.x & 31;
+  double em = __shfl_up_sync(0xffffffffu, e, 1);
+  if (lane == 0) em = 0.0;
+  const double rs = fabs(d) + fabs(e) + fabs(em);
+  const unsigned mx = __reduce_max_sync(0xffffffffu, q_mag(rs));
+  const double theta = __hiloint2double((int)mx, -1) * fabs(h);
+  const int steps = (theta <= 1e6) ? max(1, (int)ceil(theta)) : 1;  // a NaN gives NaNs either way
+  const double hs = h / steps, th = theta / steps;
+  // lane p holds hs / p; terms to th^p / p! <= 1e-18
+  const double f = lane > 0 ? hs / lane : 0.0;
+  int terms = 1;
+  double b = th;
+  while (b > 1e-18 && terms < 30) {
+    ++terms;
+    b *= th / terms;
+  }
+  yr = (lane == 0) ? 1.0 : 0.0;
+  yi = 0.0;
+  for (int s = 0; s < steps; ++s) {
+    double tr = yr, ti = yi;
+    for (int p = 1; p <= terms; ++p) {
+      const double fp = __shfl_sync(0xffffffffu, f, p);
+      const double rdn = __shfl_down_sync(0xffffffffu, tr, 1), idn = __shfl_down_sync(0xffffffffu, ti, 1);
+      const double rup = __shfl_up_sync(0xffffffffu, tr, 1), iup = __shfl_up_sync(0xffffffffu, ti, 1);
+      // e and em are 0 beyond the matrix, so the shuffles' ends drop out
+      const double kr = fma(d, tr, fma(e, rdn, em * rup)), ki = fma(d, ti, fma(e, idn, em * iup));
+      tr = fp * ki;
+      ti = -fp * kr;
+      yr += tr;
+      yi += ti;
+    }
+  }
+}
+
+template <typename MV, typename VV, int C, bool kUni, bool kPaige, bool kExp>
+__global__ void __launch_bounds__(kLanThreads, 1) lan_kernel(LanArgs<MV, VV> A) {
+  constexpr int T = kLanThreads, kPer = sizeof(VV) / sizeof(double);
+  constexpr int NV = kPaige ? 2 : 1 + 3 * kPer;
+  extern __shared__ __align__(16) unsigned char lan_smem[];
+  __shared__ LanShared<T> S;
+  __shared__ double talpha[kExp ? kLanMaxExp + 1 : 1], tnrm[kExp ? kLanMaxExp + 1 : 1], tscl[kExp ? kLanMaxExp + 1 : 1];
+  __shared__ cplx y[kExp ? kLanMaxExp : 1];
+  const int tid = threadIdx.x;
+  const int64_t r0 = A.row_first[blockIdx.x];
+  const int R = A.row_first[blockIdx.x + 1] - (int)r0;
+  VV* ring = reinterpret_cast<VV*>(lan_smem);  // V[k] of the block's rows at ring + (k % 3) rows
+  VV* Vg = A.V + r0;
+  const GridX& X = A.X;
+  const bool mute = X.hold && blockIdx.x == 0;
+  int lanes = 1;
+  while (lanes < 4 && 2 * lanes * A.rows <= (kUni ? 512 : 256)) lanes *= 2;
+  double vals[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) vals[i] = 0.0;
+  const int nact = max(1, min(T / 32, (R * lanes + 31) / 32));  // warps with rows
+  for (int i = tid; i < 8 * (T / 32); i += T) {
+    S.mx[i / (T / 32)][i % (T / 32)] = 0;
+    S.q[i / (T / 32)][i % (T / 32)] = 0;
+  }
+  if (kExp && tid == 0) S.s1 = S.s2 = 0.0;
+  // the rows of the vectors the first step reads; kExp: V[0] = psi, its norm still to come
+  if (kExp) {
+    for (int r = tid; r < R; r += T) {
+      VV v;
+      lan_make(v, A.psi[r0 + r].re, A.psi[r0 + r].im);
+      ring[r] = v;
+      Vg[r] = v;
+      vals[NV - 1] = lan_redot(v, v, vals[NV - 1]);
+    }
+  } else {
+    for (int b = 1; b <= 2; ++b) {
+      const int j = A.first - b;
+      if (j >= 0)
+        for (int r = tid; r < R; r += T) ring[(size_t)(j % 3) * A.rows + r] = Vg[(int64_t)j * A.ld + r];
+    }
+    if (!kPaige && A.first > 1) {  // <V1, V2>
+      __syncthreads();
+      VV d3 = vzero(VV{});
+      const VV *u1 = ring + (size_t)((A.first - 1) % 3) * A.rows, *u2 = ring + (size_t)((A.first - 2) % 3) * A.rows;
+      for (int r = tid; r < R; r += T) d3 = vdotfma(u1[r], u2[r], d3);
+      vals[2 * kPer] = lan_re(d3);
+      if (kPer == 2) vals[2 * kPer + 1] = lan_im(d3);
+    }
+    if (tid == 0) {
+      S.s1 = A.scl[A.first - 1];
+      S.s2 = A.first > 1 ? A.scl[A.first - 2] : 0.0;
+    }
+  }
+  __syncthreads();
+  int ov = 0, stop = 0;
+  if constexpr (kUni)
+    for (int r = tid; r < R; r += T)
+      if (!mute) x_put(A.XV + r0 + r, fx_from_double(ring[(size_t)((A.first - 1) % 3) * A.rows + r], A.F, &ov));
+  for (int k = A.first; k <= A.last; ++k) {
+    const VV* u1 = ring + (size_t)((k - 1) % 3) * A.rows;
+    const VV* u2 = ring + (size_t)((k + 1) % 3) * A.rows;  // V[k-2]
+    VV* w = ring + (size_t)(k % 3) * A.rows;
+    const bool has2 = k >= 2, known = !kExp && k == A.first;  // known: V[k-1]'s scale is from before
+    const VV* x = A.V + (int64_t)(k - 1) * A.ld;
+    if constexpr (kExp && sizeof(VV) == sizeof(cplx))
+      if (k == 1) x = reinterpret_cast<const VV*>(A.psi);
+    // w = H V1 (not scaled) and its inner products
+    {
+      VV d1 = vzero(VV{}), d2 = vzero(VV{});
+      double d2re = 0.0;
+      const int g = tid / lanes, sub = tid & (lanes - 1), per = T / lanes;
+      for (int r = g; (r & ~(32 / lanes - 1)) < R; r += per) {  // whole warps
+        const bool live = r < R;
+        VV a;
+        if constexpr (kUni)
+          a = lan_row_uniform(A, A.XV + (int64_t)(k - A.first) * A.ld, r0 + r, live, sub, lanes, live ? u1[r] : 0.0);
+        else a = lan_row(A, x, r0 + r, live, sub, lanes, k > A.first);
+        if (live && sub == 0) {
+          w[r] = a;
+          if (kPaige) {
+            d2re = lan_redot(u1[r], a, d2re);
+          } else {
+            d2 = vdotfma(u1[r], a, d2);
+            if (has2) d1 = vdotfma(u2[r], a, d1);
+          }
+        }
+      }
+      if (kPaige) {
+        vals[0] = d2re;
+      } else {
+        vals[0] = lan_re(d1);
+        vals[kPer] = lan_re(d2);
+        if (kPer == 2) {
+          vals[1] = lan_im(d1);
+          vals[kPer + 1] = lan_im(d2);
+        }
+      }
+    }
+    lan_block_sums<NV, T>(S, vals, nact);
+    __syncthreads();
+    x_sum<C>(X, A.slots + (size_t)(k - A.first) * A.xstride, S.v, NV, S.red);
+    // the scale of V1 from its norm, alpha and beta, and the update's coefficients: one chain of scalar
+    // FP64 operations (64 cycles each), what the update does not wait for on a second warp
+    if (tid == 0) {
+      const double s1 = known ? S.s1 : rsqrt(S.red[NV - 1]), s2 = S.s2;
+      double ar, ai = 0.0, br = 0.0, bi = 0.0;
+      if (kPaige) {
+        ar = (s1 * s1) * S.red[0];
+        br = !has2 ? 0.0 : (known ? 1.0 / s1 : S.red[NV - 1] * s1);  // ||V1||
+      } else {
+        const double* d = S.red;
+        const double s12 = s1 * s2;
+        br = has2 ? s12 * d[0] : 0.0;
+        ar = s1 * d[kPer];
+        if (kPer == 2) {
+          bi = has2 ? s12 * d[1] : 0.0;
+          ai = s1 * d[kPer + 1];
+        }
+        if (has2) {  // - (beta s2) <V1, V2>
+          const double pr = br * s2, pi = bi * s2, qr = d[2 * kPer], qi = kPer == 2 ? d[2 * kPer + 1] : 0.0;
+          ar = fma(-pr, qr, ar);
+          if (kPer == 2) {
+            ar = fma(pi, qi, ar);
+            ai = fma(-pr, qi, fma(-pi, qr, ai));
+          }
+        }
+        ar *= s1;
+        ai *= s1;
+      }
+      S.sw = s1;
+      S.c1[0] = ar * s1;
+      S.c1[1] = ai * s1;
+      S.c2[0] = br * s2;
+      S.c2[1] = bi * s2;
+      if (kExp) {
+        talpha[k] = ar;
+      } else if (blockIdx.x == 0) {
+        VV v;
+        lan_make(v, ar, ai);
+        A.alpha[k] = v;
+        lan_make(v, br, bi);
+        if (A.beta) A.beta[k] = v;
+      }
+    } else if (tid == T - 32) {
+      S.stop = 0;
+      if (!known) {
+        const double n2 = S.red[NV - 1], s1 = rsqrt(n2), nr = n2 > 0.0 ? n2 * s1 : n2;
+        S.stop = (k > 1 || !kExp) && nr < A.stop_below;
+        if (kExp) {
+          tnrm[k - 1] = nr;
+          tscl[k - 1] = s1;
+        } else if (blockIdx.x == 0) {
+          A.nrm[k - 1] = nr;
+          A.scl[k - 1] = s1;
+        }
+      }
+    }
+    __syncthreads();
+    if (S.stop) {
+      stop = k - 1;
+      break;
+    }
+    // V[k] = (s1 w - (beta s2) V2) - (alpha s1) V1, its norm and its overlap with V1
+    {
+      const double sw = S.sw;
+      if (tid == 0) S.s2 = S.s1 = sw;
+      VV a, b, d3 = vzero(VV{});
+      lan_make(a, S.c1[0], S.c1[1]);
+      lan_make(b, S.c2[0], S.c2[1]);
+      double n2 = 0.0;
+      VV* vk = Vg + (int64_t)k * A.ld;
+      for (int r = tid; r < R; r += T) {
+        VV o = vscale(sw, w[r]);
+        if constexpr (kPaige) {  // real coefficients
+          if (has2) o = vfma(-S.c2[0], u2[r], o);
+          o = vfma(-S.c1[0], u1[r], o);
+        } else {
+          if (has2) o = vsubmul(o, b, u2[r]);
+          o = vsubmul(o, a, u1[r]);
+        }
+        w[r] = o;
+        if constexpr (kUni) {
+          vk[r] = o;
+          if (!mute) x_put(A.XV + (int64_t)(k - A.first + 1) * A.ld + r0 + r, fx_from_double(o, A.F, &ov));
+        } else {
+          if (!mute) x_put(vk + r, o);
+        }
+        n2 = lan_redot(o, o, n2);
+        if (!kPaige) d3 = vdotfma(o, u1[r], d3);
+      }
+      vals[NV - 1] = n2;
+      if (!kPaige) {
+        vals[2 * kPer] = lan_re(d3);
+        if (kPer == 2) vals[2 * kPer + 1] = lan_im(d3);
+      }
+    }
+    __syncthreads();
+  }
+  if (kUni && ov) *A.ovf = 1;
+  if (!kExp || !stop) {
+    if (!stop) {  // the last vector's norm
+      lan_block_sums<NV, T>(S, vals, nact);
+      __syncthreads();
+      x_sum<C>(X, A.slots + (size_t)(A.last + 1 - A.first) * A.xstride, S.v, NV, S.red);
+      if (tid == 0) {
+        const double n2 = S.red[NV - 1], nr = n2 > 0.0 ? n2 * rsqrt(n2) : n2;
+        S.stop = nr < A.stop_below;
+        if (!kExp && blockIdx.x == 0) {
+          A.nrm[A.last] = nr;
+          A.scl[A.last] = rsqrt(n2);
+        }
+      }
+      __syncthreads();
+      if (S.stop) stop = A.last;
+    }
+    if (!kExp) {
+      if (blockIdx.x == 0 && tid == 0 && stop) *A.stop = stop;
+      return;
+    }
+  }
+  if constexpr (kExp) {
+    // expandBasis<0>'s count: the breaking step is kept
+    const int act = stop ? stop : A.last;
+    if (tid < 32) {
+      const double d = tid < act ? talpha[tid + 1] : 0.0, e = tid + 1 < act ? tnrm[tid + 1] : 0.0;
+      double yr, yi;
+      lan_texp(act, A.h, d, e, yr, yi);
+      if (tid < act) y[tid] = mkc(yr * tscl[tid], yi * tscl[tid]);
+    }
+    __syncthreads();
+    if (*reinterpret_cast<volatile int*>(X.abort) == kXAborted) return;
+    if (blockIdx.x == 0 && tid == 0) {
+      *A.act = act;
+      *A.matvecs += act;
+    }
+    if constexpr (sizeof(VV) == sizeof(cplx)) {
+      cplx* out = A.psi + r0;  // read by the others in the first step only
+      for (int r = tid; r < R; r += T) {
+        const cplx* v = reinterpret_cast<const cplx*>(Vg) + r;
+        cplx a = mkc(0.0, 0.0);
+        int j = 0;
+        for (; j + 4 <= act; j += 4, v += 4 * A.ld) {
+          const cplx v0 = v[0], v1 = v[A.ld], v2 = v[2 * A.ld], v3 = v[3 * A.ld];
+          a = vfma(y[j], v0, a);
+          a = vfma(y[j + 1], v1, a);
+          a = vfma(y[j + 2], v2, a);
+          a = vfma(y[j + 3], v3, a);
+        }
+        for (; j < act; ++j, v += A.ld) a = vfma(y[j], v[0], a);
+        out[r] = a;
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------- host
+// First rows of `grid` blocks of nearly equal work: a row costs about what six entries do (its share of
+// the inner products, the update and the norm).  Equal row counts left the blocks of a spin chain, whose
+// rows' lengths follow their states, waiting for the longest: 24,000 of 65,000 cycles a step at L = 20.
+__global__ void lan_rows_kernel(int64_t n, const int64_t* rowptr, int grid, int* first) {
+  const double total = (double)rowptr[n] + 6.0 * (double)n;
+  for (int b = threadIdx.x; b <= grid; b += blockDim.x) {
+    const double want = total * b / grid;
+    int64_t lo = 0, hi = n;
+    while (lo < hi) {
+      const int64_t mid = (lo + hi) >> 1;
+      if ((double)rowptr[mid] + 6.0 * (double)mid < want) lo = mid + 1;
+      else hi = mid;
+    }
+    first[b] = b == grid ? (int)n : (int)lo;
+  }
+}
+
+// The kernel of each cluster size; cfg for the one the sector takes.  False when the device does not hold
+// the grid at once, or a block its rows.
+template <typename VV, typename K>
+static bool lan_plan(qd_ham* H, K kern1, K kern4, K kern8, LanPlan& P, cudaLaunchConfig_t& cfg,
+                     cudaLaunchAttribute (&at)[2], K& kern) {
+  Ctx* ctx = H->ctx;
+  const int64_t n = H->dim;
+  const int csize = n <= 64 ? 1 : (n <= kLanWideRows ? 8 : 4);  // one block: an exchange would cost more than it saves
+  kern = csize == 1 ? kern1 : (csize == 4 ? kern4 : kern8);
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = (unsigned)csize;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  cfg.blockDim = dim3(kLanThreads);
+  cfg.stream = ctx->stream;
+  cfg.attrs = at;
+  cfg.numAttrs = csize == 1 ? 1 : 2;
+  const auto smem_of = [](int rows) { return (size_t)3 * rows * sizeof(VV); };
+  if (!P.ok) {
+    int maxsm = 0;
+    QD_CUDA(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    int ncl = csize == 1 ? 1 : (int)std::min<int64_t>(ctx->num_sms / csize, ceil_div(n, csize * kLanMinRows));
+    int rows = (int)n;
+    std::vector<int> first;
+    for (;;) {
+      const int grid = ncl * csize;
+      if (P.first.n < (size_t)grid + 1) P.first.alloc(grid + 1);
+      lan_rows_kernel<<<1, 256, 0, ctx->stream>>>(n, H->rowptr.p, grid, P.first.p);
+      QD_CHECK_LAUNCH();
+      QD_LAUNCHED(ctx);
+      if (csize > 1) {
+        first.resize(grid + 1);
+        QD_CUDA(cudaMemcpyAsync(first.data(), P.first.p, (grid + 1) * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+        QD_CUDA(cudaStreamSynchronize(ctx->stream));
+        rows = 1;
+        for (int b = 0; b < grid; ++b) rows = std::max(rows, first[b + 1] - first[b]);
+      }
+      if (smem_of(rows) + 8192 > (size_t)maxsm) return false;
+      if (csize == 1) break;
+      QD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(rows)));
+      cfg.gridDim = dim3((unsigned)grid);
+      cfg.dynamicSmemBytes = smem_of(rows);
+      cudaLaunchConfig_t q = cfg;
+      q.attrs = at + 1;
+      q.numAttrs = 1;
+      int fit = 0;
+      QD_CUDA(cudaOccupancyMaxActiveClusters(&fit, kern, &q));
+      if (fit >= ncl) break;
+      if (fit < 1) return false;
+      ncl = fit;
+    }
+    P.ok = true;
+    P.csize = csize;
+    P.ncl = ncl;
+    P.rows = rows;
+  }
+  cfg.gridDim = dim3((unsigned)(P.ncl * csize));
+  cfg.dynamicSmemBytes = smem_of(P.rows);
+  QD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes));
+  return true;
+}
+
+template <typename MV, typename VV>
+static LanArgs<MV, VV> lan_args(qd_ham* H, const MV* vals, const LanPlan& P, VV* V, int64_t ld, int first, int last,
+                                int nv, int* flags, DBuf<double>* slots, XInt* xv) {
+  Ctx* ctx = H->ctx;
+  LanArgs<MV, VV> A;
+  std::memset(&A, 0, sizeof(A));
+  A.n = H->dim;
+  A.ld = ld;
+  A.rows = P.rows;
+  A.row_first = P.first.p;
+  A.rowptr = H->rowptr.p;
+  A.colidx = H->colidx.p;
+  A.vals = vals;
+  A.V = V;
+  A.first = first;
+  A.last = last;
+  A.xstride = P.ncl * nv;
+  const size_t want = (size_t)(last + 2 - first) * A.xstride;
+  if (slots->n < want) slots->alloc(want);
+  A.slots = slots->p;
+  A.X.abort = flags + 1;
+  const unsigned wait_out = step_wait_out_polls();
+  A.X.polls = wait_out ? wait_out : kXPolls;
+  A.X.hold = wait_out != 0;
+  // everything this launch writes for the other blocks starts empty
+  QD_CUDA(cudaMemsetAsync(A.slots, kXEmptyByte, want * sizeof(double), ctx->stream));
+  if (xv)
+    QD_CUDA(cudaMemsetAsync(xv, kXEmptyByte, (size_t)(last + 2 - first) * ld * sizeof(XInt), ctx->stream));
+  else
+    QD_CUDA(cudaMemsetAsync(V + (int64_t)first * ld, kXEmptyByte, (size_t)(last + 1 - first) * ld * sizeof(VV), ctx->stream));
+  A.XV = xv;
+  return A;
+}
+
+template <typename MV, typename VV, bool kUni, bool kPaige>
+static bool lan_launch(qd_ham* H, const LanRun<MV, VV>& r) {
+  Ctx* ctx = H->ctx;
+  LanPlan& P = ham_workspace(H).lan_plan[sizeof(VV) == sizeof(double) ? (kPaige ? 1 : 0) : (kPaige ? 3 : 2)];
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[2];
+  auto kern = lan_kernel<MV, VV, 1, kUni, kPaige, false>;
+  if (!lan_plan<VV>(H, kern, lan_kernel<MV, VV, 4, kUni, kPaige, false>, lan_kernel<MV, VV, 8, kUni, kPaige, false>, P,
+                    cfg, at, kern))
+    return false;
+  constexpr int kPer = sizeof(VV) / sizeof(double);
+  const size_t nx = (size_t)(r.kdim + 1) * r.ld * sizeof(XInt);
+  if (kUni && r.xv->n < nx) r.xv->alloc(nx);
+  LanArgs<MV, VV> A =
+      lan_args(H, r.vals, P, r.V, r.ld, r.first, r.last, kPaige ? 2 : 1 + 3 * kPer, r.flags, r.slots, kUni ? reinterpret_cast<XInt*>(r.xv->p) : nullptr);
+  if (kUni) {
+    A.fxdiag = r.form->diag_zero ? nullptr : r.form->diag.p;
+    A.cF = std::ldexp(r.form->c, -r.form->F);
+    A.fxptr = r.form->colidx.p ? r.form->rowptr.p : nullptr;
+    A.fxcol = r.form->colidx.p;
+    A.F = r.form->F;
+    A.ovf = r.flags;
+  }
+  A.stop_below = r.stop_below;
+  A.alpha = r.alpha;
+  A.beta = r.beta;
+  A.nrm = r.nrm;
+  A.scl = r.scl;
+  A.stop = r.stop;
+  QD_CUDA(cudaLaunchKernelEx(&cfg, kern, A));
+  QD_LAUNCHED(ctx);
+  return true;
+}
+
+template <typename MV, typename VV>
+bool lan_res_run(qd_ham* H, const LanRun<MV, VV>& r) {
+  if constexpr (std::is_same<VV, double>::value)
+    if (r.form) return lan_launch<MV, VV, true, false>(H, r);
+  return r.rule == kLanPaige ? lan_launch<MV, VV, false, true>(H, r) : lan_launch<MV, VV, false, false>(H, r);
+}
+template bool lan_res_run<double, double>(qd_ham*, const LanRun<double, double>&);
+template bool lan_res_run<double, cplx>(qd_ham*, const LanRun<double, cplx>&);
+template bool lan_res_run<cplx, cplx>(qd_ham*, const LanRun<cplx, cplx>&);
+
+template <typename MV>
+bool lan_res_evolve(qd_ham* H, const MV* vals, cplx* psi, cplx* V, int64_t ld, int kdim, double h, int* act,
+                    long long* matvecs, int* flags, DBuf<double>* slots) {
+  Ctx* ctx = H->ctx;
+  LanPlan& P = ham_workspace(H).lan_plan[4];
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[2];
+  auto kern = lan_kernel<MV, cplx, 1, false, true, true>;
+  if (kdim > kLanMaxExp ||
+      !lan_plan<cplx>(H, kern, lan_kernel<MV, cplx, 4, false, true, true>, lan_kernel<MV, cplx, 8, false, true, true>, P,
+                      cfg, at, kern))
+    return false;
+  LanArgs<MV, cplx> A = lan_args<MV, cplx>(H, vals, P, V, ld, 1, kdim, 2, flags, slots, nullptr);
+  A.stop_below = 1e-10;
+  A.psi = psi;
+  A.h = h;
+  A.act = act;
+  A.matvecs = matvecs;
+  QD_CUDA(cudaLaunchKernelEx(&cfg, kern, A));
+  QD_LAUNCHED(ctx);
+  return true;
+}
+template bool lan_res_evolve<double>(qd_ham*, const double*, cplx*, cplx*, int64_t, int, double, int*, long long*, int*, DBuf<double>*);
+template bool lan_res_evolve<cplx>(qd_ham*, const cplx*, cplx*, cplx*, int64_t, int, double, int*, long long*, int*, DBuf<double>*);
+
+}  // namespace qd

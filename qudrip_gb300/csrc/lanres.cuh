@@ -1,0 +1,41 @@
+// lanres.cuh -- the Lanczos recurrence in one persistent launch (lanres.cu).
+#pragma once
+
+#include "krylov.cuh"
+
+namespace qd {
+
+enum LanForm { kLanLocal = 0, kLanPaige = 1 };
+
+// Steps first .. last of the recurrence on the basis V (V[first - 1] and, past the first step, V[first - 2]
+// complete; scl[first - 1] known):
+//   kLanLocal  the reference's local orthogonalisation against two vectors (sparse_algorithm.hpp:395-425)
+//   kLanPaige  alpha = <v1, H v1>, beta = ||V1|| (Hermitian::LanczosSolver; the Krylov exponential)
+// with the stopping rule norm < stop_below (*stop = the step).  `form`: the uniform-coupling form whose
+// fixed-point sums the product keeps (real vectors), or null for the FP64 product.
+template <typename MV, typename VV>
+struct LanRun {
+  const MV* vals;
+  LanForm rule;
+  const FxForm* form;
+  VV* V;
+  int64_t ld;
+  int kdim, first, last;
+  double stop_below;
+  VV *alpha, *beta;  // alpha[k], beta[k] of step k (beta may be null)
+  double *nrm, *scl;
+  int* stop;
+  int* flags;        // [0] a vector left the fixed-point range, [1] a wait ran out (both 0 before)
+  DBuf<double>* slots;
+  DBuf<char>* xv;  // `form`: the vectors' fixed-point copies
+};
+template <typename MV, typename VV>
+bool lan_res_run(qd_ham* H, const LanRun<MV, VV>& r);
+
+// One Krylov step psi <- V exp(-i h T) e_0 of dimension kdim (<= 32), psi in place.  act and the product
+// count are written on the device.  False: nothing launched.
+template <typename MV>
+bool lan_res_evolve(qd_ham* H, const MV* vals, cplx* psi, cplx* V, int64_t ld, int kdim, double h, int* act,
+                    long long* matvecs, int* flags, DBuf<double>* slots);
+
+}  // namespace qd

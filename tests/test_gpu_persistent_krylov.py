@@ -152,3 +152,117 @@ def test_a_wait_that_runs_out_is_reported_and_the_next_step_is_unchanged(ctx, mo
     sec2, H2 = objects("flux11")
     fresh, _ = evolve(sec2, H2, psi0, 12, 0.05, 1)
     assert np.array_equal(again[0], ref[0]) and np.array_equal(fresh[0], ref[0])
+
+
+def bond_chain(L, seed=3):
+    pre = q.getQbits(L)
+    gc, ga, gz = q.getBoseGate(pre), q.getBoseGate(pre), q.getBoseGate(pre)
+    gc << 0.5 * (q.pauli_x + q.II * q.pauli_y)
+    ga << 0.5 * (q.pauli_x - q.II * q.pauli_y)
+    gz << 0.5 * q.pauli_z
+    J = np.random.default_rng(seed).uniform(0.3, 0.7, L)
+    ham = q.getEmptyOperator()
+    for i in range(L):
+        j = (i + 1) % L
+        ham = ham + float(J[i]) * (gc(i) * ga(j)) + float(J[i]) * (gc(j) * ga(i)) + 0.9 * (gz(i) * gz(j))
+    return q.SectorSpec(pre, [q.getNset(pre) == L // 2]), ham
+
+
+LANCZOS = {
+    "uniform7_one_block": lambda: chains.xxz_chain(7, 1.0, 0.6, True, np.linspace(-1, 1, 7)),  # 35 rows
+    "uniform8": lambda: fields(8),             # 70 rows: one cluster, a ragged last block
+    "uniform13": lambda: chains.xy_chain(13),  # 1,716 rows
+    "uniform18": lambda: fields(18),           # 48,620 rows: every cluster, several rows a thread
+    "bonds9": lambda: bond_chain(9),
+    "bonds15": lambda: bond_chain(15),
+    "flux8": lambda: flux_chain(8),
+    "flux16": lambda: flux_chain(16),
+    "hubbard5_signs": lambda: chains.hubbard_chain(5, 2, 3, 4.0, -1.0, periodic=True),
+}
+
+
+def both_forms(monkeypatch, run):
+    out = [run()]
+    monkeypatch.setenv("QD_KRYLOV_STEP", "split")
+    monkeypatch.setenv("QD_LANCZOS_STEP", "split")
+    out.append(run())
+    monkeypatch.delenv("QD_KRYLOV_STEP")
+    monkeypatch.delenv("QD_LANCZOS_STEP")
+    return out
+
+
+@pytest.mark.parametrize("name,kdim,imag,mfree", [
+    ("uniform7_one_block", 12, False, False), ("uniform8", 20, False, True), ("uniform13", 30, False, False),
+    ("uniform18", 40, False, False), ("uniform13", 25, True, False), ("bonds9", 22, False, True),
+    ("bonds15", 40, False, False), ("flux8", 18, False, False), ("flux16", 40, True, True),
+    ("hubbard5_signs", 25, False, False), ("uniform8", 1, False, False)])
+def test_lanczos_matches_the_separate_launches(ctx, monkeypatch, name, kdim, imag, mfree):
+    """Krylov dimensions below the first spurious copy, where the recurrence is well-conditioned: the
+    eigenvalues differ by a few eps ||H|| per step at most (40 steps, ||H|| <= 30 eigenvalue units: 1e-12)."""
+    spec, ham = LANCZOS[name]()
+    sec = q.Sector(spec.index, spec.constraints)
+    v0 = q.start_vector(sec.dim, 8).astype(complex)
+    if imag:
+        v0 = v0 + 1j * q.start_vector(sec.dim, 9)
+
+    def run():
+        H = sec.lower(ham)
+        psi = q.getState(sec, 1)
+        psi.set(0, v0)
+        s = q.LanczosSolver(sec, kdim, spmv=A.QD_SPMV_MATRIX_FREE if mfree else A.QD_SPMV_CSR)
+        r = s.getGroundState(H, psi, 0)
+        return r.act_dim, s.eigenvalues(), psi.get(0)
+
+    a, b = both_forms(monkeypatch, run)
+    assert a[0] == b[0]
+    assert np.allclose(a[1], b[1], rtol=0, atol=1e-12 * np.abs(b[1]).max())
+    assert abs(abs(np.vdot(a[2], b[2])) - np.linalg.norm(a[2]) * np.linalg.norm(b[2])) <= 1e-10
+
+
+@pytest.mark.parametrize("name,m,h,steps", [("uniform7_one_block", 12, 0.2, 3), ("uniform8", 33, 0.3, 2),
+                                            ("flux8", 2, 0.05, 3), ("bonds15", 24, 0.2, 4), ("flux16", 32, 0.25, 3),
+                                            ("uniform18", 20, 0.1, 2), ("hubbard5_signs", 33, 2.5, 2)])
+def test_short_exponential_matches_the_separate_launches(ctx, monkeypatch, name, m, h, steps):
+    spec, ham = LANCZOS[name]()
+    sec = q.Sector(spec.index, spec.constraints)
+    H = sec.lower(ham)
+    rng = np.random.default_rng(m)
+    x = rng.normal(size=sec.dim) + 1j * rng.normal(size=sec.dim)
+    x /= np.linalg.norm(x)
+
+    def run():
+        st = q.getState(sec, 2)
+        st.set(0, x)
+        act = q.lanczos_evolve(H, st, 0, 1, h, m, steps)
+        return act, st.get(1), st.get(0)
+
+    a, b = both_forms(monkeypatch, run)
+    assert a[0] == b[0] and np.array_equal(a[2], x)
+    assert np.linalg.norm(a[1] - b[1]) <= (TOL if h < 1 else 1e-9)
+    if h * m < 10 and m > 12:
+        exact = sla.expm_multiply(-1j * h * steps * H.scipy().tocsc(), x)
+        assert np.linalg.norm(a[1] - exact) <= 1e-8
+
+
+@pytest.mark.parametrize("name,kdim,imag", [("uniform8", 20, False), ("bonds15", 35, False), ("flux16", 35, True),
+                                            ("hubbard5_signs", 25, True), ("uniform7_one_block", 10, False)])
+def test_hermitian_lanczos_with_its_basis_kept_matches_two_passes(ctx, monkeypatch, name, kdim, imag):
+    spec, ham = LANCZOS[name]()
+    sec = q.Sector(spec.index, spec.constraints)
+    H = sec.lower(ham)
+    v0 = q.start_vector(sec.dim, 8).astype(complex)
+    if imag:
+        v0 = v0 + 1j * q.start_vector(sec.dim, 9)
+
+    def run():
+        psi = q.getState(sec, 1)
+        psi.set(0, v0)
+        s = q.Hermitian.LanczosSolver(sec, kdim)
+        r = s.getGroundState(H, psi, 0)
+        return (r.act_dim, r.breakdown, r.matvecs), s.eigenvalues(), psi.get(0), r.err
+
+    a, b = both_forms(monkeypatch, run)
+    assert a[0] == b[0]
+    assert np.allclose(a[1], b[1], rtol=0, atol=1e-12 * np.abs(b[1]).max())
+    assert abs(abs(np.vdot(a[2], b[2])) - np.linalg.norm(a[2]) * np.linalg.norm(b[2])) <= 1e-10
+    assert abs(a[3] - b[3]) <= 1e-10
