@@ -304,7 +304,7 @@ __device__ bool arn_expm(const cplx* hs, int act, double h, bool band, cplx (*t)
   return true;
 }
 
-template <typename MV, typename VV, bool kExp, int C>
+template <typename MV, typename VV, bool kExp, bool kOne>
 __global__ void __launch_bounds__(kArnThreads, 1) arn_kernel(ArnArgs<MV, VV> A) {
   using QT = typename QVec<VV>::T;
   constexpr int T = kArnThreads;
@@ -410,7 +410,7 @@ __global__ void __launch_bounds__(kArnThreads, 1) arn_kernel(ArnArgs<MV, VV> A) 
       if (tid == 0) S.xv[J1 * kPer] = nshare;
     }
     __syncthreads();
-    x_sum<C>(X, slot1, S.xv, J1 * kPer + 1, S.red);
+    x_sum<kOne>(X, slot1, S.xv, J1 * kPer + 1, S.red);
     if (tid == 0 && !scaled) set_norm(J - 1, S.red[J1 * kPer]);
     __syncthreads();
     if (S.stop && J > 1 && !scaled) {  // sparse_algorithm.hpp:387: the breaking step counts
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(kArnThreads, 1) arn_kernel(ArnArgs<MV, VV> A) 
       __syncthreads();
       arn_dots_res<VV, T>(S, Vs, A.ldr, 0, J, wq, uw, R);
     }
-    x_sum<C>(X, slot2, S.xv, J * kPer, S.red);
+    x_sum<kOne>(X, slot2, S.xv, J * kPer, S.red);
     if (tid < J) {
       const VV c = reinterpret_cast<const VV*>(S.red)[tid];
       S.cf[tid] = vscale(S.scl[tid], c);
@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(kArnThreads, 1) arn_kernel(ArnArgs<MV, VV> A) 
   if (!stop) {  // the last vector's norm
     if (tid == 0) S.xv[0] = nshare;
     __syncthreads();
-    x_sum<C>(X, A.slots + (size_t)(2 * (A.last + 1 - A.first)) * A.xstride, S.xv, 1, S.red);
+    x_sum<kOne>(X, A.slots + (size_t)(2 * (A.last + 1 - A.first)) * A.xstride, S.xv, 1, S.red);
     if (tid == 0) set_norm(A.last, S.red[0]);
     __syncthreads();
     if (S.stop) stop = A.last;
@@ -573,7 +573,7 @@ static bool arn_launch(qd_ham* H, const MV* vals, ArnRes& B, const cplx* psi_in,
   // one block up to 64 rows (an exchange would cost more than it saves), then clusters of eight blocks
   // of at least kArnMinRows rows, as many as fit the device at once
   const bool one = n <= 64;
-  auto kern = one ? arn_kernel<MV, VV, kExp, 1> : arn_kernel<MV, VV, kExp, kArnCluster>;
+  auto kern = one ? arn_kernel<MV, VV, kExp, true> : arn_kernel<MV, VV, kExp, false>;
   int ncl = one ? 1 : (int)std::min<int64_t>(ctx->num_sms / kArnCluster, ceil_div(n, kArnCluster * kArnMinRows));
   int rows = 0;
   cudaLaunchConfig_t cfg = {};
@@ -609,8 +609,8 @@ static bool arn_launch(qd_ham* H, const MV* vals, ArnRes& B, const cplx* psi_in,
       ncl = fit;
     }
   }
-  const size_t smem = smem_of(rows), xstride = (size_t)ncl * (kPer * kdim + 1);
   const int grid = one ? 1 : ncl * kArnCluster;
+  const size_t smem = smem_of(rows), xstride = (size_t)grid * (kPer * kdim + 1);
   cfg.gridDim = dim3((unsigned)grid);
   cfg.dynamicSmemBytes = smem;
   arn_ensure(B, n, kdim, kPer == 1, (2 * (size_t)kdim + 1) * xstride);

@@ -117,48 +117,57 @@ __device__ __forceinline__ bool x_await(const GridX& X, const VV* p, VV& v) {
 }
 
 // out[q] = the sum over the grid of every block's v[q], q < nv <= kXMaxVals, the same bits in every
-// block (fixed trees over the cluster's ranks and over the clusters).  C: the cluster size, a power of
-// two; C = 1 is a grid of one block.  v and out in shared memory, not overlapping; slots: gridDim.x / C * nv
-// of them.  v must be complete for all threads, as by a block barrier, before the call; out is complete
-// for all threads on return, and v may then be written again.
+// block (fixed trees over the cluster's ranks and over the clusters).  kOne: a grid of one block.  v and out
+// in shared memory, not overlapping; slots: gridDim.x * nv of them.  v must be complete for all threads, as
+// by a block barrier, before the call; out is complete for all threads on return, and v may then be
+// written again.  The cluster's size is read, not assumed: a profiler launches a cooperative grid
+// without its clusters, and the memory of a rank that does not exist must not be read.
 constexpr int kXMaxVals = 256;
-template <int C>
+template <int CT>  // the cluster's size, 0: any power of two
+__device__ __forceinline__ void x_sum_cluster(const GridX& X, double* slots, double* v, int nv, double* out, int size) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  const int C = CT ? CT : size, tid = threadIdx.x;
+  const int rank = (int)cl.block_rank(), ncl = (int)gridDim.x / C, me = (int)blockIdx.x / C;
+  const int per = (nv + C - 1) / C;  // values per block
+  cl.sync();
+  // a value takes C lanes, or a warp where there are many clusters to collect from
+  const int L = ncl > 2 * C ? 32 : C;
+  const int l = tid & (L - 1);
+  for (int g = tid / L; (g & ~(32 / L - 1)) < per; g += blockDim.x / L) {  // whole warps
+    const int q = rank * per + g;
+    const bool on = g < per && q < nv;
+    double a = (on && l < C) ? *cl.map_shared_rank(v + q, l) : 0.0;
+#pragma unroll
+    for (int o = C / 2; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (ncl > 1) {
+      if (on && l == 0 && !(X.hold && me == 0)) x_st(slots + (size_t)me * nv + q, x_clean(a));
+      double t = 0.0;
+      if (on)
+        for (int c = l; c < ncl; c += L) {
+          double b = x_ld(slots + (size_t)c * nv + q);
+          x_wait(X, slots + (size_t)c * nv + q, b);
+          t += b;
+        }
+      for (int o = L / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      a = t;
+    }
+    if (on && l < C) *cl.map_shared_rank(out + q, l) = a;
+  }
+  cl.sync();
+}
+
+template <bool kOne>
 __device__ __forceinline__ void x_sum(const GridX& X, double* slots, double* v, int nv, double* out) {
-  const int tid = threadIdx.x;
-  if constexpr (C == 1) {
+  if constexpr (kOne) {
     __syncthreads();
-    if (tid < nv) out[tid] = v[tid];
+    if (threadIdx.x < nv) out[threadIdx.x] = v[threadIdx.x];
     __syncthreads();
   } else {
-    namespace cg = cooperative_groups;
-    cg::cluster_group cl = cg::this_cluster();
-    const int rank = (int)cl.block_rank(), ncl = (int)gridDim.x / C, me = (int)blockIdx.x / C;
-    const int per = (nv + C - 1) / C;  // values per block
-    cl.sync();
-    // a value takes C lanes, or a warp where there are many clusters to collect from
-    const int L = ncl > 2 * C ? 32 : C;
-    const int l = tid & (L - 1);
-    for (int g = tid / L; (g & ~(32 / L - 1)) < per; g += blockDim.x / L) {  // whole warps
-      const int q = rank * per + g;
-      const bool on = g < per && q < nv;
-      double a = (on && l < C) ? *cl.map_shared_rank(v + q, l) : 0.0;
-#pragma unroll
-      for (int o = C / 2; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-      if (ncl > 1) {
-        if (on && l == 0 && !(X.hold && me == 0)) x_st(slots + (size_t)me * nv + q, x_clean(a));
-        double t = 0.0;
-        if (on)
-          for (int c = l; c < ncl; c += L) {
-            double b = x_ld(slots + (size_t)c * nv + q);
-            x_wait(X, slots + (size_t)c * nv + q, b);
-            t += b;
-          }
-        for (int o = L / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        a = t;
-      }
-      if (on && l < C) *cl.map_shared_rank(out + q, l) = a;
-    }
-    cl.sync();
+    const int size = (int)cooperative_groups::this_cluster().num_blocks();
+    if (size == 8) x_sum_cluster<8>(X, slots, v, nv, out, size);
+    else if (size == 4) x_sum_cluster<4>(X, slots, v, nv, out, size);
+    else x_sum_cluster<0>(X, slots, v, nv, out, size);
   }
 }
 

@@ -259,7 +259,7 @@ __device__ __forceinline__ void lan_texp(int act, double h, double d, double e, 
   }
 }
 
-template <typename MV, typename VV, int C, bool kUni, bool kPaige, bool kExp>
+template <typename MV, typename VV, bool kOne, bool kUni, bool kPaige, bool kExp>
 __global__ void __launch_bounds__(kLanThreads, 1) lan_kernel(LanArgs<MV, VV> A) {
   constexpr int T = kLanThreads, kPer = sizeof(VV) / sizeof(double);
   constexpr int NV = kPaige ? 2 : 1 + 3 * kPer;
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(kLanThreads, 1) lan_kernel(LanArgs<MV, VV> A) 
     }
     lan_block_sums<NV, T>(S, vals, nact);
     __syncthreads();
-    x_sum<C>(X, A.slots + (size_t)(k - A.first) * A.xstride, S.v, NV, S.red);
+    x_sum<kOne>(X, A.slots + (size_t)(k - A.first) * A.xstride, S.v, NV, S.red);
     // the scale of V1 from its norm, alpha and beta, and the update's coefficients: one chain of scalar
     // FP64 operations (64 cycles each), what the update does not wait for on a second warp
     if (tid == 0) {
@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(kLanThreads, 1) lan_kernel(LanArgs<MV, VV> A) 
     if (!stop) {  // the last vector's norm
       lan_block_sums<NV, T>(S, vals, nact);
       __syncthreads();
-      x_sum<C>(X, A.slots + (size_t)(A.last + 1 - A.first) * A.xstride, S.v, NV, S.red);
+      x_sum<kOne>(X, A.slots + (size_t)(A.last + 1 - A.first) * A.xstride, S.v, NV, S.red);
       if (tid == 0) {
         const double n2 = S.red[NV - 1], nr = n2 > 0.0 ? n2 * rsqrt(n2) : n2;
         S.stop = nr < A.stop_below;
@@ -533,15 +533,15 @@ __global__ void lan_rows_kernel(int64_t n, const int64_t* rowptr, int grid, int*
   }
 }
 
-// The kernel of each cluster size; cfg for the one the sector takes.  False when the device does not hold
+// The kernel for one block or many; cfg for the grid the sector takes.  False when the device does not hold
 // the grid at once, or a block its rows.
 template <typename VV, typename K>
-static bool lan_plan(qd_ham* H, K kern1, K kern4, K kern8, LanPlan& P, cudaLaunchConfig_t& cfg,
+static bool lan_plan(qd_ham* H, K kern1, K kern_many, LanPlan& P, cudaLaunchConfig_t& cfg,
                      cudaLaunchAttribute (&at)[2], K& kern) {
   Ctx* ctx = H->ctx;
   const int64_t n = H->dim;
   const int csize = n <= 64 ? 1 : (n <= kLanWideRows ? 8 : 4);  // one block: an exchange would cost more than it saves
-  kern = csize == 1 ? kern1 : (csize == 4 ? kern4 : kern8);
+  kern = csize == 1 ? kern1 : kern_many;
   at[0].id = cudaLaunchAttributeCooperative;
   at[0].val.cooperative = 1;
   at[1].id = cudaLaunchAttributeClusterDimension;
@@ -612,7 +612,7 @@ static LanArgs<MV, VV> lan_args(qd_ham* H, const MV* vals, const LanPlan& P, VV*
   A.V = V;
   A.first = first;
   A.last = last;
-  A.xstride = P.ncl * nv;
+  A.xstride = P.ncl * P.csize * nv;
   const size_t want = (size_t)(last + 2 - first) * A.xstride;
   if (slots->n < want) slots->alloc(want);
   A.slots = slots->p;
@@ -636,10 +636,8 @@ static bool lan_launch(qd_ham* H, const LanRun<MV, VV>& r) {
   LanPlan& P = ham_workspace(H).lan_plan[sizeof(VV) == sizeof(double) ? (kPaige ? 1 : 0) : (kPaige ? 3 : 2)];
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[2];
-  auto kern = lan_kernel<MV, VV, 1, kUni, kPaige, false>;
-  if (!lan_plan<VV>(H, kern, lan_kernel<MV, VV, 4, kUni, kPaige, false>, lan_kernel<MV, VV, 8, kUni, kPaige, false>, P,
-                    cfg, at, kern))
-    return false;
+  auto kern = lan_kernel<MV, VV, true, kUni, kPaige, false>;
+  if (!lan_plan<VV>(H, kern, lan_kernel<MV, VV, false, kUni, kPaige, false>, P, cfg, at, kern)) return false;
   constexpr int kPer = sizeof(VV) / sizeof(double);
   const size_t nx = (size_t)(r.kdim + 1) * r.ld * sizeof(XInt);
   if (kUni && r.xv->n < nx) r.xv->alloc(nx);
@@ -681,10 +679,9 @@ bool lan_res_evolve(qd_ham* H, const MV* vals, cplx* psi, cplx* V, int64_t ld, i
   LanPlan& P = ham_workspace(H).lan_plan[4];
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[2];
-  auto kern = lan_kernel<MV, cplx, 1, false, true, true>;
+  auto kern = lan_kernel<MV, cplx, true, false, true, true>;
   if (kdim > kLanMaxExp ||
-      !lan_plan<cplx>(H, kern, lan_kernel<MV, cplx, 4, false, true, true>, lan_kernel<MV, cplx, 8, false, true, true>, P,
-                      cfg, at, kern))
+      !lan_plan<cplx>(H, kern, lan_kernel<MV, cplx, false, false, true, true>, P, cfg, at, kern))
     return false;
   LanArgs<MV, cplx> A = lan_args<MV, cplx>(H, vals, P, V, ld, 1, kdim, 2, flags, slots, nullptr);
   A.stop_below = 1e-10;
