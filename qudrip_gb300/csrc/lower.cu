@@ -214,24 +214,35 @@ void ham_transpose(Ctx* ctx, int64_t n, const int64_t* ptr, const int32_t* idx, 
 __global__ void analyze_kernel(int64_t n, const int64_t* rowptr, const int32_t* colidx, const cplx* vals,
                                int* flags) {
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n) return;
-  const int64_t b = rowptr[r], e = rowptr[r + 1];
-  atomicMax(flags + 2, (int)(e - b));
-  for (int64_t k = b; k < e; ++k) {
-    const cplx v = vals[k];
-    if (v.im != 0.0) atomicOr(flags + 0, 1);
-    const int32_t c = colidx[k];
-    int64_t lo = rowptr[c], hi = rowptr[c + 1];
-    while (lo < hi) {
-      const int64_t mid = (lo + hi) >> 1;
-      if (colidx[mid] < (int32_t)r) lo = mid + 1;
-      else hi = mid;
+  // one update of each flag per warp, not per row
+  int len = 0, imag = 0, herm = 0;
+  if (r < n) {
+    const int64_t b = rowptr[r], e = rowptr[r + 1];
+    len = (int)(e - b);
+    for (int64_t k = b; k < e; ++k) {
+      const cplx v = vals[k];
+      imag |= v.im != 0.0;
+      const int32_t c = colidx[k];
+      int64_t lo = rowptr[c], hi = rowptr[c + 1];
+      while (lo < hi) {
+        const int64_t mid = (lo + hi) >> 1;
+        if (colidx[mid] < (int32_t)r) lo = mid + 1;
+        else hi = mid;
+      }
+      cplx w = mkc(0.0, 0.0);
+      if (lo < rowptr[c + 1] && colidx[lo] == (int32_t)r) w = vals[lo];
+      const double dr = v.re - w.re, di = v.im + w.im;
+      const double scale = fabs(v.re) + fabs(v.im) + fabs(w.re) + fabs(w.im);
+      herm |= fabs(dr) + fabs(di) > 1e-13 * scale;
     }
-    cplx w = mkc(0.0, 0.0);
-    if (lo < rowptr[c + 1] && colidx[lo] == (int32_t)r) w = vals[lo];
-    const double dr = v.re - w.re, di = v.im + w.im;
-    const double scale = fabs(v.re) + fabs(v.im) + fabs(w.re) + fabs(w.im);
-    if (fabs(dr) + fabs(di) > 1e-13 * scale) atomicOr(flags + 1, 1);
+  }
+  len = __reduce_max_sync(0xffffffffu, len);
+  imag = __any_sync(0xffffffffu, imag);
+  herm = __any_sync(0xffffffffu, herm);
+  if ((threadIdx.x & 31) == 0) {
+    if (len > *reinterpret_cast<volatile int*>(flags + 2)) atomicMax(flags + 2, len);
+    if (imag) atomicOr(flags + 0, 1);
+    if (herm) atomicOr(flags + 1, 1);
   }
 }
 
@@ -403,8 +414,8 @@ void ham_finish(qd_ham* H) {
   if (H->flags & QD_HAM_REAL) {
     H->vals_r.alloc(nnz + 16);
     H->vals_f.alloc(nnz + 16);
-    QD_CUDA(cudaMemsetAsync(H->vals_r.p, 0, (nnz + 16) * sizeof(double), ctx->stream));
-    QD_CUDA(cudaMemsetAsync(H->vals_f.p, 0, (nnz + 16) * sizeof(float), ctx->stream));
+    QD_CUDA(cudaMemsetAsync(H->vals_r.p + nnz, 0, 16 * sizeof(double), ctx->stream));  // the padding
+    QD_CUDA(cudaMemsetAsync(H->vals_f.p + nnz, 0, 16 * sizeof(float), ctx->stream));
     if (nnz > 0) {
       real_part_kernel<<<(unsigned)ceil_div(nnz, 256), 256, 0, ctx->stream>>>(nnz, H->vals_c.p, H->vals_r.p,
                                                                              H->vals_f.p);
@@ -416,11 +427,14 @@ void ham_finish(qd_ham* H) {
 }
 
 __global__ void row_abs_max_kernel(int64_t n, const int64_t* rowptr, const cplx* vals, unsigned long long* out) {
+  unsigned long long m = 0;  // magnitudes in order as integers, a NaN above all
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
     double s = 0.0;
     for (int64_t k = rowptr[r]; k < rowptr[r + 1]; ++k) s += hypot(vals[k].re, vals[k].im);
-    atomicMax(out, (unsigned long long)__double_as_longlong(s));
+    m = max(m, (unsigned long long)__double_as_longlong(s));
   }
+  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
 
 // max_r sum_c |H(r, c)| (cached): bounds the spectral radius.
