@@ -971,7 +971,10 @@ void batch_lanczos(Ctx* ctx, qd_ham* const* hams, const double* const* v0s, int 
     ~Side() {
       if (in) cudaEventDestroy(in);
       if (done) cudaEventDestroy(done);
-      if (s) cudaStreamDestroy(s);
+      if (s) {
+        cudaStreamSynchronize(s);  // after an error its kernel may still run, and the buffers are given back next
+        cudaStreamDestroy(s);
+      }
     }
   } side;
   cudaStream_t large_stream = ctx->stream;

@@ -94,6 +94,7 @@ qd_status qd_ctx_destroy(qd_ctx* ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
+    ctx->cache->drain(true);
     for (auto& ev : ctx->events)
       if (ev) cudaEventDestroy(ev);
     cudaStreamDestroy(ctx->stream);
@@ -167,7 +168,7 @@ qd_status qd_sector_create(qd_ctx* ctx, int nbits, const qd_constraint* cons, in
                    "constraint %d: Nd needs 1 <= nsite <= 32", i);
       }
     }
-    DeviceGuard dg(ctx->device);
+    CacheGuard dg(ctx);
     auto* S = new qd_sector();
     S->ctx = ctx;
     S->nbits = nbits;
@@ -186,7 +187,7 @@ qd_status qd_sector_create(qd_ctx* ctx, int nbits, const qd_constraint* cons, in
 qd_status qd_sector_destroy(qd_sector* sec) {
   return guard([&] {
     if (!sec) return;
-    DeviceGuard dg(sec->ctx->device);
+    CacheGuard dg(sec->ctx);
     cudaStreamSynchronize(sec->ctx->stream);
     delete sec;
   });
@@ -209,7 +210,7 @@ qd_status qd_sector_rank_kind(const qd_sector* sec, int* kind) {
 qd_status qd_sector_basis(qd_sector* sec, uint64_t* host_states) {
   return guard([&] {
     QD_REQUIRE(sec && (host_states || sec->view.dim == 0), QD_ERR_INVALID, "null argument");
-    DeviceGuard dg(sec->ctx->device);
+    CacheGuard dg(sec->ctx);
     if (sec->view.dim == 0) return;
     QD_CUDA(cudaMemcpyAsync(host_states, sec->basis.p, sec->view.dim * 8, cudaMemcpyDeviceToHost,
                             sec->ctx->stream));
@@ -221,7 +222,7 @@ qd_status qd_sector_rank(qd_sector* sec, const uint64_t* host_states, int64_t n,
   return guard([&] {
     QD_REQUIRE(sec && n >= 0 && (n == 0 || (host_states && host_ranks)), QD_ERR_INVALID, "bad argument");
     if (n == 0) return;
-    DeviceGuard dg(sec->ctx->device);
+    CacheGuard dg(sec->ctx);
     DBuf<uint64_t> s(n);
     DBuf<int64_t> r(n);
     QD_CUDA(cudaMemcpyAsync(s.p, host_states, n * 8, cudaMemcpyHostToDevice, sec->ctx->stream));
@@ -238,7 +239,7 @@ qd_status qd_ham_lower(qd_sector* sec, const qd_term* terms, int nterms, const q
     QD_REQUIRE(sec && out, QD_ERR_INVALID, "qd_ham_lower: null argument");
     QD_REQUIRE(nterms >= 0 && (nterms == 0 || terms), QD_ERR_INVALID, "bad term array");
     QD_REQUIRE(ngates >= 0 && (ngates == 0 || gates), QD_ERR_INVALID, "bad gate array");
-    DeviceGuard dg(sec->ctx->device);
+    CacheGuard dg(sec->ctx);
     auto* H = new qd_ham();
     H->ctx = sec->ctx;
     H->sec = sec;
@@ -256,7 +257,7 @@ qd_status qd_ham_add(const qd_ham* a, const qd_ham* b, qd_ham** out) {
   return guard([&] {
     QD_REQUIRE(a && b && out, QD_ERR_INVALID, "qd_ham_add: null argument");
     QD_REQUIRE(a->sec == b->sec, QD_ERR_INVALID, "qd_ham_add: the operands live on different sectors");
-    DeviceGuard dg(a->ctx->device);
+    CacheGuard dg(a->ctx);
     auto* H = new qd_ham();
     H->ctx = a->ctx;
     H->sec = a->sec;
@@ -273,7 +274,7 @@ qd_status qd_ham_add(const qd_ham* a, const qd_ham* b, qd_ham** out) {
 qd_status qd_ham_copy(const qd_ham* a, qd_ham** out) {
   return guard([&] {
     QD_REQUIRE(a && out, QD_ERR_INVALID, "qd_ham_copy: null argument");
-    DeviceGuard dg(a->ctx->device);
+    CacheGuard dg(a->ctx);
     auto* H = new qd_ham();
     H->ctx = a->ctx;
     H->sec = a->sec;
@@ -290,7 +291,7 @@ qd_status qd_ham_copy(const qd_ham* a, qd_ham** out) {
 qd_status qd_ham_scale(qd_ham* ham, double re, double im) {
   return guard([&] {
     QD_REQUIRE(ham, QD_ERR_INVALID, "qd_ham_scale: null argument");
-    DeviceGuard dg(ham->ctx->device);
+    CacheGuard dg(ham->ctx);
     ham_scale(ham, mkc(re, im));
   });
 }
@@ -298,7 +299,7 @@ qd_status qd_ham_scale(qd_ham* ham, double re, double im) {
 qd_status qd_ham_destroy(qd_ham* ham) {
   return guard([&] {
     if (!ham) return;
-    DeviceGuard dg(ham->ctx->device);
+    CacheGuard dg(ham->ctx);
     cudaStreamSynchronize(ham->ctx->stream);
     delete ham;
   });
@@ -307,6 +308,7 @@ qd_status qd_ham_destroy(qd_ham* ham) {
 qd_status qd_ham_get_info(qd_ham* ham, qd_ham_info* info) {
   return guard([&] {
     QD_REQUIRE(ham && info, QD_ERR_INVALID, "null argument");
+    CacheGuard dg(ham->ctx);
     std::memset(info, 0, sizeof(*info));
     info->dim = ham->dim;
     info->nnz = ham->nnz;
@@ -325,7 +327,7 @@ qd_status qd_ham_get_info(qd_ham* ham, qd_ham_info* info) {
 qd_status qd_ham_build_matrix_free(qd_ham* ham) {
   return guard([&] {
     QD_REQUIRE(ham, QD_ERR_INVALID, "null argument");
-    DeviceGuard dg(ham->ctx->device);
+    CacheGuard dg(ham->ctx);
     ham_build_matrix_free(ham);
   });
 }
@@ -336,7 +338,7 @@ qd_status qd_ham_apply_matrix_free(qd_ham* ham, qd_state* x, int t_in, qd_state*
     QD_REQUIRE(x->dim == ham->dim && y->dim == ham->dim, QD_ERR_INVALID, "dimension mismatch");
     QD_REQUIRE(t_in >= 0 && t_in < x->nt && t_out >= 0 && t_out < y->nt, QD_ERR_INVALID, "bad column");
     QD_REQUIRE(x->col(t_in) != y->col(t_out), QD_ERR_INVALID, "in-place product");
-    DeviceGuard dg(ham->ctx->device);
+    CacheGuard dg(ham->ctx);
     mf_apply_c(ham, x->col(t_in), y->col(t_out));
     QD_CUDA(cudaStreamSynchronize(ham->ctx->stream));
   });
@@ -345,7 +347,7 @@ qd_status qd_ham_apply_matrix_free(qd_ham* ham, qd_state* x, int t_in, qd_state*
 qd_status qd_ham_download_csr(qd_ham* ham, int64_t* rowptr, int32_t* colidx, double* vals) {
   return guard([&] {
     QD_REQUIRE(ham && rowptr, QD_ERR_INVALID, "null argument");
-    DeviceGuard dg(ham->ctx->device);
+    CacheGuard dg(ham->ctx);
     cudaStream_t s = ham->ctx->stream;
     QD_CUDA(cudaMemcpyAsync(rowptr, ham->rowptr.p, (ham->dim + 1) * 8, cudaMemcpyDeviceToHost, s));
     if (ham->nnz > 0) {
@@ -360,7 +362,7 @@ qd_status qd_ham_download_csr(qd_ham* ham, int64_t* rowptr, int32_t* colidx, dou
 qd_status qd_ham_download_csc(qd_ham* ham, int64_t* colptr, int32_t* rowidx, double* vals) {
   return guard([&] {
     QD_REQUIRE(ham && colptr, QD_ERR_INVALID, "null argument");
-    DeviceGuard dg(ham->ctx->device);
+    CacheGuard dg(ham->ctx);
     cudaStream_t s = ham->ctx->stream;
     DBuf<int64_t> cp(ham->dim + 1);
     DBuf<int32_t> ri(ham->nnz + 1);
@@ -388,7 +390,12 @@ qd_status qd_state_create(qd_ctx* ctx, int64_t dim, int nt, qd_state** out) {
     st->nt = nt;
     st->ld = (dim + 31) / 32 * 32;
     try {
-      st->data.alloc((size_t)st->ld * nt);
+      try {
+        st->data.alloc((size_t)st->ld * nt);
+      } catch (const Error&) {
+        ctx->cache->drain();  // what is kept may be what is missing
+        st->data.alloc((size_t)st->ld * nt);
+      }
       QD_CUDA(cudaMemsetAsync(st->data.p, 0, st->data.bytes(), ctx->stream));  // Matrix::Zero (state.hpp:29)
       QD_CUDA(cudaStreamSynchronize(ctx->stream));
     } catch (...) {
@@ -402,7 +409,7 @@ qd_status qd_state_create(qd_ctx* ctx, int64_t dim, int nt, qd_state** out) {
 qd_status qd_state_destroy(qd_state* st) {
   return guard([&] {
     if (!st) return;
-    DeviceGuard dg(st->ctx->device);
+    CacheGuard dg(st->ctx);
     cudaStreamSynchronize(st->ctx->stream);
     delete st;
   });
@@ -411,7 +418,7 @@ qd_status qd_state_destroy(qd_state* st) {
 qd_status qd_state_upload(qd_state* st, int t, const double* host_complex) {
   return guard([&] {
     QD_REQUIRE(st && host_complex && t >= 0 && t < st->nt, QD_ERR_INVALID, "bad argument");
-    DeviceGuard dg(st->ctx->device);
+    CacheGuard dg(st->ctx);
     QD_CUDA(cudaMemcpyAsync(st->col(t), host_complex, st->dim * sizeof(cplx), cudaMemcpyHostToDevice,
                             st->ctx->stream));
     QD_CUDA(cudaStreamSynchronize(st->ctx->stream));
@@ -421,7 +428,7 @@ qd_status qd_state_upload(qd_state* st, int t, const double* host_complex) {
 qd_status qd_state_download(qd_state* st, int t, double* host_complex) {
   return guard([&] {
     QD_REQUIRE(st && host_complex && t >= 0 && t < st->nt, QD_ERR_INVALID, "bad argument");
-    DeviceGuard dg(st->ctx->device);
+    CacheGuard dg(st->ctx);
     QD_CUDA(cudaMemcpyAsync(host_complex, st->col(t), st->dim * sizeof(cplx), cudaMemcpyDeviceToHost,
                             st->ctx->stream));
     QD_CUDA(cudaStreamSynchronize(st->ctx->stream));
@@ -433,7 +440,7 @@ qd_status qd_state_copy(qd_state* src, int t_src, qd_state* dst, int t_dst) {
     QD_REQUIRE(src && dst && src->dim == dst->dim, QD_ERR_INVALID, "bad argument");
     QD_REQUIRE(t_src >= 0 && t_src < src->nt && t_dst >= 0 && t_dst < dst->nt, QD_ERR_INVALID, "bad column");
     QD_REQUIRE(src->ctx == dst->ctx, QD_ERR_INVALID, "states of different contexts");
-    DeviceGuard dg(src->ctx->device);
+    CacheGuard dg(src->ctx);
     QD_CUDA(cudaMemcpyAsync(dst->col(t_dst), src->col(t_src), src->dim * sizeof(cplx), cudaMemcpyDeviceToDevice,
                             src->ctx->stream));
   });
@@ -452,7 +459,7 @@ qd_status qd_ham_apply(qd_ham* ham, qd_state* x, int t_in, qd_state* y, int t_ou
     QD_REQUIRE(x->dim == ham->dim && y->dim == ham->dim, QD_ERR_INVALID, "dimension mismatch");
     QD_REQUIRE(t_in >= 0 && t_in < x->nt && t_out >= 0 && t_out < y->nt, QD_ERR_INVALID, "bad column");
     QD_REQUIRE(!(x == y && t_in == t_out), QD_ERR_INVALID, "qd_ham_apply cannot work in place");
-    DeviceGuard dg(ham->ctx->device);
+    CacheGuard dg(ham->ctx);
     ham_apply_c(ham, x->col(t_in), y->col(t_out));
     QD_CUDA(cudaStreamSynchronize(ham->ctx->stream));
   });
@@ -464,7 +471,7 @@ qd_status qd_state_eval(qd_state* psi, int t, qd_ham* ham, double* re_im) {
     // the reference only prints on a dimension mismatch (state.hpp:35-39); here it is an error
     QD_REQUIRE(psi->dim == ham->dim, QD_ERR_INVALID, "State::eval: dimension mismatch (%lld vs %lld)",
                (long long)psi->dim, (long long)ham->dim);
-    DeviceGuard dg(ham->ctx->device);
+    CacheGuard dg(ham->ctx);
     const cplx e = state_eval(ham, psi->col(t));
     re_im[0] = e.re;
     re_im[1] = e.im;
@@ -477,7 +484,7 @@ qd_status qd_obs_eval(qd_state* psi, int t, int nobs, qd_ham* const* obs, double
     for (int i = 0; i < nobs; ++i)
       QD_REQUIRE(obs[i] && obs[i]->dim == psi->dim && obs[i]->ctx == psi->ctx, QD_ERR_INVALID,
                  "observable %d: null, other dimension or other context", i);
-    DeviceGuard dg(psi->ctx->device);
+    CacheGuard dg(psi->ctx);
     obs_eval_many(obs, nobs, psi->col(t), reinterpret_cast<cplx*>(re_im));
   });
 }
@@ -492,7 +499,7 @@ qd_status qd_lanczos_ground(qd_ham* ham, qd_state* psi, int t, const qd_lanczos_
     QD_REQUIRE(opts->spmv == QD_SPMV_CSR || opts->spmv == QD_SPMV_MATRIX_FREE, QD_ERR_INVALID, "bad spmv kind");
     QD_REQUIRE(opts->ritz == QD_RITZ_STORED_BASIS || opts->ritz == QD_RITZ_SECOND_PASS, QD_ERR_INVALID,
                "bad ritz mode");
-    DeviceGuard dg(ham->ctx->device);
+    CacheGuard dg(ham->ctx);
     std::memset(res, 0, sizeof(*res));
     lanczos_ground(ham, psi->col(t), *opts, evals_out, res);
   });
@@ -507,7 +514,7 @@ qd_status qd_ham_time_spmv(qd_ham* ham, int spmv, int iters, double* avg_ms, dou
     const bool fused = spmv >= 2000 + kSpmvTile && spmv <= 2000 + kSpmvLast;
     const bool vec = spmv == 3001 || spmv == 3002;
     QD_REQUIRE(plain || fused || vec, QD_ERR_UNSUPPORTED, "qd_ham_time_spmv: unknown kernel code %d", spmv);
-    DeviceGuard dg(ham->ctx->device);
+    CacheGuard dg(ham->ctx);
     if (spmv % 1000 == kSpmvRowSorted) ham_ensure_row_order(ham);
     time_spmv(ham, spmv, iters, avg_ms, bytes_per_launch);
   });
@@ -518,7 +525,7 @@ qd_status qd_arnoldi_evolve(qd_ham* ham, qd_state* psi, int t_in, int t_out, dou
     QD_REQUIRE(ham && psi, QD_ERR_INVALID, "null argument");
     QD_REQUIRE(psi->dim == ham->dim, QD_ERR_INVALID, "dimension mismatch");
     QD_REQUIRE(t_in >= 0 && t_in < psi->nt && t_out >= 0 && t_out < psi->nt, QD_ERR_INVALID, "bad column");
-    DeviceGuard dg(ham->ctx->device);
+    CacheGuard dg(ham->ctx);
     arnoldi_evolve(ham, psi->col(t_in), psi->col(t_out), h, m, act_dim);
   });
 }
@@ -529,7 +536,7 @@ qd_status qd_lanczos_extend(qd_ham* ham, qd_state* psi, int t, const qd_lanczos_
     QD_REQUIRE(ham && psi && opts && res, QD_ERR_INVALID, "null argument");
     QD_REQUIRE(t >= 0 && t < psi->nt, QD_ERR_INVALID, "bad column");
     QD_REQUIRE(psi->dim == ham->dim, QD_ERR_INVALID, "dimension mismatch");
-    DeviceGuard dg(ham->ctx->device);
+    CacheGuard dg(ham->ctx);
     std::memset(res, 0, sizeof(*res));
     lanczos_extend(ham, psi->col(t), *opts, evals_out, res);
   });
@@ -540,7 +547,7 @@ static void arnoldi_ground_call(qd_ham* ham, qd_state* psi, int t, const qd_lanc
   QD_REQUIRE(ham && psi && opts && res, QD_ERR_INVALID, "null argument");
   QD_REQUIRE(t >= 0 && t < psi->nt, QD_ERR_INVALID, "bad column");
   QD_REQUIRE(psi->dim == ham->dim, QD_ERR_INVALID, "dimension mismatch");
-  DeviceGuard dg(ham->ctx->device);
+  CacheGuard dg(ham->ctx);
   const double prev = (extend && ham->arnoldi_gs) ? ham->arnoldi_gs_ritz : 0.0;
   std::memset(res, 0, sizeof(*res));
   arnoldi_ground(ham, psi->col(t), opts->krylov_dim, opts->add_dim, extend, evals_out, res);
@@ -564,7 +571,7 @@ qd_status qd_hermitian_lanczos_ground(qd_ham* ham, qd_state* psi, int t, int kry
     QD_REQUIRE(ham && psi && res, QD_ERR_INVALID, "null argument");
     QD_REQUIRE(t >= 0 && t < psi->nt, QD_ERR_INVALID, "bad column");
     QD_REQUIRE(psi->dim == ham->dim, QD_ERR_INVALID, "dimension mismatch");
-    DeviceGuard dg(ham->ctx->device);
+    CacheGuard dg(ham->ctx);
     std::memset(res, 0, sizeof(*res));
     hermitian_lanczos_ground(ham, psi->col(t), kry_dim, evals_out, res);
   });
@@ -577,7 +584,7 @@ qd_status qd_lanczos_evolve(qd_ham* ham, qd_state* psi, int t_in, int t_out, dou
     QD_REQUIRE(psi->dim == ham->dim, QD_ERR_INVALID, "dimension mismatch");
     QD_REQUIRE(t_in >= 0 && t_in < psi->nt && t_out >= 0 && t_out < psi->nt, QD_ERR_INVALID, "bad column");
     QD_REQUIRE(m >= 2 && m <= 33, QD_ERR_UNSUPPORTED, "Krylov dimension m must be in 2..33");
-    DeviceGuard dg(ham->ctx->device);
+    CacheGuard dg(ham->ctx);
     QD_REQUIRE(nsteps >= 1, QD_ERR_INVALID, "nsteps must be positive");
     lanczos_evolve(ham, psi->col(t_in), psi->col(t_out), h, m, nsteps, act_dim, nullptr);
   });
@@ -587,7 +594,7 @@ qd_status qd_batch_lanczos(qd_ctx* ctx, int ninst, qd_ham* const* hams, const do
                            double* out) {
   return guard([&] {
     QD_REQUIRE(ctx && hams && v0s && out, QD_ERR_INVALID, "null argument");
-    DeviceGuard dg(ctx->device);
+    CacheGuard dg(ctx);
     batch_lanczos(ctx, hams, v0s, ninst, steps, out);
   });
 }
@@ -598,7 +605,7 @@ qd_status qd_krylov_evolve_batch(qd_ham* ham, const double* d_X, int64_t ldx, in
     QD_REQUIRE(ham && d_Y && nvec >= 1, QD_ERR_INVALID, "bad argument");
     QD_REQUIRE(ldy >= ham->dim && (!d_X || ldx >= ham->dim), QD_ERR_INVALID, "leading dimension below dim");
     QD_REQUIRE(d_X || nvec <= ham->dim, QD_ERR_INVALID, "more unit vectors than the dimension");
-    DeviceGuard dg(ham->ctx->device);
+    CacheGuard dg(ham->ctx);
     krylov_batch(ham, reinterpret_cast<const cplx*>(d_X), ldx, nvec, h, m, reinterpret_cast<cplx*>(d_Y), nullptr,
                  ldy, act_dims);
   });
@@ -610,7 +617,7 @@ qd_status qd_traj_run(qd_ham* heff, const qd_traj_desc* desc, const double* psi0
     QD_REQUIRE(heff && desc && psi0 && (obs_mean || desc->nobs == 0), QD_ERR_INVALID, "null argument");
     QD_REQUIRE(desc->chan_bits && (desc->nobs == 0 || (desc->obs_a && desc->obs_b)), QD_ERR_INVALID,
                "null channel or observable array");
-    DeviceGuard dg(heff->ctx->device);
+    CacheGuard dg(heff->ctx);
     int64_t jumps = 0;
     double t[2] = {0, 0};
     int path[2] = {0, 0};
@@ -631,7 +638,7 @@ qd_status qd_ham_set_spmv_kernel(qd_ham* ham, int kernel) {
     QD_REQUIRE(ham && ((kernel >= kSpmvTile && kernel <= kSpmvLast) || kernel == kSpmvFx || kernel == kSpmvFxSlots ||
                        kernel == kSpmvFxBlock),
                QD_ERR_INVALID, "unknown product kernel");
-    DeviceGuard dg(ham->ctx->device);
+    CacheGuard dg(ham->ctx);
     if (kernel == kSpmvFx || kernel == kSpmvFxSlots || kernel == kSpmvFxBlock) {
       QD_REQUIRE(ham_build_fx(ham), QD_ERR_UNSUPPORTED, "the fixed-point form does not apply to this operator");
       QD_REQUIRE(kernel != kSpmvFxSlots || ham_build_fx_slots(ham), QD_ERR_UNSUPPORTED,
@@ -652,7 +659,7 @@ qd_status qd_ham_set_spmv_kernel(qd_ham* ham, int kernel) {
 qd_status qd_ham_autotune(qd_ham* ham, int iters, int* chosen, double* best_ms) {
   return guard([&] {
     QD_REQUIRE(ham && iters >= 1, QD_ERR_INVALID, "bad argument");
-    DeviceGuard dg(ham->ctx->device);
+    CacheGuard dg(ham->ctx);
     double best = 1e300, bytes = 0;
     int pick = ham->spmv_variant;
     ham_ensure_row_order(ham);

@@ -6,6 +6,9 @@
 
 #include <cstdint>
 #include <cstdio>
+#include <map>
+#include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -80,17 +83,80 @@ struct AllocStreamScope {
   ~AllocStreamScope() { alloc_stream() = prev; }
 };
 
+// Freed device buffers of one context, kept for its next allocations of about
+// their size.  Building an operator makes and frees some forty buffers, and
+// cudaMalloc and cudaFree (which waits for the device) were a third of the
+// 2.85 ms that a new 20-site operator, its sector and an energy took (2.0
+// without them).  A context's work is on one stream
+// (a side stream joins it before its buffers are freed), so a buffer taken
+// again is used after everything that used it before.  States are not taken
+// from here: their addresses are handed out, and a caller may read them on a
+// stream of its own until they are freed.  At most kDevCacheBytes are kept
+// (larger buffers never); everything is given back with the context, and when
+// an allocation fails.
+constexpr size_t kDevCacheBytes = (size_t)1 << 30;
+constexpr size_t kDevCacheBlock = (size_t)1 << 28;
+struct DevCache {
+  std::mutex lock;  // handles may be dropped on another thread than the one that works
+  std::multimap<size_t, void*> idle;
+  size_t held = 0;
+  bool closed = false;
+  // Buffers of one size class take each other's place: eighths of a power of
+  // two, 512 bytes at least; what is too large to be kept is not rounded.
+  static size_t round_up(size_t bytes) {
+    if (bytes > kDevCacheBlock) return bytes;
+    size_t step = 512;
+    while (step * 16 <= bytes) step *= 2;
+    return (bytes + step - 1) / step * step;
+  }
+  void* take(size_t bytes) {
+    std::lock_guard<std::mutex> g(lock);
+    auto it = idle.find(bytes);
+    if (it == idle.end()) return nullptr;
+    void* p = it->second;
+    idle.erase(it);
+    held -= bytes;
+    return p;
+  }
+  bool give(void* p, size_t bytes) {
+    std::lock_guard<std::mutex> g(lock);
+    if (closed || bytes > kDevCacheBlock || held + bytes > kDevCacheBytes) return false;
+    idle.emplace(bytes, p);
+    held += bytes;
+    return true;
+  }
+  void drain(bool close = false) {
+    std::lock_guard<std::mutex> g(lock);
+    for (auto& e : idle) cudaFree(e.second);
+    idle.clear();
+    held = 0;
+    closed |= close;
+  }
+  ~DevCache() { drain(true); }
+};
+// The cache that this thread's DBuf allocations come from; null: plain cudaMalloc.
+inline std::shared_ptr<DevCache>& alloc_cache() {
+  static thread_local std::shared_ptr<DevCache> c;
+  return c;
+}
+struct AllocCacheScope {
+  std::shared_ptr<DevCache> prev;
+  explicit AllocCacheScope(const std::shared_ptr<DevCache>& c) : prev(alloc_cache()) { alloc_cache() = c; }
+  ~AllocCacheScope() { alloc_cache() = std::move(prev); }
+};
+
 // Owning device buffer; never copied.
 template <typename T>
 struct DBuf {
   T* p = nullptr;
   size_t n = 0;
   cudaStream_t s = nullptr;  // stream the buffer was allocated on (stream-ordered pool), or null
+  std::shared_ptr<DevCache> c;  // the cache it goes back to, or null
   DBuf() = default;
   explicit DBuf(size_t count) { alloc(count); }
   DBuf(const DBuf&) = delete;
   DBuf& operator=(const DBuf&) = delete;
-  DBuf(DBuf&& o) noexcept : p(o.p), n(o.n), s(o.s) {
+  DBuf(DBuf&& o) noexcept : p(o.p), n(o.n), s(o.s), c(std::move(o.c)) {
     o.p = nullptr;
     o.n = 0;
     o.s = nullptr;
@@ -101,6 +167,7 @@ struct DBuf {
       p = o.p;
       n = o.n;
       s = o.s;
+      c = std::move(o.c);
       o.p = nullptr;
       o.n = 0;
       o.s = nullptr;
@@ -112,22 +179,39 @@ struct DBuf {
     release();
     if (count == 0) count = 1;
     s = alloc_stream();
-    if (s)
+    if (s) {
       QD_CUDA(cudaMallocAsync((void**)&p, count * sizeof(T), s));
-    else
+    } else if (alloc_cache()) {
+      c = alloc_cache();
+      const size_t b = DevCache::round_up(count * sizeof(T));
+      p = static_cast<T*>(c->take(b));
+      if (!p && cudaMalloc((void**)&p, b) != cudaSuccess) {
+        cudaGetLastError();
+        p = nullptr;
+        c->drain();  // what is kept may be what is missing
+        const cudaError_t e = cudaMalloc((void**)&p, b);
+        if (e != cudaSuccess) {
+          p = nullptr;
+          c.reset();
+          QD_CUDA(e);
+        }
+      }
+    } else {
       QD_CUDA(cudaMalloc((void**)&p, count * sizeof(T)));
+    }
     n = count;
   }
   void release() {
     if (p) {
       if (s)
         cudaFreeAsync(p, s);
-      else
+      else if (!c || !c->give(p, DevCache::round_up(n * sizeof(T))))
         cudaFree(p);
     }
     p = nullptr;
     n = 0;
     s = nullptr;
+    c.reset();
   }
   size_t bytes() const { return n * sizeof(T); }
 };
@@ -139,6 +223,7 @@ struct Ctx {
   int num_sms = 0;
   int64_t launches = 0;
   cudaEvent_t events[16] = {};
+  std::shared_ptr<DevCache> cache = std::make_shared<DevCache>();
 };
 
 struct DeviceGuard {
@@ -152,6 +237,13 @@ struct DeviceGuard {
     cudaGetDevice(&cur);
     if (prev >= 0 && cur != prev) cudaSetDevice(prev);
   }
+};
+
+// The context's device, and its cache for the buffers that the call makes.
+struct CacheGuard {
+  DeviceGuard dev;
+  AllocCacheScope cache;
+  explicit CacheGuard(Ctx* ctx) : dev(ctx->device), cache(ctx->cache) {}
 };
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }

@@ -66,8 +66,8 @@ void exclusive_scan_i64(Ctx* ctx, const int64_t* in, int64_t* out, int64_t n) {
     QD_CHECK_LAUNCH();
     QD_LAUNCHED(ctx);
   }
-  // keep `sums` alive until the kernels that read it have run
-  QD_CUDA(cudaStreamSynchronize(ctx->stream));
+  // a plain allocation lives until the kernels that read it have run; the others are reused in stream order
+  if (!sums.c && !sums.s) QD_CUDA(cudaStreamSynchronize(ctx->stream));
 }
 
 }  // namespace qd
