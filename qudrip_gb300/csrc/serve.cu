@@ -142,7 +142,7 @@ static int64_t held_bytes(const qd_sector* S, const qd_ham* H) {
            dbytes(W.partials_td) + dbytes(W.gpart_td) + dbytes(W.partials_tc) + dbytes(W.gpart_tc) +
            dbytes(W.tickets) + dbytes(W.lz_d.V) + dbytes(W.lz_c.V) + dbytes(W.lz_d.w) + dbytes(W.lz_c.w);
     }
-    if (H->arnoldi) b += dbytes(H->arnoldi->V) + dbytes(H->arnoldi->w) + dbytes(H->arnoldi->partials);
+    if (H->arnoldi) b += H->arnoldi->basis.bytes();
   }
   return b;
 }
