@@ -595,7 +595,7 @@ static bool arn_launch(qd_ham* H, const MV* vals, ArnRes& B, const cplx* psi_in,
       rows = (int)ceil_div(n, one ? 1 : ncl * kArnCluster);
       if (smem_of(rows) + sizeof(ArnShared<VV, kArnThreads>) + 4096 > (size_t)maxsm || rows > kArnMaxResRows) return false;
       if (one) break;
-      QD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(rows)));
+      allow_dynamic_smem(kern, ctx->device);
       cfg.gridDim = dim3((unsigned)(ncl * kArnCluster));
       cfg.dynamicSmemBytes = smem_of(rows);
       cfg.attrs = at + 1;
@@ -653,7 +653,7 @@ static bool arn_launch(qd_ham* H, const MV* vals, ArnRes& B, const cplx* psi_in,
     QD_CUDA(cudaMemsetAsync(&A.st->abort, kXEmptyByte, sizeof(int), ctx->stream));
     QD_CUDA(cudaMemsetAsync(A.slots, kXEmptyByte, slot_bytes, ctx->stream));
   }
-  QD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_dynamic_smem(kern, ctx->device);
   QD_CUDA(cudaLaunchKernelEx(&cfg, kern, A));
   QD_LAUNCHED(ctx);
   QD_CUDA(cudaMemcpyAsync(&B.host, A.st, sizeof(ArnStatus), cudaMemcpyDeviceToHost, ctx->stream));

@@ -246,6 +246,17 @@ struct CacheGuard {
   explicit CacheGuard(Ctx* ctx) : dev(ctx->device), cache(ctx->cache) {}
 };
 
+// Allows a kernel all the dynamic shared memory a block may have.  The limit belongs to the function, not to
+// the launch: set to each launch's own size, a thread with a small one would fail another thread's larger one.
+template <typename K>
+inline void allow_dynamic_smem(K kern, int device) {
+  cudaFuncAttributes a;
+  int most = 0;
+  QD_CUDA(cudaFuncGetAttributes(&a, kern));
+  QD_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+  QD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes));
+}
+
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 }  // namespace qd

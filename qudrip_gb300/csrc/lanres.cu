@@ -573,7 +573,7 @@ static bool lan_plan(qd_ham* H, K kern1, K kern_many, LanPlan& P, cudaLaunchConf
       }
       if (smem_of(rows) + 8192 > (size_t)maxsm) return false;
       if (csize == 1) break;
-      QD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(rows)));
+      allow_dynamic_smem(kern, ctx->device);
       cfg.gridDim = dim3((unsigned)grid);
       cfg.dynamicSmemBytes = smem_of(rows);
       cudaLaunchConfig_t q = cfg;
@@ -592,7 +592,7 @@ static bool lan_plan(qd_ham* H, K kern1, K kern_many, LanPlan& P, cudaLaunchConf
   }
   cfg.gridDim = dim3((unsigned)(P.ncl * csize));
   cfg.dynamicSmemBytes = smem_of(P.rows);
-  QD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes));
+  allow_dynamic_smem(kern, ctx->device);
   return true;
 }
 
