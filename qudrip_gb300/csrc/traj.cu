@@ -95,7 +95,6 @@ struct TrajResArgs {
 };
 
 struct TrajSmem {
-  float2* tb[2];
   uint16_t* ent;
   uint16_t* rid;
   uint32_t* st;
@@ -105,48 +104,86 @@ struct TrajSmem {
   const uint32_t* obs_mask;
 };
 
-__device__ __forceinline__ float traj_warp_sum(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+// Two floats at once (one issue slot for both sums of a complex addition).
+using Pair = unsigned long long;
+__device__ __forceinline__ Pair pair_add(Pair a, Pair b) {
+  Pair r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ Pair pair_fma(float a, Pair b, Pair c) {
+  Pair r, aa;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(aa) : "f"(a));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(aa), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ float2 pair_get(Pair a) {
+  float2 v;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(a));
   return v;
 }
 
 // Block sums of q_j = sum over the block's rows of |acc|^2 f_j(state), j < nq,
 // into res[0 .. nq-1]; f_j chosen by `kind`: 0 the step's quantities
 // (1, popcount(state & chanmask), observables), 1 the channel weights.
+// Eight quantities share one butterfly (each step halves the values a lane
+// keeps); a warp a quantity adds the warps' sums in FP64.
 template <int kind>
 __device__ __forceinline__ void traj_block_sums(const TrajResArgs& A, const TrajSmem& M, const float2 (&acc)[kTrajRpt],
                                                 int nq, float* res) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int q = 0; q < nq; ++q) {
-    float v = 0.f;
+  float p[kTrajRpt];
+  uint32_t st[kTrajRpt];
 #pragma unroll
-    for (int i = 0; i < kTrajRpt; ++i) {
-      const int s = warp + i * A.nwarps;
-      if (s < A.nsl) {
-        const float p = fmaf(acc[i].x, acc[i].x, acc[i].y * acc[i].y);
-        const uint32_t st = M.st[32 * s + lane];
-        float f;
-        if (kind == 0) {
-          f = (q == 0) ? 1.f
-                       : (q == 1 ? (float)__popc(st & A.chanmask)
-                                 : (((st & M.obs_mask[q - 2]) == M.obs_mask[q - 2]) ? 1.f : 0.f));
-        } else {
-          f = (float)((st >> M.chan_bit[q]) & 1u);
-        }
-        v = fmaf(p, f, v);
+  for (int i = 0; i < kTrajRpt; ++i) {
+    const int s = warp + i * A.nwarps;
+    p[i] = 0.f;
+    st[i] = 0u;
+    if (s < A.nsl) {
+      p[i] = fmaf(acc[i].x, acc[i].x, acc[i].y * acc[i].y);
+      st[i] = M.st[32 * s + lane];
+    }
+  }
+  for (int q0 = 0; q0 < nq; q0 += 8) {
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int q = q0 + j;
+      v[j] = 0.f;
+      if (q >= nq) continue;
+      if (kind == 0 && q == 0) {
+#pragma unroll
+        for (int i = 0; i < kTrajRpt; ++i) v[j] += p[i];
+      } else if (kind == 0 && q == 1) {
+#pragma unroll
+        for (int i = 0; i < kTrajRpt; ++i) v[j] = fmaf(p[i], (float)__popc(st[i] & A.chanmask), v[j]);
+      } else {
+        const uint32_t m = (kind == 0) ? M.obs_mask[q - 2] : 1u << M.chan_bit[q];
+#pragma unroll
+        for (int i = 0; i < kTrajRpt; ++i)
+          if ((st[i] & m) == m) v[j] += p[i];
       }
     }
-    v = traj_warp_sum(v);
-    if (lane == 0) M.red[warp * kTrajRedStride + q] = v;
+#pragma unroll
+    for (int h = 4; h >= 1; h >>= 1) {
+      const bool up = (lane & (4 * h)) != 0;
+#pragma unroll
+      for (int i = 0; i < h; ++i) {
+        const float send = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4 * h);
+      }
+    }
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    if ((lane & 3) == 0 && q0 + (lane >> 2) < nq) M.red[warp * kTrajRedStride + q0 + (lane >> 2)] = v[0];
   }
   __syncthreads();
-  if (threadIdx.x < nq) {
-    double t = 0.0;
-    for (int w = 0; w < A.nwarps; ++w) t += M.red[w * kTrajRedStride + threadIdx.x];
-    res[threadIdx.x] = (float)t;
+  for (int q = warp; q < nq; q += A.nwarps) {
+    double t = lane < A.nwarps ? (double)M.red[lane * kTrajRedStride + q] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) res[q] = (float)t;
   }
-  __syncthreads();
 }
 
 template <bool kSigned>
@@ -155,13 +192,13 @@ __global__ void __launch_bounds__(kTrajMaxWarps * 32, 1) traj_resident_kernel(Tr
   __shared__ float res[2 + kTrajMaxObs];
   __shared__ float resc[kTrajMaxChan];
   __shared__ int s_jump;
-  __shared__ double s_u2;
+  __shared__ double s_u1, s_u2;  // the step's random numbers
+  __shared__ float s_u1f;
   __shared__ int s_chan_bit[kTrajMaxChan];
   __shared__ uint32_t s_obs_mask[kTrajMaxObs];
   TrajSmem M;
-  M.tb[0] = reinterpret_cast<float2*>(traj_smem);
-  M.tb[1] = M.tb[0] + A.tb_len;
-  M.ent = reinterpret_cast<uint16_t*>(M.tb[1] + A.tb_len);
+  float2* const tb = reinterpret_cast<float2*>(traj_smem);  // two vectors, tb_len apart
+  M.ent = reinterpret_cast<uint16_t*>(tb + 2 * A.tb_len);
   M.rid = M.ent + A.ent_len;
   M.st = reinterpret_cast<uint32_t*>(M.rid + 32 * A.nsl);
   M.sd = reinterpret_cast<int2*>(M.st + 32 * A.nsl);
@@ -178,8 +215,8 @@ __global__ void __launch_bounds__(kTrajMaxWarps * 32, 1) traj_resident_kernel(Tr
     }
     for (int i = tid; i < A.nsl; i += blockDim.x) M.sd[i] = A.sdesc[i];
     if (tid == 0) {
-      M.tb[0][A.n] = make_float2(0.f, 0.f);
-      M.tb[1][A.n] = make_float2(0.f, 0.f);
+      tb[A.n] = make_float2(0.f, 0.f);
+      tb[A.tb_len + A.n] = make_float2(0.f, 0.f);
 #pragma unroll
       for (int j = 0; j < kTrajMaxChan; ++j) s_chan_bit[j] = A.chan_bit[j];
 #pragma unroll
@@ -197,6 +234,19 @@ __global__ void __launch_bounds__(kTrajMaxWarps * 32, 1) traj_resident_kernel(Tr
   __syncthreads();
   const int nq = 2 + A.nobs;
   unsigned long long njumps = 0;
+  const float gdt = (float)(A.gamma * A.dt);
+  // The sums of the new vector, and meanwhile the last warp draws the next step's random numbers.
+  auto sums = [&](const float2 (&acc)[kTrajRpt], int b, int next) {
+    traj_block_sums<0>(A, M, acc, nq, res);
+    if (tid == (int)blockDim.x - 1) {
+      double u1, u2;
+      philox_uniform2(A.seed, (uint32_t)b, (uint32_t)next, u1, u2);
+      s_u1 = u1;
+      s_u1f = (float)u1;
+      s_u2 = u2;
+    }
+    __syncthreads();
+  };
 
   for (int b = blockIdx.x; b < A.ntraj; b += gridDim.x) {
     float2 acc[kTrajRpt];
@@ -209,25 +259,26 @@ __global__ void __launch_bounds__(kTrajMaxWarps * 32, 1) traj_resident_kernel(Tr
         const int r = M.rid[32 * s + lane];
         if (r < A.n) {
           acc[i] = A.psi0[r];
-          M.tb[0][r] = acc[i];
+          tb[r] = acc[i];
         }
       }
     }
-    traj_block_sums<0>(A, M, acc, nq, res);
+    sums(acc, b, 1);
     if (tid < A.nobs) A.obs[(size_t)tid * A.ntraj + b] = res[2 + tid] / res[0];
 
     for (int step = 1; step <= A.nsteps; ++step) {
-      if (tid == 0) {
-        double u1, u2;
-        philox_uniform2(A.seed, (uint32_t)b, (uint32_t)step, u1, u2);
+      // jump if u1 < gamma wtot dt.  In FP32 unless that is too close to tell: in FP64 one thread's
+      // conversions and division would hold the block up for 1,500 cycles
+      const float rate = gdt * (res[1] / res[0]);
+      bool jump = s_u1f < rate;
+      if (!(fabsf(s_u1f - rate) > 1e-5f * rate)) {  // and when something is not finite
         const double wtot = (double)res[1] / (double)res[0];
-        s_jump = (wtot > 0.0 && u1 < A.gamma * wtot * A.dt) ? 1 : 0;
-        s_u2 = u2;
+        jump = wtot > 0.0 && s_u1 < A.gamma * wtot * A.dt;
       }
-      __syncthreads();
-      if (s_jump) {
+      if (jump) {
         // channel weights of the current state, then psi <- n_j psi (norm carried)
         traj_block_sums<1>(A, M, acc, A.nchan, resc);
+        __syncthreads();
         if (tid == 0) {
           // bsearch on the cumulative weights normalised by their total: the channel j
           // with wt[j] <= u2 < wt[j+1] (a scan gives the same index on a monotone table)
@@ -252,7 +303,7 @@ __global__ void __launch_bounds__(kTrajMaxWarps * 32, 1) traj_resident_kernel(Tr
             const int r = M.rid[slot];
             if (r < A.n) {
               if (!((M.st[slot] >> bit) & 1u)) acc[i] = make_float2(0.f, 0.f);
-              M.tb[cb][r] = acc[i];
+              tb[cb * A.tb_len + r] = acc[i];
             }
           }
         }
@@ -268,31 +319,27 @@ __global__ void __launch_bounds__(kTrajMaxWarps * 32, 1) traj_resident_kernel(Tr
           for (int k = 1; k <= A.K; ++k) {
             // t_k = (-i tau / k) (H - mu) t_{k-1}; t_0 = the vector in tb[cb] (times sc on the first sub-step)
             const float f = A.tau / (float)k * ((sub == 0 && k == 1) ? sc : 1.f);
-            const float2* __restrict__ src = M.tb[rb];
-            float2* __restrict__ dst = M.tb[rb ^ 1];
+            const float2* src = tb + rb * A.tb_len;
+            float2* dst = tb + (rb ^ 1) * A.tb_len;
             // Two slices at a time (i and i + 1): their entry loads and gathers interleave, so a
             // lane has four independent gathers in flight; each row keeps its own sums in entry
             // order (even entries in s, odd ones in u).
-            auto gather = [&](uint32_t pr, float& sx, float& sy, float& ux, float& uy) {
+            auto at = [&](uint32_t c) { return *reinterpret_cast<const Pair*>(src + c); };
+            auto gather = [&](uint32_t pr, Pair& sp, Pair& up) {
               const uint32_t ev = pr & 0xffffu, fv = pr >> 16;
               if (kSigned) {
-                const float2 x = src[ev & 0x7fffu], y = src[fv & 0x7fffu];
                 const float sg = __uint_as_float(0x3f800000u | ((ev & 0x8000u) << 16));
                 const float tg = __uint_as_float(0x3f800000u | ((fv & 0x8000u) << 16));
-                sx = fmaf(sg, x.x, sx);
-                sy = fmaf(sg, x.y, sy);
-                ux = fmaf(tg, y.x, ux);
-                uy = fmaf(tg, y.y, uy);
+                sp = pair_fma(sg, at(ev & 0x7fffu), sp);
+                up = pair_fma(tg, at(fv & 0x7fffu), up);
               } else {  // every entry carries +c: plain sums
-                const float2 x = src[ev], y = src[fv];
-                sx += x.x;
-                sy += x.y;
-                ux += y.x;
-                uy += y.y;
+                sp = pair_add(sp, at(ev));
+                up = pair_add(up, at(fv));
               }
             };
-            auto finish = [&](int i, int r, float sx, float sy) {
+            auto finish = [&](int i, int r, Pair sum) {
               if (r < A.n) {
+                const float sx = pair_get(sum).x, sy = pair_get(sum).y;
                 const float2 o = src[r];
                 // v = c * sum + dg * own
                 const float vx = fmaf(A.coff.x, sx, fmaf(-A.coff.y, sy, fmaf(dg[i].x, o.x, -dg[i].y * o.y)));
@@ -317,19 +364,18 @@ __global__ void __launch_bounds__(kTrajMaxWarps * 32, 1) traj_resident_kernel(Tr
                 const uint32_t* e0 = reinterpret_cast<const uint32_t*>(M.ent + d0.x) + lane;
                 const uint32_t* e1 = reinterpret_cast<const uint32_t*>(M.ent + d1.x) + lane;
                 const int w0 = d0.y >> 1, w1 = d1.y >> 1;
-                float sx0 = 0.f, sy0 = 0.f, ux0 = 0.f, uy0 = 0.f;
-                float sx1 = 0.f, sy1 = 0.f, ux1 = 0.f, uy1 = 0.f;
+                Pair sp0 = 0, up0 = 0, sp1 = 0, up1 = 0;
                 const int wm = min(w0, w1);
                 int q = 0;
                 for (; q < wm; ++q) {
                   const uint32_t p0 = e0[32 * q], p1 = e1[32 * q];
-                  gather(p0, sx0, sy0, ux0, uy0);
-                  gather(p1, sx1, sy1, ux1, uy1);
+                  gather(p0, sp0, up0);
+                  gather(p1, sp1, up1);
                 }
-                for (int q0 = q; q0 < w0; ++q0) gather(e0[32 * q0], sx0, sy0, ux0, uy0);
-                for (int q1 = q; q1 < w1; ++q1) gather(e1[32 * q1], sx1, sy1, ux1, uy1);
-                finish(i, r0, sx0 + ux0, sy0 + uy0);
-                if (has1) finish(i + 1, r1, sx1 + ux1, sy1 + uy1);
+                for (int q0 = q; q0 < w0; ++q0) gather(e0[32 * q0], sp0, up0);
+                for (int q1 = q; q1 < w1; ++q1) gather(e1[32 * q1], sp1, up1);
+                finish(i, r0, pair_add(sp0, up0));
+                if (has1) finish(i + 1, r1, pair_add(sp1, up1));
               }
             }
             __syncthreads();
@@ -342,13 +388,13 @@ __global__ void __launch_bounds__(kTrajMaxWarps * 32, 1) traj_resident_kernel(Tr
             const int s = warp + i * A.nwarps;
             if (s < A.nsl) {
               const int r = M.rid[32 * s + lane];
-              if (r < A.n) M.tb[cb][r] = acc[i];
+              if (r < A.n) tb[cb * A.tb_len + r] = acc[i];
             }
           }
           __syncthreads();
         }
       }
-      traj_block_sums<0>(A, M, acc, nq, res);
+      sums(acc, b, step + 1);
       if (tid < A.nobs) A.obs[((size_t)step * A.nobs + tid) * A.ntraj + b] = res[2 + tid] / res[0];
     }
   }
@@ -623,16 +669,23 @@ __global__ void init_states_kernel(cplx* psi, int64_t n, int64_t ld, int ntraj, 
   psi[(size_t)b * ld + i] = mkc(v.re * inv, v.im * inv);
 }
 
-// mean and standard error over trajectories (fixed order, FP64)
-__global__ void traj_reduce_kernel(const float* obs, int ntraj, int nrows, double* mean, double* stderr_) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
+// mean and standard error over trajectories (fixed order, FP64), a warp per row
+constexpr int kTrajReduceThreads = 64;
+__global__ void __launch_bounds__(kTrajReduceThreads) traj_reduce_kernel(const float* obs, int ntraj, int nrows,
+                                                                         double* mean, double* stderr_) {
+  const int row = (int)((blockIdx.x * kTrajReduceThreads + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (row >= nrows) return;
   double s = 0.0, s2 = 0.0;
-  for (int b = 0; b < ntraj; ++b) {
+  for (int b = lane; b < ntraj; b += 32) {
     const double v = obs[(size_t)row * ntraj + b];
     s += v;
-    s2 += v * v;
+    s2 = fma(v, v, s2);
   }
+  for (int o = 16; o > 0; o >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+  }
+  if (lane != 0) return;
   const double m = s / ntraj;
   mean[row] = m;
   stderr_[row] = (ntraj > 1) ? sqrt(fmax(s2 / ntraj - m * m, 0.0) / (ntraj - 1)) : 0.0;
@@ -820,7 +873,8 @@ void traj_run(qd_ham* H, const qd_traj_desc& d, const double* psi0_host, double*
   }
   if (nrows > 0) {
     DBuf<double> dm(nrows), ds(nrows);
-    traj_reduce_kernel<<<(unsigned)ceil_div(nrows, 128), 128, 0, ctx->stream>>>(obs.p, d.ntraj, nrows, dm.p, ds.p);
+    traj_reduce_kernel<<<(unsigned)ceil_div(nrows, kTrajReduceThreads / 32), kTrajReduceThreads, 0, ctx->stream>>>(
+        obs.p, d.ntraj, nrows, dm.p, ds.p);
     QD_CHECK_LAUNCH();
     QD_LAUNCHED(ctx);
     QD_CUDA(cudaMemcpyAsync(obs_mean, dm.p, nrows * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
