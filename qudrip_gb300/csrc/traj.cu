@@ -14,16 +14,16 @@
 // random numbers are Philox4x32-10 keyed by (seed, trajectory, step), so the
 // oracle replays every decision.
 //
-// GB300 form (resident kernel): one CTA per trajectory at a time, persistent
-// over the ensemble.  H_eff is shared by every trajectory and small (config:
-// Hubbard L=8, dim 4,900, 44,100 stored entries), so each CTA stages it in
-// shared memory once -- rows in 32-row slices with their columns in gather
-// order, each entry a 16-bit column with the sign of the uniform off-diagonal
-// value c in its top bit (a lane's entries 2j and 2j+1 in one 32-bit word;
-// when no entry carries -c the kernel's sums are plain adds), the diagonal
-// (shifted by the centre mu of its range) in registers --
-// together with two complex64 copies of the trajectory's vector.  A step is
-// then K products H - mu of the shared-memory vector (the gathers never leave
+// GB300 form (resident kernel): one CTA per trajectory, or per two of them, at
+// a time, persistent over the ensemble.  H_eff is shared by every trajectory and
+// small (config: Hubbard L=8, dim 4,900, 44,100 stored entries), so each CTA
+// stages it in shared memory once -- rows in 32-row slices with their columns in
+// gather order, each entry a 16-bit column with the sign of the uniform
+// off-diagonal value c in its top bit (a lane's entries 2j and 2j+1 in one
+// 32-bit word; when no entry carries -c the kernel's sums are plain adds) --
+// together with the vector that a product gathers from, in complex64; the
+// diagonal (shifted by the centre mu of its range) comes from L1 and L2.  A step
+// is then K products H - mu of the shared-memory vector (the gathers never leave
 // the SM) summed into the truncated Taylor series of exp(-i tau (H - mu)),
 // S sub-steps of tau = dt / S, with (S, K) from the series' remainder bound
 // (tau ||H - mu|| <= 1 and ||R_K|| <= theta^(K+1) / (K+1)! e^theta <= 1e-8,
@@ -33,6 +33,16 @@
 // one block reduction of the new vector per step; HBM sees only the observable
 // records.  The state's norm is carried, not divided out: the next products
 // start from psi / ||psi||.
+//
+// Two trajectories a CTA share the loads and the decoding of the entries and
+// fetch a column's two values in one 16-byte load.  2,048 trajectories of 100
+// steps at dim 4,900 (six products a step): generic addresses and one sum after
+// another 50.9 ms, shared-memory addresses, packed additions and one butterfly
+// for eight sums 41.1 ms, two trajectories a CTA 35.1 ms.  A product of two
+// takes 10,700 cycles of shared-memory bandwidth, 1,900 of them conflicts, and
+// 8,500 issue cycles in 17,000; entries ordered against the conflicts took 5%
+// off the kernel and gave it to the host.  16 warps of 10 slices and loops
+// unrolled deeper measured the same.
 //
 // Operators the resident form does not cover (dim > 5,120, registers of more
 // than 32 bits, or off-diagonal values other than +-c) run each step as a
@@ -82,7 +92,7 @@ struct TrajResArgs {
   int chan_bit[kTrajMaxChan];
   uint32_t obs_mask[kTrajMaxObs];
   // smem segment sizes (elements)
-  int tb_len;         // per vector buffer: n + 1 rounded up to 2 (slot n is a zero)
+  int tb_len;         // half the vector buffer: n + 1 rounded up to 2 (slot n is a zero)
   int ent_len;        // entries rounded up to 8
   const uint16_t* ent;   // entry k of slice row l at sdesc.x + 64 (k / 2) + 2 l + k % 2: column | sign << 15
   const uint16_t* rid;   // row of each slot (n: padding)
@@ -128,76 +138,84 @@ __device__ __forceinline__ float2 pair_get(Pair a) {
 // (1, popcount(state & chanmask), observables), 1 the channel weights.
 // Eight quantities share one butterfly (each step halves the values a lane
 // keeps); a warp a quantity adds the warps' sums in FP64.
-template <int kind>
-__device__ __forceinline__ void traj_block_sums(const TrajResArgs& A, const TrajSmem& M, const float2 (&acc)[kTrajRpt],
-                                                int nq, float* res) {
+template <int NT, int kind>
+__device__ __forceinline__ void traj_block_sums(const TrajResArgs& A, const TrajSmem& M,
+                                                const float2 (&acc)[NT][kTrajRpt], int nq, float* res, int ldres) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float p[kTrajRpt];
   uint32_t st[kTrajRpt];
 #pragma unroll
   for (int i = 0; i < kTrajRpt; ++i) {
     const int s = warp + i * A.nwarps;
-    p[i] = 0.f;
-    st[i] = 0u;
-    if (s < A.nsl) {
-      p[i] = fmaf(acc[i].x, acc[i].x, acc[i].y * acc[i].y);
-      st[i] = M.st[32 * s + lane];
-    }
+    st[i] = (s < A.nsl) ? M.st[32 * s + lane] : 0u;  // |acc|^2 is 0 there
   }
-  for (int q0 = 0; q0 < nq; q0 += 8) {
-    float v[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int q = q0 + j;
-      v[j] = 0.f;
-      if (q >= nq) continue;
-      if (kind == 0 && q == 0) {
+  for (int a = 0; a < NT; ++a) {
+    float p[kTrajRpt];
 #pragma unroll
-        for (int i = 0; i < kTrajRpt; ++i) v[j] += p[i];
-      } else if (kind == 0 && q == 1) {
-#pragma unroll
-        for (int i = 0; i < kTrajRpt; ++i) v[j] = fmaf(p[i], (float)__popc(st[i] & A.chanmask), v[j]);
-      } else {
-        const uint32_t m = (kind == 0) ? M.obs_mask[q - 2] : 1u << M.chan_bit[q];
-#pragma unroll
-        for (int i = 0; i < kTrajRpt; ++i)
-          if ((st[i] & m) == m) v[j] += p[i];
-      }
+    for (int i = 0; i < kTrajRpt; ++i) {
+      p[i] = fmaf(acc[a][i].x, acc[a][i].x, acc[a][i].y * acc[a][i].y);
     }
+    for (int q0 = 0; q0 < nq; q0 += 8) {
+      float v[8];
 #pragma unroll
-    for (int h = 4; h >= 1; h >>= 1) {
-      const bool up = (lane & (4 * h)) != 0;
+      for (int j = 0; j < 8; ++j) {
+        const int q = q0 + j;
+        v[j] = 0.f;
+        if (q >= nq) continue;
+        if (kind == 0 && q == 0) {
 #pragma unroll
-      for (int i = 0; i < h; ++i) {
-        const float send = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
-        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4 * h);
+          for (int i = 0; i < kTrajRpt; ++i) v[j] += p[i];
+        } else if (kind == 0 && q == 1) {
+#pragma unroll
+          for (int i = 0; i < kTrajRpt; ++i) v[j] = fmaf(p[i], (float)__popc(st[i] & A.chanmask), v[j]);
+        } else {
+          const uint32_t m = (kind == 0) ? M.obs_mask[q - 2] : 1u << M.chan_bit[q];
+#pragma unroll
+          for (int i = 0; i < kTrajRpt; ++i)
+            if ((st[i] & m) == m) v[j] += p[i];
+        }
       }
+#pragma unroll
+      for (int h = 4; h >= 1; h >>= 1) {
+        const bool up = (lane & (4 * h)) != 0;
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+          const float send = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
+          v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4 * h);
+        }
+      }
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+      if ((lane & 3) == 0 && q0 + (lane >> 2) < nq) M.red[(a * kTrajMaxWarps + warp) * kTrajRedStride + q0 + (lane >> 2)] = v[0];
     }
-    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
-    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-    if ((lane & 3) == 0 && q0 + (lane >> 2) < nq) M.red[warp * kTrajRedStride + q0 + (lane >> 2)] = v[0];
   }
   __syncthreads();
-  for (int q = warp; q < nq; q += A.nwarps) {
-    double t = lane < A.nwarps ? (double)M.red[lane * kTrajRedStride + q] : 0.0;
+  for (int i = warp; i < NT * nq; i += A.nwarps) {
+    const int a = i / nq, q = i - a * nq;
+    double t = lane < A.nwarps ? (double)M.red[(a * kTrajMaxWarps + lane) * kTrajRedStride + q] : 0.0;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (lane == 0) res[q] = (float)t;
+    if (lane == 0) res[a * ldres + q] = (float)t;
   }
 }
 
-template <bool kSigned>
+// NT trajectories of a CTA run side by side: they share every entry's load and
+// address, and a gather fetches the column's value of both in one 16-byte load.
+// One buffer holds the vectors t_{k-1}: a product's results stay in registers
+// until every gather of the block is done.  A trajectory that jumps sits the
+// step's products out (its factor is 0).
+template <int NT, bool kSigned>
 __global__ void __launch_bounds__(kTrajMaxWarps * 32, 1) traj_resident_kernel(TrajResArgs A) {
   extern __shared__ __align__(16) unsigned char traj_smem[];
-  __shared__ float res[2 + kTrajMaxObs];
+  __shared__ float res[NT][2 + kTrajMaxObs];
   __shared__ float resc[kTrajMaxChan];
-  __shared__ int s_jump;
-  __shared__ double s_u1, s_u2;  // the step's random numbers
-  __shared__ float s_u1f;
+  __shared__ int s_chan;
+  __shared__ double s_u1[NT], s_u2[NT];  // the step's random numbers
+  __shared__ float s_u1f[NT];
   __shared__ int s_chan_bit[kTrajMaxChan];
   __shared__ uint32_t s_obs_mask[kTrajMaxObs];
   TrajSmem M;
-  float2* const tb = reinterpret_cast<float2*>(traj_smem);  // two vectors, tb_len apart
+  Pair* const tb = reinterpret_cast<Pair*>(traj_smem);  // trajectory a's element c at NT c + a
   M.ent = reinterpret_cast<uint16_t*>(tb + 2 * A.tb_len);
   M.rid = M.ent + A.ent_len;
   M.st = reinterpret_cast<uint32_t*>(M.rid + 32 * A.nsl);
@@ -215,8 +233,8 @@ __global__ void __launch_bounds__(kTrajMaxWarps * 32, 1) traj_resident_kernel(Tr
     }
     for (int i = tid; i < A.nsl; i += blockDim.x) M.sd[i] = A.sdesc[i];
     if (tid == 0) {
-      tb[A.n] = make_float2(0.f, 0.f);
-      tb[A.tb_len + A.n] = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int a = 0; a < NT; ++a) tb[NT * A.n + a] = 0;
 #pragma unroll
       for (int j = 0; j < kTrajMaxChan; ++j) s_chan_bit[j] = A.chan_bit[j];
 #pragma unroll
@@ -225,178 +243,195 @@ __global__ void __launch_bounds__(kTrajMaxWarps * 32, 1) traj_resident_kernel(Tr
   }
   M.chan_bit = s_chan_bit;
   M.obs_mask = s_obs_mask;
-  float2 dg[kTrajRpt];
-#pragma unroll
-  for (int i = 0; i < kTrajRpt; ++i) {
-    const int s = warp + i * A.nwarps;
-    dg[i] = (s < A.nsl) ? A.dg[32 * s + lane] : make_float2(0.f, 0.f);
-  }
   __syncthreads();
   const int nq = 2 + A.nobs;
   unsigned long long njumps = 0;
   const float gdt = (float)(A.gamma * A.dt);
-  // The sums of the new vector, and meanwhile the last warp draws the next step's random numbers.
-  auto sums = [&](const float2 (&acc)[kTrajRpt], int b, int next) {
-    traj_block_sums<0>(A, M, acc, nq, res);
-    if (tid == (int)blockDim.x - 1) {
-      double u1, u2;
-      philox_uniform2(A.seed, (uint32_t)b, (uint32_t)next, u1, u2);
-      s_u1 = u1;
-      s_u1f = (float)u1;
-      s_u2 = u2;
-    }
-    __syncthreads();
-  };
-
-  for (int b = blockIdx.x; b < A.ntraj; b += gridDim.x) {
-    float2 acc[kTrajRpt];
-    int cb = 0;
+  // The vectors v into the buffer.
+  auto store = [&](const float2 (&v)[NT][kTrajRpt]) {
 #pragma unroll
     for (int i = 0; i < kTrajRpt; ++i) {
       const int s = warp + i * A.nwarps;
-      acc[i] = make_float2(0.f, 0.f);
       if (s < A.nsl) {
         const int r = M.rid[32 * s + lane];
         if (r < A.n) {
-          acc[i] = A.psi0[r];
-          tb[r] = acc[i];
+          if (NT == 2) reinterpret_cast<float4*>(traj_smem)[r] = make_float4(v[0][i].x, v[0][i].y, v[NT - 1][i].x, v[NT - 1][i].y);
+          else reinterpret_cast<float2*>(traj_smem)[r] = v[0][i];
         }
       }
     }
-    sums(acc, b, 1);
-    if (tid < A.nobs) A.obs[(size_t)tid * A.ntraj + b] = res[2 + tid] / res[0];
+  };
+
+  for (int b = NT * blockIdx.x; b < A.ntraj; b += NT * gridDim.x) {
+    float2 acc[NT][kTrajRpt], t[NT][kTrajRpt];
+    // The sums of the new vectors and the next step's random numbers.  An odd ensemble's last CTA runs
+    // its trajectory twice.
+    auto sums = [&](int next) {
+      traj_block_sums<NT, 0>(A, M, acc, nq, res[0], 2 + kTrajMaxObs);
+      if (tid >= (int)blockDim.x - NT) {
+        const int a = tid - ((int)blockDim.x - NT);
+        double u1, u2;
+        philox_uniform2(A.seed, (uint32_t)min(b + a, A.ntraj - 1), (uint32_t)next, u1, u2);
+        s_u1[a] = u1;
+        s_u1f[a] = (float)u1;
+        s_u2[a] = u2;
+      }
+      __syncthreads();
+      // observables of the step before `next`
+      for (int x = tid; x < NT * A.nobs; x += (int)blockDim.x) {
+        const int a = x / A.nobs, k = x - a * A.nobs;
+        if (b + a < A.ntraj) A.obs[((size_t)(next - 1) * A.nobs + k) * A.ntraj + b + a] = res[a][2 + k] / res[a][0];
+      }
+    };
+#pragma unroll
+    for (int i = 0; i < kTrajRpt; ++i) {
+      const int s = warp + i * A.nwarps;
+      float2 v = make_float2(0.f, 0.f);
+      if (s < A.nsl) {
+        const int r = M.rid[32 * s + lane];
+        if (r < A.n) v = A.psi0[r];
+      }
+#pragma unroll
+      for (int a = 0; a < NT; ++a) acc[a][i] = v;
+    }
+    store(acc);
+    sums(1);
 
     for (int step = 1; step <= A.nsteps; ++step) {
-      // jump if u1 < gamma wtot dt.  In FP32 unless that is too close to tell: in FP64 one thread's
-      // conversions and division would hold the block up for 1,500 cycles
-      const float rate = gdt * (res[1] / res[0]);
-      bool jump = s_u1f < rate;
-      if (!(fabsf(s_u1f - rate) > 1e-5f * rate)) {  // and when something is not finite
-        const double wtot = (double)res[1] / (double)res[0];
-        jump = wtot > 0.0 && s_u1 < A.gamma * wtot * A.dt;
+      bool jump[NT], any = false, all = true;
+      float sc[NT];
+#pragma unroll
+      for (int a = 0; a < NT; ++a) {
+        // jump if u1 < gamma wtot dt.  In FP32 unless that is too close to tell: in FP64 one thread's
+        // conversions and division would hold the block up for 1,500 cycles
+        const float rate = gdt * (res[a][1] / res[a][0]);
+        jump[a] = s_u1f[a] < rate;
+        if (!(fabsf(s_u1f[a] - rate) > 1e-5f * rate)) {  // and when something is not finite
+          const double wtot = (double)res[a][1] / (double)res[a][0];
+          jump[a] = wtot > 0.0 && s_u1[a] < A.gamma * wtot * A.dt;
+        }
+        sc[a] = jump[a] ? 1.f : rsqrtf(res[a][0]);
+        any |= jump[a];
+        all &= jump[a];
       }
-      if (jump) {
-        // channel weights of the current state, then psi <- n_j psi (norm carried)
-        traj_block_sums<1>(A, M, acc, A.nchan, resc);
-        __syncthreads();
-        if (tid == 0) {
-          // bsearch on the cumulative weights normalised by their total: the channel j
-          // with wt[j] <= u2 < wt[j+1] (a scan gives the same index on a monotone table)
-          double tot = 0.0;
-          for (int j = 0; j < A.nchan; ++j) tot += (double)resc[j];
-          double cum = 0.0;
-          int ch = 0;
-          for (int j = 1; j < A.nchan; ++j) {
-            cum += (double)resc[j - 1];
-            if (cum / tot <= s_u2) ch = j;
-          }
-          s_jump = 1 + ch;
-          ++njumps;
-        }
-        __syncthreads();
-        const int bit = s_chan_bit[s_jump - 1];
-#pragma unroll
-        for (int i = 0; i < kTrajRpt; ++i) {
-          const int s = warp + i * A.nwarps;
-          if (s < A.nsl) {
-            const int slot = 32 * s + lane;
-            const int r = M.rid[slot];
-            if (r < A.n) {
-              if (!((M.st[slot] >> bit) & 1u)) acc[i] = make_float2(0.f, 0.f);
-              tb[cb * A.tb_len + r] = acc[i];
-            }
-          }
-        }
-      } else {
+      if (!all) {
         // psi <- exp(-i dt (H - mu)) psi / ||psi||: S sub-steps of K Taylor terms
-        const float sc = rsqrtf(res[0]);
         for (int sub = 0; sub < A.S; ++sub) {
-          if (sub == 0) {
 #pragma unroll
-            for (int i = 0; i < kTrajRpt; ++i) acc[i] = make_float2(acc[i].x * sc, acc[i].y * sc);
-          }
-          int rb = cb;
+          for (int a = 0; a < NT; ++a)
+#pragma unroll
+            for (int i = 0; i < kTrajRpt; ++i) {
+              t[a][i] = acc[a][i];  // t_0; times sc on the first sub-step, in the factor
+              if (sub == 0) acc[a][i] = make_float2(acc[a][i].x * sc[a], acc[a][i].y * sc[a]);
+            }
           for (int k = 1; k <= A.K; ++k) {
-            // t_k = (-i tau / k) (H - mu) t_{k-1}; t_0 = the vector in tb[cb] (times sc on the first sub-step)
-            const float f = A.tau / (float)k * ((sub == 0 && k == 1) ? sc : 1.f);
-            const float2* src = tb + rb * A.tb_len;
-            float2* dst = tb + (rb ^ 1) * A.tb_len;
-            // Two slices at a time (i and i + 1): their entry loads and gathers interleave, so a
-            // lane has four independent gathers in flight; each row keeps its own sums in entry
-            // order (even entries in s, odd ones in u).
-            auto at = [&](uint32_t c) { return *reinterpret_cast<const Pair*>(src + c); };
-            auto gather = [&](uint32_t pr, Pair& sp, Pair& up) {
-              const uint32_t ev = pr & 0xffffu, fv = pr >> 16;
-              if (kSigned) {
-                const float sg = __uint_as_float(0x3f800000u | ((ev & 0x8000u) << 16));
-                const float tg = __uint_as_float(0x3f800000u | ((fv & 0x8000u) << 16));
-                sp = pair_fma(sg, at(ev & 0x7fffu), sp);
-                up = pair_fma(tg, at(fv & 0x7fffu), up);
-              } else {  // every entry carries +c: plain sums
-                sp = pair_add(sp, at(ev));
-                up = pair_add(up, at(fv));
+            // t_k = (-i tau / k) (H - mu) t_{k-1}
+            float f[NT];
+#pragma unroll
+            for (int a = 0; a < NT; ++a)
+              f[a] = jump[a] ? 0.f : A.tau / (float)k * ((sub == 0 && k == 1) ? sc[a] : 1.f);
+            auto gather = [&](uint32_t c, uint32_t sign, Pair (&s)[NT]) {
+              Pair x[NT];
+              if (NT == 2) {
+                const ulonglong2 xx = reinterpret_cast<const ulonglong2*>(traj_smem)[c];
+                x[0] = xx.x;
+                x[NT - 1] = xx.y;
+              } else {
+                x[0] = reinterpret_cast<const Pair*>(traj_smem)[c];
               }
-            };
-            auto finish = [&](int i, int r, Pair sum) {
-              if (r < A.n) {
-                const float sx = pair_get(sum).x, sy = pair_get(sum).y;
-                const float2 o = src[r];
-                // v = c * sum + dg * own
-                const float vx = fmaf(A.coff.x, sx, fmaf(-A.coff.y, sy, fmaf(dg[i].x, o.x, -dg[i].y * o.y)));
-                const float vy = fmaf(A.coff.x, sy, fmaf(A.coff.y, sx, fmaf(dg[i].x, o.y, dg[i].y * o.x)));
-                // t = (-i f) v = (f vy, -f vx)
-                const float2 t = make_float2(f * vy, -f * vx);
-                dst[r] = t;
-                acc[i].x += t.x;
-                acc[i].y += t.y;
-              }
+              const float sg = __uint_as_float(0x3f800000u | sign);
+#pragma unroll
+              for (int a = 0; a < NT; ++a) s[a] = kSigned ? pair_fma(sg, x[a], s[a]) : pair_add(s[a], x[a]);
             };
 #pragma unroll
-            for (int i = 0; i < kTrajRpt; i += 2) {
-              const int s0 = warp + i * A.nwarps, s1 = s0 + A.nwarps;
-              if (s0 < A.nsl) {
-                const bool has1 = s1 < A.nsl;
-                const int2 d0 = M.sd[s0];
-                const int2 d1 = has1 ? M.sd[s1] : make_int2(0, 0);
-                const int r0 = M.rid[32 * s0 + lane];
-                const int r1 = has1 ? (int)M.rid[32 * s1 + lane] : A.n;
-                // a lane's entries 2j and 2j+1 share one 32-bit word (widths are even)
-                const uint32_t* e0 = reinterpret_cast<const uint32_t*>(M.ent + d0.x) + lane;
-                const uint32_t* e1 = reinterpret_cast<const uint32_t*>(M.ent + d1.x) + lane;
-                const int w0 = d0.y >> 1, w1 = d1.y >> 1;
-                Pair sp0 = 0, up0 = 0, sp1 = 0, up1 = 0;
-                const int wm = min(w0, w1);
-                int q = 0;
-                for (; q < wm; ++q) {
-                  const uint32_t p0 = e0[32 * q], p1 = e1[32 * q];
-                  gather(p0, sp0, up0);
-                  gather(p1, sp1, up1);
+            for (int i = 0; i < kTrajRpt; ++i) {
+              const int sl = warp + i * A.nwarps;
+              if (sl < A.nsl) {
+                const int2 d = M.sd[sl];
+                const float2 dg = __ldg(A.dg + 32 * sl + lane);
+                // a lane's entries 2j and 2j+1 share one 32-bit word (widths are even); even entries' sum
+                // in s, odd ones' in u, each in entry order
+                const uint32_t* e = reinterpret_cast<const uint32_t*>(M.ent + d.x) + lane;
+                const int w = d.y >> 1;
+                Pair s[NT], u[NT];
+#pragma unroll
+                for (int a = 0; a < NT; ++a) s[a] = u[a] = 0;
+#pragma unroll 2
+                for (int q = 0; q < w; ++q) {
+                  const uint32_t pr = e[32 * q];
+                  if (kSigned) {
+                    gather(pr & 0x7fffu, (pr & 0x8000u) << 16, s);
+                    gather((pr >> 16) & 0x7fffu, pr & 0x80000000u, u);
+                  } else {  // every entry carries +c: plain sums
+                    gather(pr & 0xffffu, 0u, s);
+                    gather(pr >> 16, 0u, u);
+                  }
                 }
-                for (int q0 = q; q0 < w0; ++q0) gather(e0[32 * q0], sp0, up0);
-                for (int q1 = q; q1 < w1; ++q1) gather(e1[32 * q1], sp1, up1);
-                finish(i, r0, pair_add(sp0, up0));
-                if (has1) finish(i + 1, r1, pair_add(sp1, up1));
+#pragma unroll
+                for (int a = 0; a < NT; ++a) {
+                  const float2 g = pair_get(pair_add(s[a], u[a]));
+                  const float2 o = t[a][i];
+                  // v = c * sum + dg * own; t = (-i f) v = (f vy, -f vx)
+                  const float vx = fmaf(A.coff.x, g.x, fmaf(-A.coff.y, g.y, fmaf(dg.x, o.x, -dg.y * o.y)));
+                  const float vy = fmaf(A.coff.x, g.y, fmaf(A.coff.y, g.x, fmaf(dg.x, o.y, dg.y * o.x)));
+                  t[a][i] = make_float2(__fmul_rn(f[a], vy), __fmul_rn(-f[a], vx));
+                  acc[a][i].x = __fadd_rn(acc[a][i].x, t[a][i].x);
+                  acc[a][i].y = __fadd_rn(acc[a][i].y, t[a][i].y);
+                }
               }
             }
-            __syncthreads();
-            rb ^= 1;
+            __syncthreads();  // every gather is done
+            if (k < A.K) {
+              store(t);
+              __syncthreads();
+            }
           }
-          // the sub-step's result into the buffer that held t_{K-1} (its readers are done)
-          cb = rb ^ 1;
+          if (sub + 1 < A.S) {
+            store(acc);
+            __syncthreads();
+          }
+        }
+      }
+      if (any) {
+        for (int a = 0; a < NT; ++a) {
+          if (!(NT == 2 && a == 1 ? jump[NT - 1] : jump[0])) continue;
+          // channel weights of the trajectory's vector, then psi <- n_j psi (norm carried)
+          float2 one[1][kTrajRpt];
+#pragma unroll
+          for (int i = 0; i < kTrajRpt; ++i) one[0][i] = (NT == 2 && a == 1) ? acc[NT - 1][i] : acc[0][i];
+          traj_block_sums<1, 1>(A, M, one, A.nchan, resc, 0);
+          __syncthreads();
+          if (tid == 0) {
+            // bsearch on the cumulative weights normalised by their total: the channel j
+            // with wt[j] <= u2 < wt[j+1] (a scan gives the same index on a monotone table)
+            double tot = 0.0;
+            for (int j = 0; j < A.nchan; ++j) tot += (double)resc[j];
+            double cum = 0.0;
+            int ch = 0;
+            for (int j = 1; j < A.nchan; ++j) {
+              cum += (double)resc[j - 1];
+              if (cum / tot <= s_u2[a]) ch = j;
+            }
+            s_chan = ch;
+            if (b + a < A.ntraj) ++njumps;
+          }
+          __syncthreads();
+          const int bit = s_chan_bit[s_chan];
 #pragma unroll
           for (int i = 0; i < kTrajRpt; ++i) {
             const int s = warp + i * A.nwarps;
-            if (s < A.nsl) {
-              const int r = M.rid[32 * s + lane];
-              if (r < A.n) tb[cb * A.tb_len + r] = acc[i];
+            if (s < A.nsl && !((M.st[32 * s + lane] >> bit) & 1u)) {
+              if (NT == 2 && a == 1) acc[NT - 1][i] = make_float2(0.f, 0.f);
+              else acc[0][i] = make_float2(0.f, 0.f);
             }
           }
-          __syncthreads();
+          __syncthreads();  // s_chan and the scratch are free
         }
       }
-      sums(acc, b, step + 1);
-      if (tid < A.nobs) A.obs[((size_t)step * A.nobs + tid) * A.ntraj + b] = res[2 + tid] / res[0];
+      store(acc);  // every reader of the buffer is past a barrier
+      sums(step + 1);
     }
+    __syncthreads();
   }
   if (tid == 0 && njumps) atomicAdd(A.jumps, njumps);
 }
@@ -415,10 +450,10 @@ struct TrajHostForm {
 };
 
 // Dynamic shared memory of the resident kernel for dim n, nsl slices and ent_len entries.
-static size_t traj_smem_bytes(int n, int nsl, int ent_len) {
+static size_t traj_smem_bytes(int n, int nsl, int ent_len, int nt = 1) {
   const size_t tb_len = (size_t)(n + 2) / 2 * 2;
   return 2 * tb_len * sizeof(float2) + (size_t)ent_len * 2 + (size_t)32 * nsl * 2 + (size_t)32 * nsl * 4 +
-         (size_t)(nsl + (nsl & 1)) * sizeof(int2) + (size_t)kTrajMaxWarps * kTrajRedStride * sizeof(float);
+         (size_t)(nsl + (nsl & 1)) * sizeof(int2) + (size_t)nt * kTrajMaxWarps * kTrajRedStride * sizeof(float);
 }
 
 static bool traj_build_resident(qd_ham* H, TrajHostForm& F, size_t max_smem) {
@@ -793,15 +828,32 @@ void traj_run(qd_ham* H, const qd_traj_desc& d, const double* psi0_host, double*
     A.psi0 = p0.p;
     A.obs = obs.p;
     A.jumps = jumps_dev.p;
-    const size_t smem = traj_smem_bytes(F.n, F.nsl, A.ent_len);
-    if (smem <= smem_cap) {
-      auto kern = F.any_neg ? traj_resident_kernel<true> : traj_resident_kernel<false>;
-      QD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (traj_smem_bytes(F.n, F.nsl, A.ent_len) <= smem_cap) {
       const int threads = 32 * F.nwarps;
-      int occ = 0;
-      QD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem));
-      QD_REQUIRE(occ >= 1, QD_ERR_UNSUPPORTED, "trajectory kernel does not fit an SM");
-      const int grid = (int)std::min<int64_t>(d.ntraj, (int64_t)occ * ctx->num_sms);
+      int nt = 1, grid = 0;
+      auto kern = F.any_neg ? traj_resident_kernel<1, true> : traj_resident_kernel<1, false>;
+      auto plan = [&] {
+        const size_t bytes = traj_smem_bytes(F.n, F.nsl, A.ent_len, nt);
+        if (bytes > smem_cap) return false;
+        allow_dynamic_smem(kern, ctx->device);
+        int occ = 0;
+        QD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, bytes));
+        grid = (int)std::min<int64_t>(ceil_div(d.ntraj, nt), (int64_t)occ * ctx->num_sms);
+        return occ >= 1;
+      };
+      QD_REQUIRE(plan(), QD_ERR_UNSUPPORTED, "trajectory kernel does not fit an SM");
+      if (d.ntraj > grid) {  // more trajectories than CTAs in flight: two a CTA take less than twice one's time
+        const auto one = kern;
+        const int grid1 = grid;
+        nt = 2;
+        kern = F.any_neg ? traj_resident_kernel<2, true> : traj_resident_kernel<2, false>;
+        if (!plan()) {
+          nt = 1;
+          kern = one;
+          grid = grid1;
+        }
+      }
+      const size_t smem = traj_smem_bytes(F.n, F.nsl, A.ent_len, nt);
       QD_CUDA(cudaEventRecord(e1, ctx->stream));
       kern<<<grid, threads, smem, ctx->stream>>>(A);
       QD_CHECK_LAUNCH();
