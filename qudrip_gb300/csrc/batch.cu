@@ -2,27 +2,25 @@
 //
 // The mixed-precision form of the reference's Lanczos (sparse_algorithm.hpp:
 // 395-425, 564-585) for a packed work list of independent, uneven instances:
-//   * small instances: one CTA owns one instance at a time and takes the next
-//     one from an atomic counter;
-//   * large instances (dim >= kClusterMinDim): a thread-block cluster of
-//     8, 4 or 2 CTAs owns one instance (per call, the largest size at which
-//     every large instance of the call is resident at once, else 2: more
-//     instances side by side beat wider clusters once the device is full, and
-//     an instance's bits depend on this size); each CTA keeps a slice of the rows
-//     of every vector, and the inner products are combined through
-//     distributed shared memory (each CTA adds the CTAs' partials in rank
-//     order, so every CTA holds the same bits) between hardware cluster
-//     barriers -- one SM's memory parallelism is far too little for an
-//     instance of 10^5 rows;
+//   * an instance is owned by one CTA or by a thread-block cluster of 2 to 8,
+//     by its dimension and the work of the call (batch_widths; an instance's
+//     bits depend on this size); CTAs and clusters take the next instance of
+//     their size from an atomic counter;
+//   * each CTA of a cluster keeps a slice of the rows of every vector, and the
+//     inner products are combined through distributed shared memory (each CTA
+//     adds the CTAs' partials in rank order, so every CTA holds the same bits)
+//     between hardware cluster barriers -- one SM's memory parallelism is far
+//     too little for an instance of 10^5 rows;
 //   * the lists are sorted by decreasing nnz (longest first);
 //   * matrix values and Krylov vectors are FP32 and so is the product;
 //   * every inner product keeps FP32 partial sums over at most 64 elements per
-//     thread and adds those partials in FP64 (threads, warps, blocks, CTAs);
+//     thread (16 in the Gram-Schmidt coefficients); a warp adds them exactly, in
+//     integers (f_fix), and warps, CTAs and tiles are added in FP64;
 //   * after the three-term step (the reference's local orthogonalisation
 //     against the two previous vectors) the new vector is orthogonalised
 //     once more against the whole stored basis (classical Gram-Schmidt);
-//   * the tridiagonal matrix (FP64) is solved on the device: eigenvalues by
-//     implicit QL, the lowest eigenvector by inverse iteration;
+//   * the tridiagonal matrix (FP64) is solved on the device by the block: the
+//     lowest eigenvalue by bisection, its vector by inverse iteration;
 //   * the Ritz vector gets one FP64 refinement: E = psi^T H psi / psi^T psi with
 //     the FP64 matrix values and FP64 accumulation.
 // No CTA spins on another: the only shared state is the work counter, and the
@@ -30,13 +28,25 @@
 // hardware schedules together and every CTA of a cluster reaches the same
 // number of times (the instance index and every stopping decision are the
 // same in all of them).
+//
+// Measured (GB300), 80 steps.  With the threads' partials added in FP64, the
+// step's scalars formed in every warp, a conversion of each coefficient in the
+// update's inner loop and QL on one thread, FP64 issue (72 cycles a warp
+// instruction, conversions included) set the time: 32 chains of 12, 14, 16 and
+// 18 sites 15.2, 16.3, 23.8 and 25.7 ms; now 1.3, 2.9, 3.9 and 11.8 ms, and 96
+// mixed chains of 14 to 18 sites 37.5 -> 15.8 ms.  At 18 sites on 8 CTAs a step
+// is 300,000 cycles: the product 100,000 (its gathers and the strided reads of
+// the columns), the coefficients 70,000 and the update 65,000 (HBM), the rest
+// the barriers' waits.
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <memory>
 #include <numeric>
+#include <string>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include <cooperative_groups.h>
@@ -53,6 +63,8 @@ constexpr int kBatchThreads = 512;  // two CTAs per SM
 constexpr int kBatchMaxSteps = 256;
 constexpr int kChunk = 64;  // FP32 partial sums cover at most this many elements
 constexpr int64_t kClusterMinDim = 32768;
+constexpr int64_t kBatchSplitMinDim = 8192;  // below it an instance stays on one CTA
+constexpr int64_t kBatchMinRows = 1024;      // slices are not made shorter
 
 constexpr int kWTile = 4096;  // elements of w staged in shared memory for the Gram-Schmidt coefficients
 
@@ -60,16 +72,23 @@ struct BlockScratch {
   float wt[kWTile];
   double red[kBatchThreads / 32];
   double red3[kBatchThreads / 32][3];
+  long long fq[3][kBatchThreads / 32];    // warps' integer sums and their exponents
+  unsigned fe[3][kBatchThreads / 32];
+  float fu[kBatchThreads / 32];
   double bcast;
   double bcast3[3];
   double xp[2], bc[2];                    // this CTA's partial of a cluster sum, and the sum
-  double xp3[2][3], bc3[2][3];
+  double xp3[2][3];
+  double al, bp;                          // the step's alpha and beta before the Gram-Schmidt pass
+  float c1, c2;                           // the same on the stored vectors
+  double ga, gb;                          // bracket of the lowest eigenvalue
+  unsigned gm[4];
   double hp[2][kBatchMaxSteps + 2];       // this CTA's partials of the Gram-Schmidt coefficients
   double alpha[kBatchMaxSteps + 2];
   double beta[kBatchMaxSteps + 2];
   double y[kBatchMaxSteps + 2];
   double h[kBatchMaxSteps + 2];
-  double c[kBatchMaxSteps + 2];           // update coefficients of the stored vectors
+  float cf[kBatchMaxSteps + 2];           // update coefficients of the stored vectors, negated; Ritz coefficients
   double scl[kBatchMaxSteps + 2];         // basis vector j is scl[j] * V[j] (V stored unnormalised)
   int stop;
   int idx;
@@ -80,6 +99,54 @@ __device__ __forceinline__ unsigned long long batch_clock_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
+}
+
+// ---- sums of FP32 partials in integers
+// An FP64 instruction takes an SM quarter 64 to 76 cycles whatever its active lanes, conversions included: the
+// FP64 sums of the threads' FP32 partials took several times the products that they summed.  A warp adds them as
+// integers instead, exact down to 2^-30 of the last place of the largest (2^-54 of it: FP64 rounds its sums at
+// 2^-53), and one conversion serves a warp's sum, or a lane each the sums of many vectors.
+__device__ __forceinline__ unsigned f_mag(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+// The exponent field of the largest magnitude word of a warp.
+__device__ __forceinline__ unsigned f_top(unsigned mag) { return max(__reduce_max_sync(0xffffffffu, mag) >> 23, 1u); }
+// v as an integer in units of 2^(e - 180), e at least its exponent field: below 2^54.
+__device__ __forceinline__ long long f_fix(float v, unsigned e) {
+  const unsigned b = __float_as_uint(v);
+  const unsigned ev = (b >> 23) & 0xffu;
+  const unsigned m = (b & 0x7fffffu) | (ev ? 0x800000u : 0u);
+  const int sh = 30 - (int)(e - max(ev, 1u));
+  const long long q = sh >= 0 ? (long long)m << sh : (long long)(m >> min(-sh, 31));
+  return (int)b < 0 ? -q : q;
+}
+__device__ __forceinline__ double f_unit(unsigned e) {  // NaN when a value was not finite
+  return e == 0xffu ? __longlong_as_double(0x7ff8000000000000ll) : __hiloint2double((int)(e + 843) << 20, 0);
+}
+__device__ __forceinline__ long long f_warp_sum(long long q) {  // at most 256 values
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+  return q;
+}
+// Block sums of NV values per thread into out (shared memory), complete after the caller's next barrier.
+template <int NV>
+__device__ __forceinline__ void block_sum_f(const float (&v)[NV], BlockScratch& S, double* out) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < NV; ++q) {
+    const unsigned e = f_top(f_mag(v[q]));
+    const long long t = f_warp_sum(f_fix(v[q], e));
+    if (lane == 0) {
+      S.fq[q][warp] = t;
+      S.fe[q][warp] = e;
+    }
+  }
+  __syncthreads();
+  if (warp < NV) {  // warps 0 .. NV - 1, each on its own SM quarter
+    constexpr int nw = kBatchThreads / 32;
+    double t = lane < nw ? (double)S.fq[warp][lane] * f_unit(S.fe[warp][lane]) : 0.0;
+#pragma unroll
+    for (int o = nw / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) out[warp] = t;
+  }
 }
 
 // FP64 sum over the block of per-thread values; every thread gets the result.
@@ -156,20 +223,40 @@ __device__ double block_dot(const float* __restrict__ a, const float* __restrict
 // chains of four gathers), each summed in its entry order.  x is a basis
 // vector written earlier in the same launch (by this CTA or, for a cluster, by
 // all of its CTAs), so it is read with ordinary loads, not the read-only path.
-__device__ __forceinline__ float row_f32(const BatchInst& I, const float* x, int64_t b, int64_t e) {
-  float acc = 0.f;
-  int64_t k = b;
-  for (; k + 4 <= e; k += 4) {
-    const int32_t c0 = I.colidx[k], c1 = I.colidx[k + 1], c2 = I.colidx[k + 2], c3 = I.colidx[k + 3];
-    const float v0 = I.vals_f[k], v1 = I.vals_f[k + 1], v2 = I.vals_f[k + 2], v3 = I.vals_f[k + 3];
-    const float x0 = x[c0], x1 = x[c1], x2 = x[c2], x3 = x[c3];
-    acc = fmaf(v0, x0, acc);
-    acc = fmaf(v1, x1, acc);
-    acc = fmaf(v2, x2, acc);
-    acc = fmaf(v3, x3, acc);
+template <bool kUniform>
+__device__ __forceinline__ void rows_f32(const BatchInst& I, const float* x, int64_t b0, int m0, int64_t b1, int m1,
+                                         float& a0, float& a1) {
+  const int32_t* c0 = I.colidx + b0;
+  const int32_t* c1 = I.colidx + b1;
+  const float* v0 = I.vals_f + b0;
+  const float* v1 = I.vals_f + b1;
+  const int m = max(m0, m1);
+  for (int k = 0; k < m; k += 4) {  // eight gathers in flight, also over the ends of the rows
+    int32_t c[8];
+    float v[8], xv[8];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool p0 = k + u < m0, p1 = k + u < m1;
+      c[u] = p0 ? c0[k + u] : -1;
+      c[4 + u] = p1 ? c1[k + u] : -1;
+      if (!kUniform) {
+        v[u] = p0 ? v0[k + u] : 0.f;
+        v[4 + u] = p1 ? v1[k + u] : 0.f;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) xv[u] = c[u] >= 0 ? x[c[u]] : 0.f;
+    if (kUniform) {
+      a0 += (xv[0] + xv[1]) + (xv[2] + xv[3]);
+      a1 += (xv[4] + xv[5]) + (xv[6] + xv[7]);
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        a0 = fmaf(v[u], xv[u], a0);
+        a1 = fmaf(v[4 + u], xv[4 + u], a1);
+      }
+    }
   }
-  for (; k < e; ++k) acc = fmaf(I.vals_f[k], x[I.colidx[k]], acc);
-  return acc;
 }
 
 // The product of the step and, row by row as it is formed, this thread's
@@ -198,82 +285,28 @@ struct ProdDots {
   }
 };
 
-// The same product when every off-diagonal value is one c (uniform hopping, any
-// diagonal): y_r = c (sum of x over the row's stored columns) + e_r x_r with
-// e_r = d_r - c where the row stores its diagonal (else 0), the column indices
-// the only per-entry reads (no values).
-__device__ void block_spmv_f32_uniform(const BatchInst& I, const float* x, const float* v2, float* __restrict__ y,
-                                       int64_t lo, int64_t hi, ProdDots& pd) {
-  const float c = __ldg(I.coff);
+// kUniform: every off-diagonal value is one c (uniform hopping, any diagonal): y_r = c (sum of x over the
+// row's stored columns) + e_r x_r with e_r = d_r - c where the row stores its diagonal (else 0), the column
+// indices the only per-entry reads (no values).
+template <bool kUniform>
+__device__ void block_spmv_f32(const BatchInst& I, const float* x, const float* v2, float* __restrict__ y, int64_t lo,
+                               int64_t hi, ProdDots& pd) {
+  const float c = kUniform ? __ldg(I.coff) : 0.f;
   const int64_t bs = blockDim.x;
-  int64_t r = lo + threadIdx.x;
   auto finish = [&](int64_t row, float sum) {
-    const float yr = fmaf(c, sum, __ldg(I.diag_f + row) * x[row]);
+    const float yr = kUniform ? fmaf(c, sum, __ldg(I.diag_f + row) * x[row]) : sum;
     y[row] = yr;
     pd.add(x, v2, row, yr);
   };
-  for (; r + bs < hi; r += 2 * bs) {
-    const int64_t b0 = I.rowptr[r], e0 = I.rowptr[r + 1], b1 = I.rowptr[r + bs], e1 = I.rowptr[r + bs + 1];
+  for (int64_t r = lo + threadIdx.x; r < hi; r += 2 * bs) {
+    const bool two = r + bs < hi;
+    const int64_t b0 = I.rowptr[r], b1 = two ? I.rowptr[r + bs] : b0;
+    const int m0 = (int)(I.rowptr[r + 1] - b0), m1 = two ? (int)(I.rowptr[r + bs + 1] - b1) : 0;
     float a0 = 0.f, a1 = 0.f;
-    int64_t k0 = b0, k1 = b1;
-    for (; k0 + 4 <= e0 && k1 + 4 <= e1; k0 += 4, k1 += 4) {  // eight gathers in flight
-      const int32_t c0 = I.colidx[k0], c1 = I.colidx[k0 + 1], c2 = I.colidx[k0 + 2], c3 = I.colidx[k0 + 3];
-      const int32_t d0 = I.colidx[k1], d1 = I.colidx[k1 + 1], d2 = I.colidx[k1 + 2], d3 = I.colidx[k1 + 3];
-      a0 += (x[c0] + x[c1]) + (x[c2] + x[c3]);
-      a1 += (x[d0] + x[d1]) + (x[d2] + x[d3]);
-    }
-    for (; k0 < e0; ++k0) a0 += x[I.colidx[k0]];
-    for (; k1 < e1; ++k1) a1 += x[I.colidx[k1]];
+    rows_f32<kUniform>(I, x, b0, m0, b1, m1, a0, a1);
     finish(r, a0);
-    finish(r + bs, a1);
+    if (two) finish(r + bs, a1);
   }
-  if (r < hi) {
-    float a0 = 0.f;
-    for (int64_t k = I.rowptr[r]; k < I.rowptr[r + 1]; ++k) a0 += x[I.colidx[k]];
-    finish(r, a0);
-  }
-  pd.flush();
-}
-
-__device__ void block_spmv_f32(const BatchInst& I, const float* x, const float* v2, float* __restrict__ y, int64_t lo,
-                               int64_t hi, ProdDots& pd) {
-  const int64_t bs = blockDim.x;
-  int64_t r = lo + threadIdx.x;
-  for (; r + bs < hi; r += 2 * bs) {
-    const int64_t b0 = I.rowptr[r], e0 = I.rowptr[r + 1], b1 = I.rowptr[r + bs], e1 = I.rowptr[r + bs + 1];
-    // the two rows' groups of four interleaved: eight gathers in flight
-    float a0 = 0.f, a1 = 0.f;
-    int64_t k0 = b0, k1 = b1;
-    for (; k0 + 4 <= e0 && k1 + 4 <= e1; k0 += 4, k1 += 4) {
-      const int32_t c0 = I.colidx[k0], c1 = I.colidx[k0 + 1], c2 = I.colidx[k0 + 2], c3 = I.colidx[k0 + 3];
-      const int32_t d0 = I.colidx[k1], d1 = I.colidx[k1 + 1], d2 = I.colidx[k1 + 2], d3 = I.colidx[k1 + 3];
-      const float v0 = I.vals_f[k0], v1 = I.vals_f[k0 + 1], w2 = I.vals_f[k0 + 2], v3 = I.vals_f[k0 + 3];
-      const float u0 = I.vals_f[k1], u1 = I.vals_f[k1 + 1], u2 = I.vals_f[k1 + 2], u3 = I.vals_f[k1 + 3];
-      const float x0 = x[c0], x1 = x[c1], x2 = x[c2], x3 = x[c3];
-      const float z0 = x[d0], z1 = x[d1], z2 = x[d2], z3 = x[d3];
-      a0 = fmaf(v0, x0, a0);
-      a0 = fmaf(v1, x1, a0);
-      a0 = fmaf(w2, x2, a0);
-      a0 = fmaf(v3, x3, a0);
-      a1 = fmaf(u0, z0, a1);
-      a1 = fmaf(u1, z1, a1);
-      a1 = fmaf(u2, z2, a1);
-      a1 = fmaf(u3, z3, a1);
-    }
-    // the rest of each row, continuing its sum in entry order
-    for (; k0 < e0; ++k0) a0 = fmaf(I.vals_f[k0], x[I.colidx[k0]], a0);
-    for (; k1 < e1; ++k1) a1 = fmaf(I.vals_f[k1], x[I.colidx[k1]], a1);
-    y[r] = a0;
-    y[r + bs] = a1;
-    pd.add(x, v2, r, a0);
-    pd.add(x, v2, r + bs, a1);
-  }
-  if (r < hi) {
-    const float a0 = row_f32(I, x, I.rowptr[r], I.rowptr[r + 1]);
-    y[r] = a0;
-    pd.add(x, v2, r, a0);
-  }
-  pd.flush();
 }
 
 // ---------------------------------------------------------------- uniform check
@@ -394,107 +427,197 @@ __device__ double inst_sum(double block_total, BlockScratch& S, int& buf) {
   }
 }
 
-// The instance totals of three block totals (one cluster barrier).
-template <int C>
-__device__ void inst_sum3(double (&v)[3], BlockScratch& S, int& buf) {
-  if constexpr (C > 1) {
-    cg::cluster_group cl = cg::this_cluster();
-    if (threadIdx.x == 0) {
-#pragma unroll
-      for (int q = 0; q < 3; ++q) S.xp3[buf][q] = v[q];
+// Lowest eigenpair of tridiag(d, e) (n <= kBatchMaxSteps), by the whole block: the eigenvalue by bisection
+// (128 points a round, a warp on each SM quarter: is any leading minor of T - x not positive?), the vector by
+// three steps of inverse iteration with partial pivoting (the reorthogonalised Lanczos matrix has no spurious
+// copies).  Eigenvalues by QL and the same iteration on one thread took 5 ms at n = 80, FP64 instructions
+// taking 72 cycles each.
+constexpr int kTriWork = kBatchMaxSteps + 2;
+__device__ double block_tridiag_lowest(int n, const double* d, const double* e, double* y, BlockScratch& S) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __syncthreads();
+  double* work = reinterpret_cast<double*>(S.wt);  // the tile of w is free
+  static_assert(sizeof(float) * kWTile >= 7 * sizeof(double) * kTriWork, "scratch");
+  double *dl = work, *dd = dl + kTriWork, *du = dd + kTriWork, *du2 = du + kTriWork, *rd = du2 + kTriWork,
+         *e2 = rd + kTriWork;
+  int* piv = reinterpret_cast<int*>(e2 + kTriWork);
+  if (warp == 0) {
+    double glo = 1e300, dmin = 1e300;
+    for (int i = lane; i < n; i += 32) {
+      const double el = i > 0 ? fabs(e[i - 1]) : 0.0, er = i + 1 < n ? fabs(e[i]) : 0.0;
+      glo = fmin(glo, d[i] - (el + er));
+      dmin = fmin(dmin, d[i]);
+      e2[i] = er * er;
     }
-    cl.sync();
-    if (threadIdx.x < 3) {
-      double t = 0.0;
-      for (int r = 0; r < C; ++r) t += cl.map_shared_rank(&S.xp3[buf][0], r)[threadIdx.x];
-      S.bc3[buf][threadIdx.x] = t;
+    for (int o = 16; o > 0; o >>= 1) {
+      glo = fmin(glo, __shfl_xor_sync(0xffffffffu, glo, o));
+      dmin = fmin(dmin, __shfl_xor_sync(0xffffffffu, dmin, o));
     }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 3; ++q) v[q] = S.bc3[buf][q];
-    buf ^= 1;
+    if (lane == 0) {  // the lowest eigenvalue is at most the least diagonal element
+      S.ga = glo - 1e-15 * fabs(glo);
+      S.gb = dmin;
+    }
   }
-}
-
-// Lowest eigenpair of tridiag(d, e) (n <= kBatchMaxSteps), one thread:
-// eigenvalues by QL, eigenvector by two steps of inverse iteration with
-// partial pivoting (the reorthogonalised Lanczos matrix has no spurious copies).
-__device__ double device_tridiag_lowest(int n, const double* d_in, const double* e_in, double* y, double* work) {
-  double* d = work;
-  double* e = work + (kBatchMaxSteps + 2);
-  for (int i = 0; i < n; ++i) {
-    d[i] = d_in[i];
-    e[i] = (i + 1 < n) ? e_in[i] : 0.0;
-  }
-  tridiag_ql<double>(n, d, e, nullptr, 0);
-  const double lam = d[0];
-  // (T - sigma I) y = b, sigma just below lam; Gaussian elimination with
-  // partial pivoting on the tridiagonal band (three diagonals + fill-in)
-  double* dl = work + 2 * (kBatchMaxSteps + 2);
-  double* dd = work + 3 * (kBatchMaxSteps + 2);
-  double* du = work + 4 * (kBatchMaxSteps + 2);
-  double* du2 = work + 5 * (kBatchMaxSteps + 2);
-  int* piv = reinterpret_cast<int*>(work + 6 * (kBatchMaxSteps + 2));
-  const double scale = fmax(fabs(lam), 1.0);
-  const double sigma = lam - 1e-10 * scale;
-  for (int i = 0; i < n; ++i) y[i] = 1.0;
-  for (int it = 0; it < 3; ++it) {
-    for (int i = 0; i < n; ++i) {
-      dd[i] = d_in[i] - sigma;
-      du[i] = (i + 1 < n) ? e_in[i] : 0.0;
-      dl[i] = (i + 1 < n) ? e_in[i] : 0.0;
-      du2[i] = 0.0;
-    }
-    // factor
-    for (int i = 0; i < n - 1; ++i) {
-      if (fabs(dd[i]) >= fabs(dl[i])) {
-        piv[i] = i;
-        const double f = (dd[i] != 0.0) ? dl[i] / dd[i] : 0.0;
-        dl[i] = f;
-        dd[i + 1] -= f * du[i];
-      } else {
-        piv[i] = i + 1;
-        const double f = dd[i] / dl[i];
-        dd[i] = dl[i];
-        dl[i] = f;
-        const double t = du[i];
-        du[i] = dd[i + 1];
-        dd[i + 1] = t - f * dd[i + 1];
-        if (i < n - 2) {
-          du2[i] = du[i + 1];
-          du[i + 1] = -f * du[i + 1];
+  __syncthreads();
+  for (int round = 0; round < 9; ++round) {  // 128^9 = 2^63
+    const double a = S.ga, b = S.gb;
+    bool has = true;
+    if (threadIdx.x < 127) {
+      const double x = fma(b - a, (double)(threadIdx.x + 1) * 0.0078125, a);
+      double p0 = 1.0, p1 = d[0] - x;
+      has = !(p1 > 0.0);
+      for (int i = 1; i < n; ++i) {
+        const double p2 = fma(d[i] - x, p1, -e2[i - 1] * p0);
+        has |= !(p2 > 0.0);
+        p0 = p1;
+        p1 = p2;
+        if ((i & 3) == 0) {  // p1 back to [1, 2), p0 with it
+          const int sh = ((__double2hiint(p1) >> 20) & 0x7ff) - 1023, e0 = (__double2hiint(p0) >> 20) & 0x7ff;
+          p0 = e0 - sh > 0 && e0 - sh < 2047 ? __hiloint2double(__double2hiint(p0) - sh * (1 << 20), __double2loint(p0))
+                                             : 0.0;
+          p1 = __hiloint2double(__double2hiint(p1) - sh * (1 << 20), __double2loint(p1));
         }
       }
     }
-    // solve L U x = P b
-    for (int i = 0; i < n - 1; ++i) {
-      if (piv[i] == i) {
-        y[i + 1] -= dl[i] * y[i];
-      } else {
-        const double t = y[i];
-        y[i] = y[i + 1];
-        y[i + 1] = t - dl[i] * y[i + 1];
+    if (warp < 4) {
+      const unsigned m = __ballot_sync(0xffffffffu, has);
+      if (lane == 0) S.gm[warp] = m;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      int t = 0;  // the first point with an eigenvalue below it (the last, b, at least)
+      for (; t < 127 && !((S.gm[t >> 5] >> (t & 31)) & 1u); t = (S.gm[t >> 5] >> (t & 31)) ? t + 1 : (t | 31) + 1) {
+      }
+      if (t < 127) S.gb = fma(b - a, (double)(t + 1) * 0.0078125, a);
+      if (t > 0) S.ga = fma(b - a, (double)t * 0.0078125, a);
+    }
+    __syncthreads();
+  }
+  const double lam = S.gb;
+  // (T - sigma I) y = b, sigma just below lam; Gaussian elimination with partial pivoting on the
+  // tridiagonal band (three diagonals + fill-in), factored once
+  if (warp == 0) {
+    const double sigma = lam - 1e-10 * fmax(fabs(lam), 1.0);
+    for (int i = lane; i < n; i += 32) {
+      dd[i] = d[i] - sigma;
+      du[i] = dl[i] = (i + 1 < n) ? e[i] : 0.0;
+      du2[i] = 0.0;
+      y[i] = 1.0;
+    }
+    __syncwarp();
+    if (lane == 0) {
+      for (int i = 0; i < n - 1; ++i) {
+        if (fabs(dd[i]) >= fabs(dl[i])) {
+          piv[i] = i;
+          const double f = (dd[i] != 0.0) ? dl[i] / dd[i] : 0.0;
+          dl[i] = f;
+          dd[i + 1] -= f * du[i];
+        } else {
+          piv[i] = i + 1;
+          const double f = dd[i] / dl[i];
+          dd[i] = dl[i];
+          dl[i] = f;
+          const double t = du[i];
+          du[i] = dd[i + 1];
+          dd[i + 1] = t - f * dd[i + 1];
+          if (i < n - 2) {
+            du2[i] = du[i + 1];
+            du[i + 1] = -f * du[i + 1];
+          }
+        }
       }
     }
-    for (int i = n - 1; i >= 0; --i) {
-      double s = y[i];
-      if (i + 1 < n) s -= du[i] * y[i + 1];
-      if (i + 2 < n) s -= du2[i] * y[i + 2];
-      const double p = (dd[i] != 0.0) ? dd[i] : 1e-300;
-      y[i] = s / p;
+    __syncwarp();
+    for (int i = lane; i < n; i += 32) rd[i] = 1.0 / ((dd[i] != 0.0) ? dd[i] : 1e-300);
+    __syncwarp();
+    for (int it = 0; it < 3; ++it) {
+      if (lane == 0) {  // solve L U x = P b
+        double yi = y[0];
+        for (int i = 0; i < n - 1; ++i) {
+          const double yn = y[i + 1];
+          if (piv[i] == i) {
+            y[i] = yi;
+            yi = yn - dl[i] * yi;
+          } else {
+            y[i] = yn;
+            yi = yi - dl[i] * yn;
+          }
+        }
+        double y1 = 0.0, y2 = 0.0;  // y[i + 1], y[i + 2]
+        for (int i = n - 1; i >= 0; --i) {
+          double v = (i == n - 1) ? yi : y[i];
+          v = (v - du[i] * y1 - du2[i] * y2) * rd[i];
+          y[i] = v;
+          y2 = y1;
+          y1 = v;
+        }
+      }
+      __syncwarp();
+      double nr = 0.0;
+      for (int i = lane; i < n; i += 32) nr += y[i] * y[i];
+      for (int o = 16; o > 0; o >>= 1) nr += __shfl_xor_sync(0xffffffffu, nr, o);
+      nr = 1.0 / sqrt(nr);
+      for (int i = lane; i < n; i += 32) y[i] *= nr;
+      __syncwarp();
     }
-    double nr = 0.0;
-    for (int i = 0; i < n; ++i) nr += y[i] * y[i];
-    nr = sqrt(nr);
-    for (int i = 0; i < n; ++i) y[i] /= nr;
   }
+  __syncthreads();
   return lam;
 }
 
+// float4s on their way to a thread's own slots of a ring, kBatchRing deep: rows of `per` blocks of 32 float4s,
+// `left` of them, `stride` floats apart; lane l takes float4 l of each block, zeros from float4 `len` of a row on.
+constexpr int kBatchRing = 8;
+constexpr size_t kBatchRingBytes = (size_t)kBatchThreads * kBatchRing * sizeof(float4);
+struct BatchStream {
+  const float* p;  // the row
+  int64_t stride;
+  unsigned base, in, out;
+  int per, b, left, len;
+  __device__ __forceinline__ void fetch() {
+    if (left > 0) {
+      const int i = 32 * b + (int)(threadIdx.x & 31);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + in), "l"(p + 4 * (i < len ? i : 0)),
+                   "r"(i < len ? 16 : 0)
+                   : "memory");
+      if (++b == per) {
+        b = 0;
+        p += stride;
+        --left;
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    in = (in + 16 * kBatchThreads) & (unsigned)(kBatchRingBytes - 1);
+  }
+  __device__ __forceinline__ void begin(const float* rows, int64_t st, int count, int blocks, int length, float4* slot) {
+    p = rows;
+    stride = st;
+    left = count;
+    per = blocks;
+    len = length;
+    b = 0;
+    base = (unsigned)__cvta_generic_to_shared(slot);
+    in = out = 0;
+#pragma unroll
+    for (int i = 0; i < kBatchRing - 1; ++i) fetch();
+  }
+  __device__ __forceinline__ float4 next() {
+    fetch();  // into the slot that the float4 before left
+    asm volatile("cp.async.wait_group %0;" ::"n"(kBatchRing - 1) : "memory");
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(base + out));
+    out = (out + 16 * kBatchThreads) & (unsigned)(kBatchRingBytes - 1);
+    return v;
+  }
+};
+
 template <int C>
 __global__ void __launch_bounds__(kBatchThreads, 2) batch_lanczos_kernel(const BatchInst* __restrict__ list, int ninst,
-                                                                     unsigned* counter, double* tri_work) {
+                                                                     unsigned* counter) {
   __shared__ BlockScratch S;
+  extern __shared__ __align__(16) float4 batch_ring[];  // C > 1
   int rank = 0;
   if constexpr (C > 1) rank = (int)cg::this_cluster().block_rank();
   int buf = 0, hbuf = 0;
@@ -519,6 +642,11 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batch_lanczos_kernel(const B
     const double nrm0 = sqrt(inst_sum<C>(block_dot(I.v0, I.v0, lo, hi, S), S, buf));
     const float inv0 = (float)(1.0 / nrm0);
     for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) V[i] = I.v0[i] * inv0;
+    // the last float4s of the vectors are read whole: zeros past the end
+    const int64_t pad = (hi == n && lo < n) ? I.ld : hi;
+    for (int64_t i = hi + threadIdx.x; i < pad; i += blockDim.x) V[i] = 0.f;
+    // so few rows a thread that none of its FP32 partials spans more than kChunk elements
+    const bool few = per <= (int64_t)(kChunk - 4) * kBatchThreads;
     if (threadIdx.x == 0) {
       S.stop = 0;
       S.scl[0] = 1.0;
@@ -532,19 +660,49 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batch_lanczos_kernel(const B
     for (int k = 1; k <= I.steps; ++k) {
       const float* v1 = V + (int64_t)(k - 1) * I.ld;
       const float* v2 = (k >= 2) ? V + (int64_t)(k - 2) * I.ld : nullptr;
-      const double s1 = S.scl[k - 1], s2 = (k >= 2) ? S.scl[k - 2] : 0.0;
       ProdDots pd;
-      if (uni) block_spmv_f32_uniform(I, v1, v2, w, lo, hi, pd);
-      else block_spmv_f32(I, v1, v2, w, lo, hi, pd);
-      double d3[3] = {pd.da, pd.db, pd.dc};
-      block_sum_all3(d3, S);
-      inst_sum3<C>(d3, S, buf);
-      // bp = <v2, w>, al = <v1, w - bp v2> in the true (normalised) vectors
-      const double bp = v2 ? s2 * s1 * d3[0] : 0.0;
-      const double al = s1 * (s1 * d3[1] - bp * s2 * d3[2]);
-      const float c2 = v2 ? (float)(bp * s2 / s1) : 0.f, c1 = (float)al;
+      if (uni) block_spmv_f32<true>(I, v1, v2, w, lo, hi, pd);
+      else block_spmv_f32<false>(I, v1, v2, w, lo, hi, pd);
+      // <V2, y>, <V1, y>, <V1, V2> of the instance; the scalars of the step on one thread
+      double* d3 = S.xp3[buf];
+      if (few) {
+        const float f3[3] = {pd.fa, pd.fb, pd.fc};
+        block_sum_f<3>(f3, S, d3);
+      } else {
+        pd.flush();
+        double t3[3] = {pd.da, pd.db, pd.dc};
+        block_sum_all3(t3, S);
+        if (threadIdx.x < 3) d3[threadIdx.x] = threadIdx.x == 0 ? t3[0] : threadIdx.x == 1 ? t3[1] : t3[2];
+      }
+      inst_sync<C>();
+      if (threadIdx.x < 32) {
+        double t = 0.0;
+        if constexpr (C > 1) {
+          if (threadIdx.x < 3)
+#pragma unroll 1
+            for (int r = 0; r < C; ++r) t += cg::this_cluster().map_shared_rank(&S.xp3[buf][0], r)[threadIdx.x];
+        } else {
+          if (threadIdx.x < 3) t = d3[threadIdx.x];
+        }
+        const double ta = __shfl_sync(0xffffffffu, t, 0), tb = __shfl_sync(0xffffffffu, t, 1),
+                     tc = __shfl_sync(0xffffffffu, t, 2);
+        // bp = <v2, w>, al = <v1, w - bp v2> in the true (normalised) vectors
+        const double s1 = S.scl[k - 1], s2 = (k >= 2) ? S.scl[k - 2] : 0.0;
+        const double bp = v2 ? s2 * s1 * ta : 0.0;
+        const double al = s1 * (s1 * tb - bp * s2 * tc);
+        if (threadIdx.x == 0) {
+          S.bp = bp;
+          S.al = al;
+          S.c1 = (float)al;
+          S.c2 = (float)(s2 * s2 * ta);
+        }
+      }
+      buf ^= 1;
+      __syncthreads();
+      const float c2 = v2 ? S.c2 : 0.f, c1 = S.c1;
       // one full Gram-Schmidt pass against v_0 .. v_{k-1}
-      double nacc = 0.0;  // this thread's share of the stored V[k]'s squared norm
+      double nacc = 0.0;  // this thread's share of the stored V[k]'s squared norm, but for its last FP32 partial
+      float nshare = 0.f;
       float tk = 1.f;     // the power of two V[k] is stored with
       {
         const int64_t q0 = lo >> 2, q1 = hi >> 2;
@@ -554,13 +712,12 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batch_lanczos_kernel(const B
         // tile, eight float4 of V_j in flight per lane
         {
           const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-          for (int j = threadIdx.x; j <= k; j += blockDim.x) part[j] = 0.0;
-          double uacc = 0.0;
+          float uf = 0.f;     // ||u||^2, for its exponent alone
+          double gacc = 0.0;  // lane i: vector warp + nw i
           for (int64_t t0 = lo; t0 < hi; t0 += kWTile) {
             const int tn = (int)std::min<int64_t>(hi - t0, kWTile);
-            const int nq = tn >> 2;  // t0 is a multiple of 32: float4-aligned
-            __syncthreads();  // the previous tile's readers are done (and part is zeroed)
-            float uf = 0.f;
+            const int nq = tn >> 2, nq4 = (tn + 3) >> 2;  // t0 is a multiple of 32: float4-aligned
+            __syncthreads();  // the previous tile's readers are done
             for (int i = threadIdx.x; i < nq; i += blockDim.x) {
               float4 u = reinterpret_cast<const float4*>(w + t0)[i];
               const float4 p1 = reinterpret_cast<const float4*>(v1 + t0)[i];
@@ -582,68 +739,98 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batch_lanczos_kernel(const B
               uf = fmaf(u.z, u.z, uf);
               uf = fmaf(u.w, u.w, uf);
             }
-            for (int i = (nq << 2) + threadIdx.x; i < tn; i += blockDim.x) {
-              float u = w[t0 + i];
-              if (v2) u = fmaf(-c2, v2[t0 + i], u);
-              u = fmaf(-c1, v1[t0 + i], u);
+            for (int i = (nq << 2) + threadIdx.x; i < kWTile; i += blockDim.x) {  // the end of the rows, then zeros
+              float u = 0.f;
+              if (i < tn) {
+                u = w[t0 + i];
+                if (v2) u = fmaf(-c2, v2[t0 + i], u);
+                u = fmaf(-c1, v1[t0 + i], u);
+                w[t0 + i] = u;
+                uf = fmaf(u, u, uf);
+              }
               S.wt[i] = u;
-              w[t0 + i] = u;
-              uf = fmaf(u, u, uf);
             }
-            uacc += (double)uf;  // at most kWTile / blockDim.x = 8 elements per thread per tile
             __syncthreads();
             const float4* ws4 = reinterpret_cast<const float4*>(S.wt);
-            for (int j = warp; j < k; j += nw) {
-              const float* vj = V + (int64_t)j * I.ld + t0;
-              const float4* vj4 = reinterpret_cast<const float4*>(vj);
-              double dacc = 0.0;
-              float acc = 0.f;
-              int i = lane;
-              for (; i + 224 < nq; i += 256) {  // 8 float4 per lane: 128 elements in two FP32 chunks
-                float4 x[8];
+            long long qs = 0;
+            unsigned es = 1;
+            int mine = 0;
+            // clusters: the vectors' float4s of the tile come through a ring of asynchronous copies that each thread
+            // reads back itself, vector after vector, kBatchRing of them in flight
+            const int nc = (nq4 + 127) >> 7;
+            BatchStream ring;
+            if constexpr (C > 1)
+              ring.begin(V + (int64_t)warp * I.ld + t0, (int64_t)nw * I.ld, warp < k ? (k - warp + nw - 1) / nw : 0, 4 * nc,
+                         nq4, batch_ring + threadIdx.x);
+            for (int j = warp; j < k; j += nw, ++mine) {
+              float c[kWTile / 512];  // FP32 over 16 elements
+              unsigned mag = 0;
+              if constexpr (C > 1) {
 #pragma unroll
-                for (int q = 0; q < 8; ++q) x[q] = vj4[i + 32 * q];
+                for (int h = 0; h < kWTile / 512; ++h) {
+                  c[h] = 0.f;
+                  if (h < nc) {
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                  const float4 y = ws4[i + 32 * q];
-                  acc = fmaf(x[q].x, y.x, acc);
-                  acc = fmaf(x[q].y, y.y, acc);
-                  acc = fmaf(x[q].z, y.z, acc);
-                  acc = fmaf(x[q].w, y.w, acc);
-                  if (q == 3 || q == 7) {
-                    dacc += (double)acc;
-                    acc = 0.f;
+                    for (int q = 0; q < 4; ++q) {
+                      const float4 x = ring.next();
+                      const float4 y = ws4[128 * h + 32 * q + lane];
+                      c[h] = fmaf(x.x, y.x, c[h]);
+                      c[h] = fmaf(x.y, y.y, c[h]);
+                      c[h] = fmaf(x.z, y.z, c[h]);
+                      c[h] = fmaf(x.w, y.w, c[h]);
+                    }
+                    mag = max(mag, f_mag(c[h]));
+                  }
+                }
+              } else {
+                const float4* vj4 = reinterpret_cast<const float4*>(V + (int64_t)j * I.ld + t0);
+#pragma unroll
+                for (int h = 0; h < kWTile / 1024; ++h) {
+                  c[2 * h] = c[2 * h + 1] = 0.f;
+                  if (256 * h < nq4) {
+                    float4 x[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                      const int i = 256 * h + 32 * q + lane;
+                      x[q] = i < nq4 ? vj4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                      const float4 y = ws4[256 * h + 32 * q + lane];
+                      float acc = c[2 * h + (q >> 2)];
+                      acc = fmaf(x[q].x, y.x, acc);
+                      acc = fmaf(x[q].y, y.y, acc);
+                      acc = fmaf(x[q].z, y.z, acc);
+                      acc = fmaf(x[q].w, y.w, acc);
+                      c[2 * h + (q >> 2)] = acc;
+                    }
+                    mag = max(mag, max(f_mag(c[2 * h]), f_mag(c[2 * h + 1])));
                   }
                 }
               }
-              int cnt = 0;
-              for (; i < nq; i += 32) {
-                const float4 x = vj4[i], y = ws4[i];
-                acc = fmaf(x.x, y.x, acc);
-                acc = fmaf(x.y, y.y, acc);
-                acc = fmaf(x.z, y.z, acc);
-                acc = fmaf(x.w, y.w, acc);
-                if (++cnt == kChunk / 4) {
-                  dacc += (double)acc;
-                  acc = 0.f;
-                  cnt = 0;
-                }
+              const unsigned e = f_top(mag);
+              long long t = 0;
+#pragma unroll
+              for (int h = 0; h < kWTile / 512; ++h)
+                if (h < nc) t += f_fix(c[h], e);
+              t = f_warp_sum(t);
+              if (lane == mine) {
+                qs = t;
+                es = e;
               }
-              for (int ii = (nq << 2) + lane; ii < tn; ii += 32) acc = fmaf(vj[ii], S.wt[ii], acc);
-              dacc += (double)acc;
-              dacc = warp_sum0(dacc);
-              if (lane == 0) part[j] += dacc;  // tile by tile, in order: the same bits in every run
             }
+            gacc = fma((double)qs, f_unit(es), gacc);  // tile by tile, in order: the same bits in every run
           }
+          if (warp + nw * lane < k) part[warp + nw * lane] = gacc;
           // ||u||^2 of this CTA's rows into part[k]
-          uacc = warp_sum0(uacc);
-          __syncthreads();
-          if (lane == 0) S.red[warp] = uacc;
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) uf += __shfl_xor_sync(0xffffffffu, uf, o);
+          if (lane == 0) S.fu[warp] = uf;
           __syncthreads();
           if (threadIdx.x == 0) {
-            double t = 0.0;
-            for (int q = 0; q < nw; ++q) t += S.red[q];
-            part[k] = t;
+            float t = 0.f;
+            for (int q = 0; q < nw; ++q) t += S.fu[q];
+            part[k] = (double)t;
           }
         }
         if constexpr (C > 1) {  // the coefficients of the whole vector, the same bits in every CTA
@@ -651,6 +838,7 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batch_lanczos_kernel(const B
           cl.sync();
           for (int j = threadIdx.x; j <= k; j += blockDim.x) {
             double t = 0.0;
+#pragma unroll 1
             for (int r = 0; r < C; ++r) t += *cl.map_shared_rank(&S.hp[hbuf][j], r);
             S.h[j] = t;
           }
@@ -658,14 +846,12 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batch_lanczos_kernel(const B
         }
         __syncthreads();
         // update coefficients of the stored vectors: u' = u - sum_j scl[j]^2 g_j V[j]
-        for (int j = threadIdx.x; j < k; j += blockDim.x) S.c[j] = S.scl[j] * S.scl[j] * S.h[j];
+        for (int j = threadIdx.x; j < k; j += blockDim.x) S.cf[j] = -(float)(S.scl[j] * S.scl[j] * S.h[j]);
         {
-          int e2 = 0;
-          const double un = sqrt(S.h[k]);
-          if (un > 0.0 && std::isfinite(un)) {
-            frexp(un, &e2);
-            tk = ldexpf(1.f, -e2);  // tk ||u|| in [0.5, 1)
-          }
+          // tk ||u|| in [0.5, 1), from the exponent of ||u||^2
+          const unsigned hw = (unsigned)__double2hiint(S.h[k]);
+          const int e2 = (int)(hw >> 20) - 1022;
+          if (hw >= 0x00100000u && hw < 0x7ff00000u) tk = ldexpf(1.f, -((e2 + 1) >> 1));
         }
         __syncthreads();
         // V[k] = tk (u - sum_j c_j V[j]), and its squared norm (FP32 over at most kChunk elements)
@@ -679,7 +865,7 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batch_lanczos_kernel(const B
           float4 x = wm4[i], u = wm4[i + bs];
 #pragma unroll 4
           for (int j = 0; j < k; ++j) {
-            const float c = -(float)S.c[j];
+            const float c = S.cf[j];
             const float4* vj4 = reinterpret_cast<const float4*>(V + (int64_t)j * I.ld);
             const float4 y = vj4[i], z = vj4[i + bs];
             x.x = fmaf(c, y.x, x.x);
@@ -703,20 +889,22 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batch_lanczos_kernel(const B
           nf = fmaf(u.y, u.y, nf);
           nf = fmaf(u.z, u.z, nf);
           nf = fmaf(u.w, u.w, nf);
-          if (++ncnt == kChunk / 8) {
+          if (!few && ++ncnt == kChunk / 8) {
             nacc += (double)nf;
             nf = 0.f;
             ncnt = 0;
           }
         }
-        nacc += (double)nf;
-        nf = 0.f;
-        ncnt = 0;
+        if (!few) {
+          nacc += (double)nf;
+          nf = 0.f;
+          ncnt = 0;
+        }
         for (; i < q1; i += bs) {
           float4 x = wm4[i];
 #pragma unroll 4
           for (int j = 0; j < k; ++j) {
-            const float c = -(float)S.c[j];
+            const float c = S.cf[j];
             const float4 y = reinterpret_cast<const float4*>(V + (int64_t)j * I.ld)[i];
             x.x = fmaf(c, y.x, x.x);
             x.y = fmaf(c, y.y, x.y);
@@ -729,7 +917,7 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batch_lanczos_kernel(const B
           nf = fmaf(x.y, x.y, nf);
           nf = fmaf(x.z, x.z, nf);
           nf = fmaf(x.w, x.w, nf);
-          if (++ncnt == kChunk / 4) {
+          if (!few && ++ncnt == kChunk / 4) {
             nacc += (double)nf;
             nf = 0.f;
             ncnt = 0;
@@ -738,47 +926,63 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batch_lanczos_kernel(const B
         float* vk = V + (int64_t)k * I.ld;
         for (int64_t i = (q1 << 2) + threadIdx.x; i < hi; i += blockDim.x) {
           float wi = w[i];
-          for (int j = 0; j < k; ++j) wi = fmaf(-(float)S.c[j], V[(int64_t)j * I.ld + i], wi);
+          for (int j = 0; j < k; ++j) wi = fmaf(S.cf[j], V[(int64_t)j * I.ld + i], wi);
           wi *= tk;
           vk[i] = wi;
           nf = fmaf(wi, wi, nf);
         }
-        nacc += (double)nf;
+        for (int64_t i = hi + threadIdx.x; i < pad; i += blockDim.x) vk[i] = 0.f;
+        nshare = nf;
       }
-      const double nst = sqrt(inst_sum<C>(block_sum_all(nacc, S), S, buf));  // ||V[k]|| as stored
-      const double nr = s1 * nst / (double)tk;                               // beta_k
+      // ||V[k]||^2 as stored; the barrier also completes V[k] for the next product
+      if (few) {
+        const float f1[1] = {nshare};
+        block_sum_f<1>(f1, S, &S.xp[buf]);
+      } else {
+        const double t = block_sum_all(nacc + (double)nshare, S);
+        if (threadIdx.x == 0) S.xp[buf] = t;
+      }
+      inst_sync<C>();
       if (threadIdx.x == 0) {
-        S.alpha[k] = al + s1 * s1 * S.h[k - 1];  // al + <v_{k-1}, u> in the true vectors
+        double n2 = 0.0;
+        if constexpr (C > 1) {
+#pragma unroll 1
+          for (int r = 0; r < C; ++r) n2 += *cg::this_cluster().map_shared_rank(&S.xp[buf], r);
+        } else {
+          n2 = S.xp[buf];
+        }
+        const double rs = rsqrt(n2), nst = n2 > 0.0 ? n2 * rs : n2;
+        const double nr = S.scl[k - 1] * nst * (double)(1.f / tk);  // beta_k
+        S.alpha[k] = S.al + S.scl[k - 1] * S.scl[k - 1] * S.h[k - 1];  // al + <v_{k-1}, u> in the true vectors
         S.beta[k] = nr;
-        S.scl[k] = (nst > 0.0) ? 1.0 / nst : 0.0;
+        S.scl[k] = (nst > 0.0) ? rs : 0.0;
         // breakdown (sparse_algorithm.hpp:421): the reference's 1e-10, or the
         // FP32 resolution of the recurrence, or an exhausted space
-        const double scale = fabs(al) + fabs(bp) + (k >= 2 ? S.beta[k - 1] : 0.0);
+        const double scale = fabs(S.al) + fabs(S.bp) + (k >= 2 ? S.beta[k - 1] : 0.0);
         if (nr < 1e-10 || nr < 1e-5 * scale || k >= n) S.stop = k;
       }
+      buf ^= 1;
       __syncthreads();
       if (S.stop) {  // the same decision in every CTA of the cluster
         act = k;     // v_0 .. v_{k-1} span an invariant subspace: T_k is exact
         break;
       }
-      inst_sync<C>();  // the next product reads all of V[k]
     }
     if (act < 1) act = 1;
     // lowest Ritz pair of tridiag(alpha_1..act, beta_1..act-1), the same in every CTA
-    if (threadIdx.x == 0) {
-      double* work = tri_work + (size_t)blockIdx.x * 8 * (kBatchMaxSteps + 2);
-      const double lam = device_tridiag_lowest(act, S.alpha + 1, S.beta + 1, S.y, work);
-      if (rank == 0) {
-        I.out[0] = lam;
-        I.out[3] = act;
-        I.out[4] = S.stop ? 1 : 0;
-      }
+    const double lam = block_tridiag_lowest(act, S.alpha + 1, S.beta + 1, S.y, S);
+    if (rank == 0 && threadIdx.x == 0) {
+      I.out[0] = lam;
+      I.out[3] = act;
+      I.out[4] = S.stop ? 1 : 0;
     }
+    for (int k = threadIdx.x; k < act; k += blockDim.x) S.cf[k] = (float)(S.y[k] * S.scl[k]);
     __syncthreads();
     // Ritz vector psi = sum_k y_k v_k (FP32 storage)
     for (int64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
       float acc = 0.f;
-      for (int k = 0; k < act; ++k) acc = fmaf((float)(S.y[k] * S.scl[k]), V[(int64_t)k * I.ld + i], acc);
+#pragma unroll 8
+      for (int k = 0; k < act; ++k) acc = fmaf(S.cf[k], V[(int64_t)k * I.ld + i], acc);
       I.psi[i] = acc;
     }
     inst_sync<C>();  // the refinement reads all of psi
@@ -808,15 +1012,16 @@ __global__ void __launch_bounds__(kBatchThreads, 2) batch_lanczos_kernel(const B
 // (clusters of C CTAs for C > 1).
 template <int C>
 static void launch_batch(Ctx* ctx, cudaStream_t stream, const BatchInst* list, int count, unsigned* counter,
-                         double* tri_work, int grid) {
+                         int grid) {
   if (count <= 0) return;
+  if constexpr (C > 1) allow_dynamic_smem(batch_lanczos_kernel<C>, ctx->device);
   if constexpr (C == 1) {
-    batch_lanczos_kernel<1><<<grid, kBatchThreads, 0, stream>>>(list, count, counter, tri_work);
+    batch_lanczos_kernel<1><<<grid, kBatchThreads, 0, stream>>>(list, count, counter);
   } else {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(kBatchThreads);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = kBatchRingBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -825,7 +1030,7 @@ static void launch_batch(Ctx* ctx, cudaStream_t stream, const BatchInst* list, i
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    QD_CUDA(cudaLaunchKernelEx(&cfg, batch_lanczos_kernel<C>, list, count, counter, tri_work));
+    QD_CUDA(cudaLaunchKernelEx(&cfg, batch_lanczos_kernel<C>, list, count, counter));
   }
   QD_CHECK_LAUNCH();
   QD_LAUNCHED(ctx);
@@ -834,11 +1039,14 @@ static void launch_batch(Ctx* ctx, cudaStream_t stream, const BatchInst* list, i
 // Clusters of C CTAs the device keeps resident at once (0 if none).
 template <int C>
 static int resident_clusters(Ctx* ctx) {
+  if (C == 1) return 2 * ctx->num_sms;
   static thread_local int cached = -1;
   if (cached >= 0) return cached;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(C * 2 * ctx->num_sms));
   cfg.blockDim = dim3(kBatchThreads);
+  cfg.dynamicSmemBytes = kBatchRingBytes;
+  allow_dynamic_smem(batch_lanczos_kernel<C>, ctx->device);
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = C;
@@ -853,6 +1061,66 @@ static int resident_clusters(Ctx* ctx) {
   }
   cached = n;
   return n;
+}
+
+constexpr int kBatchSizes = 6;
+static const int kBatchSize[kBatchSizes] = {1, 2, 3, 4, 6, 8};
+
+template <typename F>
+static void batch_size(int c, F&& f) {
+  switch (c) {
+    case 2: f(std::integral_constant<int, 2>()); break;
+    case 3: f(std::integral_constant<int, 3>()); break;
+    case 4: f(std::integral_constant<int, 4>()); break;
+    case 6: f(std::integral_constant<int, 6>()); break;
+    case 8: f(std::integral_constant<int, 8>()); break;
+    default: f(std::integral_constant<int, 1>()); break;
+  }
+}
+
+// CTAs per instance.  While slots are free a call takes as long as its longest slice of rows, so the slices are
+// as short as the device has CTA slots for, down to kBatchMinRows.  32 chains each of 14, 16 and 18 sites, 80
+// steps: 19.4 ms on 1, 1 and 8 CTAs, 22.0 on 1, 4 and 4, 17.1 on 1, 2 and 6, which this takes; 32 of 16 sites
+// 11.3, 8.5, 5.6 and 4.5 ms on 1, 2, 4 and 8.  A call with more instances than slots keeps 2 CTAs for dimensions
+// from kClusterMinDim and one below: more instances side by side beat wider clusters there.
+static std::vector<int> batch_widths(Ctx* ctx, qd_ham* const* hams, int ninst) {
+  int most[kBatchSizes];
+  for (int k = 0; k < kBatchSizes; ++k)
+    batch_size(kBatchSize[k], [&](auto c) { most[k] = resident_clusters<decltype(c)::value>(ctx); });
+  const int64_t slots = most[0];
+  auto size_of = [&](int64_t dim, int64_t rows) {  // index of the least size with slices of at most `rows`
+    if (dim < kBatchSplitMinDim) return 0;
+    int k = (dim >= kClusterMinDim && most[1] > 0) ? 1 : 0;
+    while (k + 1 < kBatchSizes && dim > rows * kBatchSize[k]) ++k;
+    while (k > 0 && most[k] < 1) --k;
+    return k;
+  };
+  auto fits = [&](int64_t rows) {
+    int64_t used = 0, n[kBatchSizes] = {};
+    for (int i = 0; i < ninst; ++i) {
+      const int k = size_of(hams[i]->dim, rows);
+      used += kBatchSize[k];
+      ++n[k];
+    }
+    for (int k = 0; k < kBatchSizes; ++k)
+      if (n[k] > most[k]) return false;
+    return used <= slots;
+  };
+  std::vector<int64_t> cand;
+  for (int i = 0; i < ninst; ++i)
+    for (int k = 0; k < kBatchSizes; ++k)
+      cand.push_back(std::max<int64_t>(ceil_div(hams[i]->dim, kBatchSize[k]), kBatchMinRows));
+  std::sort(cand.begin(), cand.end());
+  cand.erase(std::unique(cand.begin(), cand.end()), cand.end());
+  size_t lo = 0, hi = cand.size() - 1;  // the least slice that fits, else the longest
+  while (lo < hi) {
+    const size_t mid = (lo + hi) / 2;
+    if (fits(cand[mid])) hi = mid;
+    else lo = mid + 1;
+  }
+  std::vector<int> width(ninst);
+  for (int i = 0; i < ninst; ++i) width[i] = kBatchSize[size_of(hams[i]->dim, cand[lo])];
+  return width;
 }
 
 void batch_lanczos(Ctx* ctx, qd_ham* const* hams, const double* const* v0s, int ninst, int steps, double* out) {
@@ -871,9 +1139,11 @@ void batch_lanczos(Ctx* ctx, qd_ham* const* hams, const double* const* v0s, int 
   const char* uenv = std::getenv("QD_BATCH_UNIFORM");
   const bool uniform_ok = !(uenv && std::strcmp(uenv, "0") == 0);
   if (uniform_ok) check_uniform(ctx, hams, ninst);
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return hams[a]->nnz > hams[b]->nnz; });
-  // large instances (a cluster each) first, each class longest first
-  std::stable_partition(order.begin(), order.end(), [&](int a) { return hams[a]->dim >= kClusterMinDim; });
+  // wider clusters first, each size longest first
+  const std::vector<int> width = batch_widths(ctx, hams, ninst);
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    return width[a] != width[b] ? width[a] > width[b] : hams[a]->nnz > hams[b]->nnz;
+  });
   // one arena for every instance's basis, work vector and Ritz vector
   std::vector<int64_t> off_V(ninst), off_w(ninst), off_psi(ninst);
   int64_t total = 0;
@@ -915,20 +1185,8 @@ void batch_lanczos(Ctx* ctx, qd_ham* const* hams, const double* const* v0s, int 
   }
   QD_CUDA(cudaMemcpyAsync(v0buf.p, h32.get(), (size_t)v0_total * sizeof(float), cudaMemcpyHostToDevice,
                           ctx->stream));
-  // the work list: large instances, then small ones
+  // the work list, one launch per cluster size
   std::vector<BatchInst> list(ninst);
-  int nlarge = 0;
-  for (int q = 0; q < ninst; ++q) nlarge += (hams[order[q]]->dim >= kClusterMinDim) ? 1 : 0;
-  // cluster size: the largest whose resident clusters hold every large instance at once, else 2
-  int ctas = 2, nclusters = resident_clusters<2>(ctx);
-  if (resident_clusters<8>(ctx) >= nlarge) {
-    ctas = 8;
-    nclusters = resident_clusters<8>(ctx);
-  } else if (resident_clusters<4>(ctx) >= nlarge) {
-    ctas = 4;
-    nclusters = resident_clusters<4>(ctx);
-  }
-  if (nclusters < 1) nlarge = 0;  // no cluster fits: every instance on one CTA
   for (int q = 0; q < ninst; ++q) {
     const int i = order[q];
     const qd_ham* H = hams[i];
@@ -952,62 +1210,66 @@ void batch_lanczos(Ctx* ctx, qd_ham* const* hams, const double* const* v0s, int 
   }
   DBuf<BatchInst> dlist(ninst);
   QD_CUDA(cudaMemcpyAsync(dlist.p, list.data(), ninst * sizeof(BatchInst), cudaMemcpyHostToDevice, ctx->stream));
-  DBuf<unsigned> counter(2);
-  QD_CUDA(cudaMemsetAsync(counter.p, 0, 2 * sizeof(unsigned), ctx->stream));
-  const int nsmall = ninst - nlarge;
-  const int grid_large = nlarge ? ctas * std::min(nlarge, nclusters) : 0;
-  const int grid_small = nsmall ? std::min(nsmall, 2 * ctx->num_sms) : 0;
-  // one scratch region per CTA of either launch (they may run at the same time)
-  DBuf<double> tri_work((size_t)std::max(grid_large + grid_small, 1) * 8 * (kBatchMaxSteps + 2));
-  double* tri_small = tri_work.p + (size_t)grid_large * 8 * (kBatchMaxSteps + 2);
-  // With both classes present the cluster launch goes on a high-priority side
-  // stream and the single-CTA launch beside it on the context's stream: the
-  // clusters are placed first, and single CTAs take the SM slots the clusters
-  // leave (and free at the end).  Every instance is computed by its own CTAs
-  // in a fixed order, so the results do not depend on the overlap.
+  DBuf<unsigned> counter(kBatchSizes);
+  QD_CUDA(cudaMemsetAsync(counter.p, 0, counter.bytes(), ctx->stream));
+  // The widest clusters go first, each size but the last on a high-priority side stream: the clusters are
+  // placed before the narrower ones and the single CTAs, which take the SM slots they leave (and free at the
+  // end).  Every instance is computed by its own CTAs in a fixed order, so the results do not depend on the
+  // overlap.
   struct Side {
     cudaStream_t s = nullptr;
-    cudaEvent_t in = nullptr, done = nullptr;
+    cudaEvent_t done = nullptr;
     ~Side() {
-      if (in) cudaEventDestroy(in);
       if (done) cudaEventDestroy(done);
       if (s) {
         cudaStreamSynchronize(s);  // after an error its kernel may still run, and the buffers are given back next
         cudaStreamDestroy(s);
       }
     }
-  } side;
-  cudaStream_t large_stream = ctx->stream;
-  if (nlarge > 0 && nsmall > 0) {
-    int least = 0, greatest = 0;
-    QD_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-    QD_CUDA(cudaStreamCreateWithPriority(&side.s, cudaStreamNonBlocking, greatest));
-    QD_CUDA(cudaEventCreateWithFlags(&side.in, cudaEventDisableTiming));
-    QD_CUDA(cudaEventCreateWithFlags(&side.done, cudaEventDisableTiming));
-    QD_CUDA(cudaEventRecord(side.in, ctx->stream));  // the list, the start vectors and the counters are in place
-    QD_CUDA(cudaStreamWaitEvent(side.s, side.in, 0));
-    large_stream = side.s;
-  }
+  } side[kBatchSizes];
+  struct InEvent {
+    cudaEvent_t e = nullptr;
+    ~InEvent() {
+      if (e) cudaEventDestroy(e);
+    }
+  } in;
   const bool timing = std::getenv("QD_TIMING") != nullptr;
   if (timing) QD_CUDA(cudaEventRecord(ctx->events[12], ctx->stream));
-  if (ctas == 8) launch_batch<8>(ctx, large_stream, dlist.p, nlarge, counter.p, tri_work.p, grid_large);
-  else if (ctas == 4) launch_batch<4>(ctx, large_stream, dlist.p, nlarge, counter.p, tri_work.p, grid_large);
-  else launch_batch<2>(ctx, large_stream, dlist.p, nlarge, counter.p, tri_work.p, grid_large);
-  launch_batch<1>(ctx, ctx->stream, dlist.p + nlarge, nsmall, counter.p + 1, tri_small, grid_small);
-  if (timing) QD_CUDA(cudaEventRecord(ctx->events[14], ctx->stream));
-  if (side.s) {
-    QD_CUDA(cudaEventRecord(side.done, side.s));
-    QD_CUDA(cudaStreamWaitEvent(ctx->stream, side.done, 0));
+  std::string plan;
+  for (int q0 = 0, li = 0; q0 < ninst; ++li) {
+    const int c = width[order[q0]];
+    int q1 = q0;
+    while (q1 < ninst && width[order[q1]] == c) ++q1;
+    cudaStream_t st = ctx->stream;
+    if (q1 < ninst) {  // not the last size
+      int least = 0, greatest = 0;
+      if (!in.e) {
+        QD_CUDA(cudaEventCreateWithFlags(&in.e, cudaEventDisableTiming));
+        QD_CUDA(cudaEventRecord(in.e, ctx->stream));  // the list, the start vectors and the counters are in place
+      }
+      QD_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+      QD_CUDA(cudaStreamCreateWithPriority(&side[li].s, cudaStreamNonBlocking, greatest));
+      QD_CUDA(cudaEventCreateWithFlags(&side[li].done, cudaEventDisableTiming));
+      QD_CUDA(cudaStreamWaitEvent(side[li].s, in.e, 0));
+      st = side[li].s;
+    }
+    batch_size(c, [&](auto k) {
+      constexpr int C = decltype(k)::value;
+      launch_batch<C>(ctx, st, dlist.p + q0, q1 - q0, counter.p + li, C * std::min(q1 - q0, resident_clusters<C>(ctx)));
+    });
+    if (side[li].s) QD_CUDA(cudaEventRecord(side[li].done, side[li].s));
+    if (timing) plan += " " + std::to_string(q1 - q0) + " x " + std::to_string(c);
+    q0 = q1;
   }
+  for (Side& sd : side)
+    if (sd.s) QD_CUDA(cudaStreamWaitEvent(ctx->stream, sd.done, 0));
   if (timing) QD_CUDA(cudaEventRecord(ctx->events[13], ctx->stream));
   QD_CUDA(cudaMemcpyAsync(out, dout.p, (size_t)ninst * 8 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   QD_CUDA(cudaStreamSynchronize(ctx->stream));
   if (timing) {
-    float a = 0.f, b = 0.f;
+    float a = 0.f;
     QD_CUDA(cudaEventElapsedTime(&a, ctx->events[12], ctx->events[13]));
-    QD_CUDA(cudaEventElapsedTime(&b, ctx->events[12], ctx->events[14]));
-    std::fprintf(stderr, "[qd timing] batch: %d large on %d clusters, %d small on %d CTAs: all done at %.3f ms, "
-                 "small done at %.3f ms (%d-CTA clusters)\n", nlarge, grid_large / ctas, nsmall, grid_small, a, b, ctas);
+    std::fprintf(stderr, "[qd timing] batch: instances x CTAs:%s: %.3f ms\n", plan.c_str(), a);
   }
 }
 
