@@ -21,9 +21,10 @@
 // forms every vector a second time for the Ritz vector.
 //
 // Measured (GB300): a step at dim 12,870 (uniform couplings) 18 -> 9 us, complex
-// at dim 184,756 61 -> 28 us (the FP64 product is 14 of them, rows of unequal
-// length in a warp and the exchange most of the rest), real couplings per bond
-// there 41 -> 22 us; Hermitian solver at dim 4,900 2.3 -> 0.42 ms a solve.
+// at dim 184,756 61 -> 24 us (the FP64 product is 12 of them, the exchange most
+// of the rest; 28 us before a block took its rows in order of their length),
+// real couplings per bond there 41 -> 19 us; Hermitian solver at dim 4,900 2.3
+// -> 0.42 ms a solve.
 // Mean error against 64-bit references over ten random cases each: ground-state
 // eigenvalues 5.4e-16 (launched step by step: 5.6e-16), evolved states 1.95e-15
 // (1.99e-15).
@@ -259,6 +260,52 @@ __device__ __forceinline__ void lan_texp(int act, double h, double d, double e, 
   }
 }
 
+// The block's rows in order of their length, longest first (lengths from kLanBins - 1 on alike; equal ones in
+// their own order), so that a warp issues as many FP64 multiply-adds as its rows have entries and not as the
+// longest of 32 neighbours has.  scratch: (R / 32 + 2) kLanBins shorts.
+constexpr int kLanBins = 64;
+template <int T>
+__device__ void lan_sort_rows(const int64_t* rowptr, int64_t r0, int R, short* order, short* scratch) {
+  const int tid = threadIdx.x, lane = tid & 31, chunks = (R + 31) / 32;
+  short* base = scratch + chunks * kLanBins;
+  for (int i = tid; i < chunks * kLanBins; i += T) scratch[i] = 0;
+  __syncthreads();
+  for (int pass = 0; pass < 2; ++pass) {
+    for (int r = tid; r - lane < R; r += T) {
+      const unsigned live = __ballot_sync(0xffffffffu, r < R);
+      if (r < R) {
+        const int len = (int)min(__ldg(rowptr + r0 + r + 1) - __ldg(rowptr + r0 + r), (int64_t)kLanBins - 1);
+        const unsigned same = __match_any_sync(live, len), before = same & ((1u << lane) - 1u);
+        short* h = scratch + (r >> 5) * kLanBins + len;
+        if (pass == 0) {
+          if (!before) *h = (short)__popc(same);
+        } else {
+          order[base[len] + *h + __popc(before)] = (short)r;
+        }
+      }
+    }
+    __syncthreads();
+    if (pass == 0) {
+      if (tid < kLanBins) {
+        int run = 0;
+        for (int c = 0; c < chunks; ++c) {
+          const int t = scratch[c * kLanBins + tid];
+          scratch[c * kLanBins + tid] = (short)run;
+          run += t;
+        }
+        base[kLanBins + tid] = (short)run;
+      }
+      __syncthreads();
+      if (tid < kLanBins) {
+        int b = 0;
+        for (int i = tid + 1; i < kLanBins; ++i) b += base[kLanBins + i];
+        base[tid] = (short)b;
+      }
+      __syncthreads();
+    }
+  }
+}
+
 template <typename MV, typename VV, bool kOne, bool kUni, bool kPaige, bool kExp>
 __global__ void __launch_bounds__(kLanThreads, 1) lan_kernel(LanArgs<MV, VV> A) {
   constexpr int T = kLanThreads, kPer = sizeof(VV) / sizeof(double);
@@ -276,6 +323,9 @@ __global__ void __launch_bounds__(kLanThreads, 1) lan_kernel(LanArgs<MV, VV> A) 
   const bool mute = X.hold && blockIdx.x == 0;
   int lanes = 1;
   while (lanes < 4 && 2 * lanes * A.rows <= (kUni ? 512 : 256)) lanes *= 2;
+  short* order = reinterpret_cast<short*>(ring + 3 * (size_t)A.rows);
+  if constexpr (!kUni)
+    if (lanes == 1) lan_sort_rows<T>(A.rowptr, r0, R, order, reinterpret_cast<short*>(ring));
   double vals[NV];
 #pragma unroll
   for (int i = 0; i < NV; ++i) vals[i] = 0.0;
@@ -331,8 +381,9 @@ __global__ void __launch_bounds__(kLanThreads, 1) lan_kernel(LanArgs<MV, VV> A) 
       VV d1 = vzero(VV{}), d2 = vzero(VV{});
       double d2re = 0.0;
       const int g = tid / lanes, sub = tid & (lanes - 1), per = T / lanes;
-      for (int r = g; (r & ~(32 / lanes - 1)) < R; r += per) {  // whole warps
-        const bool live = r < R;
+      for (int i = g; (i & ~(32 / lanes - 1)) < R; i += per) {  // whole warps
+        const bool live = i < R;
+        const int r = (!kUni && lanes == 1 && live) ? order[i] : i;
         VV a;
         if constexpr (kUni)
           a = lan_row_uniform(A, A.XV + (int64_t)(k - A.first) * A.ld, r0 + r, live, sub, lanes, live ? u1[r] : 0.0);
@@ -551,7 +602,8 @@ static bool lan_plan(qd_ham* H, K kern1, K kern_many, LanPlan& P, cudaLaunchConf
   cfg.stream = ctx->stream;
   cfg.attrs = at;
   cfg.numAttrs = csize == 1 ? 1 : 2;
-  const auto smem_of = [](int rows) { return (size_t)3 * rows * sizeof(VV); };
+  // three vectors' rows and their order by length
+  const auto smem_of = [](int rows) { return (size_t)3 * rows * sizeof(VV) + ((size_t)rows * sizeof(short) + 15) / 16 * 16; };
   if (!P.ok) {
     int maxsm = 0;
     QD_CUDA(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
