@@ -33,9 +33,10 @@ namespace qd {
 
 constexpr int kVecThreads = 256;
 // Most rows of the persistent recurrence (lan_res_takes).  Whole solves of 3 L steps, launched step by step
-// -> persistent: real couplings per bond L = 17 1,338 -> 693 us, L = 21 (352,716 rows) 2,953 -> 2,444, L = 22
-// (705,432) 4,806 -> 5,474; complex L = 21 6,523 -> 5,213, L = 22 the same: the line lies between them.
-constexpr int64_t kLanResMax = 1 << 19;
+// -> persistent: real couplings per bond L = 17 1,338 -> 693 us, L = 21 (352,716 rows) 2,983 -> 2,167, L = 22
+// (705,432) 4,788 -> 4,158; complex L = 21 6,523 -> 4,900.  The gain shrinks with the rows, and beyond the line
+// the blocks' rows soon do not fit (complex vectors from about 600,000 on, which then run step by step).
+constexpr int64_t kLanResMax = 3 << 18;
 // With the uniform-coupling form, whose one-launch step is faster: L = 12 686 -> 433 us, L = 16 906 -> 647,
 // L = 18 (48,620 rows) 1,152 -> 822, L = 19 (92,378) 1,356 -> 1,227 on the stored columns but 1,436 -> 1,682
 // matrix-free, and both keep one route so that their bits stay the same.
