@@ -24,11 +24,12 @@
 // together with the vector that a product gathers from, in complex64; the
 // diagonal (shifted by the centre mu of its range) comes from L1 and L2.  A step
 // is then K products H - mu of the shared-memory vector (the gathers never leave
-// the SM) summed into the truncated Taylor series of exp(-i tau (H - mu)),
-// S sub-steps of tau = dt / S, with (S, K) from the series' remainder bound
+// the SM) summed into a truncated series of exp(-i tau (H - mu)), S sub-steps of
+// tau = dt / S, with (S, K) from the series' remainder bound: Taylor's
 // (tau ||H - mu|| <= 1 and ||R_K|| <= theta^(K+1) / (K+1)! e^theta <= 1e-8,
 // the scheme of A. H. Al-Mohy and N. J. Higham, SIAM J. Sci. Comput. 33
-// (2011) 488-511, with one sub-step size); the factor exp(-i tau mu) is
+// (2011) 488-511, with one sub-step size), or where H - mu is Hermitian (the
+// jumps' damping is one number on the sector) Chebyshev's; the factor exp(-i tau mu) is
 // dropped with the renormalisation.  Weights, norm and observables come from
 // one block reduction of the new vector per step; HBM sees only the observable
 // records.  The state's norm is carried, not divided out: the next products
@@ -36,9 +37,10 @@
 //
 // Two trajectories a CTA share the loads and the decoding of the entries and
 // fetch a column's two values in one 16-byte load.  2,048 trajectories of 100
-// steps at dim 4,900 (six products a step): generic addresses and one sum after
-// another 50.9 ms, shared-memory addresses, packed additions and one butterfly
-// for eight sums 41.1 ms, two trajectories a CTA 35.1 ms.  A product of two
+// steps at dim 4,900: generic addresses and one sum after another 50.9 ms,
+// shared-memory addresses, packed additions and one butterfly for eight sums
+// 41.1 ms, two trajectories a CTA 35.1 ms, five products a step instead of six
+// (traj_series_plan) 30.8 ms.  A product of two
 // takes 10,700 cycles of shared-memory bandwidth, 1,900 of them conflicts, and
 // 8,500 issue cycles in 17,000; entries ordered against the conflicts took 5%
 // off the kernel and gave it to the host.  16 warps of 10 slices and loops
@@ -86,6 +88,7 @@ struct TrajResArgs {
   int K, S;
   float tau;          // dt / S
   float2 coff;        // the off-diagonal value c
+  float weight[kTrajMaxTaylor + 1];  // of each Taylor term in the sum
   double gamma, dt;
   uint64_t seed;
   uint32_t chanmask;  // union of the channel bits
@@ -322,10 +325,12 @@ __global__ void __launch_bounds__(kTrajMaxWarps * 32, 1) traj_resident_kernel(Tr
 #pragma unroll
             for (int i = 0; i < kTrajRpt; ++i) {
               t[a][i] = acc[a][i];  // t_0; times sc on the first sub-step, in the factor
-              if (sub == 0) acc[a][i] = make_float2(acc[a][i].x * sc[a], acc[a][i].y * sc[a]);
+              const float w0 = jump[a] ? 1.f : (sub == 0 ? A.weight[0] * sc[a] : A.weight[0]);
+              acc[a][i] = make_float2(acc[a][i].x * w0, acc[a][i].y * w0);
             }
           for (int k = 1; k <= A.K; ++k) {
-            // t_k = (-i tau / k) (H - mu) t_{k-1}
+            // t_k = (-i tau / k) (H - mu) t_{k-1}, added with its weight
+            const float wk = A.weight[k];
             float f[NT];
 #pragma unroll
             for (int a = 0; a < NT; ++a)
@@ -375,8 +380,8 @@ __global__ void __launch_bounds__(kTrajMaxWarps * 32, 1) traj_resident_kernel(Tr
                   const float vx = fmaf(A.coff.x, g.x, fmaf(-A.coff.y, g.y, fmaf(dg.x, o.x, -dg.y * o.y)));
                   const float vy = fmaf(A.coff.x, g.y, fmaf(A.coff.y, g.x, fmaf(dg.x, o.y, dg.y * o.x)));
                   t[a][i] = make_float2(__fmul_rn(f[a], vy), __fmul_rn(-f[a], vx));
-                  acc[a][i].x = __fadd_rn(acc[a][i].x, t[a][i].x);
-                  acc[a][i].y = __fadd_rn(acc[a][i].y, t[a][i].y);
+                  acc[a][i].x = fmaf(wk, t[a][i].x, acc[a][i].x);
+                  acc[a][i].y = fmaf(wk, t[a][i].y, acc[a][i].y);
                 }
               }
             }
@@ -447,6 +452,7 @@ struct TrajHostForm {
   cplx coff{0.0, 0.0};
   double norm = 0.0;  // bound on ||H - mu||_2: max of the 1- and infinity-norms
   bool any_neg = false;  // some entry carries -c
+  bool hermitian = false;  // H - mu is: c real, every entry with its mirror image, one imaginary part on the diagonal
 };
 
 // Dynamic shared memory of the resident kernel for dim n, nsl slices and ent_len entries.
@@ -572,6 +578,15 @@ static bool traj_build_resident(qd_ham* H, TrajHostForm& F, size_t max_smem) {
   }
   double colmax = 0.0;
   for (double x : colsum) colmax = std::max(colmax, x);
+  F.hermitian = c.im == 0.0 && imin == imax;
+  for (int64_t r = 0; r < n && F.hermitian; ++r)
+    for (int64_t k = rp[r]; k < rp[r + 1] && F.hermitian; ++k) {
+      if (ci[k] == r || (v[k].re == 0.0 && v[k].im == 0.0)) continue;
+      const int32_t* lo = ci.data() + rp[ci[k]];
+      const int32_t* hi = ci.data() + rp[ci[k] + 1];
+      const int32_t* m = std::lower_bound(lo, hi, (int32_t)r);  // columns ascend
+      F.hermitian = m < hi && *m == r && v[m - ci.data()].re == v[k].re;
+    }
   F.coff = c;
   F.norm = std::max(rowmax, colmax);
   return true;
@@ -582,24 +597,70 @@ static bool traj_build_resident(qd_ham* H, TrajHostForm& F, size_t max_smem) {
 // exponential), so the series adds no error the FP32 state would not.
 constexpr double kTrajTaylorTol = 1e-8;
 
-// (S, K) for exp(-i dt A) with ||A|| <= norm: S sub-steps of tau = dt / S with
-// theta = tau norm <= 1, K the least degree with theta^(K+1)/(K+1)! e^theta <= kTrajTaylorTol.
-static void traj_taylor_plan(double dt, double norm, int kmax, int* S, int* K) {
+// Bessel functions of the first kind for small arguments, by their power series.
+static double traj_bessel(int k, double x) {
+  double term = 1.0;
+  for (int i = 1; i <= k; ++i) term *= 0.5 * x / i;
+  double sum = 0.0;
+  for (int m = 1; m <= 20; ++m) {
+    sum += term;
+    term *= -0.25 * x * x / ((double)m * (m + k));
+  }
+  return sum;
+}
+
+// (S, K) for exp(-i dt A) with ||A|| <= norm: S sub-steps of tau = dt / S with theta = tau norm <= 1, and the
+// least K with an error of at most kTrajTaylorTol a sub-step.  In general the Taylor series, by its remainder
+// theta^(K+1)/(K+1)! e^theta.  For a Hermitian A the Chebyshev series of exp(-i theta x) on [-1, 1], sum of
+// (2 - [k = 0]) (-i)^k J_k(theta) T_k(x), cut after K: its remainder 2 (|J_{K+1}| + ...) is 2^K times smaller,
+// one product less at theta = 0.22 (six -> five).  As powers of A it is the Taylor terms times weights near 1.
+static void traj_series_plan(double dt, double norm, bool hermitian, int kmax, int* S, int* K, float* weight) {
   int s = std::max(1, (int)std::ceil(dt * norm));
+  int k = 0;
+  double th = 0.0;
+  auto remainder = [&](int deg) {  // of the Chebyshev series
+    double r = 0.0;
+    for (int j = deg + 1; j <= deg + 20; ++j) r += 2.0 * std::fabs(traj_bessel(j, th));
+    return r;
+  };
+  bool cheb = false;
   for (;; ++s) {
-    const double th = dt * norm / s;
+    th = dt * norm / s;
     double term = th;  // th^(k+1)/(k+1)! at k = 0
-    int k = 0;
+    k = 0;
     while (term * std::exp(th) > kTrajTaylorTol && k < kTrajMaxTaylor) {
       ++k;
       term *= th / (k + 1);
     }
-    if (k <= kmax) {
-      *S = s;
-      *K = std::max(k, 1);
-      return;
+    // below 1e-2 the two take the same products
+    cheb = hermitian && th >= 1e-2 && k >= 2 && remainder(k - 1) <= kTrajTaylorTol;
+    if (cheb)
+      while (k >= 2 && remainder(k - 1) <= kTrajTaylorTol) --k;
+    if (k <= kmax) break;
+  }
+  k = std::max(k, 1);
+  for (int j = 0; j <= kTrajMaxTaylor; ++j) weight[j] = 1.f;
+  if (cheb) {
+    // T_k's coefficients by T_{k+1} = 2 x T_k - T_{k-1}; weight_j = j! / theta^j times the sum over k of
+    // (2 - [k = 0]) J_k (-1)^((k-j)/2) T_k[j]
+    std::vector<double> w(k + 1, 0.0), t0(k + 2, 0.0), t1(k + 2, 0.0), t2(k + 2, 0.0);
+    t0[0] = 1.0;
+    t1[1] = 1.0;
+    for (int q = 0; q <= k; ++q) {
+      const double c = (q == 0 ? 1.0 : 2.0) * traj_bessel(q, th);
+      for (int j = q & 1; j <= q; j += 2) w[j] += c * (((q - j) / 2 & 1) ? -t0[j] : t0[j]);
+      for (int j = 0; j <= k; ++j) t2[j] = (j > 0 ? 2.0 * t1[j - 1] : 0.0) - t0[j];
+      t0 = t1;
+      t1 = t2;
+    }
+    double scale = 1.0;
+    for (int j = 0; j <= k; ++j) {
+      if (j > 0) scale *= j / th;
+      weight[j] = (float)(w[j] * scale);
     }
   }
+  *S = s;
+  *K = k;
 }
 
 // ---------------------------------------------------------------- fallback: FP64 Arnoldi steps
@@ -792,7 +853,7 @@ void traj_run(qd_ham* H, const qd_traj_desc& d, const double* psi0_host, double*
     A.nsteps = d.nsteps;
     A.nchan = d.nchan;
     A.nobs = d.nobs;
-    traj_taylor_plan(d.dt, F.norm, d.m - 1, &A.S, &A.K);
+    traj_series_plan(d.dt, F.norm, F.hermitian, d.m - 1, &A.S, &A.K, A.weight);
     if (path) path[1] = A.K * A.S;
     A.tau = (float)(d.dt / A.S);
     A.coff = make_float2((float)F.coff.re, (float)F.coff.im);
