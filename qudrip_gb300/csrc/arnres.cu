@@ -132,13 +132,11 @@ struct ArnShared {
   double xv[2 * kArnMaxVecs + 2];   // this block's sums
   double red[2 * kArnMaxVecs + 2];  // the grid's
   VV c1[kArnMaxVecs];           // projections of the first pass
-  VV cf[kArnMaxVecs];           // coefficients on the stored vectors
-  typename QVec<VV>::T cq[kArnMaxVecs];  // the same times the vectors' scales, quantised
+  typename QVec<VV>::T cq[kArnMaxVecs];  // coefficients on the quantised vectors
   double uc;                    // their scale
   double scl[kArnMaxVecs + 2];
   double u[kArnMaxVecs + 2];    // scales of the block's quantised vectors
   double us[kArnMaxVecs + 2];   // u[j] scl[j]
-  double bs[32];
   double nrm2;
   unsigned mx[32];
   int stop;
@@ -156,11 +154,9 @@ __device__ __forceinline__ unsigned arn_block_max(ArnShared<VV, T>& S, unsigned 
   return m;
 }
 
-// The update coefficients cf[j] times the scales u[j] of the vectors, quantised (J < blockDim.x).
+// The update coefficients of the quantised vectors (thread j's c, j < J < blockDim.x), quantised.
 template <typename VV, int T>
-__device__ void arn_quant_coefs(ArnShared<VV, T>& S, int j0, int J) {
-  VV c = vzero(VV{});
-  if (threadIdx.x < J) c = vscale(S.u[j0 + threadIdx.x], S.cf[threadIdx.x]);
+__device__ void arn_quant_coefs(ArnShared<VV, T>& S, VV c, int J) {
   const QScale q = q_scale(arn_block_max<VV, T>(S, q_mag(c)));
   if (threadIdx.x < J) S.cq[threadIdx.x] = q_of(c, q.E);
   if (threadIdx.x == 0) S.uc = q.u;
@@ -334,6 +330,25 @@ __global__ void __launch_bounds__(kArnThreads, 1) arn_kernel(ArnArgs<MV, VV> A) 
     return q.u;
   };
 
+  // The block's ||v||^2 of the rows just quantised on the scale u (each thread its own), in thread 0: integers
+  // again, where the sum of FP64 values over sixteen warps takes 2,000 cycles.
+  const int nact = (min(R, T) + 31) / 32;  // warps with rows
+  auto norm2 = [&](const QT* v, double u) {
+    QSum t{0, 0u};
+    if ((tid >> 5) < nact) {
+      QDot<VV> a;
+      for (int i = tid; i < R; i += T) a.add(v[i], v[i]);
+      t.set(a.re());
+      t = q_warp_sum(t);
+      if ((tid & 31) == 0) S.part[tid >> 5] = t;
+    }
+    __syncthreads();
+    if (tid < 32) {
+      t = tid < nact ? S.part[tid] : QSum{0, 0u};
+      t = q_warp_sum(t);
+    }
+    return tid == 0 ? t.value() * u * u : 0.0;
+  };
   const bool mute = X.hold && blockIdx.x == 0;
   // The norm of vector j from its square: one thread (a square root in every warp would take longer than
   // the exchange).
@@ -353,7 +368,6 @@ __global__ void __launch_bounds__(kArnThreads, 1) arn_kernel(ArnArgs<MV, VV> A) 
   double nshare = 0.0;
 
   if (A.first == 1) {
-    double acc = 0.0;
     unsigned mag = 0;
     for (int r = tid; r < R; r += T) {
       VV v;
@@ -361,11 +375,10 @@ __global__ void __launch_bounds__(kArnThreads, 1) arn_kernel(ArnArgs<MV, VV> A) 
       if (!mute) x_put(Vg + r, v);
       wd[r] = v;
       mag = max(mag, q_mag(v));
-      acc += vnorm2(v);
     }
     const double u = quantise(mag, Vs);
     if (tid == 0) S.u[0] = S.us[0] = u;
-    nshare = block_sum(acc, S.bs);
+    nshare = norm2(Vs, u);
   } else {
     for (int j = tid; j < A.first; j += T) S.scl[j] = A.st->scl[j];
     __syncthreads();
@@ -419,16 +432,17 @@ __global__ void __launch_bounds__(kArnThreads, 1) arn_kernel(ArnArgs<MV, VV> A) 
     }
     if (!kExp && S.stop && !scaled) return;  // a zero start vector: the host reports it (evolve goes on, as NaNs)
     const double sx = S.scl[J - 1];
+    VV cq = vzero(VV{});
     if (tid < J1) {
       // <v_j, w> = sx <v_j, H V[J-1]>, and v_{J-1}'s own scale, which its share above did not have
       VV c = vscale(sx, reinterpret_cast<const VV*>(S.red)[tid]);
       if (tid == J1 - 1 && !scaled) c = vscale(sx, c);
       S.c1[tid] = c;
-      S.cf[tid] = vscale(S.scl[j1 + tid], c);
+      cq = vscale(S.us[j1 + tid], c);
     }
     // 2: the first pass taken out, projections of what is left
     {
-      arn_quant_coefs<VV, T>(S, j1, J1);
+      arn_quant_coefs<VV, T>(S, cq, J1);
       unsigned mag = 0;
       arn_comb_res<VV, T>(S, Vs, A.ldr, j1, J1, R, [&](int r, long long re, long long im) {
         const VV o = q_sub(vscale(sx, wd[r]), S.uc, re, im);
@@ -440,9 +454,10 @@ __global__ void __launch_bounds__(kArnThreads, 1) arn_kernel(ArnArgs<MV, VV> A) 
       arn_dots_res<VV, T>(S, Vs, A.ldr, 0, J, wq, uw, R);
     }
     x_sum<kOne>(X, slot2, S.xv, J * kPer, S.red);
+    cq = vzero(VV{});
     if (tid < J) {
       const VV c = reinterpret_cast<const VV*>(S.red)[tid];
-      S.cf[tid] = vscale(S.scl[tid], c);
+      cq = vscale(S.us[tid], c);
       const VV hij = (tid >= j1) ? vadd(S.c1[tid - j1], c) : c;
       if (kExp) hs[(J - 1) * kArnHs + tid] = arn_c(hij);
       if (blockIdx.x == 0) {
@@ -451,23 +466,19 @@ __global__ void __launch_bounds__(kArnThreads, 1) arn_kernel(ArnArgs<MV, VV> A) 
       }
     }
     // 3: the second pass taken out, the norm, and the rows for everybody's gathers
-    double acc = 0.0;
-    {
-      arn_quant_coefs<VV, T>(S, 0, J);
-      unsigned mag = 0;
-      arn_comb_res<VV, T>(S, Vs, A.ldr, 0, J, R, [&](int r, long long re, long long im) {
-        const VV o = q_sub(wd[r], S.uc, re, im);
-        wd[r] = o;
-        if (!mute) x_put(wg + r, o);
-        mag = max(mag, q_mag(o));
-        acc += vnorm2(o);
-      });
-      if (J < A.kdim) {  // the last column's vector is projected on no more
-        const double u = quantise(mag, Vs + (size_t)J * A.ldr);
-        if (tid == 0) S.u[J] = S.us[J] = u;
-      }
-    }
-    nshare = block_sum(acc, S.bs);
+    arn_quant_coefs<VV, T>(S, cq, J);
+    unsigned mag = 0;
+    arn_comb_res<VV, T>(S, Vs, A.ldr, 0, J, R, [&](int r, long long re, long long im) {
+      const VV o = q_sub(wd[r], S.uc, re, im);
+      wd[r] = o;
+      if (!mute) x_put(wg + r, o);
+      mag = max(mag, q_mag(o));
+    });
+    // the last column's vector is projected on no more: only its norm is needed
+    QT* dst = J < A.kdim ? Vs + (size_t)J * A.ldr : wq;
+    const double u = quantise(mag, dst);
+    if (J < A.kdim && tid == 0) S.u[J] = S.us[J] = u;
+    nshare = norm2(dst, u);
   }
   if (!stop) {  // the last vector's norm
     if (tid == 0) S.xv[0] = nshare;
