@@ -181,18 +181,21 @@ __device__ void arn_dots_res(ArnShared<VV, T>& S, const typename QVec<VV>::T* Vs
   __syncthreads();
   // four lanes a value: every fourth chunk each
   constexpr int kPer = sizeof(VV) / sizeof(double);
-  const int v4 = tid >> 2, nv = kPer * J;
-  if ((tid & ~31) < 4 * nv) {  // whole warps
-    const int j = min(v4, nv - 1) / kPer, q = min(v4, nv - 1) - kPer * j;
-    QSum t{0, 0u};
-    for (int c = tid & 3; c < C; c += 4) {
-      const QSum x = S.part[2 * (c * J + j) + q];
-      t.add(x.hi, x.lo);
-    }
+  const int nv = kPer * J;
+  for (int b = 0; b < nv; b += T / 4) {
+    const int v4 = b + (tid >> 2);
+    if (b + ((tid & ~31) >> 2) < nv) {  // whole warps
+      const int j = min(v4, nv - 1) / kPer, q = min(v4, nv - 1) - kPer * j;
+      QSum t{0, 0u};
+      for (int c = tid & 3; c < C; c += 4) {
+        const QSum x = S.part[2 * (c * J + j) + q];
+        t.add(x.hi, x.lo);
+      }
 #pragma unroll
-    for (int o = 1; o < 4; o <<= 1)
-      t.add(__shfl_xor_sync(0xffffffffu, t.hi, o), __shfl_xor_sync(0xffffffffu, t.lo, o));
-    if ((tid & 3) == 0 && v4 < nv) S.xv[v4] = (uw * S.us[j0 + j]) * t.value();
+      for (int o = 1; o < 4; o <<= 1)
+        t.add(__shfl_xor_sync(0xffffffffu, t.hi, o), __shfl_xor_sync(0xffffffffu, t.lo, o));
+      if ((tid & 3) == 0 && v4 < nv) S.xv[v4] = (uw * S.us[j0 + j]) * t.value();
+    }
   }
   __syncthreads();
 }
