@@ -29,13 +29,13 @@
 // block, and the combination uses the block's own rows: evolve is one launch.
 //
 // Measured (GB300, SM clock 1.9 GHz): dim 4,900, m = 30, not Hermitian: 3.3 ms
-// -> 0.59 ms a step; dim 36, m = 20: 0.56 -> 0.19 ms; ground state of the 4 x 4
+// -> 0.57 ms a step; dim 36, m = 20: 0.56 -> 0.18 ms; ground state of the 4 x 4
 // cluster (dim 12,870, 40 columns, real vectors): 6.5 -> 1.1 ms.  A column at dim
-// 4,900 is 36,000 cycles: the two exchanges 14,000, the projections and their
-// removal 12,000, the product 3,000, the rest block barriers and the few scalar
-// FP64 operations between them.
-// Operators whose rows do not fit (about 60,000 rows at m = 30) keep the kernels
-// launched one by one (evolve.cu), as served requests do.
+// 4,900 is 35,000 cycles: the two exchanges 14,600, the projections and their
+// removal 14,000, the product 2,800, the rest scalar FP64 operations between
+// block barriers (16,000 cycles a column in all on one block of 36 rows).
+// Operators whose rows do not fit (about 60,000 rows at m = 30) take passes over
+// a basis in memory (gspass.cu), as served requests do.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
