@@ -41,9 +41,15 @@ namespace qd {
 
 constexpr int kLanThreads = 512;
 constexpr int kLanMinRows = 96;  // rows of a block before the grid covers every SM
-// Clusters of eight keep the exchange short; of four cover more SMs (148 of 152 against 120, which is
+// Clusters of eight keep the exchange short; of four cover more SMs (144 of 152 against 120, which is
 // what one block per SM and whole clusters per GPC leave), which pays once a block's rows outweigh it.
-constexpr int64_t kLanWideRows = 1 << 16;
+// Complex vectors, four steps of m = 32, on eight and four: 48,620 rows 1,881 and 1,791 us, 184,756 4,510
+// and 3,941; real, whole solves: 48,620 rows 793 and 836 us, 92,378 1,032 and 1,046, 184,756 1,478 and
+// 1,402, 705,432 5,365 and 4,220.  Clusters of two (152 SMs) were at most 2% faster and up to 10% slower.
+template <typename VV>
+constexpr int64_t lan_wide_rows() {
+  return sizeof(VV) == sizeof(double) ? 1 << 17 : 1 << 15;
+}
 constexpr int kLanMaxExp = 32;
 
 template <typename MV, typename VV>
@@ -591,7 +597,7 @@ static bool lan_plan(qd_ham* H, K kern1, K kern_many, LanPlan& P, cudaLaunchConf
                      cudaLaunchAttribute (&at)[2], K& kern) {
   Ctx* ctx = H->ctx;
   const int64_t n = H->dim;
-  const int csize = n <= 64 ? 1 : (n <= kLanWideRows ? 8 : 4);  // one block: an exchange would cost more than it saves
+  const int csize = n <= 64 ? 1 : (n <= lan_wide_rows<VV>() ? 8 : 4);  // one block: an exchange would cost more than it saves
   kern = csize == 1 ? kern1 : kern_many;
   at[0].id = cudaLaunchAttributeCooperative;
   at[0].val.cooperative = 1;
