@@ -556,7 +556,9 @@ bool arn_res_fits(qd_ham* H, int kdim) {
          arn_coop(H->ctx);
 }
 
-static void arn_ensure(ArnRes& B, int64_t n, int kdim, bool real_v, size_t slots) {
+// True if buffers moved: what an earlier launch left in them is gone.
+static bool arn_ensure(ArnRes& B, int64_t n, int kdim, bool real_v, size_t slots) {
+  bool moved = false;
   if (B.n != n || B.kdim != kdim || B.real_v != real_v) {
     B.n = n;
     B.kdim = kdim;
@@ -564,14 +566,15 @@ static void arn_ensure(ArnRes& B, int64_t n, int kdim, bool real_v, size_t slots
     B.ld = (n + 31) / 32 * 32;
     B.ncl = 0;
     B.V.alloc((size_t)(kdim + 1) * B.ld * (real_v ? sizeof(double) : sizeof(cplx)));
-    B.open = false;
+    moved = true;
   }
   if (!B.hcol.p) B.hcol.alloc((size_t)kArnLdh * (kArnMaxExp + 1));
   const size_t want = sizeof(ArnStatus) + slots * sizeof(double);
   if (B.slots.n < want) {
     B.slots.alloc(want);
-    B.open = false;  // the status holds the stored vectors' scales
+    moved = true;  // the status holds the stored vectors' scales
   }
+  return moved;
 }
 
 template <typename MV, typename VV, bool kExp>
@@ -627,7 +630,8 @@ static bool arn_launch(qd_ham* H, const MV* vals, ArnRes& B, const cplx* psi_in,
   const size_t smem = smem_of(rows), xstride = (size_t)grid * (kPer * kdim + 1);
   cfg.gridDim = dim3((unsigned)grid);
   cfg.dynamicSmemBytes = smem;
-  arn_ensure(B, n, kdim, kPer == 1, (2 * (size_t)kdim + 1) * xstride);
+  const bool moved = arn_ensure(B, n, kdim, kPer == 1, (2 * (size_t)kdim + 1) * xstride);
+  QD_REQUIRE(!moved || first == 1, QD_ERR_INVALID, "the open solve's basis is gone: start it again");
   B.ncl = ncl;
   B.rows = rows;
   ArnArgs<MV, VV> A;

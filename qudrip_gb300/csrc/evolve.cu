@@ -209,6 +209,7 @@ static bool arnoldi_ground_res(qd_ham* H, cplx* psi, int kdim, int add_dim, bool
   Ctx* ctx = H->ctx;
   if (!extend) {
     if (H->arn_gs) H->arn_gs->open = false;
+    if (H->arnoldi_gs) H->arnoldi_gs->open = false;
     if (!arn_res_fits(H, kdim)) return false;
     if (!H->arn_gs) H->arn_gs.reset(new ArnRes());
     bool has_imag = false;
@@ -229,7 +230,6 @@ static bool arnoldi_ground_res(qd_ham* H, cplx* psi, int kdim, int add_dim, bool
     B.open = false;
     if (!arn_res_steps(H, B, psi, kdim, B.real_start, B.act + 1, B.act + steps)) return false;
     B.open = true;
-    if (H->arnoldi_gs) H->arnoldi_gs->open = false;
     B.act = B.host.stop ? B.host.stop : B.act + steps;  // expandBasis<0>: the breaking step counts
     B.broke = B.host.stop != 0;
   }

@@ -128,6 +128,8 @@ void ham_scale(qd_ham* H, cplx s) {
   H->ws.reset();
   H->arnoldi.reset();
   H->arnoldi_gs.reset();
+  H->arn_ev.reset();
+  H->arn_gs.reset();
   H->fx.reset();
   H->fx_state = 0;
   H->mfx.reset();
