@@ -548,7 +548,7 @@ static void arnoldi_ground_call(qd_ham* ham, qd_state* psi, int t, const qd_lanc
   QD_REQUIRE(t >= 0 && t < psi->nt, QD_ERR_INVALID, "bad column");
   QD_REQUIRE(psi->dim == ham->dim, QD_ERR_INVALID, "dimension mismatch");
   CacheGuard dg(ham->ctx);
-  const double prev = (extend && ham->arnoldi_gs) ? ham->arnoldi_gs_ritz : 0.0;
+  const double prev = extend ? ham->arnoldi_gs_ritz : 0.0;
   std::memset(res, 0, sizeof(*res));
   arnoldi_ground(ham, psi->col(t), opts->krylov_dim, opts->add_dim, extend, evals_out, res);
   res->err = std::fabs(res->ritz_value - prev);

@@ -55,3 +55,19 @@ def test_scaling_the_operator_ends_its_open_solve(ctx, monkeypatch, system, fact
     b.getGroundState(fresh, psi2, 0, ADD)
     assert np.array_equal(a.eigenvalues(), b.eigenvalues())
     assert np.array_equal(psi.get(0), psi2.get(0))
+
+
+@pytest.mark.parametrize("system", [hubbard, xxz])
+@pytest.mark.parametrize("form", ["one", "split"])
+def test_a_grown_solve_reports_the_change_of_its_lowest_eigenvalue(ctx, monkeypatch, system, form):
+    if form == "split":
+        monkeypatch.setenv("QD_KRYLOV_STEP", "split")
+    sec, ham = system()
+    H = sec.lower(ham)
+    psi = start(sec)
+    solver = q.Arnoldi.getSolver(sec, KDIM)
+    last = 0.0
+    for _ in range(3):
+        r = solver.getGroundState(H, psi, 0, ADD)
+        assert r.err == abs(r.ritz_value - last)  # |lambda_0| first, then |lambda_0 - previous lambda_0|
+        last = r.ritz_value
