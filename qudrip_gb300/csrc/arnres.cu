@@ -560,12 +560,13 @@ bool arn_res_fits(qd_ham* H, int kdim) {
 static bool arn_ensure(ArnRes& B, int64_t n, int kdim, bool real_v, size_t slots) {
   bool moved = false;
   if (B.n != n || B.kdim != kdim || B.real_v != real_v) {
-    B.n = n;
+    B.n = 0;  // until the memory is there
     B.kdim = kdim;
     B.real_v = real_v;
     B.ld = (n + 31) / 32 * 32;
     B.ncl = 0;
     B.V.alloc((size_t)(kdim + 1) * B.ld * (real_v ? sizeof(double) : sizeof(cplx)));
+    B.n = n;
     moved = true;
   }
   if (!B.hcol.p) B.hcol.alloc((size_t)kArnLdh * (kArnMaxExp + 1));
