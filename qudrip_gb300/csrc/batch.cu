@@ -431,7 +431,7 @@ __device__ double inst_sum(double block_total, BlockScratch& S, int& buf) {
 // (128 points a round, a warp on each SM quarter: is any leading minor of T - x not positive?), the vector by
 // three steps of inverse iteration with partial pivoting (the reorthogonalised Lanczos matrix has no spurious
 // copies).  Eigenvalues by QL and the same iteration on one thread took 5 ms at n = 80, FP64 instructions
-// taking 72 cycles each.
+// taking 72 cycles each.  A matrix that is not finite has NaN for its eigenvalue.
 constexpr int kTriWork = kBatchMaxSteps + 2;
 __device__ double block_tridiag_lowest(int n, const double* d, const double* e, double* y, BlockScratch& S) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -443,8 +443,10 @@ __device__ double block_tridiag_lowest(int n, const double* d, const double* e, 
   int* piv = reinterpret_cast<int*>(e2 + kTriWork);
   if (warp == 0) {
     double glo = 1e300, dmin = 1e300;
+    bool bad = false;  // fmin drops a NaN
     for (int i = lane; i < n; i += 32) {
       const double el = i > 0 ? fabs(e[i - 1]) : 0.0, er = i + 1 < n ? fabs(e[i]) : 0.0;
+      bad |= !isfinite(d[i]) || !isfinite(er);
       glo = fmin(glo, d[i] - (el + er));
       dmin = fmin(dmin, d[i]);
       e2[i] = er * er;
@@ -453,9 +455,11 @@ __device__ double block_tridiag_lowest(int n, const double* d, const double* e, 
       glo = fmin(glo, __shfl_xor_sync(0xffffffffu, glo, o));
       dmin = fmin(dmin, __shfl_xor_sync(0xffffffffu, dmin, o));
     }
+    bad = __any_sync(0xffffffffu, bad);
     if (lane == 0) {  // the lowest eigenvalue is at most the least diagonal element
-      S.ga = glo - 1e-15 * fabs(glo);
-      S.gb = dmin;
+      const double nan = __longlong_as_double(0x7ff8000000000000ll);
+      S.ga = bad ? nan : glo - 1e-15 * fabs(glo);
+      S.gb = bad ? nan : dmin;
     }
   }
   __syncthreads();
