@@ -34,8 +34,6 @@ __device__ __forceinline__ cplx vdotfma(cplx a, cplx b, cplx acc) {
 
 __device__ __forceinline__ double vadd(double a, double b) { return a + b; }
 __device__ __forceinline__ cplx vadd(cplx a, cplx b) { return mkc(a.re + b.re, a.im + b.im); }
-__device__ __forceinline__ double vsub(double a, double b) { return a - b; }
-__device__ __forceinline__ cplx vsub(cplx a, cplx b) { return mkc(a.re - b.re, a.im - b.im); }
 __device__ __forceinline__ double vscale(double s, double x) { return s * x; }
 __device__ __forceinline__ cplx vscale(double s, cplx x) { return mkc(s * x.re, s * x.im); }
 __device__ __forceinline__ double vnorm2(double x) { return x * x; }
