@@ -23,6 +23,8 @@
 #include <cstring>
 #include <vector>
 
+#include "dense.h"
+#include "evolve.cuh"
 #include "fxstep.cuh"
 #include "krylov.cuh"
 #include "lanres.cuh"
@@ -1424,6 +1426,60 @@ struct EvolveGraph {
 
 void EvolveGraphDeleter::operator()(EvolveGraph* g) const { delete g; }
 
+// One Krylov step in place with its exponential formed on the host, the recurrence in one launch; the Krylov
+// dimension, or 0 with nothing run.
+template <typename MV>
+static int lanczos_evolve_host(qd_ham* H, const MV* vals, LanczosBuffers<cplx>& B, Workspace& W, cplx* psi, double h,
+                               int kdim, cplx* y) {
+  Ctx* ctx = H->ctx;
+  const int64_t n = H->dim;
+  bool has_imag = false;
+  state_norm2_imag(H, psi, &has_imag);
+  QD_CUDA(cudaMemsetAsync(B.stop.p, 0, sizeof(int), ctx->stream));
+  const double one = 1.0;
+  QD_CUDA(cudaMemcpyAsync(B.scl.p, &one, sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  init_v0_kernel<cplx><<<vec_grid(ctx, n), kVecThreads, 0, ctx->stream>>>(n, psi, W.start_nrm2.p, B.V.p);
+  QD_CHECK_LAUNCH();
+  QD_LAUNCHED(ctx);
+  LanRun<MV, cplx> r{};
+  r.vals = vals;
+  r.rule = kLanPaige;
+  r.V = B.V.p;
+  r.ld = B.ld;
+  r.kdim = kdim;
+  r.first = 1;
+  r.last = kdim;
+  r.stop_below = 1e-10;
+  r.alpha = B.alpha.p;
+  r.nrm = B.nrm.p;
+  r.scl = B.scl.p;
+  r.stop = B.stop.p;
+  r.flags = lan_flags(W);
+  r.slots = &W.lan_slots;
+  if (!lan_res_run(H, r)) return 0;
+  std::vector<cplx> alpha(kdim + 1);
+  std::vector<double> nrm(kdim + 1), scl(kdim + 1);
+  int stop = 0;
+  QD_CUDA(cudaMemcpyAsync(alpha.data(), B.alpha.p, (kdim + 1) * sizeof(cplx), cudaMemcpyDeviceToHost, ctx->stream));
+  QD_CUDA(cudaMemcpyAsync(nrm.data(), B.nrm.p, (kdim + 1) * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  QD_CUDA(cudaMemcpyAsync(scl.data(), B.scl.p, (kdim + 1) * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  QD_CUDA(cudaMemcpyAsync(&stop, B.stop.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  fx_flags(ctx, W.lan_flags.p);
+  const int act = stop ? stop : kdim;  // expandBasis<0>'s count: the breaking step is kept
+  dense::Mat K((size_t)act * act, dense::cd(0.0, 0.0)), E;
+  for (int i = 0; i < act; ++i) {
+    K[(size_t)i * act + i] = dense::cd(0.0, -h * alpha[i + 1].re);
+    if (i + 1 < act) K[(size_t)i * act + i + 1] = K[(size_t)(i + 1) * act + i] = dense::cd(0.0, -h * nrm[i + 1]);
+  }
+  QD_REQUIRE(dense::expm(K, act, E), QD_ERR_INVALID, "matrix exponential failed");
+  std::vector<cplx> e(act);
+  for (int j = 0; j < act; ++j) e[j] = mkc(E[j].real() * scl[j], E[j].imag() * scl[j]);
+  QD_CUDA(cudaMemcpyAsync(y, e.data(), act * sizeof(cplx), cudaMemcpyHostToDevice, ctx->stream));
+  launch_ev_combine(ctx, n, B.V.p, B.ld, act, y, psi);
+  QD_CUDA(cudaStreamSynchronize(ctx->stream));
+  return act;
+}
+
 template <typename MV>
 static void lanczos_evolve_steps(qd_ham* H, cplx* psi, double h, int m, int nsteps, int* act_out,
                                  int64_t* matvecs_out) {
@@ -1450,6 +1506,20 @@ static void lanczos_evolve_steps(qd_ham* H, cplx* psi, double h, int m, int nste
   QD_CUDA(cudaMemsetAsync(G.matvecs.p, 0, sizeof(long long), ctx->stream));
   // one launch per Krylov step (lanres.cu) where the recurrence fits the grid
   bool res_run = lan_res_takes(H, false);
+  if (res_run && !(std::fabs(h) * 3.0 * ham_norm_inf(H) <= kLanMaxTheta)) {
+    int act = 1;
+    int64_t mv = 0;
+    for (int s = 0; s < nsteps && act; ++s, mv += act) {
+      act = lanczos_evolve_host<MV>(H, vals, B, W, psi, h, kdim, G.y.p);
+      QD_REQUIRE(act || s == 0, QD_ERR_UNSUPPORTED, "the persistent recurrence's grid does not fit any more");
+    }
+    if (act) {
+      if (act_out) *act_out = act;
+      if (matvecs_out) *matvecs_out = mv;
+      return;
+    }
+    res_run = false;
+  }
   if (res_run) {
     int* flags = lan_flags(W);
     for (int s = 0; s < nsteps && res_run; ++s) {

@@ -230,7 +230,8 @@ __device__ __forceinline__ double lan_redot(cplx a, cplx b, double acc) {
 }
 
 // y = exp(-i h T) e_0, T = tridiag(al[0 .. act), be[1 .. act)), by one warp: Taylor terms on sub-steps of
-// infinity-norm at most 1 (as texp_kernel, krylov.cu, with its terms counted from the remainder bound).
+// infinity-norm at most 1 (as texp_kernel, krylov.cu, with its terms counted from the remainder bound).  The
+// caller bounds ||h T|| (kLanMaxTheta, krylov.cu).
 __device__ __forceinline__ void lan_texp(int act, double h, double d, double e, double& yr, double& yi) {
   const int lane = threadIdx.x & 31;
   double em = __shfl_up_sync(0xffffffffu, e, 1);
@@ -238,7 +239,8 @@ __device__ __forceinline__ void lan_texp(int act, double h, double d, double e, 
   const double rs = fabs(d) + fabs(e) + fabs(em);
   const unsigned mx = __reduce_max_sync(0xffffffffu, q_mag(rs));
   const double theta = __hiloint2double((int)mx, -1) * fabs(h);
-  const int steps = (theta <= 1e6) ? max(1, (int)ceil(theta)) : 1;  // a NaN gives NaNs either way
+  // one for a NaN and for what a run leaves whose wait has run out (its result is discarded)
+  const int steps = (theta <= 2.0 * kLanMaxTheta) ? max(1, (int)ceil(theta)) : 1;
   const double hs = h / steps, th = theta / steps;
   // lane p holds hs / p; terms to th^p / p! <= 1e-18
   const double f = lane > 0 ? hs / lane : 0.0;
