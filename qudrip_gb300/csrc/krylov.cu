@@ -1506,7 +1506,8 @@ static void lanczos_evolve_steps(qd_ham* H, cplx* psi, double h, int m, int nste
   QD_CUDA(cudaMemsetAsync(G.matvecs.p, 0, sizeof(long long), ctx->stream));
   // one launch per Krylov step (lanres.cu) where the recurrence fits the grid
   bool res_run = lan_res_takes(H, false);
-  if (res_run && !(std::fabs(h) * 3.0 * ham_norm_inf(H) <= kLanMaxTheta)) {
+  const double theta = res_run ? std::fabs(h) * 3.0 * ham_norm_inf(H) : 0.0;
+  if (theta > kLanMaxTheta && std::isfinite(theta)) {
     int act = 1;
     int64_t mv = 0;
     for (int s = 0; s < nsteps && act; ++s, mv += act) {

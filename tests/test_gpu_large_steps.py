@@ -32,3 +32,14 @@ def test_a_long_step_on_a_closed_space(ctx, system, rows, theta):
     assert act == 3
     ref = v @ (np.exp(-2j * h * w) * (v.conj().T @ x))
     assert np.linalg.norm(st.get(1) - ref) <= 2 * (2 * rows + 33) * 2.3e-16 * theta
+
+
+@pytest.mark.parametrize("h", [np.nan, np.inf])
+def test_a_step_that_is_not_finite_gives_nan(ctx, h):
+    spec, ham = chains.xxz_chain(10, 1.0, 0.7, True, np.linspace(-1, 1, 10))
+    sec = q.Sector(spec.index, spec.constraints)
+    H = sec.lower(ham)
+    st = q.getState(sec, 2)
+    st.set(0, q.start_vector(sec.dim, 1).astype(complex))
+    q.lanczos_evolve(H, st, 0, 1, h, 12, 1)
+    assert np.isnan(st.get(1)).all()
