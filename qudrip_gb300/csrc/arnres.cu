@@ -500,10 +500,10 @@ __global__ void __launch_bounds__(kArnThreads, 1) arn_kernel(ArnArgs<MV, VV> A) 
   __syncthreads();
   const bool ok = arn_expm(hs, act, A.h, A.herm != 0, tt, y, S.red);
   if (blockIdx.x == 0 && tid == 0) A.st->need_host = ok ? 0 : 1;
-  if (!ok || *reinterpret_cast<volatile int*>(X.abort) == kXAborted) return;
+  if (!ok) return;
   if (tid < act) y[tid] = vscale(S.scl[tid], y[tid]);
   __syncthreads();
-  // psi_out = sum_j y_j v_j on the block's rows (psi_in is read no more: every block has passed step 1)
+  // psi_out = sum_j y_j v_j on the block's rows
   if constexpr (kPer == 2) {
     cplx* out = A.psi_out + r0;
     const int JC = R > 0 ? min(min(T / R, act), 8) : 1;
@@ -652,7 +652,10 @@ static bool arn_launch(qd_ham* H, const MV* vals, ArnRes& B, const cplx* psi_in,
   A.first = first;
   A.last = last;
   A.herm = (H->flags & QD_HAM_HERMITIAN) ? 1 : 0;
-  A.psi_out = psi_out;
+  // the blocks write their rows one by one: apart from the caller's state until none of them has given up a wait
+  const bool apart = kExp && !one;
+  if (apart && B.out.n < (size_t)n) B.out.alloc(n);
+  A.psi_out = apart ? B.out.p : psi_out;
   A.h = h;
   A.slots = reinterpret_cast<double*>(B.slots.p + sizeof(ArnStatus));
   A.xstride = xstride;
@@ -675,6 +678,7 @@ static bool arn_launch(qd_ham* H, const MV* vals, ArnRes& B, const cplx* psi_in,
   allow_dynamic_smem(kern, ctx->device);
   QD_CUDA(cudaLaunchKernelEx(&cfg, kern, A));
   QD_LAUNCHED(ctx);
+  if (apart) launch_commit(ctx, n, B.out.p, psi_out, &A.st->abort, &A.st->need_host);
   QD_CUDA(cudaMemcpyAsync(&B.host, A.st, sizeof(ArnStatus), cudaMemcpyDeviceToHost, ctx->stream));
   QD_CUDA(cudaStreamSynchronize(ctx->stream));
   QD_REQUIRE(B.host.abort != kXAborted, QD_ERR_TIMEOUT, "an Arnoldi step's blocks did not meet within the wait limit");

@@ -29,6 +29,7 @@ struct ArnRes {
   bool real_v = false; // V holds reals
   int ncl = 0, rows = 0;  // clusters of the grid and rows per block (0: not chosen yet)
   DBuf<char> V;        // (kdim + 1) x ld, unnormalised
+  DBuf<cplx> out;      // the evolved state before it replaces the caller's
   DBuf<cplx> hcol;     // Hessenberg column i at i * (kArnMaxVecs + 1)
   DBuf<char> slots;    // ArnStatus, then the exchange slots (gridx.cuh)
   ArnStatus host{};    // the last run's status

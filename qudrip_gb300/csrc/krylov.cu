@@ -315,6 +315,19 @@ __global__ void __launch_bounds__(kVecThreads) ritz_kernel(int64_t n, const VV* 
   }
 }
 
+__global__ void __launch_bounds__(kVecThreads) commit_kernel(int64_t n, const cplx* src, cplx* dst, const int* abort,
+                                                             const int* other) {
+  if (*abort == 1 || (other && *other != 0)) return;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    dst[i] = src[i];
+}
+
+void launch_commit(Ctx* ctx, int64_t n, const cplx* src, cplx* dst, const int* abort, const int* other) {
+  commit_kernel<<<vec_grid(ctx, n), kVecThreads, 0, ctx->stream>>>(n, src, dst, abort, other);
+  QD_CHECK_LAUNCH();
+  QD_LAUNCHED(ctx);
+}
+
 void launch_ritz(Ctx* ctx, int64_t n, const void* V, bool real_v, int64_t ld, const double* y, int act, cplx* psi) {
   const int vg = vec_grid(ctx, n);
   if (real_v)
@@ -1418,6 +1431,7 @@ struct EvolveGraph {
   DBuf<double> nrm2;
   DBuf<int> has_im, act;
   DBuf<cplx> y;
+  DBuf<cplx> state;  // the persistent form's state between its first step and the end of the call
   DBuf<long long> matvecs;
   ~EvolveGraph() {
     if (exec) cudaGraphExecDestroy(exec);
@@ -1426,11 +1440,11 @@ struct EvolveGraph {
 
 void EvolveGraphDeleter::operator()(EvolveGraph* g) const { delete g; }
 
-// One Krylov step in place with its exponential formed on the host, the recurrence in one launch; the Krylov
-// dimension, or 0 with nothing run.
+// One Krylov step out <- V exp(-i h T) e_0 from psi (out may be psi) with its exponential formed on the host, the
+// recurrence in one launch; the Krylov dimension, or 0 with nothing run.
 template <typename MV>
-static int lanczos_evolve_host(qd_ham* H, const MV* vals, LanczosBuffers<cplx>& B, Workspace& W, cplx* psi, double h,
-                               int kdim, cplx* y) {
+static int lanczos_evolve_host(qd_ham* H, const MV* vals, LanczosBuffers<cplx>& B, Workspace& W, const cplx* psi,
+                               cplx* out, double h, int kdim, cplx* y) {
   Ctx* ctx = H->ctx;
   const int64_t n = H->dim;
   bool has_imag = false;
@@ -1475,13 +1489,13 @@ static int lanczos_evolve_host(qd_ham* H, const MV* vals, LanczosBuffers<cplx>& 
   std::vector<cplx> e(act);
   for (int j = 0; j < act; ++j) e[j] = mkc(E[j].real() * scl[j], E[j].imag() * scl[j]);
   QD_CUDA(cudaMemcpyAsync(y, e.data(), act * sizeof(cplx), cudaMemcpyHostToDevice, ctx->stream));
-  launch_ev_combine(ctx, n, B.V.p, B.ld, act, y, psi);
+  launch_ev_combine(ctx, n, B.V.p, B.ld, act, y, out);
   QD_CUDA(cudaStreamSynchronize(ctx->stream));
   return act;
 }
 
 template <typename MV>
-static void lanczos_evolve_steps(qd_ham* H, cplx* psi, double h, int m, int nsteps, int* act_out,
+static void lanczos_evolve_steps(qd_ham* H, const cplx* psi_in, cplx* psi, double h, int m, int nsteps, int* act_out,
                                  int64_t* matvecs_out) {
   Ctx* ctx = H->ctx;
   const int64_t n = H->dim;
@@ -1511,7 +1525,7 @@ static void lanczos_evolve_steps(qd_ham* H, cplx* psi, double h, int m, int nste
     int act = 1;
     int64_t mv = 0;
     for (int s = 0; s < nsteps && act; ++s, mv += act) {
-      act = lanczos_evolve_host<MV>(H, vals, B, W, psi, h, kdim, G.y.p);
+      act = lanczos_evolve_host<MV>(H, vals, B, W, s ? psi : psi_in, psi, h, kdim, G.y.p);
       QD_REQUIRE(act || s == 0, QD_ERR_UNSUPPORTED, "the persistent recurrence's grid does not fit any more");
     }
     if (act) {
@@ -1523,10 +1537,16 @@ static void lanczos_evolve_steps(qd_ham* H, cplx* psi, double h, int m, int nste
   }
   if (res_run) {
     int* flags = lan_flags(W);
+    // the steps' state is apart until all of them are done: a wait that runs out leaves the caller's as it was
+    const bool apart = n > kLanOneBlock;
+    if (apart && G.state.n < (size_t)n) G.state.alloc(n);
+    cplx* st = apart ? G.state.p : psi;
     for (int s = 0; s < nsteps && res_run; ++s) {
-      res_run = lan_res_evolve<MV>(H, vals, psi, B.V.p, B.ld, kdim, h, G.act.p, G.matvecs.p, flags, &W.lan_slots);
+      res_run = lan_res_evolve<MV>(H, vals, s ? st : psi_in, st, B.V.p, B.ld, kdim, h, G.act.p, G.matvecs.p, flags,
+                                   &W.lan_slots);
       QD_REQUIRE(res_run || s == 0, QD_ERR_UNSUPPORTED, "the persistent recurrence's grid does not fit any more");
     }
+    if (res_run && apart) launch_commit(ctx, n, st, psi, flags + 1, nullptr);
   }
   if (res_run) {
     int act = 0;
@@ -1538,6 +1558,8 @@ static void lanczos_evolve_steps(qd_ham* H, cplx* psi, double h, int m, int nste
     if (matvecs_out) *matvecs_out = mv;
     return;
   }
+  if (psi != psi_in)
+    QD_CUDA(cudaMemcpyAsync(psi, psi_in, n * sizeof(cplx), cudaMemcpyDeviceToDevice, ctx->stream));
   QD_CUDA(cudaMemcpyAsync(B.scl.p, &one, sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
   if (B.kind != 0) {
     B.drop_graph();
@@ -1614,12 +1636,10 @@ void lanczos_evolve(qd_ham* H, const cplx* psi_in, cplx* psi_out, double h, int 
   bool has_imag = false;
   const double hn = state_norm2_imag(H, psi_in, &has_imag);
   QD_REQUIRE(hn > 0.0 && std::isfinite(hn), QD_ERR_INVALID, "input state has zero or non-finite norm");
-  if (psi_out != psi_in)
-    QD_CUDA(cudaMemcpyAsync(psi_out, psi_in, n * sizeof(cplx), cudaMemcpyDeviceToDevice, ctx->stream));
   if (H->flags & QD_HAM_REAL)
-    lanczos_evolve_steps<double>(H, psi_out, h, m, nsteps, act_out, matvecs_out);
+    lanczos_evolve_steps<double>(H, psi_in, psi_out, h, m, nsteps, act_out, matvecs_out);
   else
-    lanczos_evolve_steps<cplx>(H, psi_out, h, m, nsteps, act_out, matvecs_out);
+    lanczos_evolve_steps<cplx>(H, psi_in, psi_out, h, m, nsteps, act_out, matvecs_out);
 }
 
 }  // namespace qd

@@ -159,6 +159,9 @@ Workspace& ham_workspace(qd_ham* H);
 unsigned step_wait_out_polls();
 // ||psi||^2 and whether psi has an imaginary part, on the host.
 double state_norm2_imag(qd_ham* H, const cplx* psi, bool* has_imag);
+// dst = src unless *abort is 1 or *other is not 0 (other may be null): a result that blocks wrote one by one
+// replaces a state only once none of them has given up.
+void launch_commit(Ctx* ctx, int64_t n, const cplx* src, cplx* dst, const int* abort, const int* other);
 // psi = sum_{k < act} y_k V[k] for a basis of reals or complex numbers.
 void launch_ritz(Ctx* ctx, int64_t n, const void* V, bool real_v, int64_t ld, const double* y, int act, cplx* psi);
 void ham_apply_c(qd_ham* H, const cplx* x, cplx* y);

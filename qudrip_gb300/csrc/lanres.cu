@@ -73,7 +73,8 @@ struct LanArgs {
   int* stop;
   int* ovf;
   // the Krylov exponential
-  cplx* psi;
+  const cplx* psi;  // the state, read in the first step only
+  cplx* out;        // the new one; may be psi
   double h;
   int* act;
   long long* matvecs;
@@ -549,13 +550,12 @@ __global__ void __launch_bounds__(kLanThreads, 1) lan_kernel(LanArgs<MV, VV> A) 
       if (tid < act) y[tid] = mkc(yr * tscl[tid], yi * tscl[tid]);
     }
     __syncthreads();
-    if (*reinterpret_cast<volatile int*>(X.abort) == kXAborted) return;
     if (blockIdx.x == 0 && tid == 0) {
       *A.act = act;
       *A.matvecs += act;
     }
     if constexpr (sizeof(VV) == sizeof(cplx)) {
-      cplx* out = A.psi + r0;  // read by the others in the first step only
+      cplx* out = A.out + r0;
       for (int r = tid; r < R; r += T) {
         const cplx* v = reinterpret_cast<const cplx*>(Vg) + r;
         cplx a = mkc(0.0, 0.0);
@@ -599,7 +599,7 @@ static bool lan_plan(qd_ham* H, K kern1, K kern_many, LanPlan& P, cudaLaunchConf
                      cudaLaunchAttribute (&at)[2], K& kern) {
   Ctx* ctx = H->ctx;
   const int64_t n = H->dim;
-  const int csize = n <= 64 ? 1 : (n <= lan_wide_rows<VV>() ? 8 : 4);  // one block: an exchange would cost more than it saves
+  const int csize = n <= kLanOneBlock ? 1 : (n <= lan_wide_rows<VV>() ? 8 : 4);  // one block: an exchange would cost more than it saves
   kern = csize == 1 ? kern1 : kern_many;
   at[0].id = cudaLaunchAttributeCooperative;
   at[0].val.cooperative = 1;
@@ -733,8 +733,8 @@ template bool lan_res_run<double, cplx>(qd_ham*, const LanRun<double, cplx>&);
 template bool lan_res_run<cplx, cplx>(qd_ham*, const LanRun<cplx, cplx>&);
 
 template <typename MV>
-bool lan_res_evolve(qd_ham* H, const MV* vals, cplx* psi, cplx* V, int64_t ld, int kdim, double h, int* act,
-                    long long* matvecs, int* flags, DBuf<double>* slots) {
+bool lan_res_evolve(qd_ham* H, const MV* vals, const cplx* psi, cplx* out, cplx* V, int64_t ld, int kdim, double h,
+                    int* act, long long* matvecs, int* flags, DBuf<double>* slots) {
   Ctx* ctx = H->ctx;
   LanPlan& P = ham_workspace(H).lan_plan[4];
   cudaLaunchConfig_t cfg = {};
@@ -746,6 +746,7 @@ bool lan_res_evolve(qd_ham* H, const MV* vals, cplx* psi, cplx* V, int64_t ld, i
   LanArgs<MV, cplx> A = lan_args<MV, cplx>(H, vals, P, V, ld, 1, kdim, 2, flags, slots, nullptr);
   A.stop_below = 1e-10;
   A.psi = psi;
+  A.out = out;
   A.h = h;
   A.act = act;
   A.matvecs = matvecs;
@@ -753,7 +754,7 @@ bool lan_res_evolve(qd_ham* H, const MV* vals, cplx* psi, cplx* V, int64_t ld, i
   QD_LAUNCHED(ctx);
   return true;
 }
-template bool lan_res_evolve<double>(qd_ham*, const double*, cplx*, cplx*, int64_t, int, double, int*, long long*, int*, DBuf<double>*);
-template bool lan_res_evolve<cplx>(qd_ham*, const cplx*, cplx*, cplx*, int64_t, int, double, int*, long long*, int*, DBuf<double>*);
+template bool lan_res_evolve<double>(qd_ham*, const double*, const cplx*, cplx*, cplx*, int64_t, int, double, int*, long long*, int*, DBuf<double>*);
+template bool lan_res_evolve<cplx>(qd_ham*, const cplx*, const cplx*, cplx*, cplx*, int64_t, int, double, int*, long long*, int*, DBuf<double>*);
 
 }  // namespace qd

@@ -38,10 +38,14 @@ struct LanRun {
 template <typename MV, typename VV>
 bool lan_res_run(qd_ham* H, const LanRun<MV, VV>& r);
 
-// One Krylov step psi <- V exp(-i h T) e_0 of dimension kdim (<= 32), psi in place.  act and the product
-// count are written on the device.  False: nothing launched.
+// Sectors of so few rows run on one block, which waits for no other.
+constexpr int64_t kLanOneBlock = 64;
+
+// One Krylov step out <- V exp(-i h T) e_0 of dimension kdim (<= 32) from psi; out may be psi.  A run whose wait
+// runs out leaves rows of two times in out.  act and the product count are written on the device.  False:
+// nothing launched.
 template <typename MV>
-bool lan_res_evolve(qd_ham* H, const MV* vals, cplx* psi, cplx* V, int64_t ld, int kdim, double h, int* act,
-                    long long* matvecs, int* flags, DBuf<double>* slots);
+bool lan_res_evolve(qd_ham* H, const MV* vals, const cplx* psi, cplx* out, cplx* V, int64_t ld, int kdim, double h,
+                    int* act, long long* matvecs, int* flags, DBuf<double>* slots);
 
 }  // namespace qd
