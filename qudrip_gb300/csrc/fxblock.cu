@@ -30,6 +30,7 @@
 #include <cstring>
 #include <vector>
 
+#include "fxblock.cuh"
 #include "fxstep.cuh"
 #include "fxsum.cuh"
 #include "ham.cuh"
@@ -37,20 +38,10 @@
 
 namespace qd {
 
-constexpr int kBlkMaxCross = 8;
 constexpr int kBlkMaxBits = 16;  // per part: tables of 2^16 entries at most
 
-struct BlockRows {
-  const uint32_t* state;     // the basis in 32 bits
-  const int32_t* off;        // 2^highbits: first row of block h
-  const uint16_t* rank_low;  // 2^lowbits: rank of l among the low parts of its popcount
-  const uint8_t* ldeg;       // 2^lowbits: low targets of l
-  const uint16_t* ladj;      // 2^lowbits x lstride: their positions in the block
-  const uint8_t* hdeg;       // 2^highbits: high targets of h
-  const int32_t* hadj;       // 2^highbits x hstride: first row of each target block
+struct BlockRows : BlockTables {
   const __int128* X;
-  int lowbits, lstride, hstride, ncross;
-  uint32_t cross[3 * kBlkMaxCross];  // support, input pattern, flip
   __device__ const BlockRows& bind(unsigned char*) const { return *this; }
   __device__ __forceinline__ __int128 row_sum(int64_t r) const {
     const uint32_t s = __ldcs(state + r);
@@ -446,8 +437,8 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) lz_fx_blkstep_kerne
   }
 }
 
-static BlockRows block_rows(const FxForm& f, const __int128* X) {
-  BlockRows B;
+BlockTables block_tables(const FxForm& f) {
+  BlockTables B;
   std::memset(&B, 0, sizeof(B));
   B.state = f.blk_state32.p;
   B.off = f.blk_off.p;
@@ -456,12 +447,18 @@ static BlockRows block_rows(const FxForm& f, const __int128* X) {
   B.ladj = f.blk_ladj.p;
   B.hdeg = f.blk_hdeg.p;
   B.hadj = f.blk_hadj.p;
-  B.X = X;
   B.lowbits = f.blk_lowbits;
   B.lstride = f.blk_lstride;
   B.hstride = f.blk_hstride;
   B.ncross = f.blk_ncross;
   for (int q = 0; q < 3 * kBlkMaxCross; ++q) B.cross[q] = f.blk_cross[q];
+  return B;
+}
+
+static BlockRows block_rows(const FxForm& f, const __int128* X) {
+  BlockRows B;
+  static_cast<BlockTables&>(B) = block_tables(f);
+  B.X = X;
   return B;
 }
 

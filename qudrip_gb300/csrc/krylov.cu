@@ -40,9 +40,14 @@ constexpr int kVecThreads = 256;
 // the blocks' rows soon do not fit (complex vectors from about 600,000 on, which then run step by step).
 constexpr int64_t kLanResMax = 3 << 18;
 // With the uniform-coupling form, whose one-launch step is faster: L = 12 686 -> 433 us, L = 16 906 -> 647,
-// L = 18 (48,620 rows) 1,152 -> 822, L = 19 (92,378) 1,356 -> 1,227 on the stored columns but 1,436 -> 1,682
-// matrix-free, and both keep one route so that their bits stay the same.
+// L = 18 (48,620 rows) 1,152 -> 822, L = 20 (184,756) 1,832 -> 1,672.  The copies of the vectors for the sums
+// take 16 bytes a row and step here and two vectors' there; the line is where that is 100 MB at 100 steps.
 constexpr int64_t kLanResMaxUniform = 1 << 16;
+// With the FP64 product of the compiled transitions on real vectors, whose integer work the launched product
+// spreads over more threads: couplings per bond L = 10 761 -> 390 us, L = 16 1,414 -> 880, L = 18 1,604 ->
+// 1,061, L = 20 (184,756 rows) 2,506 -> 2,198, but L = 21 (352,716) 3,473 -> 3,609.  Complex vectors gain up to
+// kLanResMax: L = 21 7,537 -> 5,950.
+constexpr int64_t kLanResMaxMf = 1 << 18;
 // Hermitian::LanczosSolver keeps its basis up to this size instead of forming it twice
 constexpr int64_t kHermBasisBytes = 256ll << 20;
 
@@ -770,18 +775,18 @@ void time_spmv(qd_ham* H, int spmv, int iters, double* avg_ms, double* bytes_per
 }
 
 // ---------------------------------------------------------------- Lanczos
-// Whether a solve takes the persistent recurrence (lanres.cu): sectors up to kLanResMax rows, where the
+// Whether a solve takes the persistent recurrence (lanres.cu): sectors up to `most` rows, where the
 // launches and reductions of a step outweigh its memory traffic.  Served requests keep the
 // separate launches (a co-resident grid waits for room beside the other lanes' kernels), and so do
 // QD_KRYLOV_STEP=split and QD_LANCZOS_STEP=split.
-static bool lan_res_takes(const qd_ham* H, bool uniform) {
+static bool lan_res_takes(const qd_ham* H, int64_t most) {
   const char* e = std::getenv("QD_KRYLOV_STEP");
   if (H->one_shot || !fx_one_launch_step() || (e && std::strcmp(e, "split") == 0)) return false;
   static const bool coop = [&] {  // once per process (thread-safe initialisation)
     int v = 0;
     return cudaDeviceGetAttribute(&v, cudaDevAttrCooperativeLaunch, H->ctx->device) == cudaSuccess && v != 0;
   }();
-  return coop && H->dim >= 1 && H->dim <= (uniform ? kLanResMaxUniform : kLanResMax);
+  return coop && H->dim >= 1 && H->dim <= most;
 }
 
 // The flags of a persistent run, cleared on the stream.
@@ -793,10 +798,20 @@ static int* lan_flags(Workspace& W) {
 
 // Steps k_first .. k_last in one persistent launch; false: not launched.
 template <typename MV, typename VV>
-static bool lanczos_run_res(qd_ham* H, const MV* vals, LanczosBuffers<VV>& B, int k_first, int k_last, Workspace& W,
-                            const FxForm* form) {
+static bool lanczos_run_res(qd_ham* H, const MV* vals, bool mf, LanczosBuffers<VV>& B, int k_first, int k_last,
+                            Workspace& W, const FxForm* form) {
   LanRun<MV, VV> r{};
   r.vals = vals;
+  r.mf = mf;
+  // the uniform form's columns computed where they are for the launched step (codes 121 and 122)
+  if (!mf && form && ((form->use_slots && form->slots_state > 0) || (form->use_blk && form->blk_state > 0))) {
+    try {
+      ham_build_matrix_free(H);
+      r.mf = true;
+    } catch (const Error&) {  // more transitions than the compiled form keeps: the stored columns
+      clear_error();
+    }
+  }
   r.rule = kLanLocal;
   r.form = form;
   r.V = B.V.p;
@@ -944,7 +959,8 @@ static void lanczos_ground_impl(qd_ham* H, cplx* psi, const double* psi_nrm2, co
   fxk = form ? 1 : 0;
   const bool fx = fxk == 1;
   const int steps = (o.add_dim > 0 && o.add_dim < kdim) ? o.add_dim : kdim;  // add_dim of an incremental start
-  const bool res_run = lan_res_takes(H, fx) && lanczos_run_res<MV, VV>(H, vals, B, 1, steps, W, form);
+  const int64_t most = fx ? kLanResMaxUniform : (mf && std::is_same<VV, double>::value ? kLanResMaxMf : kLanResMax);
+  const bool res_run = lan_res_takes(H, most) && lanczos_run_res<MV, VV>(H, vals, mf, B, 1, steps, W, form);
   const int fxF = fx ? form->F : 0;
   const bool one_launch = fx && fx_one_launch_step() && !H->one_shot;
   // the column source of the fixed-point form is part of what a captured recurrence launches
@@ -1033,7 +1049,7 @@ static void lanczos_finish(qd_ham* H, cplx* psi, const double* psi_nrm2, const q
     QD_LAUNCHED(ctx);
     QD_CUDA(cudaMemsetAsync(B.stop.p, 0, sizeof(int), ctx->stream));
     if (res_run) {
-      QD_REQUIRE((lanczos_run_res<MV, VV>(H, vals, B, 1, act, W, form)), QD_ERR_UNSUPPORTED,
+      QD_REQUIRE((lanczos_run_res<MV, VV>(H, vals, mf, B, 1, act, W, form)), QD_ERR_UNSUPPORTED,
                  "the persistent recurrence's grid does not fit any more");
       fx_flags(ctx, W.lan_flags.p);
     } else {
@@ -1084,7 +1100,7 @@ static void lanczos_extend_impl(qd_ham* H, cplx* psi, const qd_lanczos_opts& o, 
   const FxForm* form = W.lz_fxk == 1 ? (W.lz_mf ? H->mfx.get() : H->fx.get()) : nullptr;
   if (!stop && add > 0) {
     if (W.lz_res)
-      QD_REQUIRE((lanczos_run_res<MV, VV>(H, vals, B, B.done + 1, B.done + add, W, form)), QD_ERR_UNSUPPORTED,
+      QD_REQUIRE((lanczos_run_res<MV, VV>(H, vals, W.lz_mf != 0, B, B.done + 1, B.done + add, W, form)), QD_ERR_UNSUPPORTED,
                  "the persistent recurrence's grid does not fit any more");
     else
       lanczos_run<MV, VV>(H, vals, B, B.done + 1, B.done + add, W, W.lz_mf, W.lz_fxk, form);
@@ -1215,7 +1231,7 @@ static void herm_lanczos_impl(qd_ham* H, cplx* psi, const double* psi_nrm2, int 
   const int vg = vec_grid(ctx, n);
   // the basis kept, in one persistent launch (lanres.cu): the second pass would form the same vectors again
   const int64_t ldv = (n + 31) / 32 * 32;
-  if (lan_res_takes(H, false) && (int64_t)(kdim + 2) * ldv * (int64_t)sizeof(VV) <= kHermBasisBytes) {
+  if (lan_res_takes(H, kLanResMax) && (int64_t)(kdim + 2) * ldv * (int64_t)sizeof(VV) <= kHermBasisBytes) {
     LanczosBuffers<VV>& B = herm_buffers<VV>(W);
     B.ensure(n, kdim + 1);
     QD_CUDA(cudaMemsetAsync(B.stop.p, 0, sizeof(int), ctx->stream));
@@ -1519,7 +1535,7 @@ static void lanczos_evolve_steps(qd_ham* H, const cplx* psi_in, cplx* psi, doubl
   const double one = 1.0;
   QD_CUDA(cudaMemsetAsync(G.matvecs.p, 0, sizeof(long long), ctx->stream));
   // one launch per Krylov step (lanres.cu) where the recurrence fits the grid
-  bool res_run = lan_res_takes(H, false);
+  bool res_run = lan_res_takes(H, kLanResMax);
   const double theta = res_run ? std::fabs(h) * 3.0 * ham_norm_inf(H) : 0.0;
   if (theta > kLanMaxTheta && std::isfinite(theta)) {
     int act = 1;

@@ -122,7 +122,7 @@ struct Workspace {
   LanczosBuffers<cplx> lz_c;
   LanczosBuffers<double> hl_d;  // Hermitian::LanczosSolver's, apart from an open incremental solve
   LanczosBuffers<cplx> hl_c;
-  LanPlan lan_plan[5];          // real and complex, local and Paige's rule, the exponential
+  LanPlan lan_plan[7];          // real and complex: local and Paige's rule; the exponential; real and complex matrix-free
   DBuf<double> lan_slots;
   DBuf<char> lan_x;             // fixed-point copies of the basis (uniform couplings)
   DBuf<int> lan_flags;

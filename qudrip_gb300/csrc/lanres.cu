@@ -25,6 +25,11 @@
 // of the rest; 28 us before a block took its rows in order of their length),
 // real couplings per bond there 41 -> 19 us; Hermitian solver at dim 4,900 2.3
 // -> 0.42 ms a solve.
+//
+// A matrix-free solve forms its rows from the compiled transitions (couplings that differ: a test per
+// transition and a rank per entry, 33 us a step at dim 184,756 against 19 on the stored matrix) or from the
+// block tables of the sector (uniform couplings: 917 us a solve at 18 sites against 830 on the stored columns,
+// the same bits); it reads no stored matrix.
 // Mean error against 64-bit references over ten random cases each: ground-state
 // eigenvalues 5.4e-16 (launched step by step: 5.6e-16), evolved states 1.95e-15
 // (1.99e-15).
@@ -33,9 +38,12 @@
 #include <cstring>
 #include <vector>
 
+#include "fxblock.cuh"
 #include "gridx.cuh"
 #include "lanres.cuh"
+#include "mfrow.cuh"
 #include "qvec.cuh"
+#include "scan.cuh"
 
 namespace qd {
 
@@ -51,6 +59,14 @@ constexpr int64_t lan_wide_rows() {
   return sizeof(VV) == sizeof(double) ? 1 << 17 : 1 << 15;
 }
 constexpr int kLanMaxExp = 32;
+// A block's rows of three vectors and their order by length; the transitions' 16-byte words follow.
+template <typename VV>
+__host__ __device__ constexpr size_t lan_rows_smem(int rows) {
+  return ((size_t)rows * (3 * sizeof(VV) + sizeof(short)) + 15) / 16 * 16;
+}
+static_assert(sizeof(MfEntry) % 16 == 0 && alignof(MfEntry) <= 16 &&
+                  2 * sizeof(uint2) + sizeof(cplx) <= sizeof(MfEntry),
+              "staged behind the rows in either form, aligned");
 
 template <typename MV, typename VV>
 struct LanArgs {
@@ -63,7 +79,7 @@ struct LanArgs {
   const double* fxdiag;  // uniform couplings: the diagonal (null: zero), c 2^-F and F
   double cF;
   int F;
-  const int32_t *fxptr, *fxcol;  // its off-diagonal columns (null: from the CSR rows)
+  const int32_t *fxptr, *fxcol;  // its off-diagonal columns
   XInt* XV;              // fixed-point copy of V[k] at XV + (k - first + 1) ld
   VV* V;
   int first, last;
@@ -82,6 +98,17 @@ struct LanArgs {
   int xstride;
   GridX X;
 };
+
+// Columns from the compiled transitions: no stored matrix is read.
+template <typename MV, typename VV>
+struct LanMfArgs : LanArgs<MV, VV> {
+  MfRows mf;
+  Mf32 mf32;        // the ranking in 32 bits where that holds (nf > 0)
+  BlockTables blk;  // uniform couplings: the sector's block tables instead (state not null)
+  const MV* diag;   // the diagonal beside them (FP64 product)
+};
+template <typename MV, typename VV, bool kMf>
+using LanArgsOf = std::conditional_t<kMf, LanMfArgs<MV, VV>, LanArgs<MV, VV>>;
 
 __device__ __forceinline__ __int128 lan_shfl(__int128 v, int o) {
   const unsigned long long lo = __shfl_xor_sync(0xffffffffu, (unsigned long long)v, o);
@@ -122,35 +149,172 @@ __device__ __forceinline__ VV lan_row(const LanArgs<MV, VV>& A, const VV* x, int
   return acc;
 }
 
-// The same for uniform couplings: the 128-bit fixed-point copies (fxsum.cuh) that the blocks keep beside
-// their rows, summed exactly and rounded once; the diagonal apart.  Every off-diagonal value is one c,
-// explicit zeros skipped.  (Converting each gathered double instead took twice the FP64 product's time.)
-__device__ __forceinline__ double lan_row_uniform(const LanArgs<double, double>& A, const XInt* x, int64_t r,
-                                                  bool live, int sub, int lanes, double own) {
-  __int128 acc = 0;
-  if (live) {
-    const bool listed = A.fxptr != nullptr;  // the form's own list of off-diagonal columns
-    const int32_t* col = listed ? A.fxcol : A.colidx;
-    const int64_t e = listed ? (int64_t)__ldg(A.fxptr + r + 1) : __ldg(A.rowptr + r + 1);
-    for (int64_t k = (listed ? (int64_t)__ldg(A.fxptr + r) : __ldg(A.rowptr + r)) + sub; k < e; k += 4 * lanes) {
+// The transitions in shared memory, and which of the two ranks holds.
+template <typename MV>
+struct LanEnt {
+  const MfEntry* ent;          // 64-bit form
+  const uint2 *test, *move;    // 32-bit form: (support, output pattern), (flip, sign mask)
+  const MV* amp;
+};
+
+// The columns of row r from the transitions: take(c, a, on) with up to four at a time, in entry order,
+// every lanes-th transition from sub.  kUni: transitions of amplitude zero are no columns.
+template <bool kUni, typename MV, typename VV, typename F>
+__device__ __forceinline__ void lan_mf_columns(const LanMfArgs<MV, VV>& A, const LanEnt<MV>& E, int64_t r, int sub, int lanes,
+                                               F&& take) {
+  const uint64_t s = __ldg(A.mf.basis + r);
+  const int nent = A.mf.nent;
+  const bool narrow = A.mf32.nf > 0;
+  for (int e0 = 0; e0 < nent; e0 += 32) {
+    unsigned mask = 0;
+    if (narrow) {
+      for (int q = sub; q < 32 && e0 + q < nent; q += lanes) {
+        const uint2 t = E.test[e0 + q];
+        mask |= (unsigned)(((uint32_t)s & t.x) == t.y) << q;
+      }
+    } else {
+      for (int q = sub; q < 32 && e0 + q < nent; q += lanes)
+        mask |= (unsigned)((s & E.ent[e0 + q].sup) == E.ent[e0 + q].outb) << q;
+    }
+    while (mask) {
       int32_t c[4];
-      XInt xv[4];
+      MV a[4];
       bool on[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        on[u] = k + u * lanes < e;
-        if (on[u]) c[u] = __ldg(col + k + u * lanes);
-        if (!listed && on[u]) on[u] = c[u] != (int32_t)r && __ldg(A.vals + k + u * lanes) != 0.0;
+        on[u] = mask != 0;
+        if (on[u]) {
+          const int e = e0 + __ffs(mask) - 1;
+          mask &= mask - 1;
+          bool odd;
+          if (narrow) {
+            const uint2 m = E.move[e];
+            const uint32_t t = (uint32_t)s ^ m.x;
+            uint32_t col;
+            on[u] = mf_rank32(A.mf32, t, col);
+            c[u] = (int32_t)col;
+            a[u] = E.amp[e];
+            odd = __popc(t & m.y) & 1;
+          } else {
+            const uint64_t t = s ^ E.ent[e].flip;
+            const int64_t col = mf_rank(A.mf, t);
+            on[u] = col < A.mf.dim;
+            c[u] = (int32_t)col;
+            a[u] = amp_of((MV*)nullptr, E.ent[e].amp);
+            odd = __popcll(t & E.ent[e].jw) & 1;
+          }
+          if constexpr (kUni) on[u] = on[u] && a[u] != 0.0;
+          else if (odd) a[u] = vneg(a[u]);
+        }
       }
+      take(c, a, on);
+    }
+  }
+}
+
+// The same from the block tables.
+template <typename F>
+__device__ __forceinline__ void lan_block_columns(const BlockTables& B, int64_t r, int sub, int lanes, F&& take) {
+  const uint32_t s = __ldg(B.state + r), lmask = (1u << B.lowbits) - 1u;
+  const uint32_t h = s >> B.lowbits, l = s & lmask;
+  const int base = __ldg(B.off + h), i = (int)r - base, dl = __ldg(B.ldeg + l), d = dl + __ldg(B.hdeg + h);
+  const uint16_t* la = B.ladj + (size_t)l * B.lstride;
+  const int32_t* ha = B.hadj + (size_t)h * B.hstride - dl;
+  const double none[4] = {};
+  for (int j = sub; j < d; j += 4 * lanes) {
+    int32_t c[4];
+    bool on[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int q = j + u * lanes;
+      on[u] = q < d;
+      if (on[u]) c[u] = q < dl ? base + (int)__ldg(la + q) : __ldg(ha + q) + i;
+    }
+    take(c, none, on);
+  }
+  for (int t = sub; t < B.ncross; t += lanes) {
+    if ((s & B.cross[3 * t]) != B.cross[3 * t + 1]) continue;
+    const uint32_t c = s ^ B.cross[3 * t + 2];
+    const int32_t col[4] = {__ldg(B.off + (c >> B.lowbits)) + (int)__ldg(B.rank_low + (c & lmask)), 0, 0, 0};
+    const bool on[4] = {true, false, false, false};
+    take(col, none, on);
+  }
+}
+
+// One row of H x from the transitions; own = x of the row.
+template <typename MV, typename VV>
+__device__ __forceinline__ VV lan_row_mf(const LanMfArgs<MV, VV>& A, const LanEnt<MV>& ent, const VV* x, int64_t r,
+                                         bool live, int sub, int lanes, bool wait, VV own) {
+  VV acc = vzero(VV{});
+  if (live) {
+    if (sub == 0) acc = vfma(ld_ro(A.diag + r), own, acc);
+    lan_mf_columns<false>(A, ent, r, sub, lanes, [&](const int32_t (&c)[4], const MV (&a)[4], const bool (&on)[4]) {
+      VV xv[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u)
         if (on[u]) xv[u] = x_peek(x + c[u]);
 #pragma unroll
       for (int u = 0; u < 4; ++u)
         if (on[u]) {
-          x_await(A.X, x + c[u], xv[u]);
-          acc += x_value(xv[u]);
+          if (wait) x_await(A.X, x + c[u], xv[u]);
+          acc = vfma(a[u], xv[u], acc);
         }
+    });
+  }
+  for (int o = lanes >> 1; o > 0; o >>= 1) acc = vadd(acc, shfl_xor(acc, o));
+  return acc;
+}
+
+// The same for uniform couplings: the 128-bit fixed-point copies (fxsum.cuh) that the blocks keep beside
+// their rows, summed exactly and rounded once, so that the bits do not depend on where the columns come from
+// (the form's list, block tables or the transitions); the diagonal apart.  Every off-diagonal value is one c.  (Converting
+// each gathered double instead took twice the FP64 product's time.)
+template <bool kMf>
+__device__ __forceinline__ double lan_row_uniform(const LanArgsOf<double, double, kMf>& A, const LanEnt<double>& ent,
+                                                  const XInt* x, int64_t r, bool live, int sub, int lanes, double own) {
+  __int128 acc = 0;
+  if (live) {
+    if constexpr (kMf) {
+      auto add = [&](const int32_t (&c)[4], const double (&)[4], const bool (&on)[4]) {
+        XInt xv[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (on[u]) xv[u] = x_peek(x + c[u]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (on[u]) {
+            x_await(A.X, x + c[u], xv[u]);
+            acc += x_value(xv[u]);
+          }
+      };
+      if (A.blk.state) lan_block_columns(A.blk, r, sub, lanes, add);
+      else lan_mf_columns<true>(A, ent, r, sub, lanes, add);
+    } else {
+      // the form's own list of off-diagonal columns, or the stored rows, explicit zeros skipped (with the list
+      // alone the compiler's schedule takes 9.1 us a step at dim 12,870, with both 8.8)
+      const bool listed = A.fxptr != nullptr;
+      const int32_t* col = listed ? A.fxcol : A.colidx;
+      const int64_t e = listed ? (int64_t)__ldg(A.fxptr + r + 1) : __ldg(A.rowptr + r + 1);
+      for (int64_t k = (listed ? (int64_t)__ldg(A.fxptr + r) : __ldg(A.rowptr + r)) + sub; k < e; k += 4 * lanes) {
+        int32_t c[4];
+        XInt xv[4];
+        bool on[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          on[u] = k + u * lanes < e;
+          if (on[u]) c[u] = __ldg(col + k + u * lanes);
+          if (!listed && on[u]) on[u] = c[u] != (int32_t)r && __ldg(A.vals + k + u * lanes) != 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (on[u]) xv[u] = x_peek(x + c[u]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (on[u]) {
+            x_await(A.X, x + c[u], xv[u]);
+            acc += x_value(xv[u]);
+          }
+      }
     }
   }
   for (int o = lanes >> 1; o > 0; o >>= 1) acc += lan_shfl(acc, o);
@@ -273,8 +437,8 @@ __device__ __forceinline__ void lan_texp(int act, double h, double d, double e, 
 // their own order), so that a warp issues as many FP64 multiply-adds as its rows have entries and not as the
 // longest of 32 neighbours has.  scratch: (R / 32 + 2) kLanBins shorts.
 constexpr int kLanBins = 64;
-template <int T>
-__device__ void lan_sort_rows(const int64_t* rowptr, int64_t r0, int R, short* order, short* scratch) {
+template <int T, typename F>
+__device__ void lan_sort_rows(F&& length, int R, short* order, short* scratch) {
   const int tid = threadIdx.x, lane = tid & 31, chunks = (R + 31) / 32;
   short* base = scratch + chunks * kLanBins;
   for (int i = tid; i < chunks * kLanBins; i += T) scratch[i] = 0;
@@ -283,7 +447,7 @@ __device__ void lan_sort_rows(const int64_t* rowptr, int64_t r0, int R, short* o
     for (int r = tid; r - lane < R; r += T) {
       const unsigned live = __ballot_sync(0xffffffffu, r < R);
       if (r < R) {
-        const int len = (int)min(__ldg(rowptr + r0 + r + 1) - __ldg(rowptr + r0 + r), (int64_t)kLanBins - 1);
+        const int len = (int)min(length(r), (int64_t)kLanBins - 1);
         const unsigned same = __match_any_sync(live, len), before = same & ((1u << lane) - 1u);
         short* h = scratch + (r >> 5) * kLanBins + len;
         if (pass == 0) {
@@ -315,8 +479,20 @@ __device__ void lan_sort_rows(const int64_t* rowptr, int64_t r0, int R, short* o
   }
 }
 
-template <typename MV, typename VV, bool kOne, bool kUni, bool kPaige, bool kExp>
-__global__ void __launch_bounds__(kLanThreads, 1) lan_kernel(LanArgs<MV, VV> A) {
+// Transitions of a row (its length but for the diagonal's entry and what leaves the sector).
+template <typename MV, typename VV>
+__device__ __forceinline__ int64_t lan_mf_length(const LanMfArgs<MV, VV>& A, const LanEnt<MV>& E, int64_t r) {
+  const uint64_t s = __ldg(A.mf.basis + r);
+  int n = 0;
+  if (A.mf32.nf > 0)
+    for (int e = 0; e < A.mf.nent; ++e) n += ((uint32_t)s & E.test[e].x) == E.test[e].y;
+  else
+    for (int e = 0; e < A.mf.nent; ++e) n += (s & E.ent[e].sup) == E.ent[e].outb;
+  return n;
+}
+
+template <typename MV, typename VV, bool kOne, bool kUni, bool kPaige, bool kExp, bool kMf>
+__global__ void __launch_bounds__(kLanThreads, 1) lan_kernel(LanArgsOf<MV, VV, kMf> A) {
   constexpr int T = kLanThreads, kPer = sizeof(VV) / sizeof(double);
   constexpr int NV = kPaige ? 2 : 1 + 3 * kPer;
   extern __shared__ __align__(16) unsigned char lan_smem[];
@@ -333,8 +509,37 @@ __global__ void __launch_bounds__(kLanThreads, 1) lan_kernel(LanArgs<MV, VV> A) 
   int lanes = 1;
   while (lanes < 4 && 2 * lanes * A.rows <= (kUni ? 512 : 256)) lanes *= 2;
   short* order = reinterpret_cast<short*>(ring + 3 * (size_t)A.rows);
+  LanEnt<MV> ent{};
+  if constexpr (kMf) {
+    unsigned char* p = lan_smem + lan_rows_smem<VV>(A.rows);
+    const int nent = A.mf.nent;
+    if (A.mf32.nf > 0) {
+      uint2 *test = reinterpret_cast<uint2*>(p), *move = test + nent;
+      MV* amp = reinterpret_cast<MV*>(move + nent);
+      for (int i = tid; i < nent; i += T) {
+        const MfEntry E = A.mf.ent[i];
+        test[i] = make_uint2((uint32_t)E.sup, (uint32_t)E.outb);
+        move[i] = make_uint2((uint32_t)E.flip, (uint32_t)E.jw);
+        amp[i] = amp_of((MV*)nullptr, E.amp);
+      }
+      ent.test = test;
+      ent.move = move;
+      ent.amp = amp;
+    } else {
+      MfEntry* e = reinterpret_cast<MfEntry*>(p);
+      for (int i = tid; i < nent; i += T) e[i] = A.mf.ent[i];
+      ent.ent = e;
+    }
+    __syncthreads();
+  }
   if constexpr (!kUni)
-    if (lanes == 1) lan_sort_rows<T>(A.rowptr, r0, R, order, reinterpret_cast<short*>(ring));
+    if (lanes == 1)
+      lan_sort_rows<T>(
+          [&](int r) -> int64_t {
+            if constexpr (kMf) return lan_mf_length(A, ent, r0 + r);
+            else return __ldg(A.rowptr + r0 + r + 1) - __ldg(A.rowptr + r0 + r);
+          },
+          R, order, reinterpret_cast<short*>(ring));
   double vals[NV];
 #pragma unroll
   for (int i = 0; i < NV; ++i) vals[i] = 0.0;
@@ -395,7 +600,10 @@ __global__ void __launch_bounds__(kLanThreads, 1) lan_kernel(LanArgs<MV, VV> A) 
         const int r = (!kUni && lanes == 1 && live) ? order[i] : i;
         VV a;
         if constexpr (kUni)
-          a = lan_row_uniform(A, A.XV + (int64_t)(k - A.first) * A.ld, r0 + r, live, sub, lanes, live ? u1[r] : 0.0);
+          a = lan_row_uniform<kMf>(A, ent, A.XV + (int64_t)(k - A.first) * A.ld, r0 + r, live, sub, lanes,
+                                   live ? u1[r] : 0.0);
+        else if constexpr (kMf)
+          a = lan_row_mf(A, ent, x, r0 + r, live, sub, lanes, k > A.first, live ? u1[r] : vzero(VV{}));
         else a = lan_row(A, x, r0 + r, live, sub, lanes, k > A.first);
         if (live && sub == 0) {
           w[r] = a;
@@ -592,10 +800,27 @@ __global__ void lan_rows_kernel(int64_t n, const int64_t* rowptr, int grid, int*
   }
 }
 
+// The rows' lengths as the stored matrix has them (an entry of the diagonal where one of its nd transitions
+// dia applies), so that solves on either split the rows alike.
+__global__ void lan_mf_lengths_kernel(const __grid_constant__ MfRows M, const MfEntry* dia, int nd, int64_t* len) {
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r <= M.dim; r += (int64_t)gridDim.x * blockDim.x) {
+    int64_t n = 0;
+    if (r < M.dim) {
+      const uint64_t s = __ldg(M.basis + r);
+      for (int e = 0; e < M.nent; ++e)
+        if ((s & M.ent[e].sup) == M.ent[e].outb) n += mf_rank(M, s ^ M.ent[e].flip) < M.dim;
+      bool diag = false;
+      for (int e = 0; e < nd; ++e) diag |= (s & dia[e].sup) == dia[e].outb;
+      n += diag;
+    }
+    len[r] = n;
+  }
+}
+
 // The kernel for one block or many; cfg for the grid the sector takes.  False when the device does not hold
 // the grid at once, or a block its rows.
 template <typename VV, typename K>
-static bool lan_plan(qd_ham* H, K kern1, K kern_many, LanPlan& P, cudaLaunchConfig_t& cfg,
+static bool lan_plan(qd_ham* H, bool mf, K kern1, K kern_many, LanPlan& P, cudaLaunchConfig_t& cfg,
                      cudaLaunchAttribute (&at)[2], K& kern) {
   Ctx* ctx = H->ctx;
   const int64_t n = H->dim;
@@ -610,18 +835,33 @@ static bool lan_plan(qd_ham* H, K kern1, K kern_many, LanPlan& P, cudaLaunchConf
   cfg.stream = ctx->stream;
   cfg.attrs = at;
   cfg.numAttrs = csize == 1 ? 1 : 2;
-  // three vectors' rows and their order by length
-  const auto smem_of = [](int rows) { return (size_t)3 * rows * sizeof(VV) + ((size_t)rows * sizeof(short) + 15) / 16 * 16; };
+  const auto smem_of = [&](int rows) { return lan_rows_smem<VV>(rows) + (mf ? H->mf_nent * sizeof(MfEntry) : 0); };
   if (!P.ok) {
     int maxsm = 0;
     QD_CUDA(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
     int ncl = csize == 1 ? 1 : (int)std::min<int64_t>(ctx->num_sms / csize, ceil_div(n, csize * kLanMinRows));
     int rows = (int)n;
     std::vector<int> first;
+    const int64_t* rowptr = H->rowptr.p;
+    DBuf<int64_t> len;
+    if (mf) {  // the lengths that the transitions give, summed
+      std::vector<MfEntry> off, dia;
+      compile_terms(H, off, dia);
+      DBuf<MfEntry> ddia(dia.size());
+      if (!dia.empty())
+        QD_CUDA(cudaMemcpyAsync(ddia.p, dia.data(), dia.size() * sizeof(MfEntry), cudaMemcpyHostToDevice, ctx->stream));
+      len.alloc(n + 1);
+      lan_mf_lengths_kernel<<<(unsigned)ceil_div(n + 1, 256), 256, 0, ctx->stream>>>(mf_rows(H), ddia.p, (int)dia.size(),
+                                                                                    len.p);
+      QD_CHECK_LAUNCH();
+      QD_LAUNCHED(ctx);
+      exclusive_scan_i64(ctx, len.p, len.p, n + 1);
+      rowptr = len.p;
+    }
     for (;;) {
       const int grid = ncl * csize;
       if (P.first.n < (size_t)grid + 1) P.first.alloc(grid + 1);
-      lan_rows_kernel<<<1, 256, 0, ctx->stream>>>(n, H->rowptr.p, grid, P.first.p);
+      lan_rows_kernel<<<1, 256, 0, ctx->stream>>>(n, rowptr, grid, P.first.p);
       QD_CHECK_LAUNCH();
       QD_LAUNCHED(ctx);
       if (csize > 1) {
@@ -657,7 +897,7 @@ static bool lan_plan(qd_ham* H, K kern1, K kern_many, LanPlan& P, cudaLaunchConf
 }
 
 template <typename MV, typename VV>
-static LanArgs<MV, VV> lan_args(qd_ham* H, const MV* vals, const LanPlan& P, VV* V, int64_t ld, int first, int last,
+static LanArgs<MV, VV> lan_args(qd_ham* H, const MV* vals, bool mf, const LanPlan& P, VV* V, int64_t ld, int first, int last,
                                 int nv, int* flags, DBuf<double>* slots, XInt* xv) {
   Ctx* ctx = H->ctx;
   LanArgs<MV, VV> A;
@@ -666,9 +906,11 @@ static LanArgs<MV, VV> lan_args(qd_ham* H, const MV* vals, const LanPlan& P, VV*
   A.ld = ld;
   A.rows = P.rows;
   A.row_first = P.first.p;
-  A.rowptr = H->rowptr.p;
-  A.colidx = H->colidx.p;
-  A.vals = vals;
+  if (!mf) {
+    A.rowptr = H->rowptr.p;
+    A.colidx = H->colidx.p;
+    A.vals = vals;
+  }
   A.V = V;
   A.first = first;
   A.last = last;
@@ -690,24 +932,27 @@ static LanArgs<MV, VV> lan_args(qd_ham* H, const MV* vals, const LanPlan& P, VV*
   return A;
 }
 
-template <typename MV, typename VV, bool kUni, bool kPaige>
+template <typename MV, typename VV, bool kUni, bool kPaige, bool kMf>
 static bool lan_launch(qd_ham* H, const LanRun<MV, VV>& r) {
   Ctx* ctx = H->ctx;
-  LanPlan& P = ham_workspace(H).lan_plan[sizeof(VV) == sizeof(double) ? (kPaige ? 1 : 0) : (kPaige ? 3 : 2)];
+  constexpr int kC = sizeof(VV) == sizeof(cplx);
+  LanPlan& P = ham_workspace(H).lan_plan[kMf ? 5 + kC : 2 * kC + kPaige];
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[2];
-  auto kern = lan_kernel<MV, VV, true, kUni, kPaige, false>;
-  if (!lan_plan<VV>(H, kern, lan_kernel<MV, VV, false, kUni, kPaige, false>, P, cfg, at, kern)) return false;
+  auto kern = lan_kernel<MV, VV, true, kUni, kPaige, false, kMf>;
+  if (!lan_plan<VV>(H, kMf, kern, lan_kernel<MV, VV, false, kUni, kPaige, false, kMf>, P, cfg, at, kern)) return false;
   constexpr int kPer = sizeof(VV) / sizeof(double);
   const size_t nx = (size_t)(r.kdim + 1) * r.ld * sizeof(XInt);
   if (kUni && r.xv->n < nx) r.xv->alloc(nx);
   LanArgs<MV, VV> A =
-      lan_args(H, r.vals, P, r.V, r.ld, r.first, r.last, kPaige ? 2 : 1 + 3 * kPer, r.flags, r.slots, kUni ? reinterpret_cast<XInt*>(r.xv->p) : nullptr);
+      lan_args(H, r.vals, kMf, P, r.V, r.ld, r.first, r.last, kPaige ? 2 : 1 + 3 * kPer, r.flags, r.slots, kUni ? reinterpret_cast<XInt*>(r.xv->p) : nullptr);
   if (kUni) {
     A.fxdiag = r.form->diag_zero ? nullptr : r.form->diag.p;
     A.cF = std::ldexp(r.form->c, -r.form->F);
-    A.fxptr = r.form->colidx.p ? r.form->rowptr.p : nullptr;
-    A.fxcol = r.form->colidx.p;
+    if (!kMf) {
+      A.fxptr = r.form->rowptr.p;
+      A.fxcol = r.form->colidx.p;
+    }
     A.F = r.form->F;
     A.ovf = r.flags;
   }
@@ -717,7 +962,19 @@ static bool lan_launch(qd_ham* H, const LanRun<MV, VV>& r) {
   A.nrm = r.nrm;
   A.scl = r.scl;
   A.stop = r.stop;
-  QD_CUDA(cudaLaunchKernelEx(&cfg, kern, A));
+  if constexpr (kMf) {
+    LanMfArgs<MV, VV> M;
+    std::memset(&M, 0, sizeof(M));
+    static_cast<LanArgs<MV, VV>&>(M) = A;
+    M.mf = mf_rows(H);
+    if (!mf32_prepare(H, M.mf32)) M.mf32.nf = 0;
+    if constexpr (std::is_same<MV, double>::value) M.diag = H->diag_r.p;
+    else M.diag = H->diag_c.p;
+    if (kUni && r.form->use_blk && r.form->blk_state > 0) M.blk = block_tables(*r.form);
+    QD_CUDA(cudaLaunchKernelEx(&cfg, kern, M));
+  } else {
+    QD_CUDA(cudaLaunchKernelEx(&cfg, kern, A));
+  }
   QD_LAUNCHED(ctx);
   return true;
 }
@@ -725,8 +982,9 @@ static bool lan_launch(qd_ham* H, const LanRun<MV, VV>& r) {
 template <typename MV, typename VV>
 bool lan_res_run(qd_ham* H, const LanRun<MV, VV>& r) {
   if constexpr (std::is_same<VV, double>::value)
-    if (r.form) return lan_launch<MV, VV, true, false>(H, r);
-  return r.rule == kLanPaige ? lan_launch<MV, VV, false, true>(H, r) : lan_launch<MV, VV, false, false>(H, r);
+    if (r.form) return r.mf ? lan_launch<MV, VV, true, false, true>(H, r) : lan_launch<MV, VV, true, false, false>(H, r);
+  if (r.rule == kLanPaige) return lan_launch<MV, VV, false, true, false>(H, r);
+  return r.mf ? lan_launch<MV, VV, false, false, true>(H, r) : lan_launch<MV, VV, false, false, false>(H, r);
 }
 template bool lan_res_run<double, double>(qd_ham*, const LanRun<double, double>&);
 template bool lan_res_run<double, cplx>(qd_ham*, const LanRun<double, cplx>&);
@@ -739,11 +997,11 @@ bool lan_res_evolve(qd_ham* H, const MV* vals, const cplx* psi, cplx* out, cplx*
   LanPlan& P = ham_workspace(H).lan_plan[4];
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[2];
-  auto kern = lan_kernel<MV, cplx, true, false, true, true>;
+  auto kern = lan_kernel<MV, cplx, true, false, true, true, false>;
   if (kdim > kLanMaxExp ||
-      !lan_plan<cplx>(H, kern, lan_kernel<MV, cplx, false, false, true, true>, P, cfg, at, kern))
+      !lan_plan<cplx>(H, false, kern, lan_kernel<MV, cplx, false, false, true, true, false>, P, cfg, at, kern))
     return false;
-  LanArgs<MV, cplx> A = lan_args<MV, cplx>(H, vals, P, V, ld, 1, kdim, 2, flags, slots, nullptr);
+  LanArgs<MV, cplx> A = lan_args<MV, cplx>(H, vals, false, P, V, ld, 1, kdim, 2, flags, slots, nullptr);
   A.stop_below = 1e-10;
   A.psi = psi;
   A.out = out;

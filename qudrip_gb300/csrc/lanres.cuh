@@ -18,11 +18,13 @@ enum LanForm { kLanLocal = 0, kLanPaige = 1 };
 //   kLanLocal  the reference's local orthogonalisation against two vectors (sparse_algorithm.hpp:395-425)
 //   kLanPaige  alpha = <v1, H v1>, beta = ||V1|| (Hermitian::LanczosSolver; the Krylov exponential)
 // with the stopping rule norm < stop_below (*stop = the step).  `form`: the uniform-coupling form whose
-// fixed-point sums the product keeps (real vectors), or null for the FP64 product.
+// fixed-point sums the product keeps (real vectors), or null for the FP64 product.  `mf`: the product's
+// columns and values from the compiled transitions (kLanLocal; ham_build_matrix_free has run).
 template <typename MV, typename VV>
 struct LanRun {
   const MV* vals;
   LanForm rule;
+  bool mf;
   const FxForm* form;
   VV* V;
   int64_t ld;

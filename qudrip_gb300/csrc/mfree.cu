@@ -28,6 +28,7 @@
 
 #include "ham.cuh"
 #include "krylov.cuh"
+#include "mfrow.cuh"
 #include "scan.cuh"
 #include "spmv.cuh"
 
@@ -212,37 +213,6 @@ struct MfArgs {
 };
 
 template <typename AV, typename VV>
-__device__ __forceinline__ int64_t mf_rank(const MfArgs<AV, VV>& A, uint64_t c) {
-  if (!A.use_tables) return sector_rank(A.S, c);
-  int64_t r = 0;
-  for (int f = 0; f < A.rk.nf; ++f) {
-    const int w = A.rk.width[f];
-    const uint64_t v = (c >> A.rk.lo[f]) & ((w >= 64) ? ~0ull : ((1ull << w) - 1));
-    if (A.rk.is_free[f]) {
-      r += (int64_t)v * A.rk.stride[f];
-      continue;
-    }
-    const int k = A.rk.k[f];
-    if (__popcll(v) != k) return A.dim;
-    const int64_t* T = A.rk.tab + A.rk.off[f];
-    int64_t acc = 0;
-    int cb = 0;
-    for (int b = 0; b < A.rk.nb[f]; ++b) {
-      const unsigned byte = (unsigned)(v >> (8 * b)) & 255u;
-      acc += __ldg(T + ((int64_t)b * 256 + byte) * (k + 1) + cb);
-      cb += __popc(byte);
-    }
-    r += acc * A.rk.stride[f];
-  }
-  return r;
-}
-
-__device__ __forceinline__ double amp_of(double*, cplx a) { return a.re; }
-__device__ __forceinline__ cplx amp_of(cplx*, cplx a) { return a; }
-__device__ __forceinline__ double vneg(double a) { return -a; }
-__device__ __forceinline__ cplx vneg(cplx a) { return mkc(-a.re, -a.im); }
-
-template <typename AV, typename VV>
 __global__ void __launch_bounds__(256) mf_spmv_kernel(MfArgs<AV, VV> A) {
   extern __shared__ __align__(16) unsigned char mf_smem[];
   uint64_t* s_sup = reinterpret_cast<uint64_t*>(mf_smem);
@@ -375,19 +345,7 @@ void ham_build_matrix_free(qd_ham* H) {
   H->has_mf = true;
 }
 
-// 32-bit form of the product for registers of at most 32 bits ranked by
-// tables (every model of the configurations): states, masks and table entries
-// in 32-bit integers, the fields unrolled, so a row costs about half the
-// integer instructions of the 64-bit form.
-struct Mf32 {
-  int nf;
-  int lo[2], k[2], nb[2];
-  uint32_t wmask[2];
-  uint32_t stride[2];
-  int off[2];
-  const uint32_t* tab;
-};
-
+// 32-bit form of the product (Mf32): a row costs about half the integer instructions of the 64-bit form.
 template <typename AV, typename VV, int NF>
 __global__ void __launch_bounds__(256) mf_spmv32_kernel(int64_t dim, const uint64_t* __restrict__ basis,
                                                         const AV* __restrict__ diag, const MfEntry* __restrict__ ent,
@@ -457,9 +415,7 @@ __global__ void __launch_bounds__(256) mf_spmv32_kernel(int64_t dim, const uint6
   }
 }
 
-// Builds the 32-bit form when the register has at most 32 bits, the sector is
-// a product of at most two fields and the dimension fits in 32 bits.
-static bool mf32_prepare(qd_ham* H, Mf32& R) {
+bool mf32_prepare(const qd_ham* H, Mf32& R) {
   const SectorView& V = H->sec->view;
   if (!H->mf_tables || V.nbits > 32 || H->dim >= (1ll << 31)) return false;
   int nf = 0;
@@ -581,31 +537,6 @@ struct PullArgs {
   SectorView S;
 };
 
-__device__ __forceinline__ int64_t pull_rank(const PullArgs& A, uint64_t c) {
-  if (!A.use_tables) return sector_rank(A.S, c);
-  int64_t r = 0;
-  for (int f = 0; f < A.rk.nf; ++f) {
-    const int w = A.rk.width[f];
-    const uint64_t v = (c >> A.rk.lo[f]) & ((w >= 64) ? ~0ull : ((1ull << w) - 1));
-    if (A.rk.is_free[f]) {
-      r += (int64_t)v * A.rk.stride[f];
-      continue;
-    }
-    const int k = A.rk.k[f];
-    if (__popcll(v) != k) return A.dim;
-    const int64_t* T = A.rk.tab + A.rk.off[f];
-    int64_t acc = 0;
-    int cb = 0;
-    for (int b = 0; b < A.rk.nb[f]; ++b) {
-      const unsigned byte = (unsigned)(v >> (8 * b)) & 255u;
-      acc += __ldg(T + ((int64_t)b * 256 + byte) * (k + 1) + cb);
-      cb += __popc(byte);
-    }
-    r += acc * A.rk.stride[f];
-  }
-  return r;
-}
-
 // Whether c is a state of a product sector.
 __device__ __forceinline__ bool pull_inside(const PullArgs& A, uint64_t c) {
   for (int f = 0; f < A.rk.nf; ++f) {
@@ -665,7 +596,7 @@ __global__ void __launch_bounds__(128) pull_lower_kernel(const __grid_constant__
       n += pull_inside(A, c);
       continue;
     }
-    const int64_t col = diag ? r : pull_rank(A, c);
+    const int64_t col = diag ? r : mf_rank(A, c);
     if (col >= A.dim) continue;  // outside the sector (operator.hpp:196-199)
     if (kFill) {
       int q = n;
