@@ -384,28 +384,8 @@ __global__ void __launch_bounds__(256) mf_spmv32_kernel(int64_t dim, const uint6
         const int e = e0 + __ffs(mask) - 1;
         mask &= mask - 1;
         const uint32_t c = s ^ s_flip[e];
-        uint32_t col = 0;
-        bool in = true;
-#pragma unroll
-        for (int f = 0; f < NF; ++f) {
-          const uint32_t v = (c >> R.lo[f]) & R.wmask[f];
-          in &= (__popc(v) == R.k[f]);
-          const uint32_t* T = R.tab + R.off[f];
-          const int kk = R.k[f] + 1;
-          uint32_t a = __ldg(T + (v & 255u) * kk);
-          int cb = __popc(v & 255u);
-          if (R.nb[f] > 1) {
-            a += __ldg(T + (256u + ((v >> 8) & 255u)) * kk + cb);
-            cb += __popc((v >> 8) & 255u);
-          }
-          if (R.nb[f] > 2) {
-            a += __ldg(T + (512u + ((v >> 16) & 255u)) * kk + cb);
-            cb += __popc((v >> 16) & 255u);
-          }
-          if (R.nb[f] > 3) a += __ldg(T + (768u + (v >> 24)) * kk + cb);
-          col += a * R.stride[f];
-        }
-        if (!in) continue;
+        uint32_t col;
+        if (!mf_rank32<NF>(R, c, col)) continue;
         AV a = s_amp[e];
         if (__popc(c & s_jw[e]) & 1) a = vneg(a);
         acc = vfma(a, ld_ro(x + col), acc);

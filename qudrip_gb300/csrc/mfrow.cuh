@@ -45,15 +45,16 @@ bool mf32_prepare(const qd_ham* H, Mf32& R);
 
 #ifdef __CUDACC__
 // The rank of state c into col; false, with no table read, when it is not in the sector (the tables end at k
-// set bits).
+// set bits).  NF fields, 0: one or two.
+template <int NF = 0>
 __device__ __forceinline__ bool mf_rank32(const Mf32& R, uint32_t c, uint32_t& col) {
   bool in = __popc((c >> R.lo[0]) & R.wmask[0]) == R.k[0];
-  if (R.nf > 1) in &= __popc((c >> R.lo[1]) & R.wmask[1]) == R.k[1];
+  if (NF == 2 || (NF == 0 && R.nf > 1)) in &= __popc((c >> R.lo[1]) & R.wmask[1]) == R.k[1];
   if (!in) return false;
   col = 0;
 #pragma unroll
-  for (int f = 0; f < 2; ++f) {
-    if (f >= R.nf) break;
+  for (int f = 0; f < (NF ? NF : 2); ++f) {
+    if (NF == 0 && f >= R.nf) break;
     const uint32_t v = (c >> R.lo[f]) & R.wmask[f];
     const uint32_t* T = R.tab + R.off[f];
     const int kk = R.k[f] + 1;

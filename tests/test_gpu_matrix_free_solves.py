@@ -78,3 +78,21 @@ def test_uniform_couplings_carry_the_same_bits_from_every_source_of_columns(ctx,
         got.append(solve(sec, H, v0, 24, A.QD_SPMV_CSR))
     for ev, psi in got:
         assert np.array_equal(ev, ref[0]) and np.array_equal(psi, ref[1])
+
+
+@pytest.mark.parametrize("make", [lambda: chains.xy_chain(9), lambda: two_species_xy(4, False)])
+def test_targets_outside_the_sector_are_dropped(ctx, make):
+    """Terms that raise two sites leave the sector from every state they apply to."""
+    spec, ham = make()
+    gp = q.getBoseGate(spec.index)
+    gp << 0.5 * (q.pauli_x + q.II * q.pauli_y)
+    for i in range(spec.index.nbits - 1):
+        ham = ham + 0.3 * (gp(i) * gp(i + 1))
+    sec = q.Sector(spec.index, spec.constraints)
+    H = sec.lower(ham)
+    st = q.getState(sec, 2)
+    x = q.start_vector(sec.dim, 2) + 1j * q.start_vector(sec.dim, 3)
+    st.set(0, x)
+    q.apply(H, st, 0, st, 1, matrix_free=True)
+    ref = H.scipy() @ x
+    assert np.max(np.abs(st.get(1) - ref)) <= 1e-14 * np.abs(H.scipy()).sum(axis=1).max() * np.abs(x).max()
