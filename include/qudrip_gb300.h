@@ -167,8 +167,9 @@ typedef struct {
   int32_t product_kernel;  /* product the real Lanczos path launches (codes of qd_ham_set_spmv_kernel) */
   int32_t step_launches;   /* kernel launches per Lanczos step of the last real solve on the      */
                            /* uniform-coupling form: 1 (product, dots, update and norm in one    */
-                           /* cooperative launch) or 2 (QD_LANCZOS_STEP=split, or a step too big */
-                           /* to be resident at once); 0 before such a solve                    */
+                           /* cooperative launch, or all steps in one, up to 65,536 rows) or 2   */
+                           /* (QD_LANCZOS_STEP=split, or a step too big to be resident at once);  */
+                           /* 0 before such a solve                                             */
 } qd_ham_info;
 
 qd_status qd_ham_lower(qd_sector *sec, const qd_term *terms, int nterms,
@@ -424,12 +425,21 @@ qd_status qd_ham_time_spmv(qd_ham *ham, int spmv, int iters, double *avg_ms,
  * the fly from the operator's terms instead of read (product sectors of at
  * most 32 bits; kept only after a build-time check that every row's columns
  * equal its stored ones, so 121 and 120 give bit-identical solves).  All
- * give the same products up to rounding. */
+ * give the same products up to rounding.
+ * Without a choice, solves on small and medium sectors (up to some hundred
+ * thousand rows), Krylov steps and operator lists run kernels with a product
+ * of their own; a CSR code given here is launched for every product instead,
+ * step by step.  On the uniform-coupling form such a solve (up to 65,536 rows)
+ * takes its columns from where the code says: stored (120), the transitions
+ * (121), the block tables of the sector (122); the sums are exact, so the bits
+ * are the same.  QD_KRYLOV_STEP=split launches step by step whatever the
+ * choice. */
 qd_status qd_ham_set_spmv_kernel(qd_ham *ham, int kernel);
 /* Time every product kernel on this Hamiltonian (120 and 121 included where
  * they apply, timed as the recurrence launches them, with its inner products)
- * and keep the fastest for the solvers (the autotuner); returns the choice
- * and its average ms. */
+ * and keep the fastest for the solvers' launched products (the autotuner);
+ * returns the choice and its average ms.  It is no choice of the caller's:
+ * calls with a product of their own keep it. */
 qd_status qd_ham_autotune(qd_ham *ham, int iters, int *chosen, double *best_ms);
 
 /* <psi|H|psi> for a CSR Hamiltonian, with no device allocation at all.

@@ -548,11 +548,12 @@ static bool arn_coop(Ctx* ctx) {
 }
 
 // Served requests keep the kernels launched one by one: a co-resident grid waits for room beside
-// the other lanes' kernels.  QD_KRYLOV_STEP=split keeps them for every call.
+// the other lanes' kernels, and an operator with a product kernel of the caller's choice launches that.
+// QD_KRYLOV_STEP=split keeps them for every call.
 bool arn_res_fits(qd_ham* H, int kdim) {
   const char* e = std::getenv("QD_KRYLOV_STEP");
   if (e && std::strcmp(e, "split") == 0) return false;
-  return !H->one_shot && kdim >= 1 && kdim < kArnMaxVecs && H->dim >= 1 && H->dim < (int64_t)1 << 30 &&
+  return !H->one_shot && !H->spmv_chosen && kdim >= 1 && kdim < kArnMaxVecs && H->dim >= 1 && H->dim < (int64_t)1 << 30 &&
          arn_coop(H->ctx);
 }
 

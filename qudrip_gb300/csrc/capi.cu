@@ -648,10 +648,12 @@ qd_status qd_ham_set_spmv_kernel(qd_ham* ham, int kernel) {
       ham->fx->use_slots = (kernel == kSpmvFxSlots);
       ham->fx->use_blk = (kernel == kSpmvFxBlock);
       ham->fx_allowed = true;
+      ham->spmv_chosen = false;
       return;
     }
     if (kernel == kSpmvRowSorted) ham_ensure_row_order(ham);
     ham->spmv_variant = kernel;
+    ham->spmv_chosen = true;
     ham->fx_allowed = false;
   });
 }
@@ -672,6 +674,7 @@ qd_status qd_ham_autotune(qd_ham* ham, int iters, int* chosen, double* best_ms) 
       }
     }
     ham->spmv_variant = pick;
+    ham->spmv_chosen = false;
     ham->fx_allowed = false;
     if ((ham->flags & QD_HAM_REAL) && ham_build_fx(ham)) {
       // the fixed-point forms as the recurrence launches them (fused with the step's inner products,

@@ -87,7 +87,7 @@ void arnoldi_evolve(qd_ham* H, const cplx* psi_in, cplx* psi_out, double h, int 
   }
   if (!H->arnoldi) H->arnoldi.reset(new ArnoldiBuffers());
   ArnoldiBuffers& B = *H->arnoldi;
-  if (B.basis.ensure(ctx, n, m, (H->flags & QD_HAM_HERMITIAN) != 0, !H->one_shot)) B.drop_graph();  // the buffers moved
+  if (B.basis.ensure(ctx, n, m, (H->flags & QD_HAM_HERMITIAN) && !H->spmv_chosen, !H->one_shot)) B.drop_graph();  // the buffers moved
   if (!B.hcol.p) {
     B.hcol.alloc((size_t)33 * 64);
     B.e.alloc(64);
@@ -270,7 +270,7 @@ void arnoldi_ground(qd_ham* H, cplx* psi, int kdim, int add_dim, bool extend, do
     if (!H->arnoldi_gs) H->arnoldi_gs.reset(new ArnoldiGround());
     ArnoldiGround& B = *H->arnoldi_gs;
     B.open = false;
-    B.basis.ensure(ctx, n, kdim + 1, (H->flags & QD_HAM_HERMITIAN) != 0, !H->one_shot);
+    B.basis.ensure(ctx, n, kdim + 1, (H->flags & QD_HAM_HERMITIAN) && !H->spmv_chosen, !H->one_shot);
     if (B.kdim != kdim) {
       B.kdim = 0;
       B.ldh = kdim + 1;

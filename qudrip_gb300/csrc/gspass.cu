@@ -447,7 +447,7 @@ static void gs_zero_tails(T* p, int64_t n, int64_t ld, int vecs, cudaStream_t s)
 }
 
 bool GsBasis::ensure(Ctx* ctx, int64_t n_, int vecs_, bool herm, bool copies) {
-  if (n_ == n && vecs_ == vecs) return false;
+  if (n_ == n && vecs_ == vecs && herm == (dots.p != nullptr)) return false;
   n = 0;  // until every buffer is there
   // Tiles of 128 rows amortise their conversions better, tiles of 64 fill the SMs' warps sooner: two steps
   // of m = 16 (m = 30) at 48,620 rows 1.05 (2.56) against 1.00 ms (2.39), 92,378 rows 1.30 against 1.27,

@@ -88,6 +88,8 @@ struct qd_ham {
   int max_row_nnz = 0;
   double norm_inf = -1.0;  // max row sum of |H| (ham_norm_inf), -1 until computed
   int spmv_variant = 110;  // CSR product kernel the solvers launch (krylov.cuh SpmvVariant)
+  bool spmv_chosen = false;  // ... by the caller: calls with a product of their own (the persistent recurrences,
+                             // the Hermitian Arnoldi step, operator lists) launch it instead
   qd::DBuf<int64_t> rowptr;
   qd::DBuf<int32_t> colidx;
   qd::DBuf<cplx> vals_c;

@@ -114,6 +114,7 @@ void ham_copy(const qd_ham* A, qd_ham* H) {
   H->host_gates = A->host_gates;
   H->from_terms = A->from_terms;
   H->spmv_variant = A->spmv_variant;
+  H->spmv_chosen = A->spmv_chosen;
   ham_finish(H);
 }
 

@@ -430,6 +430,7 @@ struct ObsOp {
   const int64_t* rowptr;
   const int32_t* colidx;
   const void* vals;  // double or cplx
+  cplx* out;
   int real;
 };
 struct ObsArgs {
@@ -437,7 +438,6 @@ struct ObsArgs {
   const cplx* psi;
   cplx* partials;     // gridDim.x per operator
   unsigned* tickets;  // one per operator, 0 at rest
-  cplx* out;
   ObsOp op[kObsBatch];
 };
 
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(kVecThreads) obs_kernel(const __grid_constant_
   const ObsOp& O = A.op[blockIdx.y];
   const cplx acc = O.real ? obs_rows<double>(A, O) : obs_rows<cplx>(A, O);
   GridRed<cplx> red{A.partials + (size_t)blockIdx.y * gridDim.x, A.tickets + blockIdx.y};
-  grid_sum_flat(acc, red, A.out + blockIdx.y);
+  grid_sum_flat(acc, red, O.out);
 }
 
 void obs_eval_many(qd_ham* const* obs, int nobs, const cplx* psi, cplx* out_host) {
@@ -495,21 +495,34 @@ void obs_eval_many(qd_ham* const* obs, int nobs, const cplx* psi, cplx* out_host
   A.psi = psi;
   A.partials = W.partials_c.p;
   A.tickets = W.obs_tickets.p;
-  for (int i0 = 0; i0 < nobs; i0 += kObsBatch) {
-    const int cnt = std::min(kObsBatch, nobs - i0);
-    for (int i = 0; i < cnt; ++i) {
-      const qd_ham* H = obs[i0 + i];
-      const bool real = (H->flags & QD_HAM_REAL) != 0;
-      A.op[i] = ObsOp{H->rowptr.p, H->colidx.p, real ? (const void*)H->vals_r.p : (const void*)H->vals_c.p, real};
-    }
-    A.out = W.obs_out.p + i0;
+  int cnt = 0;
+  auto launch = [&] {
+    if (!cnt) return;
     // enough blocks for eight per SM over all operators, one row per thread at least
     const int64_t gx = std::max<int64_t>(
         1, std::min<int64_t>(ceil_div(n, kVecThreads), std::max<int64_t>(1, (int64_t)ctx->num_sms * 8 / cnt)));
     obs_kernel<<<dim3((unsigned)gx, (unsigned)cnt), kVecThreads, 0, ctx->stream>>>(A);
     QD_CHECK_LAUNCH();
     QD_LAUNCHED(ctx);
+    cnt = 0;
+  };
+  for (int i = 0; i < nobs; ++i) {
+    qd_ham* H = obs[i];
+    const bool real = (H->flags & QD_HAM_REAL) != 0;
+    cplx* out = W.obs_out.p + i;
+    if (H->spmv_chosen) {  // its own product, the inner product fused with it
+      Workspace& WH = ham_workspace(H);
+      if (WH.eval_y.n < (size_t)n + 1) WH.eval_y.alloc(n + 1);
+      if (real)
+        launch_spmv<double, cplx>(ctx, H, H->vals_r.p, psi, WH.eval_y.p, 1.0, psi, WH.red_c(0), out, nullptr, 0, -1);
+      else
+        launch_spmv<cplx, cplx>(ctx, H, H->vals_c.p, psi, WH.eval_y.p, 1.0, psi, WH.red_c(0), out, nullptr, 0, -1);
+      continue;
+    }
+    A.op[cnt++] = ObsOp{H->rowptr.p, H->colidx.p, real ? (const void*)H->vals_r.p : (const void*)H->vals_c.p, out, real};
+    if (cnt == kObsBatch) launch();
   }
+  launch();
   QD_CUDA(cudaMemcpyAsync(out_host, W.obs_out.p, nobs * sizeof(cplx), cudaMemcpyDeviceToHost, ctx->stream));
   QD_CUDA(cudaStreamSynchronize(ctx->stream));
 }
@@ -777,11 +790,11 @@ void time_spmv(qd_ham* H, int spmv, int iters, double* avg_ms, double* bytes_per
 // ---------------------------------------------------------------- Lanczos
 // Whether a solve takes the persistent recurrence (lanres.cu): sectors up to `most` rows, where the
 // launches and reductions of a step outweigh its memory traffic.  Served requests keep the
-// separate launches (a co-resident grid waits for room beside the other lanes' kernels), and so do
-// QD_KRYLOV_STEP=split and QD_LANCZOS_STEP=split.
+// separate launches (a co-resident grid waits for room beside the other lanes' kernels), and so do operators
+// with a CSR kernel of the caller's choice, QD_KRYLOV_STEP=split and QD_LANCZOS_STEP=split.
 static bool lan_res_takes(const qd_ham* H, int64_t most) {
   const char* e = std::getenv("QD_KRYLOV_STEP");
-  if (H->one_shot || !fx_one_launch_step() || (e && std::strcmp(e, "split") == 0)) return false;
+  if (H->one_shot || H->spmv_chosen || !fx_one_launch_step() || (e && std::strcmp(e, "split") == 0)) return false;
   static const bool coop = [&] {  // once per process (thread-safe initialisation)
     int v = 0;
     return cudaDeviceGetAttribute(&v, cudaDevAttrCooperativeLaunch, H->ctx->device) == cudaSuccess && v != 0;
