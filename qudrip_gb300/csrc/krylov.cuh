@@ -100,7 +100,7 @@ struct EvolveGraphDeleter {
 
 // The grid of a persistent Lanczos recurrence (lanres.cu), chosen on its first run on an operator.
 struct LanPlan {
-  bool ok = false;
+  bool ok = false, none = false;  // chosen; found that no grid holds the rows
   int csize = 1, ncl = 1;  // blocks per cluster, clusters
   int rows = 0;            // most rows of a block
   DBuf<int> first;         // first row of each block, and the number of rows

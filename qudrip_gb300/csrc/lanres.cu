@@ -836,6 +836,7 @@ static bool lan_plan(qd_ham* H, bool mf, K kern1, K kern_many, LanPlan& P, cudaL
   cfg.attrs = at;
   cfg.numAttrs = csize == 1 ? 1 : 2;
   const auto smem_of = [&](int rows) { return lan_rows_smem<VV>(rows) + (mf ? H->mf_nent * sizeof(MfEntry) : 0); };
+  if (P.none) return false;
   if (!P.ok) {
     int maxsm = 0;
     QD_CUDA(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
@@ -871,7 +872,8 @@ static bool lan_plan(qd_ham* H, bool mf, K kern1, K kern_many, LanPlan& P, cudaL
         rows = 1;
         for (int b = 0; b < grid; ++b) rows = std::max(rows, first[b + 1] - first[b]);
       }
-      if (smem_of(rows) + 8192 > (size_t)maxsm) return false;
+      P.none = smem_of(rows) + 8192 > (size_t)maxsm;
+      if (P.none) return false;
       if (csize == 1) break;
       allow_dynamic_smem(kern, ctx->device);
       cfg.gridDim = dim3((unsigned)grid);
@@ -882,7 +884,8 @@ static bool lan_plan(qd_ham* H, bool mf, K kern1, K kern_many, LanPlan& P, cudaL
       int fit = 0;
       QD_CUDA(cudaOccupancyMaxActiveClusters(&fit, kern, &q));
       if (fit >= ncl) break;
-      if (fit < 1) return false;
+      P.none = fit < 1;
+      if (P.none) return false;
       ncl = fit;
     }
     P.ok = true;
