@@ -840,7 +840,6 @@ static bool lanczos_run_res(qd_ham* H, const MV* vals, bool mf, LanczosBuffers<V
   r.stop = B.stop.p;
   r.flags = lan_flags(W);
   r.slots = &W.lan_slots;
-  r.xv = &W.lan_x;
   if (!lan_res_run(H, r)) return false;
   if (form) form->step_fused = 1;
   return true;

@@ -124,7 +124,6 @@ struct Workspace {
   LanczosBuffers<cplx> hl_c;
   LanPlan lan_plan[7];          // real and complex: local and Paige's rule; the exponential; real and complex matrix-free
   DBuf<double> lan_slots;
-  DBuf<char> lan_x;             // fixed-point copies of the basis (uniform couplings)
   DBuf<int> lan_flags;
   // H psi and the result of state_eval, kept between calls (a device allocation
   // and free per call would wait for the whole device)

@@ -59,6 +59,9 @@ constexpr int64_t lan_wide_rows() {
   return sizeof(VV) == sizeof(double) ? 1 << 17 : 1 << 15;
 }
 constexpr int kLanMaxExp = 32;
+// Fixed-point copies of the basis during a run on uniform couplings (given back at its end): 122 steps a launch
+// at 65,536 rows.
+constexpr int64_t kLanCopyBytes = 128ll << 20;
 // A block's rows of three vectors and their order by length; the transitions' 16-byte words follow.
 template <typename VV>
 __host__ __device__ constexpr size_t lan_rows_smem(int rows) {
@@ -505,6 +508,7 @@ __global__ void __launch_bounds__(kLanThreads, 1) lan_kernel(LanArgsOf<MV, VV, k
   VV* ring = reinterpret_cast<VV*>(lan_smem);  // V[k] of the block's rows at ring + (k % 3) rows
   VV* Vg = A.V + r0;
   const GridX& X = A.X;
+  if (kUni && A.first > 1 && *A.stop != 0) return;  // an earlier launch of the run broke down
   const bool mute = X.hold && blockIdx.x == 0;
   int lanes = 1;
   while (lanes < 4 && 2 * lanes * A.rows <= (kUni ? 512 : 256)) lanes *= 2;
@@ -935,20 +939,14 @@ static LanArgs<MV, VV> lan_args(qd_ham* H, const MV* vals, bool mf, const LanPla
   return A;
 }
 
-template <typename MV, typename VV, bool kUni, bool kPaige, bool kMf>
-static bool lan_launch(qd_ham* H, const LanRun<MV, VV>& r) {
+// Steps first .. last of r in one launch.
+template <typename MV, typename VV, bool kUni, bool kPaige, bool kMf, typename K>
+static void lan_launch_steps(qd_ham* H, const LanRun<MV, VV>& r, const LanPlan& P, const cudaLaunchConfig_t& cfg, K kern,
+                             XInt* xv, int first, int last) {
   Ctx* ctx = H->ctx;
-  constexpr int kC = sizeof(VV) == sizeof(cplx);
-  LanPlan& P = ham_workspace(H).lan_plan[kMf ? 5 + kC : 2 * kC + kPaige];
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute at[2];
-  auto kern = lan_kernel<MV, VV, true, kUni, kPaige, false, kMf>;
-  if (!lan_plan<VV>(H, kMf, kern, lan_kernel<MV, VV, false, kUni, kPaige, false, kMf>, P, cfg, at, kern)) return false;
   constexpr int kPer = sizeof(VV) / sizeof(double);
-  const size_t nx = (size_t)(r.kdim + 1) * r.ld * sizeof(XInt);
-  if (kUni && r.xv->n < nx) r.xv->alloc(nx);
   LanArgs<MV, VV> A =
-      lan_args(H, r.vals, kMf, P, r.V, r.ld, r.first, r.last, kPaige ? 2 : 1 + 3 * kPer, r.flags, r.slots, kUni ? reinterpret_cast<XInt*>(r.xv->p) : nullptr);
+      lan_args(H, r.vals, kMf, P, r.V, r.ld, first, last, kPaige ? 2 : 1 + 3 * kPer, r.flags, r.slots, xv);
   if (kUni) {
     A.fxdiag = r.form->diag_zero ? nullptr : r.form->diag.p;
     A.cF = std::ldexp(r.form->c, -r.form->F);
@@ -979,6 +977,31 @@ static bool lan_launch(qd_ham* H, const LanRun<MV, VV>& r) {
     QD_CUDA(cudaLaunchKernelEx(&cfg, kern, A));
   }
   QD_LAUNCHED(ctx);
+}
+
+template <typename MV, typename VV, bool kUni, bool kPaige, bool kMf>
+static bool lan_launch(qd_ham* H, const LanRun<MV, VV>& r) {
+  constexpr int kC = sizeof(VV) == sizeof(cplx);
+  LanPlan& P = ham_workspace(H).lan_plan[kMf ? 5 + kC : 2 * kC + kPaige];
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[2];
+  auto kern = lan_kernel<MV, VV, true, kUni, kPaige, false, kMf>;
+  if (!lan_plan<VV>(H, kMf, kern, lan_kernel<MV, VV, false, kUni, kPaige, false, kMf>, P, cfg, at, kern)) return false;
+  // as many steps a launch as the copies' memory holds; a later launch makes the first copy again, and its
+  // bits are those of one launch
+  int most = r.last + 1 - r.first;
+  DBuf<XInt> xv;
+  if (kUni) {
+    most = (int)std::min<int64_t>(most, std::max<int64_t>(kLanCopyBytes / (r.ld * (int64_t)sizeof(XInt)) - 1, 1));
+    try {
+      xv.alloc((size_t)(most + 1) * r.ld);
+    } catch (const Error&) {  // the steps launched one by one need two copies
+      clear_error();
+      return false;
+    }
+  }
+  for (int first = r.first; first <= r.last; first += most)
+    lan_launch_steps<MV, VV, kUni, kPaige, kMf>(H, r, P, cfg, kern, xv.p, first, std::min(r.last, first + most - 1));
   return true;
 }
 

@@ -35,7 +35,6 @@ struct LanRun {
   int* stop;
   int* flags;        // [0] a vector left the fixed-point range, [1] a wait ran out (both 0 before)
   DBuf<double>* slots;
-  DBuf<char>* xv;  // `form`: the vectors' fixed-point copies
 };
 template <typename MV, typename VV>
 bool lan_res_run(qd_ham* H, const LanRun<MV, VV>& r);

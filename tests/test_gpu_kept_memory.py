@@ -27,3 +27,26 @@ def test_a_sector_too_large_for_the_persistent_form_is_looked_at_once(ctx, monke
             q.lanczos_evolve(H, psi, 0, 1, 0.05, 4, 1)
             count[split] = ctx.launches() - n0
     assert count[False] == count[True]
+
+
+def lowest(sec, H, kdim, add=-1):
+    psi = q.getState(sec, 1)
+    psi.set(0, q.start_vector(sec.dim, 3).astype(complex))
+    s = q.LanczosSolver(sec, kdim)
+    while s.act_dim() < kdim:
+        s.getGroundState(H, psi, 0, add)
+    return s.eigenvalues(), psi.get(0)
+
+
+def test_long_uniform_solves_run_in_pieces_with_the_same_bits(ctx):
+    """48,620 rows: the fixed-point copies of 171 steps are the limit of one launch.  One call (two pieces), a
+    call a few steps short of the limit and grown over it, and pieces of the caller's."""
+    spec, ham = chains.xxz_chain(18, 1.0, 0.7, True)
+    sec = q.Sector(spec.index, spec.constraints)
+    H = sec.lower(ham)
+    n0 = ctx.launches()
+    ref = lowest(sec, H, 180)
+    assert ctx.launches() - n0 < 20
+    for add in (165, 60):
+        got = lowest(sec, sec.lower(ham), 180, add)
+        assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])
