@@ -1225,12 +1225,6 @@ __global__ void __launch_bounds__(kVecThreads) herm_accum_kernel(int64_t n, doub
   }
 }
 
-template <typename VV>
-static LanczosBuffers<VV>& herm_buffers(Workspace& W) {
-  if constexpr (std::is_same<VV, double>::value) return W.hl_d;
-  else return W.hl_c;
-}
-
 template <typename MV, typename VV>
 static void herm_lanczos_impl(qd_ham* H, cplx* psi, const double* psi_nrm2, int kdim, double* evals_out,
                               qd_lanczos_result* res) {
@@ -1243,9 +1237,18 @@ static void herm_lanczos_impl(qd_ham* H, cplx* psi, const double* psi_nrm2, int 
   const int vg = vec_grid(ctx, n);
   // the basis kept, in one persistent launch (lanres.cu): the second pass would form the same vectors again
   const int64_t ldv = (n + 31) / 32 * 32;
+  std::unique_ptr<LanczosBuffers<VV>> keep;  // the call's: the operator holds no basis afterwards
   if (lan_res_takes(H, kLanResMax) && (int64_t)(kdim + 2) * ldv * (int64_t)sizeof(VV) <= kHermBasisBytes) {
-    LanczosBuffers<VV>& B = herm_buffers<VV>(W);
-    B.ensure(n, kdim + 1);
+    keep.reset(new LanczosBuffers<VV>());
+    try {
+      keep->ensure(n, kdim + 1);
+    } catch (const Error&) {  // the two passes need three vectors
+      clear_error();
+      keep.reset();
+    }
+  }
+  if (keep) {
+    LanczosBuffers<VV>& B = *keep;
     QD_CUDA(cudaMemsetAsync(B.stop.p, 0, sizeof(int), ctx->stream));
     const double one = 1.0;
     QD_CUDA(cudaMemcpyAsync(B.scl.p, &one, sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
@@ -1296,6 +1299,7 @@ static void herm_lanczos_impl(qd_ham* H, cplx* psi, const double* psi_nrm2, int 
       res->err = hn[K];
       return;
     }
+    keep.reset();
   }
   DBuf<VV> v(n), w(n), h(n), a(kdim + 2);
   DBuf<double> nn(kdim + 2);

@@ -120,8 +120,6 @@ struct Workspace {
   DBuf<unsigned> tickets;
   LanczosBuffers<double> lz_d;
   LanczosBuffers<cplx> lz_c;
-  LanczosBuffers<double> hl_d;  // Hermitian::LanczosSolver's, apart from an open incremental solve
-  LanczosBuffers<cplx> hl_c;
   LanPlan lan_plan[7];          // real and complex: local and Paige's rule; the exponential; real and complex matrix-free
   DBuf<double> lan_slots;
   DBuf<int> lan_flags;

@@ -50,3 +50,35 @@ def test_long_uniform_solves_run_in_pieces_with_the_same_bits(ctx):
     for add in (165, 60):
         got = lowest(sec, sec.lower(ham), 180, add)
         assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])
+
+
+def used():
+    torch = pytest.importorskip("torch")
+    free, total = torch.cuda.mem_get_info()
+    return total - free
+
+
+def test_an_operator_keeps_no_basis_after_a_solve(ctx):
+    """Memory that 24 operators hold beyond their matrices after a Hermitian and a uniform Lanczos solve:
+    the basis of the open solve (a later call may grow it), not the Hermitian solver's or the copies."""
+    spec, ham = chains.xxz_chain(18, 1.0, 0.7, True)
+    sec = q.Sector(spec.index, spec.constraints)
+    c = q.Context()
+    sec = q.Sector(spec.index, spec.constraints, ctx=c)
+    hams = [sec.lower(ham) for _ in range(24)]
+    vec = sec.dim * 8
+    psi = q.getState(sec, 1)
+
+    def solve(H):
+        psi.set(0, q.start_vector(sec.dim, 3).astype(complex))
+        q.Hermitian.LanczosSolver(sec, 60).getGroundState(H, psi, 0)
+        psi.set(0, q.start_vector(sec.dim, 3).astype(complex))
+        q.LanczosSolver(sec, 60).getGroundState(H, psi, 0)
+
+    solve(hams[0])  # the shared buffers
+    u0 = used()
+    for H in hams[1:]:
+        solve(H)
+    # 61 vectors of the open solve and some thirty of workspace an operator; the Hermitian basis would add 62
+    # and the copies 122
+    assert (used() - u0) / 23 < 110 * vec
