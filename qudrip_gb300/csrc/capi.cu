@@ -390,12 +390,7 @@ qd_status qd_state_create(qd_ctx* ctx, int64_t dim, int nt, qd_state** out) {
     st->nt = nt;
     st->ld = (dim + 31) / 32 * 32;
     try {
-      try {
-        st->data.alloc((size_t)st->ld * nt);
-      } catch (const Error&) {
-        ctx->cache->drain();  // what is kept may be what is missing
-        st->data.alloc((size_t)st->ld * nt);
-      }
+      st->data.alloc((size_t)st->ld * nt);
       QD_CUDA(cudaMemsetAsync(st->data.p, 0, st->data.bytes(), ctx->stream));  // Matrix::Zero (state.hpp:29)
       QD_CUDA(cudaStreamSynchronize(ctx->stream));
     } catch (...) {

@@ -92,8 +92,8 @@ struct AllocStreamScope {
 // again is used after everything that used it before.  States are not taken
 // from here: their addresses are handed out, and a caller may read them on a
 // stream of its own until they are freed.  At most kDevCacheBytes are kept
-// (larger buffers never); everything is given back with the context, and when
-// an allocation fails.
+// (larger buffers never); everything is given back with the context, and every
+// context's when an allocation of any of them, or of a server's pool, fails.
 constexpr size_t kDevCacheBytes = (size_t)1 << 30;
 constexpr size_t kDevCacheBlock = (size_t)1 << 28;
 struct DevCache {
@@ -133,6 +133,35 @@ struct DevCache {
     closed |= close;
   }
   ~DevCache() { drain(true); }
+};
+// The caches of all contexts: what one keeps may be what another misses.  (Never destroyed, so that contexts
+// may go at any time.)
+struct DevCaches {
+  std::mutex lock;
+  std::vector<std::weak_ptr<DevCache>> all;
+  static DevCaches& get() {
+    static DevCaches* c = new DevCaches;
+    return *c;
+  }
+  std::shared_ptr<DevCache> make() {
+    auto c = std::make_shared<DevCache>();
+    std::lock_guard<std::mutex> g(lock);
+    size_t k = 0;
+    for (auto& w : all)
+      if (!w.expired()) all[k++] = w;
+    all.resize(k);
+    all.push_back(c);
+    return c;
+  }
+  void drain() {
+    std::vector<std::shared_ptr<DevCache>> live;
+    {
+      std::lock_guard<std::mutex> g(lock);
+      for (auto& w : all)
+        if (auto c = w.lock()) live.push_back(std::move(c));
+    }
+    for (auto& c : live) c->drain();
+  }
 };
 // The cache that this thread's DBuf allocations come from; null: plain cudaMalloc.
 inline std::shared_ptr<DevCache>& alloc_cache() {
@@ -179,25 +208,22 @@ struct DBuf {
     release();
     if (count == 0) count = 1;
     s = alloc_stream();
-    if (s) {
-      QD_CUDA(cudaMallocAsync((void**)&p, count * sizeof(T), s));
-    } else if (alloc_cache()) {
+    size_t b = count * sizeof(T);
+    if (!s && alloc_cache()) {
       c = alloc_cache();
-      const size_t b = DevCache::round_up(count * sizeof(T));
+      b = DevCache::round_up(b);
       p = static_cast<T*>(c->take(b));
-      if (!p && cudaMalloc((void**)&p, b) != cudaSuccess) {
-        cudaGetLastError();
+    }
+    auto get = [&] { return s ? cudaMallocAsync((void**)&p, b, s) : cudaMalloc((void**)&p, b); };
+    if (!p && get() != cudaSuccess) {
+      cudaGetLastError();
+      DevCaches::get().drain();
+      const cudaError_t e = get();
+      if (e != cudaSuccess) {
         p = nullptr;
-        c->drain();  // what is kept may be what is missing
-        const cudaError_t e = cudaMalloc((void**)&p, b);
-        if (e != cudaSuccess) {
-          p = nullptr;
-          c.reset();
-          QD_CUDA(e);
-        }
+        c.reset();
+        QD_CUDA(e);
       }
-    } else {
-      QD_CUDA(cudaMalloc((void**)&p, count * sizeof(T)));
     }
     n = count;
   }
@@ -223,7 +249,7 @@ struct Ctx {
   int num_sms = 0;
   int64_t launches = 0;
   cudaEvent_t events[16] = {};
-  std::shared_ptr<DevCache> cache = std::make_shared<DevCache>();
+  std::shared_ptr<DevCache> cache = DevCaches::get().make();
 };
 
 struct DeviceGuard {

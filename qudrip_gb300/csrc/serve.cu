@@ -514,7 +514,7 @@ qd_status qd_server_create(qd_ctx* ctx_, const qd_server_opts* opts, qd_server**
     QD_REQUIRE(o.small_lanes + o.large_lanes + o.batch_lanes <= 64, QD_ERR_INVALID, "at most 64 lanes");
     if (o.hbm_budget <= 0) {
       size_t fr = 0, tot = 0;
-      ctx->cache->drain();  // idle buffers count as free
+      DevCaches::get().drain();  // idle buffers count as free
       QD_CUDA(cudaMemGetInfo(&fr, &tot));
       o.hbm_budget = (int64_t)(0.8 * (double)fr);
     }

@@ -82,3 +82,24 @@ def test_an_operator_keeps_no_basis_after_a_solve(ctx):
     # 61 vectors of the open solve and some thirty of workspace an operator; the Hermitian basis would add 62
     # and the copies 122
     assert (used() - u0) / 23 < 110 * vec
+
+
+def test_idle_memory_of_one_context_serves_another(ctx):
+    """A context keeps freed buffers (two 22-site operators': some 600 MB); when the device is full but for
+    150 MB, another context's state of 400 MB takes their place."""
+    torch = pytest.importorskip("torch")
+    spec, ham = chains.xxz_chain(22, 1.0, 0.7, True, np.linspace(-1, 1, 22))
+    a, b = q.Context(), q.Context()
+    sec = q.Sector(spec.index, spec.constraints, ctx=a)
+    for H in [sec.lower(ham), sec.lower(ham)]:
+        H.close()
+    small, _ = chains.xy_chain(20)  # 184,756 rows: 2.96 MB a column
+    other = q.Sector(small.index, small.constraints, ctx=b)
+    free, _ = torch.cuda.mem_get_info()
+    block = torch.empty(free - (150 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        st = q.getState(other, 135)
+        st.close()
+    finally:
+        del block
+        torch.cuda.empty_cache()
