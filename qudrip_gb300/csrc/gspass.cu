@@ -472,8 +472,13 @@ bool GsBasis::ensure(Ctx* ctx, int64_t n_, int vecs_, bool herm, bool copies) {
   Vq.release();
   size_t fr = 0, total = 0;
   if (copies && cudaMemGetInfo(&fr, &total) == cudaSuccess && (size_t)vecs_ * ld * sizeof(int4) <= fr / 4) {
-    Vq.alloc((size_t)vecs_ * ld);
-    gs_zero_tails(Vq.p, n_, ld, vecs_, ctx->stream);
+    try {
+      Vq.alloc((size_t)vecs_ * ld);
+      gs_zero_tails(Vq.p, n_, ld, vecs_, ctx->stream);
+    } catch (const Error&) {  // another thread took the memory meanwhile
+      clear_error();
+      Vq.release();
+    }
   }
   vecs = vecs_;
   n = n_;
