@@ -17,23 +17,27 @@
 // rounding left on all of them: the same two-fold orthogonality for half the
 // work.  The basis is stored unnormalised with its scales.
 //
-// The projections and their removal run in integer arithmetic on 55-bit copies
-// of the block's rows in shared memory (qvec.cuh); the product, the norm and
-// the combination stay in FP64.  Over 32 evolutions, 108 damped or unitary
-// quench states and 12 ground states of random sizes the mean error against 64-bit
-// references is 3.9e-16, 7.2e-16 and 6.5e-16 (kernels launched one by one:
-// 4.3e-16, 7.8e-16 and 6.5e-16).
+// The projections and norms run in integer arithmetic on 55-bit copies of the
+// block's rows in shared memory (qvec.cuh): a sum rounds relative to its largest
+// terms in FP64 as well.  The product, the removal of the projections (on the
+// vectors themselves, from L1 and L2) and the combination are FP64, so that what
+// is stored keeps the relative accuracy of each row; with the removal on the
+// copies, amplitudes of a localised state some 1e-14 below its largest were lost.
+// Over 41 evolutions, 137 damped or unitary quench states and 16 ground states of
+// random sizes the mean error against 64-bit references is 3.9e-16, 6.7e-16 and
+// 6.0e-16 (passes over a basis in memory: 4.3e-16, 7.6e-16 and 6.3e-16).
 //
 // The exponential of the small Hessenberg matrix (act <= 32) is a Taylor series
 // of exp(-i h K) e_0 on sub-steps of norm <= 1, formed redundantly by every
 // block, and the combination uses the block's own rows: evolve is one launch.
 //
 // Measured (GB300, SM clock 1.9 GHz): dim 4,900, m = 30, not Hermitian: 3.3 ms
-// -> 0.57 ms a step; dim 36, m = 20: 0.56 -> 0.18 ms; ground state of the 4 x 4
+// -> 0.65 ms a step; dim 36, m = 20: 0.56 -> 0.18 ms; ground state of the 4 x 4
 // cluster (dim 12,870, 40 columns, real vectors): 6.5 -> 1.1 ms.  A column at dim
-// 4,900 is 35,000 cycles: the two exchanges 14,600, the projections and their
-// removal 14,000, the product 2,800, the rest scalar FP64 operations between
-// block barriers (16,000 cycles a column in all on one block of 36 rows).
+// 4,900 is 40,000 cycles: the two exchanges 14,600, the projections and their
+// removal 19,000 (14,000 with the removal in integers), the product 2,800, the
+// rest scalar FP64 operations between block barriers (16,000 cycles a column in
+// all on one block of 36 rows).
 // Operators whose rows do not fit (about 60,000 rows at m = 30) take passes over
 // a basis in memory (gspass.cu), as served requests do.
 #include <algorithm>
@@ -56,6 +60,7 @@ constexpr int kArnCluster = 8;  // blocks per cluster
 constexpr int kArnLdh = kArnMaxVecs + 1;
 constexpr int kArnHs = kArnMaxExp + 1;
 constexpr int kArnMaxSubsteps = 64;
+constexpr double kArnTerms = 1e-24;  // the last Taylor term's bound: small components keep their own accuracy
 constexpr int kArnMinRows = 64;     // rows of a block before the grid covers every SM
 constexpr int kArnMaxResRows = 3800;  // rows of a resident block: its sums stay within 128 terms a thread
 
@@ -132,8 +137,7 @@ struct ArnShared {
   double xv[2 * kArnMaxVecs + 2];   // this block's sums
   double red[2 * kArnMaxVecs + 2];  // the grid's
   VV c1[kArnMaxVecs];           // projections of the first pass
-  typename QVec<VV>::T cq[kArnMaxVecs];  // coefficients on the quantised vectors
-  double uc;                    // their scale
+  VV cf[kArnMaxVecs];           // coefficients on the stored vectors
   double scl[kArnMaxVecs + 2];
   double u[kArnMaxVecs + 2];    // scales of the block's quantised vectors
   double us[kArnMaxVecs + 2];   // u[j] scl[j]
@@ -152,15 +156,6 @@ __device__ __forceinline__ unsigned arn_block_max(ArnShared<VV, T>& S, unsigned 
   m = __reduce_max_sync(0xffffffffu, lane < T / 32 ? S.mx[lane] : 0u);
   __syncthreads();
   return m;
-}
-
-// The update coefficients of the quantised vectors (thread j's c, j < J < blockDim.x), quantised.
-template <typename VV, int T>
-__device__ void arn_quant_coefs(ArnShared<VV, T>& S, VV c, int J) {
-  const QScale q = q_scale(arn_block_max<VV, T>(S, q_mag(c)));
-  if (threadIdx.x < J) S.cq[threadIdx.x] = q_of(c, q.E);
-  if (threadIdx.x == 0) S.uc = q.u;
-  __syncthreads();
 }
 
 // The block's share of the projections <v_{j0+j}, w>, j < J, into S.xv: resident vectors.
@@ -200,35 +195,39 @@ __device__ void arn_dots_res(ArnShared<VV, T>& S, const typename QVec<VV>::T* Vs
   __syncthreads();
 }
 
-// put(r, re, im) of sum_j cq[j] V_{j0+j}[r] on the block's rows: resident vectors; thread (r, c) takes
-// every JC-th vector when the rows alone leave threads idle.
+// put(r, sum_j cf[j] V_j[r]) on the block's rows, J vectors of stride ld from V, in FP64 from the vectors in memory
+// (L1 and L2); thread (r, c) takes every JC-th vector when the rows alone leave threads idle.
 template <typename VV, int T, typename F>
-__device__ void arn_comb_res(ArnShared<VV, T>& S, const typename QVec<VV>::T* Vs, int ldr, int j0, int J, int R,
-                             F&& put) {
+__device__ void arn_comb(ArnShared<VV, T>& S, const VV* V, int64_t ld, int J, int R, F&& put) {
   const int tid = threadIdx.x;
-  const int JC = R > 0 ? min(min(T / R, J), 8) : 1;
+  const int JC = R > 0 ? max(1, min(min(T / R, J), 8)) : 1;
+  auto row = [&](int r, int c) {
+    const VV* v = V + r + (int64_t)c * ld;
+    const int64_t hop = (int64_t)JC * ld;
+    VV a = vzero(VV{});
+    int j = c;
+    for (; j + 3 * JC < J; j += 4 * JC, v += 4 * hop) {
+      const VV v0 = v[0], v1 = v[hop], v2 = v[2 * hop], v3 = v[3 * hop];
+      a = vfma(S.cf[j], v0, a);
+      a = vfma(S.cf[j + JC], v1, a);
+      a = vfma(S.cf[j + 2 * JC], v2, a);
+      a = vfma(S.cf[j + 3 * JC], v3, a);
+    }
+    // (the rest in one predicated batch issues FP64 instructions for lanes that are done: a step at dim 36 took
+    // 10% longer)
+    for (; j < J; j += JC, v += hop) a = vfma(S.cf[j], v[0], a);
+    return a;
+  };
   if (JC < 2) {
-    for (int r = tid; r < R; r += T) {
-      QComb<VV> a;
-      for (int j = 0; j < J; ++j) a.add(S.cq[j], Vs[(size_t)(j0 + j) * ldr + r]);
-      put(r, a.re(), a.im());
-    }
+    for (int r = tid; r < R; r += T) put(r, row(r, 0));
   } else {
-    if (tid < R * JC) {
-      const int c = tid / R, r = tid - c * R;
-      QComb<VV> a;
-      for (int j = c; j < J; j += JC) a.add(S.cq[j], Vs[(size_t)(j0 + j) * ldr + r]);
-      S.part[2 * tid].hi = a.re();
-      S.part[2 * tid + 1].hi = a.im();
-    }
+    VV* part = reinterpret_cast<VV*>(S.part);
+    if (tid < R * JC) part[tid] = row(tid % R, tid / R);
     __syncthreads();
     if (tid < R) {
-      long long re = 0, im = 0;  // one sum over J < 96 terms of at most 2^55: no overflow
-      for (int c = 0; c < JC; ++c) {
-        re += S.part[2 * (c * R + tid)].hi;
-        im += S.part[2 * (c * R + tid) + 1].hi;
-      }
-      put(tid, re, im);
+      VV a = part[tid];
+      for (int c = 1; c < JC; ++c) a = vadd(a, part[c * R + tid]);
+      put(tid, a);
     }
   }
 }
@@ -269,7 +268,7 @@ __device__ bool arn_expm(const cplx* hs, int act, double h, bool band, cplx (*t)
       double b = 1.0;  // th^i / i!
       for (int i = 1; i <= 30; ++i) {
         b *= th * kArnInv[i];
-        if (b <= 1e-18) break;
+        if (b <= kArnTerms) break;
         tm = i;
       }
       fac[tid] = (tid >= 1) ? hst * kArnInv[tid] : 0.0;
@@ -435,20 +434,19 @@ __global__ void __launch_bounds__(kArnThreads, 1) arn_kernel(ArnArgs<MV, VV> A) 
     }
     if (!kExp && S.stop && !scaled) return;  // a zero start vector: the host reports it (evolve goes on, as NaNs)
     const double sx = S.scl[J - 1];
-    VV cq = vzero(VV{});
     if (tid < J1) {
       // <v_j, w> = sx <v_j, H V[J-1]>, and v_{J-1}'s own scale, which its share above did not have
       VV c = vscale(sx, reinterpret_cast<const VV*>(S.red)[tid]);
       if (tid == J1 - 1 && !scaled) c = vscale(sx, c);
       S.c1[tid] = c;
-      cq = vscale(S.us[j1 + tid], c);
+      S.cf[tid] = vscale(S.scl[j1 + tid], c);
     }
+    __syncthreads();
     // 2: the first pass taken out, projections of what is left
     {
-      arn_quant_coefs<VV, T>(S, cq, J1);
       unsigned mag = 0;
-      arn_comb_res<VV, T>(S, Vs, A.ldr, j1, J1, R, [&](int r, long long re, long long im) {
-        const VV o = q_sub(vscale(sx, wd[r]), S.uc, re, im);
+      arn_comb<VV, T>(S, Vg + (int64_t)j1 * A.ld, A.ld, J1, R, [&](int r, VV sum) {
+        const VV o = vfma(sx, wd[r], vscale(-1.0, sum));
         wd[r] = o;
         mag = max(mag, q_mag(o));
       });
@@ -457,10 +455,9 @@ __global__ void __launch_bounds__(kArnThreads, 1) arn_kernel(ArnArgs<MV, VV> A) 
       arn_dots_res<VV, T>(S, Vs, A.ldr, 0, J, wq, uw, R);
     }
     x_sum<kOne>(X, slot2, S.xv, J * kPer, S.red);
-    cq = vzero(VV{});
     if (tid < J) {
       const VV c = reinterpret_cast<const VV*>(S.red)[tid];
-      cq = vscale(S.us[tid], c);
+      S.cf[tid] = vscale(S.scl[tid], c);
       const VV hij = (tid >= j1) ? vadd(S.c1[tid - j1], c) : c;
       if (kExp) hs[(J - 1) * kArnHs + tid] = arn_c(hij);
       if (blockIdx.x == 0) {
@@ -469,10 +466,10 @@ __global__ void __launch_bounds__(kArnThreads, 1) arn_kernel(ArnArgs<MV, VV> A) 
       }
     }
     // 3: the second pass taken out, the norm, and the rows for everybody's gathers
-    arn_quant_coefs<VV, T>(S, cq, J);
+    __syncthreads();
     unsigned mag = 0;
-    arn_comb_res<VV, T>(S, Vs, A.ldr, 0, J, R, [&](int r, long long re, long long im) {
-      const VV o = q_sub(wd[r], S.uc, re, im);
+    arn_comb<VV, T>(S, Vg, A.ld, J, R, [&](int r, VV sum) {
+      const VV o = vadd(wd[r], vscale(-1.0, sum));
       wd[r] = o;
       if (!mute) x_put(wg + r, o);
       mag = max(mag, q_mag(o));
@@ -505,35 +502,10 @@ __global__ void __launch_bounds__(kArnThreads, 1) arn_kernel(ArnArgs<MV, VV> A) 
   __syncthreads();
   // psi_out = sum_j y_j v_j on the block's rows
   if constexpr (kPer == 2) {
+    if (tid < act) S.cf[tid] = y[tid];
+    __syncthreads();
     cplx* out = A.psi_out + r0;
-    const int JC = R > 0 ? min(min(T / R, act), 8) : 1;
-    cplx* part = reinterpret_cast<cplx*>(S.part);
-    auto row = [&](int r, int c, int by) {
-      const VV* v = Vg + r + (int64_t)c * A.ld;
-      const int64_t hop = (int64_t)by * A.ld;
-      cplx a = mkc(0.0, 0.0);
-      int j = c;
-      for (; j + 3 * by < act; j += 4 * by, v += 4 * hop) {
-        const cplx v0 = v[0], v1 = v[hop], v2 = v[2 * hop], v3 = v[3 * hop];
-        a = vfma(y[j], v0, a);
-        a = vfma(y[j + by], v1, a);
-        a = vfma(y[j + 2 * by], v2, a);
-        a = vfma(y[j + 3 * by], v3, a);
-      }
-      for (; j < act; j += by, v += hop) a = vfma(y[j], v[0], a);
-      return a;
-    };
-    if (JC < 2) {
-      for (int r = tid; r < R; r += T) out[r] = row(r, 0, 1);
-    } else {
-      if (tid < R * JC) part[tid] = row(tid % R, tid / R, JC);
-      __syncthreads();
-      if (tid < R) {
-        cplx a = part[tid];
-        for (int c = 1; c < JC; ++c) a = vadd(a, part[c * R + tid]);
-        out[tid] = a;
-      }
-    }
+    arn_comb<VV, T>(S, Vg, A.ld, act, R, [&](int r, VV sum) { out[r] = sum; });
   }
 }
 

@@ -4,15 +4,15 @@
 //
 // In FP64 the projections and their removal are bound by FP64 issue (76 cycles
 // a warp instruction and SM quarter): at 705,432 rows and 16 columns they took
-// 94 and 44 us a launch where the vectors' bytes take 14.  Here both run on
-// 55-bit integers (qvec.cuh), with one scale per vector and tile of rows:
+// 94 and 44 us a launch where the vectors' bytes take 14.  The projections run
+// on 55-bit integers here (qvec.cuh), with one scale per vector and tile of rows:
 //   dots    c_j = <V_j, w>: a warp owns a tile, holds its rows of w quantised in
 //           registers and passes over the vectors, four vectors' totals to one
 //           warp sum; lane j then keeps vector j's total in FP64, one
 //           conversion per tile.
-//   update  w -= sum_j c_j V_j: the coefficients times the vectors' scales are
-//           quantised per tile (lane j its own), one conversion and one FMA per
-//           real at the end.
+//   update  w -= sum_j c_j V_j in FP64, on the vectors themselves: what is stored
+//           keeps the relative accuracy of each row, also where a tile's largest
+//           is orders of magnitude above it (a localised state).
 // A vector's rows come through a ring of asynchronous copies that each thread
 // reads back itself, no barrier.
 // Pass 1 is dots; its update runs in the same launch as pass 2's dots, and pass
@@ -25,12 +25,13 @@
 // scales, which saves a pass; the product's own scale applies them.
 //
 // Measured (GB300), two steps of the recurrence and exponential, Hermitian:
-// 705,432 rows, m = 16: 10.4 -> 4.29 ms; 184,756 rows, m = 30: 10.2 -> 3.8 ms;
-// 2,704,156 rows, m = 30: 94.8 -> 29.3 ms.  At 705,432 rows a step's product is
-// 62 us (bound by FP64 issue and its gathers), the dots 52 and the update 40 us
-// at 12 vectors, bound by the latencies between a warp's integer instructions
-// (a third of the issue slots) with HBM at half its rate: more warps, deeper
-// rings and smaller tiles measured the same.
+// 705,432 rows, m = 16: 10.4 -> 4.87 ms; 184,756 rows, m = 30: 10.2 -> 4.6 ms;
+// 2,704,156 rows, m = 30: 94.8 -> 37.8 ms (4.25, 3.7 and 29.5 with the removal on
+// the integer copies).  At 705,432 rows a step's product is 62 us (bound by FP64
+// issue and its gathers), the dots 52 us at 12 vectors, bound by the latencies
+// between a warp's integer instructions (a third of the issue slots) with HBM at
+// half its rate (more warps, deeper rings and smaller tiles measured the same),
+// the update 70, bound by FP64 issue.
 #include <algorithm>
 
 #include "gspass.cuh"
@@ -100,16 +101,17 @@ __device__ __forceinline__ int gs_exp(double u) {
   const int e = (int)(((unsigned)__double2hiint(u) >> 20) & 0x7ff);
   return e ? e - 1023 + 27 : 1 << 20;
 }
-template <bool kQ>
-__device__ __forceinline__ int4 gs_read(unsigned slot, int E) {
-  if (kQ) {
-    int4 v;
-    asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(slot));
-    return v;
-  }
+__device__ __forceinline__ cplx gs_read_fp(unsigned slot) {
   double re, im;
   asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(re), "=d"(im) : "r"(slot));
-  return q_of(mkc(re, im), E);
+  return mkc(re, im);
+}
+template <bool kQ>
+__device__ __forceinline__ int4 gs_read(unsigned slot, int E) {
+  if (!kQ) return q_of(gs_read_fp(slot), E);
+  int4 v;
+  asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(slot));
+  return v;
 }
 
 // A tile's rows of J vectors in turn, their copies ahead: begin() starts them (what is computed up to the
@@ -147,44 +149,31 @@ struct GsStream {
   }
 };
 
-// w -= sum over j0 <= j < j1 of cu[j] V_j on tile t
-template <int RPL, bool kQ>
-__device__ __forceinline__ void gs_remove(const GsArgs& A, GsStream<RPL, kQ>& S, int64_t t, cplx* w, int4* cq,
+// w -= sum over j0 <= j < j1 of cu[j] V_j on tile t, in FP64 from the vectors themselves: the copies' scales
+// are their tiles', and what is stored keeps the accuracy of each row.
+template <int RPL>
+__device__ __forceinline__ void gs_remove(const GsArgs& A, unsigned ring, int64_t t, cplx* w, cplx* cf,
                                           double alpha = 0.0) {
   const int lane = threadIdx.x & 31;
   const int64_t r0 = t * (32 * RPL);
+  GsStream<RPL, false> S;
+  S.ring = ring;
   for (int c0 = A.j0; c0 < A.j1; c0 += kGsChunk) {
     const int J = min(kGsChunk, A.j1 - c0);
     S.begin(A, c0, J, r0);
-    cplx c = mkc(0.0, 0.0);
-    double uj = 0.0;
+    __syncwarp();
     if (lane < J) {
       const int j = c0 + lane;
-      uj = A.u[(int64_t)j * A.ntiles + t];
-      if (A.ndots) c = mkc(A.scl[j] * (j == A.step - 1 ? alpha : A.nrm[A.step - 1]), 0.0);
-      else c = A.cu[j];
-      c = vscale(uj, c);
+      if (A.ndots) cf[lane] = mkc(A.scl[j] * (j == A.step - 1 ? alpha : A.nrm[A.step - 1]), 0.0);
+      else cf[lane] = A.cu[j];
     }
-    const QScale q = q_scale(__reduce_max_sync(0xffffffffu, q_mag(c)));
     __syncwarp();
-    cq[lane] = q_of(c, q.E);
-    __syncwarp();
-    QAcc re[RPL], im[RPL];
     for (int j = 0; j < J; ++j) {
       const unsigned v = S.next();
-      const int E = kQ ? 0 : gs_exp(__shfl_sync(0xffffffffu, uj, j));
-      const int4 cj = cq[j];
+      const cplx c = cf[j];
 #pragma unroll
-      for (int i = 0; i < RPL; ++i) {
-        const int4 x = gs_read<kQ>(v + 512 * i, E);
-        re[i].mac(cj.x, cj.y, x.x, x.y);
-        re[i].mac(-cj.z, -cj.w, x.z, x.w);
-        im[i].mac(cj.x, cj.y, x.z, x.w);
-        im[i].mac(cj.z, cj.w, x.x, x.y);
-      }
+      for (int i = 0; i < RPL; ++i) w[i] = vsubmul(w[i], c, gs_read_fp(v + 512 * i));
     }
-#pragma unroll
-    for (int i = 0; i < RPL; ++i) w[i] = q_sub(w[i], q.u, re[i].value(), im[i].value());
   }
 }
 
@@ -223,7 +212,7 @@ template <int RPL, bool kUpd, bool kQ>
 __global__ void __launch_bounds__(kGsThreads, 1) gs_dots_kernel(GsArgs A) {
   if (gs_stopped(A)) return;
   extern __shared__ __align__(16) int4 gs_ring[];
-  __shared__ int4 cq[kGsWarps][kGsChunk];
+  __shared__ cplx cf[kGsWarps][kGsChunk];
   __shared__ long long tot[kGsWarps][2 * kGsChunk];
   __shared__ double bs[kGsWarps][2 * kGsChunk];
   __shared__ double sum[2 * kGsChunk];
@@ -249,7 +238,7 @@ __global__ void __launch_bounds__(kGsThreads, 1) gs_dots_kernel(GsArgs A) {
       w[i] = (r < A.n) ? A.src[r] : mkc(0.0, 0.0);
     }
     const double uj = (lane < A.J) ? A.u[(int64_t)(A.d0 + lane) * A.ntiles + t] : 0.0;
-    if (kUpd) gs_remove<RPL, kQ>(A, S, t, w, cq[warp], alpha);
+    if (kUpd) gs_remove<RPL>(A, S.ring, t, w, cf[warp], alpha);
     S.begin(A, A.d0, A.J, r0);
     unsigned mag = 0;
 #pragma unroll
@@ -330,12 +319,11 @@ template <int RPL, bool kQ>
 __global__ void __launch_bounds__(kGsThreads, 1) gs_update_kernel(GsArgs A) {
   if (gs_stopped(A)) return;
   extern __shared__ __align__(16) int4 gs_ring[];
-  __shared__ int4 cq[kGsWarps][kGsChunk];
+  __shared__ cplx cf[kGsWarps][kGsChunk];
   __shared__ double bs[kGsWarps];
   __shared__ double sum[1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  GsStream<RPL, kQ> S;
-  S.ring = (unsigned)__cvta_generic_to_shared(gs_ring + warp * (32 * kGsRing) + lane);
+  const unsigned ring = (unsigned)__cvta_generic_to_shared(gs_ring + warp * (32 * kGsRing) + lane);
   double acc = 0.0;
   // from the last tile down: the dots that ran before left the last tiles in L2
   for (int64_t t = A.ntiles - 1 - gs_first_tile(); t >= 0; t -= (int64_t)gridDim.x * kGsWarps) {
@@ -346,7 +334,7 @@ __global__ void __launch_bounds__(kGsThreads, 1) gs_update_kernel(GsArgs A) {
       const int64_t r = r0 + 32 * i + lane;
       w[i] = (r < A.n) ? A.src[r] : mkc(0.0, 0.0);
     }
-    gs_remove<RPL, kQ>(A, S, t, w, cq[warp]);
+    gs_remove<RPL>(A, ring, t, w, cf[warp]);
     unsigned mag = 0;
 #pragma unroll
     for (int i = 0; i < RPL; ++i) mag = max(mag, q_mag(w[i]));
@@ -450,8 +438,8 @@ bool GsBasis::ensure(Ctx* ctx, int64_t n_, int vecs_, bool herm, bool copies) {
   if (n_ == n && vecs_ == vecs && herm == (dots.p != nullptr)) return false;
   n = 0;  // until every buffer is there
   // Tiles of 128 rows amortise their conversions better, tiles of 64 fill the SMs' warps sooner: two steps
-  // of m = 16 (m = 30) at 48,620 rows 1.05 (2.56) against 1.00 ms (2.39), 92,378 rows 1.30 against 1.27,
-  // 184,756 rows 1.70 (3.80) against 1.80 ms (4.02).
+  // of m = 16 (m = 30) at 12,870 rows 1.11 against 1.02 ms, 48,620 rows (2.81) against (2.50), 92,378 rows 1.37
+  // against 1.32, 184,756 rows 1.89 (4.56) against 1.96 ms (4.77).
   rpl = (n_ >= 64 * (int64_t)ctx->num_sms * kGsWarps) ? 4 : 2;
   ntiles = ceil_div(n_, 32 * rpl);
   grid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)ctx->num_sms));

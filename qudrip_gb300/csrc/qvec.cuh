@@ -1,5 +1,4 @@
-// qvec.cuh -- inner products and linear combinations of FP64 vectors in
-// integer arithmetic.
+// qvec.cuh -- inner products of FP64 vectors in integer arithmetic.
 //
 // GB300 issues one warp-wide FP64 instruction per 76 cycles and SM quarter
 // (measured; the same for one active lane as for 32), but a 32 x 32 -> 64-bit
@@ -10,9 +9,10 @@
 // overflow over 128 complex terms (h h' and h l' + l h'; the dropped l l' is
 // below 2^-56 of the scale), so a real multiply-add costs 12 cycles instead of
 // 76, and sums across threads are integer adds.  Each element is within 2^-56
-// of the tile's largest (FP64: 2^-54 of the element at worst), and the sum is
-// exact up to that and one rounding of the 2^-54 unit per thread: below the
-// rounding of an FP64 sum of the same terms.
+// of the tile's largest, so a sum is within some 2^-56 of the product of its
+// vectors' norms: what an inner product of FP64 vectors is accurate to.  (An
+// element far below its tile's largest keeps fewer bits than FP64 gives it.
+// Sums do not need them; stored vectors do, and are not formed from these.)
 #pragma once
 
 #include "vec.cuh"
@@ -131,35 +131,5 @@ struct QDot<cplx> {
   __device__ __forceinline__ long long re() const { return r.value(); }
   __device__ __forceinline__ long long im() const { return a.value() - b.value(); }
 };
-// sum of c v
-template <typename VV>
-struct QComb;
-template <>
-struct QComb<double> {
-  QAcc r;
-  __device__ __forceinline__ void add(int2 c, int2 v) { r.mac(c.x, c.y, v.x, v.y); }
-  __device__ __forceinline__ long long re() const { return r.value(); }
-  __device__ __forceinline__ long long im() const { return 0; }
-};
-template <>
-struct QComb<cplx> {
-  QAcc a, b, m;
-  __device__ __forceinline__ void add(int4 c, int4 v) {
-    a.mac(c.x, c.y, v.x, v.y);
-    b.mac(c.z, c.w, v.z, v.w);
-    m.mac(c.x, c.y, v.z, v.w);
-    m.mac(c.z, c.w, v.x, v.y);
-  }
-  __device__ __forceinline__ long long re() const { return a.value() - b.value(); }
-  __device__ __forceinline__ long long im() const { return m.value(); }
-};
-
-// w - u (re, im): one conversion and one FMA per real
-__device__ __forceinline__ double q_sub(double w, double u, long long re, long long) {
-  return fma(-u, (double)re, w);
-}
-__device__ __forceinline__ cplx q_sub(cplx w, double u, long long re, long long im) {
-  return mkc(fma(-u, (double)re, w.re), fma(-u, (double)im, w.im));
-}
 
 }  // namespace qd
