@@ -14,8 +14,9 @@
 //
 // The block's sums of its threads' partial sums are integer adds: a warp-wide
 // FP64 add takes 76 cycles on GB300 and a butterfly of seven values over
-// sixteen warps 10,600; as 53-bit integers on the scale of the largest partial
-// sum it is 2,200, and each partial sum keeps what an FP64 sum would round.
+// sixteen warps 10,600; as 57-bit integers on the scale of the largest partial
+// sum (53 bits across warps) it is 2,200: one rounding at 2^-54 of the largest a
+// warp and at 2^-58 a thread, where the tree of FP64 adds has nine.
 //
 // Hermitian::LanczosSolver runs here with its basis kept, where the reference
 // forms every vector a second time for the Ritz vector.
@@ -325,13 +326,13 @@ __device__ __forceinline__ double lan_row_uniform(const LanArgsOf<double, double
   return fma(A.cF, (double)acc, dx);
 }
 
-// v on the scale 2^E (|v| < 2^E) in units of 2^(E - 53)
+// v on the scale 2^E (|v| < 2^E) in units of 2^(E - 57): a warp's sum fits 64 bits
 __device__ __forceinline__ long long lan_fix(double v, int E) {
   const long long b = __double_as_longlong(v);
   const int e = (int)((b >> 52) & 0x7ff);
   const unsigned long long m = ((unsigned long long)b & 0xfffffffffffffull) | 0x10000000000000ull;
-  const int sh = E + 1022 - e;  // >= 0
-  long long q = (e == 0 || sh > 53) ? 0ll : (long long)(sh > 0 ? (m + (1ull << (sh - 1))) >> sh : m);
+  const int sh = E + 1018 - e;  // >= -4
+  long long q = (e == 0 || sh > 53) ? 0ll : (long long)(sh > 0 ? (m + (1ull << (sh - 1))) >> sh : m << -sh);
   return b < 0 ? -q : q;
 }
 
@@ -367,7 +368,7 @@ __device__ __forceinline__ void lan_block_sums(LanShared<T>& S, const double (&v
       long long q = lan_fix(v[i], (int)(mag[i] >> 20) - 1022);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
-      if (lane == 0) S.q[i][warp] = q;
+      if (lane == 0) S.q[i][warp] = (q + 8) >> 4;  // units of 2^(E - 53): the block's sum fits as well
     }
   }
   __syncthreads();
