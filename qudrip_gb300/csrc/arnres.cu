@@ -32,10 +32,10 @@
 // block, and the combination uses the block's own rows: evolve is one launch.
 //
 // Measured (GB300, SM clock 1.9 GHz): dim 4,900, m = 30, not Hermitian: 3.3 ms
-// -> 0.65 ms a step; dim 36, m = 20: 0.56 -> 0.18 ms; ground state of the 4 x 4
+// -> 0.60 ms a step; dim 36, m = 20: 0.56 -> 0.18 ms; ground state of the 4 x 4
 // cluster (dim 12,870, 40 columns, real vectors): 6.5 -> 1.1 ms.  A column at dim
-// 4,900 is 40,000 cycles: the two exchanges 14,600, the projections and their
-// removal 19,000 (14,000 with the removal in integers), the product 2,800, the
+// 4,900 is 38,000 cycles: the two exchanges 14,600, the projections and their
+// removal 17,000 (14,000 with the removal in integers), the product 2,800, the
 // rest scalar FP64 operations between block barriers (16,000 cycles a column in
 // all on one block of 36 rows).
 // Operators whose rows do not fit (about 60,000 rows at m = 30) take passes over
@@ -196,11 +196,12 @@ __device__ void arn_dots_res(ArnShared<VV, T>& S, const typename QVec<VV>::T* Vs
 }
 
 // put(r, sum_j cf[j] V_j[r]) on the block's rows, J vectors of stride ld from V, in FP64 from the vectors in memory
-// (L1 and L2); thread (r, c) takes every JC-th vector when the rows alone leave threads idle.
+// (L1 and L2); thread (r, c) takes every JC-th vector when the rows alone leave threads idle (an evolution of m =
+// 30 at dim 4,900: 647 us with one thread a row, 601 with two to four, 613 with eight).
 template <typename VV, int T, typename F>
 __device__ void arn_comb(ArnShared<VV, T>& S, const VV* V, int64_t ld, int J, int R, F&& put) {
   const int tid = threadIdx.x;
-  const int JC = R > 0 ? max(1, min(min(T / R, J), 8)) : 1;
+  const int JC = R > 0 ? max(1, min(min(T / R, J), 4)) : 1;
   auto row = [&](int r, int c) {
     const VV* v = V + r + (int64_t)c * ld;
     const int64_t hop = (int64_t)JC * ld;
@@ -213,9 +214,17 @@ __device__ void arn_comb(ArnShared<VV, T>& S, const VV* V, int64_t ld, int J, in
       a = vfma(S.cf[j + 2 * JC], v2, a);
       a = vfma(S.cf[j + 3 * JC], v3, a);
     }
-    // (the rest in one predicated batch issues FP64 instructions for lanes that are done: a step at dim 36 took
-    // 10% longer)
-    for (; j < J; j += JC, v += hop) a = vfma(S.cf[j], v[0], a);
+    // the last three at most: their loads in flight together, as many multiply-adds as the warp has (predicated
+    // ones issue as well)
+    if (j < J) {
+      const VV v0 = v[0];
+      VV v1 = v0, v2 = v0;
+      if (j + JC < J) v1 = v[hop];
+      if (j + 2 * JC < J) v2 = v[2 * hop];
+      a = vfma(S.cf[j], v0, a);
+#pragma unroll 1
+      for (int u = 1; j + u * JC < J; ++u) a = vfma(S.cf[j + u * JC], u == 1 ? v1 : v2, a);
+    }
     return a;
   };
   if (JC < 2) {
