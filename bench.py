@@ -584,8 +584,8 @@ def trajectory_ensemble(ctx, with_oracle=True, ntraj=4096, nsteps=1000):
     t0 = time.perf_counter()
     mean, err, st = q.traj_run(Heff, psi0, ntraj, nsteps, dt, gamma, seed, m, chan, obs)
     wall = time.perf_counter() - t0
-    form = {0: "resident: one CTA per trajectory, operator and complex64 vectors in shared memory, "
-               "truncated Taylor exp(-i dt (H - mu)) with the degree from its remainder bound",
+    form = {0: "resident: one or two trajectories per CTA, operator and complex64 vectors in shared memory, "
+               "truncated series of exp(-i dt (H - mu)) with the degree from its remainder bound",
             1: "FP64 Arnoldi exponential per trajectory and step (batched kernel)"}[int(st.path)]
     out = {"workload": f"dissipative Hubbard L=8 (dim 4900), {ntraj} trajectories x {nsteps} steps, m=30, dt=0.01",
            "trajectory_steps_per_s": ntraj * nsteps / wall, "wall_s": wall, "form": form,

@@ -233,7 +233,8 @@ qd_status qd_ham_apply(qd_ham *ham, qd_state *x, int t_in, qd_state *y,
 qd_status qd_state_eval(qd_state *psi, int t, qd_ham *ham, double *re_im);
 /* <psi(:,t)|O_i|psi(:,t)> for nobs operators of psi's sector and context
  * (replaces the loop of McManager::incrAllObs, mc_manager.hpp:88-106):
- * re_im receives 2*nobs doubles; the fused products run back to back with
+ * re_im receives 2*nobs doubles; one launch evaluates up to 32 operators
+ * (those with a CSR kernel of the caller's choice launch it, one each), with
  * one copy of the results. */
 qd_status qd_obs_eval(qd_state *psi, int t, int nobs, qd_ham *const *obs, double *re_im);
 
@@ -286,6 +287,8 @@ qd_status qd_lanczos_extend(qd_ham *ham, qd_state *psi, int t, const qd_lanczos_
 /* psi(:, t_out) = V exp(-i K h) e_0 with m-1 Arnoldi products from      */
 /* psi(:, t_in) normalised; unit norm for Hermitian H.  t_out may equal  */
 /* t_in.  act_dim (may be NULL) receives the Krylov dimension used.      */
+/* After QD_ERR_TIMEOUT (a wait of the persistent form ran out) psi is    */
+/* as it was, here and in qd_lanczos_evolve.                              */
 /* m (the solver's kry_dim) must be in 2..33.                           */
 /* ------------------------------------------------------------------ */
 qd_status qd_arnoldi_evolve(qd_ham *ham, qd_state *psi, int t_in, int t_out,
@@ -363,8 +366,9 @@ qd_status qd_krylov_evolve_batch(qd_ham *ham, const double *d_X, int64_t ldx,
 /* doubles (row = step).  Where heff has dim <= 5120 on at most 32 bits  */
 /* and one off-diagonal value +-c, each trajectory runs in one SM's      */
 /* shared memory (complex64 vectors, exp(-i heff dt) by a truncated      */
-/* Taylor series whose degree and sub-steps follow the series' remainder */
-/* bound, at most m-1 products per sub-step); otherwise every step is an */
+/* series whose degree and sub-steps follow its remainder bound, at most */
+/* m-1 products per sub-step: Chebyshev's where heff is Hermitian but for */
+/* one damping, else Taylor's); otherwise every step is an               */
 /* FP64 Arnoldi exponential with m vectors per trajectory.  The          */
 /* environment variable QD_TRAJ_ARNOLDI=1 selects the second form.       */
 /* ------------------------------------------------------------------ */
@@ -387,8 +391,8 @@ typedef struct {
   int64_t jumps;        /* jumps over all trajectories */
   double setup_ms;      /* building and uploading the resident form */
   double ensemble_ms;   /* the nsteps steps of all trajectories */
-  int32_t path;         /* 0: resident Taylor kernel, 1: FP64 Arnoldi steps */
-  int32_t products;     /* sparse products per trajectory step (Taylor terms x sub-steps, or m - 1) */
+  int32_t path;         /* 0: resident kernel, 1: FP64 Arnoldi steps */
+  int32_t products;     /* sparse products per trajectory step (series terms x sub-steps, or m - 1) */
 } qd_traj_stats;
 
 qd_status qd_traj_run(qd_ham *heff, const qd_traj_desc *desc, const double *psi0,
@@ -463,8 +467,9 @@ qd_status qd_csr_expect_noalloc(const int64_t *d_rowptr, const int32_t *d_colidx
 /*   replaces Hermitian::LanczosSolver::getGroundState                */
 /*   (sparse_algorithm.hpp:287-301) with getKrylovReprAd (:72-122)    */
 /*   and getKrylovGS (:206-238)                                       */
-/* Two-vector recurrence (no stored basis), stop once ||r||^2 <= 1e-10; */
-/* the ground-state vector is rebuilt by a second pass and written to    */
+/* Two-vector recurrence, stop once ||r||^2 <= 1e-10; the ground-state   */
+/* vector, from the vectors kept for the call up to 256 MB of them, else  */
+/* rebuilt by a second pass, is written to                               */
 /* psi(:, t).  Up to kry_dim + 1 Lanczos coefficients, as the reference's */
 /* loop; evals_out (NULL or kry_dim + 1 doubles) receives res->act_dim     */
 /* eigenvalues of the tridiagonal matrix; one product per step and pass. */
