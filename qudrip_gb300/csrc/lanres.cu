@@ -31,9 +31,9 @@
 // transition and a rank per entry, 33 us a step at dim 184,756 against 19 on the stored matrix) or from the
 // block tables of the sector (uniform couplings: 917 us a solve at 18 sites against 830 on the stored columns,
 // the same bits); it reads no stored matrix.
-// Mean error against 64-bit references over ten random cases each: ground-state
-// eigenvalues 5.4e-16 (launched step by step: 5.6e-16), evolved states 1.95e-15
-// (1.99e-15).
+// Mean error against 64-bit references over 24 random cases each: ground-state
+// eigenvalues 7.2e-16 (launched step by step: 8.1e-16), evolved states 2.19e-15
+// (2.24e-15), the Hermitian solver's eigenvalues 4.7e-16 (5.2e-16).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
