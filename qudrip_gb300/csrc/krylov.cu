@@ -1552,15 +1552,23 @@ static void lanczos_evolve_steps(qd_ham* H, const cplx* psi_in, cplx* psi, doubl
   QD_CUDA(cudaMemsetAsync(G.matvecs.p, 0, sizeof(long long), ctx->stream));
   // one launch per Krylov step (lanres.cu) where the recurrence fits the grid
   bool res_run = lan_res_takes(H, kLanResMax);
+  // the steps' state is apart until all of them are done: a wait that runs out leaves the caller's as it was
+  const bool apart = res_run && n > kLanOneBlock;
+  if (apart && G.state.n < (size_t)n) G.state.alloc(n);
+  cplx* st = apart ? G.state.p : psi;
   const double theta = res_run ? std::fabs(h) * 3.0 * ham_norm_inf(H) : 0.0;
   if (theta > kLanMaxTheta && std::isfinite(theta)) {
     int act = 1;
     int64_t mv = 0;
     for (int s = 0; s < nsteps && act; ++s, mv += act) {
-      act = lanczos_evolve_host<MV>(H, vals, B, W, s ? psi : psi_in, psi, h, kdim, G.y.p);
+      act = lanczos_evolve_host<MV>(H, vals, B, W, s ? st : psi_in, st, h, kdim, G.y.p);
       QD_REQUIRE(act || s == 0, QD_ERR_UNSUPPORTED, "the persistent recurrence's grid does not fit any more");
     }
     if (act) {
+      if (apart) {
+        QD_CUDA(cudaMemcpyAsync(psi, st, n * sizeof(cplx), cudaMemcpyDeviceToDevice, ctx->stream));
+        QD_CUDA(cudaStreamSynchronize(ctx->stream));
+      }
       if (act_out) *act_out = act;
       if (matvecs_out) *matvecs_out = mv;
       return;
@@ -1569,10 +1577,6 @@ static void lanczos_evolve_steps(qd_ham* H, const cplx* psi_in, cplx* psi, doubl
   }
   if (res_run) {
     int* flags = lan_flags(W);
-    // the steps' state is apart until all of them are done: a wait that runs out leaves the caller's as it was
-    const bool apart = n > kLanOneBlock;
-    if (apart && G.state.n < (size_t)n) G.state.alloc(n);
-    cplx* st = apart ? G.state.p : psi;
     for (int s = 0; s < nsteps && res_run; ++s) {
       res_run = lan_res_evolve<MV>(H, vals, s ? st : psi_in, st, B.V.p, B.ld, kdim, h, G.act.p, G.matvecs.p, flags,
                                    &W.lan_slots);
