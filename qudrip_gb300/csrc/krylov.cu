@@ -978,7 +978,7 @@ static void lanczos_ground_impl(qd_ham* H, cplx* psi, const double* psi_nrm2, co
   // the column source of the fixed-point form is part of what a captured recurrence launches
   const int src = !fx ? 0 : ((form->blk_state > 0 && form->use_blk) ? 2 : ((form->slots_state > 0 && form->use_slots) ? 1 : 0));
   const int kind = (mf ? 1 : 0) + 2 * fxk + (one_launch ? 4 : 0) + ((one_launch && step_wait_out_polls()) ? 8 : 0) +
-                   16 * src;
+                   16 * src + 64 * H->spmv_variant;
   if (B.kind != kind) {
     B.drop_graph();
     B.kind = kind;
@@ -1458,7 +1458,7 @@ struct EvolveGraph {
   cudaGraphExec_t exec = nullptr;
   const cplx* psi = nullptr;
   double h = 0.0;
-  int m = 0, mv_kind = 0;
+  int m = 0, mv_kind = 0, variant = 0;
   int64_t kernels = 0;
   DBuf<double> nrm2;
   DBuf<int> has_im, act;
@@ -1622,7 +1622,8 @@ static void lanczos_evolve_steps(qd_ham* H, const cplx* psi_in, cplx* psi, doubl
   };
   if (H->one_shot) {  // solved once: capturing a graph would cost more than it saves
     for (int s = 0; s < nsteps; ++s) step();
-  } else if (!G.exec || G.psi != psi || G.h != h || G.m != m || G.mv_kind != mv_kind) {
+  } else if (!G.exec || G.psi != psi || G.h != h || G.m != m || G.mv_kind != mv_kind ||
+             G.variant != H->spmv_variant) {
     if (G.exec) cudaGraphExecDestroy(G.exec);
     G.exec = nullptr;
     cudaGraph_t g = nullptr;
@@ -1646,6 +1647,7 @@ static void lanczos_evolve_steps(qd_ham* H, const cplx* psi_in, cplx* psi, doubl
     G.h = h;
     G.m = m;
     G.mv_kind = mv_kind;
+    G.variant = H->spmv_variant;
   }
   if (!H->one_shot)
     for (int s = 0; s < nsteps; ++s) {

@@ -32,7 +32,8 @@ struct LanczosBuffers {
   DBuf<unsigned> epoch;  // launch parity of the one-launch steps (fxstep.cuh, fxblock.cu)
   DBuf<double> mbox;     // their alpha and beta mailbox (kMboxDoubles entries)
   cudaGraphExec_t exec = nullptr;
-  int kind = 0;  // product the captured graph launches (0 CSR, 1 matrix-free, 2 fixed-point, +4 one-launch step)
+  int kind = 0;  // product the captured graph launches (0 CSR, 1 matrix-free, 2 fixed-point, +4 one-launch step,
+                 // 64 times the CSR kernel's code)
   int done = 0;  // Lanczos steps run on the stored basis (incremental solves continue from here)
   void ensure_fx(cudaStream_t s) {  // stream-ordered: a legacy-stream call would wait for every lane
     if (!X.p) {

@@ -99,3 +99,29 @@ def test_the_autotuner_keeps_the_faster_form(ctx):
         ground(sec, op, psi)
         out.append(psi.get(0))
     assert np.array_equal(*out)
+
+
+@pytest.mark.parametrize("call", ["ground", "short", "evolve"])
+def test_a_later_choice_replaces_what_a_graph_launches(ctx, call):
+    """Recurrences are captured once and replayed; another choice on the same operator gives the bits of that
+    kernel on a fresh one (104 adds a row's entries over eight lanes, 110 in their order)."""
+    spec, ham = SYSTEMS["bonds12"]()
+    sec = q.Sector(spec.index, spec.constraints)
+    fn = {"ground": ground,
+          "short": lambda sec, H, psi: q.lanczos_evolve(H, psi, 0, 0, 0.1, 12, 2),
+          "evolve": CALLS["evolve"][0]}[call]
+    psi = q.getState(sec, 1)
+
+    def run(H, kernel):
+        A.call("qd_ham_set_spmv_kernel", H.handle, kernel)
+        for _ in range(3):  # the first runs may not be captured yet
+            psi.set(0, q.start_vector(sec.dim, 3).astype(complex))
+            fn(sec, H, psi)
+        return psi.get(0)
+
+    H = sec.lower(ham)
+    first = run(H, 110)
+    second = run(H, 104)
+    assert not np.array_equal(first, second)
+    assert np.array_equal(second, run(sec.lower(ham), 104))
+    assert np.array_equal(first, run(H, 110))
